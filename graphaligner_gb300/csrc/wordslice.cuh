@@ -291,12 +291,13 @@ GA_HD i32 ws_changed_min(const WS& w, const WS& old)
 
 // One Myers (1999) column step with horizontal inputs hinP/hinN
 // (GraphAlignerBitvectorCommon::getNextSlice, Common.h:242-262).
-// Ph/Mh receive the full horizontal delta words.
-GA_HD WS myers_step(u64 eq, WS s, u64 hinP, u64 hinN, u64& Ph, u64& Mh)
+// Ph/Mh receive the full horizontal delta words; Xh (with the old VN) the rows whose score
+// equals their upper left neighbour's.
+GA_HD WS myers_step(u64 eq, WS s, u64 hinP, u64 hinN, u64& Ph, u64& Mh, u64& Xh)
 {
     u64 Xv = eq | s.VN;
     eq |= hinN;
-    u64 Xh = (((eq & s.VP) + s.VP) ^ s.VP) | eq;
+    Xh = (((eq & s.VP) + s.VP) ^ s.VP) | eq;
     Ph = s.VN | ~(Xh | s.VP);
     Mh = s.VP & Xh;
     u64 shM = (Mh << 1) | hinN;
@@ -306,6 +307,31 @@ GA_HD WS myers_step(u64 eq, WS s, u64 hinP, u64 hinN, u64& Ph, u64& Mh)
     r.VN = shP & Xv;
     r.end = wadd(wsub(s.end, (i32)(Mh >> 63)), (i32)(Ph >> 63));
     return r;
+}
+
+GA_HD WS myers_step(u64 eq, WS s, u64 hinP, u64 hinN, u64& Ph, u64& Mh)
+{
+    u64 Xh;
+    return myers_step(eq, s, hinP, hinN, Ph, Mh, Xh);
+}
+
+// The rows of a column from which the traceback's diagonal step is open
+// (pickBacktraceInside, Common.h:770-815): the upper left score equals this one where the
+// characters match, and is one less where they do not.  xh and oldVN are the step's that made
+// the column; row 0 is not among the rows the walk inside a node-slice asks for.
+GA_HD u64 diagonal_rows(u64 eq, u64 xh, u64 oldVN) { return ~(xh | oldVN) | eq; }
+
+// How many rows the traceback steps up from `row` (>= 1) of a column: the run of +1 deltas that
+// ends there, not past row 0.
+GA_HD u32 up_run(u64 vp, u32 row)
+{
+    const u64 below = ~(vp << (63 - row));
+#ifdef __CUDA_ARCH__
+    const u32 run = (u32)__clzll((long long)below);
+#else
+    const u32 run = below ? (u32)__builtin_clzll(below) : 64;
+#endif
+    return run < row ? run : row;
 }
 
 // column entering from a row-above score (getSourceSliceFromScore, Common.h:1056-1060)
