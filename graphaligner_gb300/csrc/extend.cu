@@ -76,8 +76,19 @@ struct __align__(16) Col
     u64 Mh;             // horizontal -1 deltas of the step (the X-score's candidate mask); in the
                         // traceback's recomputation the rows with an open diagonal step
     i32 end;
-    u32 phTop;          // horizontal +1 delta out of the last row
+    u32 pad;
 };
+
+// A warp's recorded columns and the match mask of each column of its current node, in shared
+// memory in every kernel: dynamic shared memory starts with one of these per warp of the block.
+struct __align__(16) NodeCols
+{
+    Col cols[64];
+    u64 eqcol[64 + 2];  // [64] is read ahead of the last column
+};
+extern __shared__ __align__(16) uint8_t dsmem[];
+
+__device__ __forceinline__ NodeCols& node_cols() { return ((NodeCols*)dsmem)[threadIdx.x >> 5]; }
 
 __device__ __forceinline__ u32 hash_node(u32 node)
 {
@@ -94,9 +105,7 @@ struct WSpace
     NodeVal* val[2];
     HeapItem* heap;
     Extra* extras;
-    Col* cols;          // [64]
-    u64* eqcol;         // [64] match mask of each column of the current node
-    u64* ring;          // [64] trace items not yet written out
+    u64* ring;          // the traceback: [64] trace items not yet written out
     struct SliceSlot* slots;   // [2] the traceback's cached slices (odd and even)
     i32* nodeMax;       // multiseed DP: [band] each band node's best exact-end-position X-score
 };
@@ -111,7 +120,6 @@ __host__ __device__ inline u64 wspace_bytes(const Caps& c, bool multi = false)
     b += 2 * align16((u64)c.hash * sizeof(NodeVal));
     b += align16((u64)c.heap * sizeof(HeapItem));
     b += align16((u64)c.extras * sizeof(Extra));
-    b += 64 * sizeof(Col) + 64 * 8 + 64 * 8;
     return align16(b);
 }
 
@@ -127,9 +135,7 @@ __device__ __forceinline__ WSpace wspace_at(uint8_t* base, const Caps& c)
     w.val[1] = (NodeVal*)(base + off); off += align16((u64)c.hash * sizeof(NodeVal));
     w.heap = (HeapItem*)(base + off); off += align16((u64)c.heap * sizeof(HeapItem));
     w.extras = (Extra*)(base + off); off += align16((u64)c.extras * sizeof(Extra));
-    w.cols = (Col*)(base + off); off += 64 * sizeof(Col);
-    w.eqcol = (u64*)(base + off); off += 64 * 8;
-    w.ring = (u64*)(base + off); off += 64 * 8;
+    w.ring = nullptr;
     w.nodeMax = (i32*)(base + off);    // inside the stride only when it was sized for the multiseed DP
     w.slots = nullptr;
     return w;
@@ -461,11 +467,26 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
 // Fill = false: recalcNodeWordslice (no early leave); columns 0..lastColumn land in cols.
 // The column loop runs the Myers recurrence warp-uniformly and records every column; the
 // per-column minimum, X-score and horizontal output bits are then taken across the lanes.
+//
+// What bounds the loop is its chain: a warp alone waits about 4 cycles for each instruction
+// that needs the last one, and a full SM has no issue slots left.  So a column does only the
+// recurrence, on 32-bit halves: the horizontal -1 input is already in the column's match mask
+// (where it is set the row's bits of VP and VN do not depend on the mask), the +1 input enters
+// through the funnel shift that moves Ph down a row, the next mask is loaded a column ahead, and
+// the bottom-row deltas are read off the recorded scores afterwards.  The reference forces the
+// first row's delta to -1 where the row above the slice is cheaper than the band above
+// (forceMask); there the input is +1 and the column before it has that delta already, so the
+// recurrence gives it by itself (the first column's merges keep it: the cheaper row above wins
+// the minimum in both rows).  Only a seed start's columns need the force.
+// Against 64-bit steps with inputs, force and deltas shifted out of words per column and the
+// records behind generic pointers: 50,000 extensions (250 Mbp) 115.6 -> 102.9 ms, one seed of a
+// 10 kbp read 13 % less.
 template <bool Fill, bool Multi = false>
 __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i, Item& slice, const EqV4& eqv, const PrevInfo& prev,
-    const Extra* pool, uint16_t head, const WS* singleIncoming, bool singleInPrevBand, i32 seqOffset, Col* cols, u64* eqcol,
-    u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
+    const Extra* pool, uint16_t head, const WS* singleIncoming, bool singleInPrevBand, i32 seqOffset, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
 {
+    Col* const cols = node_cols().cols;
+    u64* const eqcol = node_cols().eqcol;
     const bool hasExtra = Multi && extra != nullptr;
     bool forceCalculation = false;
     const bool boundOk = seqOffset < kXBoundOffsetLimit;
@@ -490,18 +511,12 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
         a0 = a[0]; a1 = a[1]; a2 = a[2]; a3 = a[3];
     }
     const u32 inDeg = g.inOff[i + 1] - g.inOff[i];
-    // the match mask of every column (lane k: columns k and k + 32)
-    __syncwarp();
-    #pragma unroll 1
-    for (u32 pos = lane; pos < nodeLength; pos += 32)
+    auto mask_at = [&](u32 pos) -> u64
     {
-        u64 e;
-        if (!amb) e = eq_pick(eqv, (u32)(((pos < 32 ? c0 : c1) >> ((pos & 31) * 2)) & 3));
-        else e = eq_amb(eqv, (u32)(((a0 >> pos) & 1) | (((a1 >> pos) & 1) << 1) | (((a2 >> pos) & 1) << 2) | (((a3 >> pos) & 1) << 3)));
-        eqcol[pos] = e;
-    }
-    __syncwarp();
-    const u64 eq0 = eqcol[0];
+        if (!amb) return eq_pick(eqv, (u32)(((pos < 32 ? c0 : c1) >> ((pos & 31) * 2)) & 3));
+        return eq_amb(eqv, (u32)(((a0 >> pos) & 1) | (((a1 >> pos) & 1) << 1) | (((a2 >> pos) & 1) << 2) | (((a3 >> pos) & 1) << 3)));
+    };
+    const u64 eq0 = mask_at(0);
 
     WS ws = ws_make(0, 0, 0);
     bool hasWs = false;
@@ -595,58 +610,102 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     slice.sVN = ws.VN;
     slice.sEnd = ws.end;
     slice.node = i | kExists | (slice.node & kSeedStart);
-    {
-        // Fill: column 0 as it enters the node, its X-score over every row; the traceback's
-        // recomputation: column 0 after the merges
-        Col c;
-        c.VP = Fill ? ws0.VP : ws.VP;
-        c.VN = Fill ? ws0.VN : ws.VN;
-        c.Mh = kAllOnes;
-        c.end = Fill ? ws0.end : ws.end;
-        c.phTop = 0;
-        cols[0] = c;
-    }
     const u64 forceEq = prev.exists ? kAllOnes : (kAllOnes ^ 1);
     // the traceback's recomputation stops at the column it needs last
     const u32 columns = Fill ? nodeLength : (lastColumn + 1 < nodeLength ? lastColumn + 1 : nodeLength);
-    u64 hp = fixedHP >> 1, hn = fixedHN >> 1, fm = forceMask >> 1;   // bit 0: column 1
+    const i32 startEnd = ws.end;
+    // the match mask of every column (lane k: columns k and k + 32), with the horizontal -1 input
+    __syncwarp();
     #pragma unroll 1
-    for (u32 pos = 1; pos < columns; pos++)
+    for (u32 pos = lane; pos < columns; pos += 32)
     {
-        const u64 eq = eqcol[pos] & forceEq;
-        u64 Ph, Mh, Xh;
-        WS nw = myers_step(eq, ws, hp & 1, hn & 1, Ph, Mh, Xh);
-        const u64 rows = Fill ? Mh : diagonal_rows(eq, Xh, ws.VN);
-        if (fm & 1)
-        {
-            nw.VP &= kAllOnes ^ 1;
-            nw.VN |= 1;
-        }
-        hp >>= 1;
-        hn >>= 1;
-        fm >>= 1;
-        // the multiseed DP keeps both bottom-row deltas in phTop (bit 0 +1, bit 1 -1): with a
-        // seed start they come from the merged column's last-row score
-        u32 top = (u32)(Ph >> 63);
-        if (Multi)
-        {
-            if (hasExtra)
-            {
-                const WS m = merge_w(nw, *extra, lane);
-                top = (m.end == ws.end + 1 ? 1u : 0u) | (m.end == ws.end - 1 ? 2u : 0u);
-                nw = m;
-            }
-            else top |= (u32)(Mh >> 63) << 1;
-        }
-        ws = nw;
+        const u64 e = mask_at(pos);
+        eqcol[pos] = pos == 0 ? e : (e & forceEq) | ((fixedHN >> pos) & 1);
+    }
+    if (!Fill)
+    {
+        // the recomputation's column 0, after the merges
         Col c;
         c.VP = ws.VP;
         c.VN = ws.VN;
-        c.Mh = rows;
+        c.Mh = kAllOnes;
         c.end = ws.end;
-        c.phTop = top;
-        cols[pos] = c;
+        c.pad = 0;
+        cols[0] = c;
     }
+    __syncwarp();
+    if (!hasExtra)
+    {
+        u32 vpl = (u32)ws.VP, vph = (u32)(ws.VP >> 32), vnl = (u32)ws.VN, vnh = (u32)(ws.VN >> 32);
+        i32 end = ws.end;
+        u32 pos = 1;
+        u64 eq = eqcol[1];
+        #pragma unroll 1
+        for (u32 half = 0; half < 2; half++)
+        {
+            // the horizontal inputs of columns 1..32, then 33..63, the next one in the top bit
+            u32 hp = __brev((u32)(fixedHP >> (half ? 33 : 1)));
+            u32 hn = __brev((u32)(fixedHN >> (half ? 33 : 1)));
+            const u32 stop = half ? columns : (columns < 33 ? columns : 33);
+            #pragma unroll 2
+            for (; pos < stop; pos++)
+            {
+                const u32 eql = (u32)eq, eqh = (u32)(eq >> 32);
+                eq = eqcol[pos + 1];
+                const u64 sum = (((u64)(eqh & vph) << 32) | (eql & vpl)) + (((u64)vph << 32) | vpl);
+                const u32 xhl = ((u32)sum ^ vpl) | eql, xhh = ((u32)(sum >> 32) ^ vph) | eqh;
+                const u32 pl = vnl | ~(xhl | vpl), ph = vnh | ~(xhh | vph);
+                const u32 ml = vpl & xhl, mh = vph & xhh;
+                const u32 spl = __funnelshift_l(hp, pl, 1), sph = __funnelshift_l(pl, ph, 1);
+                const u32 sml = __funnelshift_l(hn, ml, 1), smh = __funnelshift_l(ml, mh, 1);
+                hp <<= 1;
+                hn <<= 1;
+                const u32 xvl = eql | vnl, xvh = eqh | vnh;
+                Col c;
+                c.Mh = Fill ? ((u64)mh << 32) | ml : ((u64)(~(xhh | vnh) | eqh) << 32) | (~(xhl | vnl) | eql);
+                vpl = sml | ~(xvl | spl);
+                vph = smh | ~(xvh | sph);
+                vnl = spl & xvl;
+                vnh = sph & xvh;
+                end = end + (i32)(ph >> 31) - (i32)(mh >> 31);
+                c.VP = ((u64)vph << 32) | vpl;
+                c.VN = ((u64)vnh << 32) | vnl;
+                c.end = end;
+                c.pad = 0;
+                cols[pos] = c;
+            }
+        }
+        ws = ws_make(((u64)vph << 32) | vpl, ((u64)vnh << 32) | vnl, end);
+    }
+    else
+    {
+        // a seed start of the multiseed DP: its column joins every column
+        u64 hp = fixedHP >> 1, hn = fixedHN >> 1, fm = forceMask >> 1;   // bit 0: column 1
+        #pragma unroll 1
+        for (u32 pos = 1; pos < columns; pos++)
+        {
+            const u64 eq = eqcol[pos];
+            u64 Ph, Mh;
+            WS nw = myers_step(eq, ws, hp & 1, hn & 1, Ph, Mh);
+            if (fm & 1)
+            {
+                nw.VP &= kAllOnes ^ 1;
+                nw.VN |= 1;
+            }
+            hp >>= 1;
+            hn >>= 1;
+            fm >>= 1;
+            ws = merge_w(nw, *extra, lane);
+            Col c;
+            c.VP = ws.VP;
+            c.VN = ws.VN;
+            c.Mh = Mh;
+            c.end = ws.end;
+            c.pad = 0;
+            cols[pos] = c;
+        }
+    }
+    __syncwarp();
     steps += columns - 1;
     result.cells = columns;
     if (Fill)
@@ -658,35 +717,49 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
         // X-score is skipped; every column above that bound is scored exactly.
         u32 loKey = 0xffffffffu, hiKey = 0xffffffffu;
         i32 lmax = kIntMin;
-        u32 hpLo = 0, hpHi = 0, hnLo = 0, hnHi = 0;
+        i32 loEnd = startEnd, hiEnd = 0;    // the columns' last-row scores (column 0's after the merges)
 #pragma unroll
         for (u32 h = 0; h < 2; h++)
         {
             const u32 pos = lane + 32 * h;
             if (pos < columns)
             {
-                const Col c = cols[pos];
+                Col c = cols[pos];
+                if (pos == 0)
+                {
+                    // column 0 as it enters the node, every row a candidate
+                    c.VP = ws0.VP;
+                    c.VN = ws0.VN;
+                    c.Mh = kAllOnes;
+                    c.end = ws0.end;
+                }
+                else if (h == 0) loEnd = c.end;
+                else hiEnd = c.end;
                 // column 0's X-score is taken after the seed start's column joins it
                 const WS cw = (Multi && pos == 0) ? wsX : ws_make(c.VP, c.VN, c.end);
                 const u32 key = (u32)c.end ^ 0x80000000u;   // signed order as unsigned
                 if (h == 0) loKey = key; else hiKey = key;
                 if (!boundOk || xscore_bound(cw, seqOffset, cost) > (int64_t)sliceMaxX)
                     lmax = imax(lmax, ws_max_xscore(cw, seqOffset, cost, 64, c.Mh));
-                if (pos >= 1)
-                {
-                    const u32 tp = Multi ? (c.phTop & 1) : c.phTop;
-                    const u32 tn = Multi ? ((c.phTop >> 1) & 1) : (u32)(c.Mh >> 63);
-                    if (h == 0) { hpLo = tp; hnLo = tn; }
-                    else { hpHi = tp; hnHi = tn; }
-                }
             }
         }
+        // the bottom-row delta of a column is its last-row score less the one before
+        i32 loBefore = __shfl_up_sync(kFull, loEnd, 1);
+        i32 hiBefore = __shfl_up_sync(kFull, hiEnd, 1);
+        const i32 end31 = __shfl_sync(kFull, loEnd, 31);
+        if (lane == 0)
+        {
+            loBefore = loEnd;
+            hiBefore = end31;
+        }
+        const i32 loDelta = lane < columns ? wsub(loEnd, loBefore) : 0;
+        const i32 hiDelta = lane + 32 < columns ? wsub(hiEnd, hiBefore) : 0;
         const u32 gkey = __reduce_min_sync(kFull, loKey < hiKey ? loKey : hiKey);
         const i32 gmax = __reduce_max_sync(kFull, lmax);
         const u32 onLo = __ballot_sync(kFull, loKey == gkey);
         const u32 onHi = __ballot_sync(kFull, hiKey == gkey);
-        const u64 outHP = (u64)__ballot_sync(kFull, hpLo) | ((u64)__ballot_sync(kFull, hpHi) << 32);
-        const u64 outHN = (u64)__ballot_sync(kFull, hnLo) | ((u64)__ballot_sync(kFull, hnHi) << 32);
+        const u64 outHP = (u64)__ballot_sync(kFull, loDelta == 1) | ((u64)__ballot_sync(kFull, hiDelta == 1) << 32);
+        const u64 outHN = (u64)__ballot_sync(kFull, loDelta == -1) | ((u64)__ballot_sync(kFull, hiDelta == -1) << 32);
         // column 0 always takes part, so the key is a real score
         result.minScore = (i32)(gkey ^ 0x80000000u);
         result.minScoreOffset = onLo ? (u32)(__ffs((int)onLo) - 1) : (u32)(32 + __ffs((int)onHi) - 1);
@@ -1061,7 +1134,7 @@ __device__ SliceResult fill_slice(const FillArgs& a, const WSpace& w, int cur, u
         // changes neither, so the node computation may skip its exact X-score
         const i32 skipBelow = Multi ? imin(res.maxX, w.nodeMax[s.band]) : res.maxX;
         NodeCalc nc = node_calc<true, Multi>(g, a.cost, i, thisNode, eqv, prev, w.extras, s.head, nullptr, singleInPrev, seqOffset,
-            w.cols, w.eqcol, steps, err, lane, skipBelow, 63, extra);
+            steps, err, lane, skipBelow, 63, extra);
         if (err) return res;
         if (Multi) w.nodeMax[s.band] = imax(nc.maxX, w.nodeMax[s.band]);
         heap_pop(w.heap, heapN);
@@ -1594,9 +1667,10 @@ __device__ __noinline__ TStep bt_corner(const DevGraph& g, const uint8_t* seq, T
 // after the one it enters at).  When every column is recomputed the last one must equal
 // the stored end column, as the reference asserts.  Returns 0 or the error status.
 template <bool Multi = false>
-__device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, u32 node, const EqV4& eqv, Col* cols, u64* eqcol,
-    u32 lane, u32 lastColumn, WS extra = fake_ws())
+__device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, u32 node, const EqV4& eqv, u32 lane, u32 lastColumn,
+    WS extra = fake_ws())
 {
+    const Col* const cols = node_cols().cols;
     const Item* it = t.template find<Multi>(s, node);
     if (!it) return GA_ASSERT;
     PrevInfo prev;
@@ -1608,7 +1682,7 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
     u64 steps = 0;
     int err = 0;
     int64_t j = ((int64_t)s - 1) * 64;
-    node_calc<false, Multi>(g, cost, node, copy, eqv, prev, nullptr, kNil, &start, false, (i32)j, cols, eqcol, steps, err, lane, kIntMin, lastColumn,
+    node_calc<false, Multi>(g, cost, node, copy, eqv, prev, nullptr, kNil, &start, false, (i32)j, steps, err, lane, kIntMin, lastColumn,
         (Multi && extra.end != kIntMax) ? &extra : nullptr);
     if (err) return err;
     u32 L = g.len[node];
@@ -1621,9 +1695,9 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
 // pickBacktraceVerticalCrossing (Common.h:886-934), the step out of (p.node, p.off > 0, row 0)
 // into the previous slice; pself is the node's entry there
 template <bool Multi>
-__device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* seq, Table t, u32 curSlice, const Item* pself, const Col* cols,
-    TPos p, int& err, WS extra)
+__device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* seq, Table t, u32 curSlice, const Item* pself, TPos p, int& err, WS extra)
 {
+    const Col* const cols = node_cols().cols;
     TStep second;
     second.pos = p;
     second.sw = false;
@@ -1728,8 +1802,9 @@ struct EndCell
 // k + 32 of its best node) the cell of greatest row among those scoring the slice's
 // X-score, the first column on ties.  The node's columns are left in cols.
 __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint8_t* arena, Table t, u32 committed, const uint8_t* seq,
-    u32 seqLen, Col* cols, u64* eqcol, u32 lane)
+    u32 seqLen, u32 lane)
 {
+    const Col* const cols = node_cols().cols;
     EndCell ec;
     ec.err = 0;
     ec.nodeOffset = 0xffffffffu;
@@ -1751,7 +1826,7 @@ __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint
     const int64_t j = ec.j;
     EqV4 eqv;
     if (!eq_vector(seq, seqLen, j, eqv, lane)) { ec.err = GA_ASSERT; return ec; }
-    ec.err = recalc(g, cost, t, best, ec.node, eqv, cols, eqcol, lane, 63);
+    ec.err = recalc(g, cost, t, best, ec.node, eqv, lane, 63);
     if (ec.err) return ec;
     const int cells = (int)((int64_t)seqLen - j < 64 ? (int64_t)seqLen - j : 64);
     const u32 L = g.len[ec.node];
@@ -1859,7 +1934,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     TPos start, i32 startScore, i32& resultScore, u32 lane)
 {
     int err = 0;
-    Col* cols = w.cols;
+    const Col* const cols = node_cols().cols;
     const u64 guardMax = (u64)((Multi && to.counting) ? (1u << 26) : to.cap) * 4 + 1024;
     resultScore = startScore;
     to.push(start, false);
@@ -1894,7 +1969,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 if (!here) { err = GA_ASSERT; break; }
                 extra = (here->node & kSeedStart) ? seed_ws(((int64_t)curSlice - 1) * 64, seqLen, cost) : fake_ws();
             }
-            err = recalc<Multi>(g, cost, t, curSlice, curNode, eqv, cols, w.eqcol, lane, b.off, extra);
+            err = recalc<Multi>(g, cost, t, curSlice, curNode, eqv, lane, b.off, extra);
             if (err) break;
             colsUpTo = b.off;
             curLen = g.len[curNode];
@@ -1928,7 +2003,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             // highest failing column at or below b.off (column 0 always ends it)
             TPos p = b;
             p.off = row0_run_start(cols, b.off, lane);
-            TStep second = p.off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : vertical_step<Multi>(g, seq, t, curSlice, pself, cols, p, err, extra);
+            TStep second = p.off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : vertical_step<Multi>(g, seq, t, curSlice, pself, p, err, extra);
             if (err) break;
             if (second.pos.seq == b.seq && col_value(cols[second.pos.off], (int)mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
             if (p.off != b.off) to.push_run(TPos { p.node, b.off - 1, p.seq }, -1, 0, b.off - p.off);
@@ -2020,7 +2095,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             u32 hori = b.off;
             u32 vert = row;
             // the recomputation left each column's match mask (the fill's Eq) in eqcol
-            const u64* eqcol = w.eqcol;
+            const u64* eqcol = node_cols().eqcol;
             if (hori > 0 && vert > 0)
             {
                 WS colH = ws_make(cols[hori].VP, cols[hori].VN, cols[hori].end);
@@ -2114,7 +2189,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
     t.lane = lane;
     t.slots = w.slots;
     t.init();
-    Col* cols = w.cols;
+    const Col* const cols = node_cols().cols;
     TraceOut to;
     to.items = out;
     to.ring = w.ring;
@@ -2124,7 +2199,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
     to.overflow = false;
     int err = 0;
     i32 resultScore = 0;
-    const EndCell ec = end_cell(g, a.cost, a.arena, t, st.committed, seq, seqLen, cols, w.eqcol, lane);
+    const EndCell ec = end_cell(g, a.cost, a.arena, t, st.committed, seq, seqLen, lane);
     err = ec.err;
     if (!err)
     {
@@ -2261,9 +2336,9 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const WSpace& w,
     EqV4 eqv;
     if (!eq_vector(seq, seqLen, j, eqv, lane)) return GA_ASSERT;
     const WS extra = (items[c.index].node & kSeedStart) ? seed_ws(j, seqLen, a.cost) : fake_ws();
-    int err = recalc<true>(g, a.cost, t, c.slice, node, eqv, w.cols, w.eqcol, lane, 63, extra);
+    int err = recalc<true>(g, a.cost, t, c.slice, node, eqv, lane, 63, extra);
     if (err) return err;
-    const Col* cols = w.cols;
+    const Col* cols = node_cols().cols;
     const i32 score = c.score;
     const int cells = (int)((int64_t)seqLen - j < 64 ? (int64_t)seqLen - j : 64);
     const u32 L = g.len[node];
@@ -2525,12 +2600,12 @@ __device__ __forceinline__ bool next_extension(u32* counter, u32 num, const u32*
 // per warp.
 __global__ void __launch_bounds__(128, 4) fill_kernel(FillArgs fa, u32* counter)
 {
-    extern __shared__ __align__(16) uint8_t dsmem[];
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
     const u32 warpInBlock = threadIdx.x >> 5;
     const u64 gwarp = (u64)blockIdx.x * (blockDim.x >> 5) + warpInBlock;
-    uint8_t* base = fa.workspace ? fa.workspace + gwarp * fa.workspaceStride : dsmem + (u64)warpInBlock * fa.workspaceStride;
+    uint8_t* base = fa.workspace ? fa.workspace + gwarp * fa.workspaceStride
+        : dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (u64)warpInBlock * fa.workspaceStride;
     const WSpace w = wspace_at(base, fa.caps);
     // generation 0 marks every node-table slot empty
 #pragma unroll 1
@@ -2569,21 +2644,19 @@ __global__ void __launch_bounds__(128, 4) fill_kernel(FillArgs fa, u32* counter)
     if (lane == 0 && arena.used) atomicAdd(fa.arenaCursor + 1, (unsigned long long)arena.used);
 }
 
-static constexpr u32 kTraceSpaceBytes = 64 * sizeof(Col) + 64 * 8 + 64 * 8 + 2 * sizeof(SliceSlot);
+// the traceback's shared memory of one warp behind the block's NodeCols
+static constexpr u32 kTraceSpaceBytes = 64 * 8 + 2 * sizeof(SliceSlot);
 
 // The traceback: a warp takes the next filled extension and walks its table back.  Its
 // shared memory holds the recomputed columns, the match masks and the trace staging.
 __global__ void __launch_bounds__(128, 6) trace_kernel(TraceArgs ta, u32* counter)
 {
-    extern __shared__ __align__(16) uint8_t dsmem[];
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
-    uint8_t* base = dsmem + (u64)(threadIdx.x >> 5) * kTraceSpaceBytes;
+    uint8_t* base = dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (threadIdx.x >> 5) * kTraceSpaceBytes;
     WSpace w {};
-    w.cols = (Col*)base;
-    w.eqcol = (u64*)(base + 64 * sizeof(Col));
-    w.ring = (u64*)(base + 64 * sizeof(Col) + 64 * 8);
-    w.slots = (SliceSlot*)(base + 64 * sizeof(Col) + 64 * 8 + 64 * 8);
+    w.ring = (u64*)base;
+    w.slots = (SliceSlot*)(base + 64 * 8);
     u32 ext;
 #pragma unroll 1
     while (next_extension(counter, ta.num, ta.order, ta.prevStatus, lane, ext))
@@ -2688,15 +2761,12 @@ __global__ void __launch_bounds__(128, 6) ms_resolve_kernel(MultiTraceArgs ta, u
 // as it has walks in the round.
 __global__ void __launch_bounds__(128, 6) ms_trace_kernel(MultiTraceArgs ta, u32* counter, int write)
 {
-    extern __shared__ __align__(16) uint8_t dsmem[];
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
-    uint8_t* base = dsmem + (u64)(threadIdx.x >> 5) * kTraceSpaceBytes;
+    uint8_t* base = dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (threadIdx.x >> 5) * kTraceSpaceBytes;
     WSpace w {};
-    w.cols = (Col*)base;
-    w.eqcol = (u64*)(base + 64 * sizeof(Col));
-    w.ring = (u64*)(base + 64 * sizeof(Col) + 64 * 8);
-    w.slots = (SliceSlot*)(base + 64 * sizeof(Col) + 64 * 8 + 64 * 8);
+    w.ring = (u64*)base;
+    w.slots = (SliceSlot*)(base + 64 * 8);
     const u64 total = write ? (*ta.candTotal < ta.candCap ? *ta.candTotal : ta.candCap) : *ta.workCount;
 #pragma unroll 1
     while (true)
@@ -2711,6 +2781,11 @@ __global__ void __launch_bounds__(128, 6) ms_trace_kernel(MultiTraceArgs ta, u32
 }
 }
 
+// dynamic shared memory of a block of the fill kernels (tables: bytes of a warp's tables kept
+// there) and of the traceback kernels
+static size_t fill_smem(int warpsPerBlock, size_t tables) { return (sizeof(gadev::NodeCols) + tables) * warpsPerBlock; }
+static size_t trace_smem(int warpsPerBlock) { return (sizeof(gadev::NodeCols) + gadev::kTraceSpaceBytes) * warpsPerBlock; }
+
 uint64_t ga_warp_tables_bytes(const gadev::Caps& c) { return gadev::wspace_bytes(c); }
 uint64_t ga_multiseed_tables_bytes(const gadev::Caps& c) { return gadev::wspace_bytes(c, true); }
 
@@ -2721,7 +2796,7 @@ static bool set_smem(const void* kernel, size_t smem)
 
 int ga_fill_blocks_per_sm(int warpsPerBlock, const gadev::Caps& caps, bool shared)
 {
-    const size_t smem = shared ? (size_t)gadev::wspace_bytes(caps) * warpsPerBlock : 0;
+    const size_t smem = fill_smem(warpsPerBlock, shared ? (size_t)gadev::wspace_bytes(caps) : 0);
     if (!set_smem((const void*)gadev::fill_kernel, smem)) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gadev::fill_kernel, warpsPerBlock * 32, smem) != cudaSuccess) return 0;
@@ -2730,7 +2805,7 @@ int ga_fill_blocks_per_sm(int warpsPerBlock, const gadev::Caps& caps, bool share
 
 int ga_trace_blocks_per_sm(int warpsPerBlock)
 {
-    const size_t smem = (size_t)gadev::kTraceSpaceBytes * warpsPerBlock;
+    const size_t smem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)gadev::trace_kernel, smem)) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gadev::trace_kernel, warpsPerBlock * 32, smem) != cudaSuccess) return 0;
@@ -2740,8 +2815,8 @@ int ga_trace_blocks_per_sm(int warpsPerBlock)
 int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int traceBlocks,
     int warpsPerBlock, void* stream)
 {
-    const size_t fillSmem = fa.workspace ? 0 : (size_t)fa.workspaceStride * warpsPerBlock;
-    const size_t traceSmem = (size_t)gadev::kTraceSpaceBytes * warpsPerBlock;
+    const size_t fillSmem = fill_smem(warpsPerBlock, fa.workspace ? 0 : (size_t)fa.workspaceStride);
+    const size_t traceSmem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)gadev::fill_kernel, fillSmem) || !set_smem((const void*)gadev::trace_kernel, traceSmem)) return -1;
     gadev::fill_kernel<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;
@@ -2753,7 +2828,9 @@ int ga_launch_multiseed_fill(const gadev::FillArgs& fa, const gadev::MultiTraceA
     int warpsPerBlock, void* stream)
 {
     if (!fa.workspace) return -1;
-    gadev::fill_multiseed_kernel<<<fillBlocks, warpsPerBlock * 32, 0, (cudaStream_t)stream>>>(fa, counters);
+    const size_t fillSmem = fill_smem(warpsPerBlock, 0);
+    if (!set_smem((const void*)gadev::fill_multiseed_kernel, fillSmem)) return -1;
+    gadev::fill_multiseed_kernel<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;
     gadev::ms_candidates_kernel<<<readBlocks, warpsPerBlock * 32, 0, (cudaStream_t)stream>>>(ta, counters + 1, 0);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -2779,7 +2856,7 @@ int ga_launch_multiseed_resolve(const gadev::MultiTraceArgs& ta, uint32_t* count
 
 int ga_launch_multiseed_walk(const gadev::MultiTraceArgs& ta, uint32_t* counters, int candBlocks, int warpsPerBlock, void* stream)
 {
-    const size_t traceSmem = (size_t)gadev::kTraceSpaceBytes * warpsPerBlock;
+    const size_t traceSmem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)gadev::ms_trace_kernel, traceSmem)) return -1;
     gadev::ms_trace_kernel<<<candBlocks, warpsPerBlock * 32, traceSmem, (cudaStream_t)stream>>>(ta, counters + 5, 0);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -2787,7 +2864,7 @@ int ga_launch_multiseed_walk(const gadev::MultiTraceArgs& ta, uint32_t* counters
 
 int ga_launch_multiseed_write(const gadev::MultiTraceArgs& ta, uint32_t* counters, int candBlocks, int warpsPerBlock, void* stream)
 {
-    const size_t traceSmem = (size_t)gadev::kTraceSpaceBytes * warpsPerBlock;
+    const size_t traceSmem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)gadev::ms_trace_kernel, traceSmem)) return -1;
     gadev::ms_trace_kernel<<<candBlocks, warpsPerBlock * 32, traceSmem, (cudaStream_t)stream>>>(ta, counters + 6, 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
