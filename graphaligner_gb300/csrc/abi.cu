@@ -239,6 +239,20 @@ extern "C" int ga_graph_upload(const ga_graph_desc* desc, int device, ga_graph_t
     g->d.outNb = (const uint32_t*)outNb;
     g->d.lin = (const uint8_t*)lin;
     g->d.comp = (const uint32_t*)comp;
+    // the nodes' records; without room for them the kernels gather each from the arrays
+    void* rec = nullptr;
+    if (cudaMalloc(&rec, (size_t)N * sizeof(gadev::NodeRec)) == cudaSuccess)
+    {
+        g->allocations.push_back(rec);
+        if (ga_build_node_records(g->d, (gadev::NodeRec*)rec, nullptr) != 0 || (e = cudaStreamSynchronize(nullptr)) != cudaSuccess)
+        {
+            for (void* p : g->allocations) cudaFree(p);
+            delete g;
+            return fail(GA_ERR_CUDA, "node records");
+        }
+        g->d.rec = (const gadev::NodeRec*)rec;
+    }
+    else cudaGetLastError();
     *out = g;
     return GA_OK;
 }
@@ -276,7 +290,7 @@ static bool shape_ok(const ga_launch_shape& sh)
 static gadev::Caps layout_caps(int layout)
 {
     gadev::Caps c;
-    if (layout == 0) { c.band = 32; c.hash = 64; c.heap = 32; c.extras = 64; }
+    if (layout == 0) { c.band = gadev::kSmallBand; c.hash = 0; c.heap = gadev::kSmallHeap; c.extras = gadev::kSmallExtras; }
     else if (layout == 1) { c.band = 512; c.hash = 1024; c.heap = 512; c.extras = 1024; }
     else { c.band = 16384; c.hash = 65536; c.heap = 16384; c.extras = 32768; }
     return c;
@@ -408,7 +422,7 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
         const bool shared = layout == 0;
         const gadev::Caps caps = layout_caps(layout);
         const uint64_t stride = ga_warp_tables_bytes(caps);
-        int fillPerSm = ga_fill_blocks_per_sm(wpb, caps, shared);
+        int fillPerSm = ga_fill_blocks_per_sm(wpb, shared);
         int tracePerSm = ga_trace_blocks_per_sm(wpb);
         if (fillPerSm <= 0 || tracePerSm <= 0) return fail(GA_ERR_CUDA, "the extension kernels do not fit an SM with this launch shape");
         if (sh.blocks_per_sm > 0)

@@ -55,7 +55,7 @@ struct Extra
     u64 VP, VN;
     i32 end;
     uint16_t next;
-    uint16_t skip;      // EdgeWithPriority::skipFirst
+    uint16_t skip;      // bit 0 EdgeWithPriority::skipFirst, bit 1 ::forceCalculation
 };
 
 static constexpr uint16_t kNil = 0xffff;
@@ -96,7 +96,63 @@ __device__ __forceinline__ u32 hash_node(u32 node)
     return h ^ (h >> 15);
 }
 
-// One warp's tables.  A node-table key is (generation << 32) | node; a slot whose
+// A node's record put together from the graph's arrays (a graph without records).
+__device__ __noinline__ void gather_record(const DevGraph& g, u32 node, NodeRec& r)
+{
+    const u32 in = g.inOff[node], inN = g.inOff[node + 1] - in;
+    const u32 out = g.outOff[node], outN = g.outOff[node + 1] - out;
+    r.seq[0] = node < g.firstAmbiguous ? g.seq2[(u64)node * 2] : 0;
+    r.seq[1] = node < g.firstAmbiguous ? g.seq2[(u64)node * 2 + 1] : 0;
+    r.comp = g.comp[node];
+    r.meta = g.len[node] | (g.lin[node] ? kRecLinearizable : 0) | ((inN < kRecDegree ? inN : kRecDegree) << 8)
+        | ((outN < kRecDegree ? outN : kRecDegree) << 20);
+    r.inOff = in;
+    r.outOff = out;
+    for (u32 k = 0; k < kRecIn; k++) r.inNb[k] = k < inN ? g.inNb[in + k] : 0xffffffffu;
+    for (u32 k = 0; k < kRecOut; k++)
+    {
+        r.outNb[k] = k < outN ? g.outNb[out + k] : 0xffffffffu;
+        r.outComp[k] = k < outN ? g.comp[r.outNb[k]] : 0;
+    }
+}
+
+__global__ void node_records_kernel(DevGraph g, NodeRec* rec)
+{
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < g.N; i += gridDim.x * blockDim.x) gather_record(g, i, rec[i]);
+}
+
+__device__ __forceinline__ NodeRec node_record(const DevGraph& g, u32 node)
+{
+    NodeRec r;
+    if (g.rec)
+    {
+        const uint4* src = (const uint4*)(g.rec + node);
+        uint4* dst = (uint4*)&r;
+#pragma unroll
+        for (u32 k = 0; k < 4; k++) dst[k] = __ldg(src + k);
+    }
+    else
+    {
+        NodeRec x;          // its address is taken, r stays in registers
+        gather_record(g, node, x);
+        r = x;
+    }
+    return r;
+}
+
+// in- and out-degree (beyond what the record's field holds: from the arrays)
+__device__ __forceinline__ u32 in_degree(const DevGraph& g, u32 node, const NodeRec& r)
+{
+    const u32 n = rec_in_degree(r.meta);
+    return n < kRecDegree ? n : g.inOff[node + 1] - r.inOff;
+}
+__device__ __forceinline__ u32 out_degree(const DevGraph& g, u32 node, const NodeRec& r)
+{
+    const u32 n = rec_out_degree(r.meta);
+    return n < kRecDegree ? n : g.outOff[node + 1] - r.outOff;
+}
+
+// One warp's tables in global memory.  A node-table key is (generation << 32) | node; a slot whose
 // generation is not the slice's is empty, so tables are never cleared between slices.
 struct WSpace
 {
@@ -105,8 +161,6 @@ struct WSpace
     NodeVal* val[2];
     HeapItem* heap;
     Extra* extras;
-    u64* ring;          // the traceback: [64] trace items not yet written out
-    struct SliceSlot* slots;   // [2] the traceback's cached slices (odd and even)
     i32* nodeMax;       // multiseed DP: [band] each band node's best exact-end-position X-score
 };
 
@@ -135,9 +189,7 @@ __device__ __forceinline__ WSpace wspace_at(uint8_t* base, const Caps& c)
     w.val[1] = (NodeVal*)(base + off); off += align16((u64)c.hash * sizeof(NodeVal));
     w.heap = (HeapItem*)(base + off); off += align16((u64)c.heap * sizeof(HeapItem));
     w.extras = (Extra*)(base + off); off += align16((u64)c.extras * sizeof(Extra));
-    w.ring = nullptr;
     w.nodeMax = (i32*)(base + off);    // inside the stride only when it was sized for the multiseed DP
-    w.slots = nullptr;
     return w;
 }
 
@@ -197,6 +249,255 @@ __device__ __forceinline__ int tbl_get_or_add(u64* key, NodeVal* val, u32 cap, u
     return -1;
 }
 
+// ---- the two forms of the fill's frontier tables ----
+//
+// Both give a slice a node table (slot: the node's place in the band, whether it is queued, its
+// pending columns in order), the band of this slice and the one before, the heap of the
+// component queue and the pool of pending columns.  next() starts a slice: the current band
+// becomes the previous one.
+
+struct SmallSpace
+{
+    Item band[2][kSmallBand];
+    NodeRec rec[32];       // records of the slots' nodes
+    HeapItem heap[kSmallHeap];
+    Extra extras[kSmallExtras];
+};
+
+__device__ __forceinline__ SmallSpace& small_space()
+{
+    return ((SmallSpace*)(dsmem + (blockDim.x >> 5) * sizeof(NodeCols)))[threadIdx.x >> 5];
+}
+
+// The tables of a warp whose bands hold at most 32 nodes: slot k of the node table is lane k's
+// registers, a lookup one ballot, and the nodes' records are copied into shared memory while
+// they wait in the queue.  With a hash table and the records' fields read from global memory
+// the pops and inserts took 17k of the fill's 45k cycles per slice of an extension alone.
+// This form against that: 50,000 extensions (250 Mbp) 102.9 -> 92.7 ms, one seed of a 10 kbp
+// read 8 % less, 1,000 tangled extensions of 20 kbp reads 14 % less.
+struct SmallTables
+{
+    static constexpr uint16_t kNoExtra = 0xff;
+    static constexpr u32 kFresh = 0x00ffffffu;     // bits 0-7 band, 8-15 first and 16-23 last pending column (0xff: none), 24 queued
+    static constexpr u32 kQueued = 1u << 24;
+    static constexpr u32 kLinear = 1u << 25;       // the node is linearizable
+    u32 lane;
+    u32 id, val, comp;     // this lane's slot
+    u32 bandSlot;          // the slot of band entry `lane`
+    u32 prevId, prevComp;  // the previous band's entry `lane`
+    bool prevLinear;
+    u32 used, heapN, poolN, count, prevCount, side;
+
+    __device__ __forceinline__ SmallTables(const FillArgs&, u64, u32 lane_) : lane(lane_), id(0), val(0), comp(0), bandSlot(0), prevId(0), prevComp(0),
+        prevLinear(false), used(0), heapN(0), poolN(0), count(0), prevCount(0), side(0) {}
+    __device__ __forceinline__ Item* band() const { return small_space().band[side]; }
+    __device__ __forceinline__ const Item* prev_band() const { return small_space().band[side ^ 1]; }
+    __device__ __forceinline__ HeapItem* heap() const { return small_space().heap; }
+    __device__ __forceinline__ Extra* extras() const { return small_space().extras; }
+    __device__ __forceinline__ i32* node_max() const { return nullptr; }
+    __device__ __forceinline__ void restart() { count = 0; }
+    __device__ __forceinline__ void next()
+    {
+        // a record that was asked for and not used may still be on its way to its slot
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        prevId = __shfl_sync(kFull, id, (int)bandSlot);
+        prevComp = __shfl_sync(kFull, comp, (int)bandSlot);
+        prevLinear = (__shfl_sync(kFull, val, (int)bandSlot) & kLinear) != 0;
+        prevCount = count;
+        side ^= 1;
+        used = heapN = poolN = count = 0;
+    }
+    // band index of node in the previous slice, or -1
+    __device__ __forceinline__ int prev_of(u32 node) const
+    {
+        return __ffs((int)__ballot_sync(kFull, lane < prevCount && prevId == node)) - 1;
+    }
+    __device__ __forceinline__ int add(const DevGraph& g, u32 node, u32 component)
+    {
+        if (used >= 32) return -1;
+        const u32 slot = used++;
+        if (lane == slot)
+        {
+            id = node;
+            comp = component;
+            val = kFresh;
+        }
+        NodeRec& r = small_space().rec[slot];
+        if (g.rec)
+        {
+            if (lane < 4)
+            {
+                const u32 to = (u32)__cvta_generic_to_shared((uint4*)&r + lane);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" :: "r"(to), "l"((const uint4*)(g.rec + node) + lane) : "memory");
+            }
+        }
+        else gather_record(g, node, r);
+        return (int)slot;
+    }
+    __device__ __forceinline__ int slot_of(const DevGraph& g, u32 node, u32 component)
+    {
+        const u32 hit = __ballot_sync(kFull, lane < used && id == node);
+        return hit ? __ffs((int)hit) - 1 : add(g, node, component);
+    }
+    // one more pending column of `slot`; false when a table is full
+    __device__ __forceinline__ bool queue(int slot, u32 node, u32 component, i32 score, const Extra& x)
+    {
+        u32 v = __shfl_sync(kFull, val, slot);
+        if (!(v & kQueued))
+        {
+            if (heapN >= kSmallHeap) return false;
+            HeapItem h;
+            h.component = component; h.score = score; h.node = node; h.slot = (u32)slot;
+            heap_push(heap(), heapN, h);
+            v = (v & (kLinear | 0xffu)) | 0xffff00u | kQueued;
+        }
+        if (poolN >= kSmallExtras) return false;
+        const u32 e = poolN++;
+        extras()[e] = x;
+        const u32 last = (v >> 16) & 0xff;
+        if (last == 0xff) v = (v & ~0xff00u) | (e << 8);
+        else extras()[last].next = (uint16_t)e;
+        v = (v & ~0xff0000u) | (e << 16);
+        if (lane == (u32)slot) val = v;
+        return true;
+    }
+    // takes the node off the queue; its first pending column
+    __device__ __forceinline__ uint16_t take(u32 slot, int& bandIndex)
+    {
+        heap_pop(heap(), heapN);
+        const u32 v = __shfl_sync(kFull, val, (int)slot);
+        if (lane == slot) val = (v & (kLinear | 0xffu)) | 0xffff00u;
+        bandIndex = (v & 0xff) == 0xff ? -1 : (int)(v & 0xff);
+        return (uint16_t)((v >> 8) & 0xff);
+    }
+    // the node's band entry; -1 when the band is full
+    __device__ __forceinline__ int enter(u32 slot)
+    {
+        if (count >= kSmallBand) return -1;
+        if (lane == slot) val = (val & ~0xffu) | count;
+        if (lane == count) bandSlot = slot;
+        return (int)count++;
+    }
+    __device__ __forceinline__ int band_of(u32 slot) const
+    {
+        const u32 b = __shfl_sync(kFull, val, (int)slot) & 0xff;
+        return b == 0xff ? -1 : (int)b;
+    }
+    __device__ __forceinline__ NodeRec record(const DevGraph&, u32 slot, u32)
+    {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        const NodeRec r = small_space().rec[slot];
+        if ((r.meta & kRecLinearizable) && lane == slot) val |= kLinear;
+        return r;
+    }
+    __device__ __forceinline__ u32 prev_component(const DevGraph&, u32 k, u32) const { return __shfl_sync(kFull, prevComp, (int)k); }
+    __device__ __forceinline__ bool prev_linear(const DevGraph&, u32 k, u32) const { return __shfl_sync(kFull, (int)prevLinear, (int)k) != 0; }
+};
+
+// The tables in global memory: a hash table with generation stamps.
+struct LargeTables
+{
+    static constexpr uint16_t kNoExtra = kNil;
+    WSpace w;
+    Caps caps;
+    u32 lane;
+    u32 gen, prevGen;
+    u32 used, heapN, poolN, count, prevCount, side;
+
+    __device__ __forceinline__ LargeTables(const FillArgs& a, u64 gwarp, u32 lane_) : w(wspace_at(a.workspace + gwarp * a.workspaceStride, a.caps)),
+        caps(a.caps), lane(lane_), gen(0), prevGen(0), used(0), heapN(0), poolN(0), count(0), prevCount(0), side(0)
+    {
+        clear();
+    }
+    // generation 0 marks every node-table slot empty
+    __device__ __forceinline__ void clear()
+    {
+        __syncwarp();
+#pragma unroll 1
+        for (u32 k = lane; k < caps.hash; k += 32)
+        {
+            w.key[0][k] = 0;
+            w.key[1][k] = 0;
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ Item* band() const { return w.band[side]; }
+    __device__ __forceinline__ const Item* prev_band() const { return w.band[side ^ 1]; }
+    __device__ __forceinline__ HeapItem* heap() const { return w.heap; }
+    __device__ __forceinline__ Extra* extras() const { return w.extras; }
+    __device__ __forceinline__ i32* node_max() const { return w.nodeMax; }
+    __device__ __forceinline__ void restart()
+    {
+        count = 0;
+        if (gen > 0xF0000000u)
+        {
+            // generation stamps are about to wrap: clear this warp's tables
+            clear();
+            gen = 0;
+        }
+    }
+    __device__ __forceinline__ void next()
+    {
+        prevGen = gen++;
+        prevCount = count;
+        side ^= 1;
+        used = heapN = poolN = count = 0;
+    }
+    __device__ __forceinline__ int prev_of(u32 node) const
+    {
+        const int s = tbl_find(w.key[side ^ 1], caps.hash, prevGen, node, lane);
+        return s < 0 ? -1 : (int)w.val[side ^ 1][s].band;
+    }
+    __device__ __forceinline__ int add(const DevGraph& g, u32 node, u32 component) { return slot_of(g, node, component); }
+    __device__ __forceinline__ int slot_of(const DevGraph&, u32 node, u32)
+    {
+        return tbl_get_or_add(w.key[side], w.val[side], caps.hash, gen, node, used, lane);
+    }
+    __device__ __forceinline__ bool queue(int slot, u32 node, u32 component, i32 score, const Extra& x)
+    {
+        NodeVal& s = w.val[side][slot];
+        if (!s.active)
+        {
+            if (heapN >= caps.heap) return false;
+            HeapItem h;
+            h.component = component; h.score = score; h.node = node; h.slot = (u32)slot;
+            heap_push(w.heap, heapN, h);
+            s.active = 1;
+            s.head = kNil;
+            s.tail = kNil;
+        }
+        if (poolN >= caps.extras) return false;
+        const uint16_t e = (uint16_t)poolN++;
+        w.extras[e] = x;
+        if (s.head == kNil) s.head = e;
+        else w.extras[s.tail].next = e;
+        s.tail = e;
+        return true;
+    }
+    __device__ __forceinline__ uint16_t take(u32 slot, int& bandIndex)
+    {
+        heap_pop(w.heap, heapN);
+        NodeVal& s = w.val[side][slot];
+        const uint16_t head = s.head;
+        bandIndex = s.band;
+        s.active = 0;
+        s.head = kNil;
+        s.tail = kNil;
+        return head;
+    }
+    __device__ __forceinline__ int enter(u32 slot)
+    {
+        if (count >= caps.band || count >= 32767) return -1;
+        w.val[side][slot].band = (int16_t)count;
+        return (int)count++;
+    }
+    __device__ __forceinline__ int band_of(u32 slot) const { return w.val[side][slot].band; }
+    __device__ __forceinline__ NodeRec record(const DevGraph& g, u32, u32 node) { return node_record(g, node); }
+    __device__ __forceinline__ u32 prev_component(const DevGraph& g, u32, u32 node) const { return g.comp[node]; }
+    __device__ __forceinline__ bool prev_linear(const DevGraph& g, u32, u32 node) const { return g.lin[node] != 0; }
+};
+
 // IUPAC membership of every byte value (bit0 A, bit1 C, bit2 G, bit3 T; 0 = '-',
 // -1 = not a sequence character), filled from iupac_mask on the host at load time and
 // copied into shared memory by every block (lanes index it by data: the constant
@@ -211,22 +512,36 @@ __device__ __forceinline__ void load_iupac_table()
     __syncthreads();
 }
 
-// Match masks of the 64 rows starting at read position j (getEqVector, Common.h:279-318):
-// lane k reads rows k and k + 32 and the masks come from ballots.  False when a row holds
-// a non-sequence byte, or a gap inside a full 64-row window (the reference asserts).
-__device__ __noinline__ bool eq_vector(const uint8_t* seq, u32 len, int64_t j, EqV4& eq, u32 lane)
+// The read's bytes at rows lane and lane + 32 of the slice at j, -1 past the read's end
+struct RowBytes
 {
-    const bool full = j + 64 <= (int64_t)len;
+    int lo, hi;
+};
+
+__device__ __forceinline__ RowBytes row_bytes(const uint8_t* seq, u32 len, int64_t j, u32 lane)
+{
+    RowBytes r;
+    r.lo = j + lane < (int64_t)len ? seq[j + lane] : -1;
+    r.hi = j + lane + 32 < (int64_t)len ? seq[j + lane + 32] : -1;
+    return r;
+}
+
+// Match masks of 64 rows (getEqVector, Common.h:279-318): the masks come from ballots.  False
+// when a row holds a non-sequence byte, or a gap inside a full 64-row window (the reference
+// asserts).
+__device__ __forceinline__ bool eq_of_rows(const RowBytes& r, EqV4& eq)
+{
+    const bool full = __ballot_sync(kFull, r.hi < 0) == 0;
     int m0 = 0, m1 = 0;
     bool bad = false;
-    if (j + lane < (int64_t)len)
+    if (r.lo >= 0)
     {
-        m0 = s_iupac[seq[j + lane]];
+        m0 = s_iupac[r.lo];
         bad |= m0 < 0 || (m0 == 0 && full);
     }
-    if (j + lane + 32 < (int64_t)len)
+    if (r.hi >= 0)
     {
-        m1 = s_iupac[seq[j + lane + 32]];
+        m1 = s_iupac[r.hi];
         bad |= m1 < 0 || (m1 == 0 && full);
     }
     eq.a = (u64)__ballot_sync(kFull, m0 & 1) | ((u64)__ballot_sync(kFull, m1 & 1) << 32);
@@ -234,6 +549,11 @@ __device__ __noinline__ bool eq_vector(const uint8_t* seq, u32 len, int64_t j, E
     eq.g = (u64)__ballot_sync(kFull, m0 & 4) | ((u64)__ballot_sync(kFull, m1 & 4) << 32);
     eq.t = (u64)__ballot_sync(kFull, m0 & 8) | ((u64)__ballot_sync(kFull, m1 & 8) << 32);
     return __ballot_sync(kFull, bad) == 0;
+}
+
+__device__ __noinline__ bool eq_vector(const uint8_t* seq, u32 len, int64_t j, EqV4& eq, u32 lane)
+{
+    return eq_of_rows(row_bytes(seq, len, j, lane), eq);
 }
 
 // graph character of node n at pos (AlignmentGraph::NodeSequences) as an IUPAC mask
@@ -459,7 +779,10 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
     return true;
 }
 
-// calculateNodeInner (Common.h:1113-1478).  Multi = false: the single-seed path, whose extra
+// calculateNodeInner (Common.h:1113-1478).  nodeLength, c0, c1: the node's length and 2-bit
+// sequence.  flags: the band entry's, 0 for a node that has none yet.  singleInPrevBand: the
+// node's only in-neighbour is in the previous band.  endColumn: the node's last column in this
+// slice.  Multi = false: the single-seed path, whose extra
 // slice is always the fake one.  Multi = true: the multiseed DP, where `extra` (non-null for
 // a node that is a seed start in this slice) is merged into every column and an incoming
 // column that starts a seed forces the computation (EdgeWithPriority::forceCalculation).
@@ -482,8 +805,9 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
 // records behind generic pointers: 50,000 extensions (250 Mbp) 115.6 -> 102.9 ms, one seed of a
 // 10 kbp read 13 % less.
 template <bool Fill, bool Multi = false>
-__device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i, Item& slice, const EqV4& eqv, const PrevInfo& prev,
-    const Extra* pool, uint16_t head, const WS* singleIncoming, bool singleInPrevBand, i32 seqOffset, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
+__device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i, u32 nodeLength, u64 c0, u64 c1, Item& slice, u32 flags,
+    const EqV4& eqv, const PrevInfo& prev, const Extra* pool, uint16_t head, uint16_t nil, const WS* singleIncoming, bool singleInPrevBand,
+    i32 seqOffset, WS& endColumn, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
 {
     Col* const cols = node_cols().cols;
     u64* const eqcol = node_cols().eqcol;
@@ -497,20 +821,13 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     result.maxX = kIntMin;
     result.maxXNode = 0xffffffffu;
     result.cells = 0;
-    const u32 nodeLength = g.len[i];
     const bool amb = i >= g.firstAmbiguous;
-    u64 c0 = 0, c1 = 0, a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-    if (!amb)
-    {
-        c0 = g.seq2[(u64)i * 2];
-        c1 = g.seq2[(u64)i * 2 + 1];
-    }
-    else
+    u64 a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+    if (amb)
     {
         const u64* a = g.seqAmb + (u64)(i - g.firstAmbiguous) * 4;
         a0 = a[0]; a1 = a[1]; a2 = a[2]; a3 = a[3];
     }
-    const u32 inDeg = g.inOff[i + 1] - g.inOff[i];
     auto mask_at = [&](u32 pos) -> u64
     {
         if (!amb) return eq_pick(eqv, (u32)(((pos < 32 ? c0 : c1) >> ((pos & 31) * 2)) & 3));
@@ -530,9 +847,10 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     else
     {
         #pragma unroll 1
-        for (uint16_t e = head; e != kNil; e = pool[e].next)
+        for (uint16_t e = head; e != nil;)
         {
-            const Extra& inc = pool[e];
+            const Extra inc = pool[e];
+            e = inc.next;
             WS incWs = ws_make(inc.VP, inc.VN, inc.end);
             result.cells++;
             if (Multi && (inc.skip & 2)) forceCalculation = true;
@@ -573,8 +891,9 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     if (hasExtra) ws = merge_w(ws, *extra, lane);
     const WS wsX = ws;
     // (the recomputation starts from the stored first column, whose merge with itself changes nothing)
-    if (Fill && !forceCalculation && (slice.node & kExists) != 0 && merge_existing(ws, slice, hasSkipless, inDeg == 1 && singleInPrevBand, lane))
+    if (Fill && !forceCalculation && (flags & kExists) != 0 && merge_existing(ws, slice, hasSkipless, singleInPrevBand, lane))
     {
+        endColumn = ws_make(slice.eVP, slice.eVN, slice.eEnd);
         if (!boundOk || xscore_bound(wsX, seqOffset, cost) > (int64_t)sliceMaxX)
             result.maxX = ws_max_xscore(wsX, seqOffset, cost, 64, kAllOnes);
         return result;
@@ -609,7 +928,7 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     slice.sVP = ws.VP;
     slice.sVN = ws.VN;
     slice.sEnd = ws.end;
-    slice.node = i | kExists | (slice.node & kSeedStart);
+    slice.node = i | kExists | (flags & kSeedStart);
     const u64 forceEq = prev.exists ? kAllOnes : (kAllOnes ^ 1);
     // the traceback's recomputation stops at the column it needs last
     const u32 columns = Fill ? nodeLength : (lastColumn + 1 < nodeLength ? lastColumn + 1 : nodeLength);
@@ -770,6 +1089,7 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     slice.eVP = ws.VP;
     slice.eVN = ws.VN;
     slice.eEnd = ws.end;
+    endColumn = ws;
     return result;
 }
 
@@ -961,10 +1281,11 @@ struct SliceSeeds
 
 // calculateSlice (GraphAlignerBitvectorBanded.h:255-511), component-queue branch.  Multi:
 // the multiseed DP's slice, whose seeds enter the band first (addSeedHitToScoresAndQueue,
-// :228-253) and whose nodes keep their best exact-end-position X-score in w.nodeMax.
-template <bool Multi = false>
-__device__ SliceResult fill_slice(const FillArgs& a, const WSpace& w, int cur, u32 curGen, u32 prevGen, u32& curCount, u32 prevCount,
-    const uint8_t* seq, u32 seqLen, int64_t j, i32 prevQuit, i32 prevMin, u64& steps, int& err, u32 lane, const SliceSeeds* seeds = nullptr)
+// :228-253) and whose nodes keep their best exact-end-position X-score in the tables' node_max.
+// rows: the slice's read bytes on entry, the next slice's on return (loaded while this one runs).
+template <class Tables, bool Multi = false>
+__device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, const uint8_t* seq, u32 seqLen, RowBytes& rows, int64_t j,
+    i32 prevQuit, i32 prevMin, u64& steps, int& err, u32 lane, const SliceSeeds* seeds = nullptr)
 {
     if (Multi)
     {
@@ -981,14 +1302,11 @@ __device__ SliceResult fill_slice(const FillArgs& a, const WSpace& w, int cur, u
     }
     const DevGraph& g = a.g;
     const int bw = (int)a.bandwidth;
-    const int prv = cur ^ 1;
-    Item* curBand = w.band[cur];
-    const Item* prevBand = w.band[prv];
-    u64* curKey = w.key[cur];
-    NodeVal* curVal = w.val[cur];
-    const u64* prevKey = w.key[prv];
-    const NodeVal* prevVal = w.val[prv];
-    const u32 hcap = a.caps.hash;
+    t.next();
+    Item* const band = t.band();
+    const Item* const prevBand = t.prev_band();
+    i32* const nodeMax = t.node_max();
+    const uint16_t nil = Tables::kNoExtra;
     SliceResult res;
     res.minScore = kIntMax - bw - 1;
     res.minScoreNode = 0xffffffffu;
@@ -996,70 +1314,59 @@ __device__ SliceResult fill_slice(const FillArgs& a, const WSpace& w, int cur, u
     res.maxXNode = 0;
     res.cells = 0;
     EqV4 eqv;
-    if (!eq_vector(seq, seqLen, j, eqv, lane)) { err = GA_ASSERT; return res; }
-    u32 heapN = 0;
-    u32 poolN = 0;
-    u32 used = 0;
-    curCount = 0;
+    if (!eq_of_rows(rows, eqv)) { err = GA_ASSERT; return res; }
+    rows = row_bytes(seq, seqLen, j + 64, lane);
 
-    // band index of node in the previous slice, or -1
-    auto prevBandOf = [&](u32 node) -> int
+    auto insert = [&](int slot, u32 node, u32 component, i32 score, const WS& c, bool skip, bool force) -> bool
     {
-        const int s = tbl_find(prevKey, hcap, prevGen, node, lane);
-        return s < 0 ? -1 : (int)prevVal[s].band;
-    };
-
-    auto insert = [&](u32 target, i32 score, u64 vp, u64 vn, i32 end, bool skip, bool force) -> bool
-    {
-        const int slot = tbl_get_or_add(curKey, curVal, hcap, curGen, target, used, lane);
         if (slot < 0) return false;
-        NodeVal& s = curVal[slot];
-        if (!s.active)
-        {
-            if (heapN >= a.caps.heap) return false;
-            HeapItem hi; hi.component = g.comp[target]; hi.score = score; hi.node = target;
-            heap_push(w.heap, heapN, hi);
-            s.active = 1;
-            s.head = kNil;
-            s.tail = kNil;
-        }
-        if (poolN >= a.caps.extras) return false;
-        uint16_t e = (uint16_t)poolN++;
         Extra x;
-        x.VP = vp; x.VN = vn; x.end = end; x.next = kNil; x.skip = (skip ? 1 : 0) | (force ? 2 : 0);
-        w.extras[e] = x;
-        if (s.head == kNil) s.head = e;
-        else w.extras[s.tail].next = e;
-        s.tail = e;
-        return true;
+        x.VP = c.VP; x.VN = c.VN; x.end = c.end; x.next = nil; x.skip = (skip ? 1 : 0) | (force ? 2 : 0);
+        return t.queue(slot, node, component, score, x);
     };
 
+    // the previous band's nodes that are within its quit score, 32 entries at a time
     #pragma unroll 1
-    for (u32 k = 0; k < prevCount; k++)
+    for (u32 from = 0; from < t.prevCount; from += 32)
     {
-        const Item& it = prevBand[k];
-        u32 node = it.node & kNodeMask;
-        if (j == 0)
+        i32 minScore = kIntMax, sEnd = 0;
+        u32 id = 0;
+        if (from + lane < t.prevCount)
         {
-            if (it.minScore > prevQuit) { err = GA_ASSERT; return res; }
+            const Item& it = prevBand[from + lane];
+            minScore = it.minScore;
+            sEnd = it.sEnd;
+            id = it.node & kNodeMask;
         }
-        else
+        const u32 have = t.prevCount - from < 32 ? (1u << (t.prevCount - from)) - 1u : kFull;
+        u32 admitted = __ballot_sync(kFull, minScore <= prevQuit) & have;
+        if (j == 0 && admitted != have) { err = GA_ASSERT; return res; }
+        #pragma unroll 1
+        while (admitted)
         {
-            if (it.minScore > prevQuit) continue;
-            if (g.lin[node])
+            const u32 k = (u32)__ffs((int)admitted) - 1;
+            admitted &= admitted - 1;
+            const u32 node = __shfl_sync(kFull, id, (int)k);
+            if (j != 0 && t.prev_linear(g, from + k, node))
             {
-                const int pb = prevBandOf(g.inNb[g.inOff[node]]);
+                const int pb = t.prev_of(g.inNb[g.inOff[node]]);
                 if (pb >= 0)
                 {
                     const Item& pn = prevBand[pb];
                     if (pn.eEnd < prevQuit && pn.minScore < prevQuit) continue;
                 }
             }
+            const u32 component = t.prev_component(g, from + k, node);
+            const WS src = ws_source(__shfl_sync(kFull, sEnd, (int)k));
+            // the band's nodes are distinct and the table is still empty of them
+            if (!insert(t.add(g, node, component), node, component, __shfl_sync(kFull, minScore, (int)k), src, true, false))
+            {
+                err = GA_CAPACITY;
+                return res;
+            }
         }
-        WS src = ws_source(it.sEnd);
-        if (!insert(node, it.minScore, src.VP, src.VN, src.end, true, false)) { err = GA_CAPACITY; return res; }
     }
-    if (!Multi && heapN == 0) { err = GA_ASSERT; return res; }
+    if (!Multi && t.heapN == 0) { err = GA_ASSERT; return res; }
     if (Multi && ws_before(seeds->ws) < wadd(prevQuit, 64))
     {
         // the seed starts: in the band before any node of the queue, computed first among equals
@@ -1067,94 +1374,97 @@ __device__ SliceResult fill_slice(const FillArgs& a, const WSpace& w, int cur, u
         for (u32 k = 0; k < seeds->count; k++)
         {
             const u32 node = seeds->nodes[k];
-            const int slot = tbl_get_or_add(curKey, curVal, hcap, curGen, node, used, lane);
+            const u32 component = g.comp[node];
+            const int slot = t.slot_of(g, node, component);
             if (slot < 0) { err = GA_CAPACITY; return res; }
-            NodeVal& sv = curVal[slot];
-            if (sv.band >= 0) { err = GA_ASSERT; return res; }
-            if (curCount >= a.caps.band || curCount >= 32767) { err = GA_CAPACITY; return res; }
-            sv.band = (int16_t)curCount;
+            if (t.band_of((u32)slot) >= 0) { err = GA_ASSERT; return res; }
+            const int at = t.enter((u32)slot);
+            if (at < 0) { err = GA_CAPACITY; return res; }
             Item ni;
             ni.sVP = seeds->ws.VP; ni.sVN = seeds->ws.VN; ni.sEnd = seeds->ws.end;
             ni.eVP = seeds->ws.VP; ni.eVN = seeds->ws.VN; ni.eEnd = seeds->ws.end;
             ni.HP = 0; ni.HN = 0;
             ni.minScore = seeds->ws.end;
             ni.node = node | kExists | kSeedStart;
-            curBand[curCount] = ni;
-            w.nodeMax[curCount] = 0;
-            curCount++;
-            if (!insert(node, ws_value(seeds->ws, 0), seeds->ws.VP, seeds->ws.VN, seeds->ws.end, true, true)) { err = GA_CAPACITY; return res; }
+            band[at] = ni;
+            nodeMax[at] = 0;
+            if (!insert(slot, node, component, ws_value(seeds->ws, 0), seeds->ws, true, true)) { err = GA_CAPACITY; return res; }
         }
     }
     i32 curMin = res.minScore;
     const i32 seqOffset = (i32)j;
     #pragma unroll 1
-    while (heapN > 0)
+    while (t.heapN > 0)
     {
-        u32 i = w.heap[0].node;
-        const int slot = tbl_find(curKey, hcap, curGen, i, lane);
-        if (slot < 0) { err = GA_ASSERT; return res; }
-        NodeVal& s = curVal[slot];
-        if (s.band < 0)
+        const u32 i = t.heap()[0].node;
+        const u32 slot = t.heap()[0].slot;
+        const NodeRec rec = t.record(g, slot, i);
+        int at;
+        const uint16_t head = t.take(slot, at);
+        const bool fresh = at < 0;
+        if (fresh)
         {
-            if (curCount >= a.caps.band || curCount >= 32767) { err = GA_CAPACITY; return res; }
-            s.band = (int16_t)curCount;
-            Item ni;
-            ni.sVP = 0; ni.sVN = 0; ni.sEnd = kIntMax;
-            ni.eVP = 0; ni.eVN = 0; ni.eEnd = kIntMax;
-            ni.HP = 0; ni.HN = 0;
-            ni.minScore = kIntMax;
-            ni.node = i;
-            if (Multi) w.nodeMax[curCount] = 0;
-            curBand[curCount++] = ni;
+            at = t.enter(slot);
+            if (at < 0) { err = GA_CAPACITY; return res; }
+            if (Multi) nodeMax[at] = 0;
         }
-        Item& thisNode = curBand[s.band];
-        WS oldEnd = (thisNode.node & kExists) ? ws_make(thisNode.eVP, thisNode.eVN, thisNode.eEnd) : ws_make(0, 0, kIntMax);
-        const WS* extra = (Multi && (thisNode.node & kSeedStart)) ? &seeds->ws : nullptr;
+        Item& thisNode = band[at];
+        const u32 flags = fresh ? 0 : thisNode.node & (kExists | kSeedStart);
+        WS oldEnd = (flags & kExists) ? ws_make(thisNode.eVP, thisNode.eVN, thisNode.eEnd) : ws_make(0, 0, kIntMax);
+        const WS* extra = (Multi && (flags & kSeedStart)) ? &seeds->ws : nullptr;
         if (Multi && extra) oldEnd = merge_w(oldEnd, *extra, lane);
         PrevInfo prev;
-        const int pb = prevBandOf(i);
+        const int pb = t.prev_of(i);
+        prev.exists = pb >= 0;
+        prev.sEnd = 0;
+        prev.HP = kAllOnes;
+        prev.HN = 0;
         if (pb >= 0)
         {
             const Item& pi = prevBand[pb];
-            prev.exists = true;
             prev.sEnd = pi.sEnd;
             prev.HP = pi.HP;
             prev.HN = pi.HN;
         }
-        else
-        {
-            prev.exists = false;
-            prev.sEnd = 0;
-            prev.HP = kAllOnes;
-            prev.HN = 0;
-        }
-        bool singleInPrev = false;
-        if (g.inOff[i + 1] - g.inOff[i] == 1) singleInPrev = prevBandOf(g.inNb[g.inOff[i]]) >= 0;
+        // asked for only when a node is computed again
+        const bool singleInPrev = (flags & kExists) && rec_in_degree(rec.meta) == 1 && t.prev_of(rec.inNb[0]) >= 0;
         // a column whose X-score bound is at most both the slice's and the node's best so far
         // changes neither, so the node computation may skip its exact X-score
-        const i32 skipBelow = Multi ? imin(res.maxX, w.nodeMax[s.band]) : res.maxX;
-        NodeCalc nc = node_calc<true, Multi>(g, a.cost, i, thisNode, eqv, prev, w.extras, s.head, nullptr, singleInPrev, seqOffset,
-            steps, err, lane, skipBelow, 63, extra);
+        const i32 skipBelow = Multi ? imin(res.maxX, nodeMax[at]) : res.maxX;
+        WS newEnd;
+        const NodeCalc nc = node_calc<true, Multi>(g, a.cost, i, rec_len(rec.meta), rec.seq[0], rec.seq[1], thisNode, flags, eqv, prev, t.extras(), head,
+            nil, nullptr, singleInPrev, seqOffset, newEnd, steps, err, lane, skipBelow, 63, extra);
         if (err) return res;
-        if (Multi) w.nodeMax[s.band] = imax(nc.maxX, w.nodeMax[s.band]);
-        heap_pop(w.heap, heapN);
-        s.active = 0;
-        s.head = kNil;
-        s.tail = kNil;
+        if (Multi) nodeMax[at] = imax(nc.maxX, nodeMax[at]);
         if (nc.minScore > wadd(wadd(seqOffset, bw), 128)) { err = GA_ASSERT; return res; }
         curMin = imin(curMin, nc.minScore);
-        if (nc.minScore < thisNode.minScore) thisNode.minScore = nc.minScore;
-        WS newEnd = ws_make(thisNode.eVP, thisNode.eVN, thisNode.eEnd);
+        if (fresh || nc.minScore < thisNode.minScore) thisNode.minScore = nc.minScore;
         if (!ws_eq(newEnd, oldEnd))
         {
-            i32 newEndMin = changed_min_w(newEnd, oldEnd, lane);
+            const i32 newEndMin = changed_min_w(newEnd, oldEnd, lane);
             if (newEndMin == kIntMax) { err = GA_ASSERT; return res; }
             if (newEndMin <= wadd(curMin, bw))
             {
+                const u32 degree = out_degree(g, i, rec);
                 #pragma unroll 1
-                for (u32 e = g.outOff[i]; e < g.outOff[i + 1]; e++)
+                for (u32 e = 0; e < degree; e++)
                 {
-                    if (!insert(g.outNb[e], newEndMin, newEnd.VP, newEnd.VN, newEnd.end, false, false)) { err = GA_CAPACITY; return res; }
+                    u32 target, component;
+                    if (e < kRecOut)
+                    {
+                        target = e == 0 ? rec.outNb[0] : e == 1 ? rec.outNb[1] : rec.outNb[2];
+                        component = e == 0 ? rec.outComp[0] : e == 1 ? rec.outComp[1] : rec.outComp[2];
+                    }
+                    else
+                    {
+                        target = g.outNb[rec.outOff + e];
+                        component = g.comp[target];
+                    }
+                    if (!insert(t.slot_of(g, target, component), target, component, newEndMin, newEnd, false, false))
+                    {
+                        err = GA_CAPACITY;
+                        return res;
+                    }
                 }
             }
         }
@@ -1176,7 +1486,8 @@ __device__ SliceResult fill_slice(const FillArgs& a, const WSpace& w, int cur, u
     return res;
 }
 
-__device__ ExtState fill_extension(const FillArgs& a, const WSpace& w, u32& gen, ArenaCursor& arena, u32 ext, u32 lane)
+template <class Tables>
+__device__ __forceinline__ ExtState fill_extension(const FillArgs& a, Tables& t, ArenaCursor& arena, u32 ext, u32 lane)
 {
     const DevGraph& g = a.g;
     ExtState st;
@@ -1184,6 +1495,7 @@ __device__ ExtState fill_extension(const FillArgs& a, const WSpace& w, u32& gen,
     st.committed = 0;
     st.status = GA_OK;
     st.steps = 0;
+    st.aux = 0;
     const uint8_t* seq = a.seq + a.seqOff[ext];
     const u32 seqLen = a.seqLen[ext];
     const u32 startNode = a.startNode[ext];
@@ -1203,10 +1515,10 @@ __device__ ExtState fill_extension(const FillArgs& a, const WSpace& w, u32& gen,
     }
     u64* dir = (u64*)(a.arena + dirOff);
     st.dir = dirOff;
+    RowBytes rows = row_bytes(seq, seqLen, 0, lane);
     // start slice (getInitialSliceExactPosition, Common.h:1551-1587): one node, scores = distance from the offset
-    int prv = 0;
-    gen++;
-    u32 prevGen = gen;
+    t.restart();
+    t.next();
     {
         Item it;
         u32 L = g.len[startNode];
@@ -1214,24 +1526,19 @@ __device__ ExtState fill_extension(const FillArgs& a, const WSpace& w, u32& gen,
         it.eVP = 0; it.eVN = 0; it.eEnd = (i32)L - 1 - (i32)startOff;
         it.minScore = 0;
         it.node = startNode | kExists;
-        u64 hn = 0, hp = 0;
-        #pragma unroll 1
-        for (u32 k = 1; k <= startOff; k++) hn |= 1ULL << k;
-        #pragma unroll 1
-        for (u32 k = startOff + 1; k < L; k++) hp |= 1ULL << k;
-        it.HP = hp;
-        it.HN = hn;
-        w.band[prv][0] = it;
-        u32 used = 0;
-        const int s = tbl_get_or_add(w.key[prv], w.val[prv], a.caps.hash, prevGen, startNode, used, lane);
-        w.val[prv][s].band = 0;
-        if (!commit_slice(a, arena, dir, 0, w.band[prv], 1, 0, 1, 0, startNode, false, lane))
+        // -1 along columns 1..startOff, +1 after them
+        const u64 upToL = (L == 64 ? kAllOnes : (1ULL << L) - 1) & ~1ULL;
+        it.HN = upToL & (startOff == 63 ? kAllOnes : (2ULL << startOff) - 1);
+        it.HP = upToL & ~it.HN;
+        const int slot = t.add(g, startNode, g.comp[startNode]);
+        const int at = t.enter((u32)slot);
+        t.band()[at] = it;
+        if (!commit_slice(a, arena, dir, 0, t.band(), 1, 0, 1, 0, startNode, false, lane))
         {
             st.status = GA_CAPACITY;
             return st;
         }
     }
-    u32 prevCount = 1;
     u32 committed = 1;
     i32 bestX = 0;
     i32 lastMin = 0;
@@ -1239,27 +1546,20 @@ __device__ ExtState fill_extension(const FillArgs& a, const WSpace& w, u32& gen,
     #pragma unroll 1
     for (u32 s = 0; s < numSlices; s++)
     {
-        const int cur = prv ^ 1;
-        gen++;
-        const u32 curGen = gen;
-        u32 curCount = 0;
         const int64_t j = (int64_t)s * 64;
-        SliceResult r = fill_slice(a, w, cur, curGen, prevGen, curCount, prevCount, seq, seqLen, j, lastQuit, lastMin, st.steps, err, lane);
+        SliceResult r = fill_slice(a, t, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane);
         if (err) break;
         if (r.maxX > bestX) bestX = r.maxX;
         const bool notValid = r.cells >= a.maxCells;
         if ((int64_t)r.maxX < (int64_t)bestX - (int64_t)a.xdrop) break;
         if (r.minScore < lastMin) { err = GA_ASSERT; break; }
         const i32 quit = wadd(r.minScore, (i32)a.bandwidth);
-        if (!commit_slice(a, arena, dir, committed, w.band[cur], curCount, r.minScore, quit, r.maxX, r.maxXNode, notValid, lane))
+        if (!commit_slice(a, arena, dir, committed, t.band(), t.count, r.minScore, quit, r.maxX, r.maxXNode, notValid, lane))
         {
             err = GA_CAPACITY;
             break;
         }
         committed++;
-        prv = cur;
-        prevGen = curGen;
-        prevCount = curCount;
         lastMin = r.minScore;
         lastQuit = quit;
     }
@@ -1273,7 +1573,7 @@ __device__ ExtState fill_extension(const FillArgs& a, const WSpace& w, u32& gen,
 // slice of read r from the empty initial slice, each slice's seeds started in it.  Each slice's
 // best X-score also goes to a per-read array (st.aux) that the traceback lowers as it finds
 // traces.
-__device__ ExtState fill_multiseed(const FillArgs& a, const WSpace& w, u32& gen, ArenaCursor& arena, u32 r, u32 lane)
+__device__ ExtState fill_multiseed(const FillArgs& a, LargeTables& t, ArenaCursor& arena, u32 r, u32 lane)
 {
     ExtState st;
     st.dir = 0;
@@ -1296,29 +1596,24 @@ __device__ ExtState fill_multiseed(const FillArgs& a, const WSpace& w, u32& gen,
     st.dir = dirOff;
     st.aux = auxOff;
     // getInitialEmptySlice (Common.h:1541-1549): no nodes, minimum 0, bandwidth 1
-    if (!commit_slice(a, arena, dir, 0, w.band[0], 0, 0, 1, kIntMin, 0xffffffffu, false, lane, w.nodeMax))
+    t.restart();
+    t.next();
+    if (!commit_slice(a, arena, dir, 0, t.band(), 0, 0, 1, kIntMin, 0xffffffffu, false, lane, t.node_max()))
     {
         st.status = GA_CAPACITY;
         return st;
     }
     if (lane == 0) sliceMax[0] = kIntMin;
-    int prv = 0;
-    gen++;
-    u32 prevGen = gen;
-    u32 prevCount = 0;
     u32 committed = 1;
     i32 lastMin = 0;
     i32 lastQuit = 1;
     u64 k = a.seedOff[r];
     const u64 kEnd = a.seedOff[r + 1];
     int err = 0;
+    RowBytes rows = row_bytes(seq, seqLen, 0, lane);
     #pragma unroll 1
     for (u32 s = 0; s < numSlices; s++)
     {
-        const int cur = prv ^ 1;
-        gen++;
-        const u32 curGen = gen;
-        u32 curCount = 0;
         const int64_t j = (int64_t)s * 64;
         u64 next = k;
         while (next < kEnd && a.seedSlice[next] == s) next++;
@@ -1327,7 +1622,7 @@ __device__ ExtState fill_multiseed(const FillArgs& a, const WSpace& w, u32& gen,
         seeds.count = (u32)(next - k);
         seeds.ws = seed_ws(j, seqLen, a.cost);
         k = next;
-        SliceResult res = fill_slice<true>(a, w, cur, curGen, prevGen, curCount, prevCount, seq, seqLen, j, lastQuit, lastMin, st.steps, err, lane, &seeds);
+        SliceResult res = fill_slice<LargeTables, true>(a, t, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane, &seeds);
         if (err) break;
         // fillDPSlice's checks of a slice that started seeds (GraphAlignerBitvectorBanded.h:543-549)
         if (seeds.count > 0)
@@ -1338,16 +1633,13 @@ __device__ ExtState fill_multiseed(const FillArgs& a, const WSpace& w, u32& gen,
         if (!(res.minScore >= lastMin || res.minScore >= ws_value(seeds.ws, 0) || lastMin == kIntMax - bw - 1)) { err = GA_ASSERT; break; }
         const bool notValid = res.cells >= a.maxCells;
         const i32 quit = wadd(res.minScore, bw);
-        if (!commit_slice(a, arena, dir, committed, w.band[cur], curCount, res.minScore, quit, res.maxX, res.maxXNode, notValid, lane, w.nodeMax))
+        if (!commit_slice(a, arena, dir, committed, t.band(), t.count, res.minScore, quit, res.maxX, res.maxXNode, notValid, lane, t.node_max()))
         {
             err = GA_CAPACITY;
             break;
         }
         if (lane == 0) sliceMax[committed] = res.maxX;
         committed++;
-        prv = cur;
-        prevGen = curGen;
-        prevCount = curCount;
         lastMin = res.minScore;
         lastQuit = quit;
     }
@@ -1394,6 +1686,13 @@ __device__ __noinline__ const SliceRec* load_slice(const uint8_t* arena, const u
     __syncwarp();
     return &sl.rec;
 }
+
+// One warp's shared memory of the traceback, besides its columns
+struct TraceSpace
+{
+    u64* ring;             // [64] trace items not yet written out
+    SliceSlot* slots;      // [2] cached slices (odd and even)
+};
 
 struct Table
 {
@@ -1466,7 +1765,6 @@ __device__ __noinline__ u32 emit_run(u64* items, u64* ring, u32 n, u32 cap, u64 
 
 static constexpr u64 kStepLeft = ~(1ULL << 32) + 1;                 // one column left
 static constexpr u64 kStepUp = ~(1ULL << 39) + 1;                   // one row up
-static constexpr u64 kStepDiagonal = kStepLeft + kStepUp;
 
 // Trace items go to a 64-entry ring in shared memory and out to the caller's buffer 32 at a
 // time, one item per lane.  A run of steps inside one node goes in at once.
@@ -1677,15 +1975,17 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
     const Item* pi = t.template find<Multi>(s - 1, node);
     if (pi) { prev.exists = true; prev.sEnd = pi->sEnd; prev.HP = pi->HP; prev.HN = pi->HN; }
     else { prev.exists = false; prev.sEnd = 0; prev.HP = kAllOnes; prev.HN = 0; }
-    Item copy = *it;
+    Item copy;
     WS start = ws_make(it->sVP, it->sVN, it->sEnd);
+    WS last;
     u64 steps = 0;
     int err = 0;
     int64_t j = ((int64_t)s - 1) * 64;
-    node_calc<false, Multi>(g, cost, node, copy, eqv, prev, nullptr, kNil, &start, false, (i32)j, steps, err, lane, kIntMin, lastColumn,
-        (Multi && extra.end != kIntMax) ? &extra : nullptr);
+    const NodeRec rec = node_record(g, node);
+    const u32 L = rec_len(rec.meta);
+    node_calc<false, Multi>(g, cost, node, L, rec.seq[0], rec.seq[1], copy, it->node, eqv, prev, nullptr, kNil, kNil, &start, false, (i32)j, last,
+        steps, err, lane, kIntMin, lastColumn, (Multi && extra.end != kIntMax) ? &extra : nullptr);
     if (err) return err;
-    u32 L = g.len[node];
     if (!ws_eq(ws_make(cols[0].VP, cols[0].VN, cols[0].end), start)) return GA_ASSERT;
     if (lastColumn + 1 >= L && !ws_eq(ws_make(cols[L - 1].VP, cols[L - 1].VN, cols[L - 1].end), ws_make(it->eVP, it->eVN, it->eEnd)))
         return GA_ASSERT;
@@ -1930,7 +2230,7 @@ __device__ __forceinline__ u32 row0_run_start(const Col* cols, u32 off, u32 lane
 // up to the row above the read or, in the multiseed DP (Multi), to a seed start.  resultScore:
 // the trace's OnewayTrace::score.  Returns 0 or the error status.
 template <bool Multi>
-__device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uint8_t* seq, u32 seqLen, u32 committed, Table& t, TraceOutT<Multi>& to, const WSpace& w,
+__device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uint8_t* seq, u32 seqLen, u32 committed, Table& t, TraceOutT<Multi>& to, const TraceSpace& w,
     TPos start, i32 startScore, i32& resultScore, u32 lane)
 {
     int err = 0;
@@ -2164,7 +2464,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     return err;
 }
 
-__device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st, const WSpace& w, u32 lane)
+__device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st, const TraceSpace& w, u32 lane)
 {
     const DevGraph& g = a.g;
     u64* out = a.traceItems + a.traceOffset[ext];
@@ -2325,7 +2625,7 @@ __device__ void ms_candidates(const MultiTraceArgs& a, u32 r, const ExtState& st
 // The first cell of a candidate's trace (getLocalMaximaTracesFromTable): among the node's
 // columns, recomputed with its seed start, the cell of greatest row that scores the node's
 // best X-score (the first column on ties); a cell above it is GA_ASSERT.
-__device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const WSpace& w, const uint8_t* seq, u32 seqLen, const MsCand& c,
+__device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const TraceSpace& w, const uint8_t* seq, u32 seqLen, const MsCand& c,
     TPos& start, i32& startScore, u32 lane)
 {
     const DevGraph& g = a.g;
@@ -2381,7 +2681,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const WSpace& w,
 // span and last cell.  write = true (a kept trace of a read whose traces all fit and, with
 // exact room, that removeDuplicateTraces kept): walks it again into the read's output at
 // the place the read's selection (or the host, with exact room) gave it.
-__device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const WSpace& w, bool write, u32 lane)
+__device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const TraceSpace& w, bool write, u32 lane)
 {
     const MsCand c = *cp;
     const u32 r = c.read;
@@ -2595,27 +2895,13 @@ __device__ __forceinline__ bool next_extension(u32* counter, u32 num, const u32*
 }
 
 // The fill: a warp takes the next extension of the longest-first order, fills its DP table
-// into the arena and records where it is, then takes the next.  The frontier tables are in
-// dynamic shared memory (fa.workspace == nullptr) or in the global workspace, one stride
-// per warp.
-__global__ void __launch_bounds__(128, 4) fill_kernel(FillArgs fa, u32* counter)
+// into the arena and records where it is, then takes the next.
+template <class Tables>
+__device__ __forceinline__ void fill_extensions(const FillArgs& fa, u32* counter)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
-    const u32 warpInBlock = threadIdx.x >> 5;
-    const u64 gwarp = (u64)blockIdx.x * (blockDim.x >> 5) + warpInBlock;
-    uint8_t* base = fa.workspace ? fa.workspace + gwarp * fa.workspaceStride
-        : dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (u64)warpInBlock * fa.workspaceStride;
-    const WSpace w = wspace_at(base, fa.caps);
-    // generation 0 marks every node-table slot empty
-#pragma unroll 1
-    for (u32 k = lane; k < fa.caps.hash; k += 32)
-    {
-        w.key[0][k] = 0;
-        w.key[1][k] = 0;
-    }
-    __syncwarp();
-    u32 gen = 0;
+    Tables t(fa, (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane);
     ArenaCursor arena;
     arena.pos = 0;
     arena.end = 0;
@@ -2625,24 +2911,14 @@ __global__ void __launch_bounds__(128, 4) fill_kernel(FillArgs fa, u32* counter)
     while (next_extension(counter, fa.num, fa.order, fa.prevStatus, lane, ext))
     {
         __syncwarp();
-        const ExtState st = fill_extension(fa, w, gen, arena, ext, lane);
+        const ExtState st = fill_extension(fa, t, arena, ext, lane);
         if (lane == 0) fa.states[ext] = st;
-        if (gen > 0xF0000000u)
-        {
-            // generation stamps are about to wrap: clear this warp's tables
-            __syncwarp();
-#pragma unroll 1
-            for (u32 k2 = lane; k2 < fa.caps.hash; k2 += 32)
-            {
-                w.key[0][k2] = 0;
-                w.key[1][k2] = 0;
-            }
-            __syncwarp();
-            gen = 0;
-        }
     }
     if (lane == 0 && arena.used) atomicAdd(fa.arenaCursor + 1, (unsigned long long)arena.used);
 }
+
+__global__ void __launch_bounds__(128, 4) fill_kernel(FillArgs fa, u32* counter) { fill_extensions<SmallTables>(fa, counter); }
+__global__ void __launch_bounds__(128, 4) fill_large_kernel(FillArgs fa, u32* counter) { fill_extensions<LargeTables>(fa, counter); }
 
 // the traceback's shared memory of one warp behind the block's NodeCols
 static constexpr u32 kTraceSpaceBytes = 64 * 8 + 2 * sizeof(SliceSlot);
@@ -2654,7 +2930,7 @@ __global__ void __launch_bounds__(128, 6) trace_kernel(TraceArgs ta, u32* counte
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
     uint8_t* base = dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (threadIdx.x >> 5) * kTraceSpaceBytes;
-    WSpace w {};
+    TraceSpace w;
     w.ring = (u64*)base;
     w.slots = (SliceSlot*)(base + 64 * 8);
     u32 ext;
@@ -2673,16 +2949,7 @@ __global__ void __launch_bounds__(128, 4) fill_multiseed_kernel(FillArgs fa, u32
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
-    const u64 gwarp = (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const WSpace w = wspace_at(fa.workspace + gwarp * fa.workspaceStride, fa.caps);
-#pragma unroll 1
-    for (u32 k = lane; k < fa.caps.hash; k += 32)
-    {
-        w.key[0][k] = 0;
-        w.key[1][k] = 0;
-    }
-    __syncwarp();
-    u32 gen = 0;
+    LargeTables t(fa, (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane);
     ArenaCursor arena;
     arena.pos = 0;
     arena.end = 0;
@@ -2692,20 +2959,8 @@ __global__ void __launch_bounds__(128, 4) fill_multiseed_kernel(FillArgs fa, u32
     while (next_extension(counter, fa.num, fa.order, fa.prevStatus, lane, r))
     {
         __syncwarp();
-        const ExtState st = fill_multiseed(fa, w, gen, arena, r, lane);
+        const ExtState st = fill_multiseed(fa, t, arena, r, lane);
         if (lane == 0) fa.states[r] = st;
-        if (gen > 0xF0000000u)
-        {
-            __syncwarp();
-#pragma unroll 1
-            for (u32 k2 = lane; k2 < fa.caps.hash; k2 += 32)
-            {
-                w.key[0][k2] = 0;
-                w.key[1][k2] = 0;
-            }
-            __syncwarp();
-            gen = 0;
-        }
     }
     if (lane == 0 && arena.used) atomicAdd(fa.arenaCursor + 1, (unsigned long long)arena.used);
 }
@@ -2764,7 +3019,7 @@ __global__ void __launch_bounds__(128, 6) ms_trace_kernel(MultiTraceArgs ta, u32
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
     uint8_t* base = dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (threadIdx.x >> 5) * kTraceSpaceBytes;
-    WSpace w {};
+    TraceSpace w;
     w.ring = (u64*)base;
     w.slots = (SliceSlot*)(base + 64 * 8);
     const u64 total = write ? (*ta.candTotal < ta.candCap ? *ta.candTotal : ta.candCap) : *ta.workCount;
@@ -2781,9 +3036,9 @@ __global__ void __launch_bounds__(128, 6) ms_trace_kernel(MultiTraceArgs ta, u32
 }
 }
 
-// dynamic shared memory of a block of the fill kernels (tables: bytes of a warp's tables kept
-// there) and of the traceback kernels
-static size_t fill_smem(int warpsPerBlock, size_t tables) { return (sizeof(gadev::NodeCols) + tables) * warpsPerBlock; }
+// dynamic shared memory of a block of the fill kernels (shared: with its frontier tables) and of
+// the traceback kernels
+static size_t fill_smem(int warpsPerBlock, bool shared) { return (sizeof(gadev::NodeCols) + (shared ? sizeof(gadev::SmallSpace) : 0)) * warpsPerBlock; }
 static size_t trace_smem(int warpsPerBlock) { return (sizeof(gadev::NodeCols) + gadev::kTraceSpaceBytes) * warpsPerBlock; }
 
 uint64_t ga_warp_tables_bytes(const gadev::Caps& c) { return gadev::wspace_bytes(c); }
@@ -2794,12 +3049,13 @@ static bool set_smem(const void* kernel, size_t smem)
     return smem <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
 }
 
-int ga_fill_blocks_per_sm(int warpsPerBlock, const gadev::Caps& caps, bool shared)
+int ga_fill_blocks_per_sm(int warpsPerBlock, bool shared)
 {
-    const size_t smem = fill_smem(warpsPerBlock, shared ? (size_t)gadev::wspace_bytes(caps) : 0);
-    if (!set_smem((const void*)gadev::fill_kernel, smem)) return 0;
+    const size_t smem = fill_smem(warpsPerBlock, shared);
+    const auto kernel = shared ? gadev::fill_kernel : gadev::fill_large_kernel;
+    if (!set_smem((const void*)kernel, smem)) return 0;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gadev::fill_kernel, warpsPerBlock * 32, smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, warpsPerBlock * 32, smem) != cudaSuccess) return 0;
     return n;
 }
 
@@ -2815,10 +3071,11 @@ int ga_trace_blocks_per_sm(int warpsPerBlock)
 int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int traceBlocks,
     int warpsPerBlock, void* stream)
 {
-    const size_t fillSmem = fill_smem(warpsPerBlock, fa.workspace ? 0 : (size_t)fa.workspaceStride);
+    const size_t fillSmem = fill_smem(warpsPerBlock, fa.workspace == nullptr);
+    const auto fill = fa.workspace ? gadev::fill_large_kernel : gadev::fill_kernel;
     const size_t traceSmem = trace_smem(warpsPerBlock);
-    if (!set_smem((const void*)gadev::fill_kernel, fillSmem) || !set_smem((const void*)gadev::trace_kernel, traceSmem)) return -1;
-    gadev::fill_kernel<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
+    if (!set_smem((const void*)fill, fillSmem) || !set_smem((const void*)gadev::trace_kernel, traceSmem)) return -1;
+    fill<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;
     gadev::trace_kernel<<<traceBlocks, warpsPerBlock * 32, traceSmem, (cudaStream_t)stream>>>(ta, counters + 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -2828,7 +3085,7 @@ int ga_launch_multiseed_fill(const gadev::FillArgs& fa, const gadev::MultiTraceA
     int warpsPerBlock, void* stream)
 {
     if (!fa.workspace) return -1;
-    const size_t fillSmem = fill_smem(warpsPerBlock, 0);
+    const size_t fillSmem = fill_smem(warpsPerBlock, false);
     if (!set_smem((const void*)gadev::fill_multiseed_kernel, fillSmem)) return -1;
     gadev::fill_multiseed_kernel<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;
@@ -2867,6 +3124,12 @@ int ga_launch_multiseed_write(const gadev::MultiTraceArgs& ta, uint32_t* counter
     const size_t traceSmem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)gadev::ms_trace_kernel, traceSmem)) return -1;
     gadev::ms_trace_kernel<<<candBlocks, warpsPerBlock * 32, traceSmem, (cudaStream_t)stream>>>(ta, counters + 6, 1);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int ga_build_node_records(const gadev::DevGraph& g, gadev::NodeRec* rec, void* stream)
+{
+    gadev::node_records_kernel<<<(g.N + 255) / 256, 256, 0, (cudaStream_t)stream>>>(g, rec);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -6,9 +6,30 @@
 namespace gadev
 {
 
+// What the DP needs of one node, in one 64-byte record: read field by field from the arrays
+// below, a node's computation waited for five loads in a row (offsets, then neighbours, then
+// their components), about 600 cycles each from L2 for a warp alone.
+struct __align__(16) NodeRec
+{
+    u64 seq[2];            // 2-bit sequence; not set for an ambiguous node
+    u32 comp;
+    u32 meta;              // bits 0-6 length, 7 linearizable, 8-19 in-degree, 20-31 out-degree (each 4095 at most)
+    u32 inOff;
+    u32 outOff;
+    u32 inNb[2];           // the first neighbours, the others are read from the arrays
+    u32 outNb[3];
+    u32 outComp[3];        // components of outNb
+};
+static constexpr u32 kRecIn = 2, kRecOut = 3, kRecDegree = 4095;
+static constexpr u32 kRecLinearizable = 0x80;
+GA_HD u32 rec_len(u32 meta) { return meta & 0x7f; }
+GA_HD u32 rec_in_degree(u32 meta) { return (meta >> 8) & kRecDegree; }
+GA_HD u32 rec_out_degree(u32 meta) { return meta >> 20; }
+
 // AlignmentGraph fields the DP reads (AlignmentGraph.h:121-139), device copies.
 struct DevGraph
 {
+    const NodeRec* rec;    // [N], or null: the records are put together from the arrays as they are needed
     u32 N;
     u32 firstAmbiguous;
     const u32* len;
@@ -69,7 +90,11 @@ struct ExtState
     u64 aux;               // multiseed DP: arena offset of the per-slice best X-scores (i32 [committed])
 };
 
-// Capacities of one warp's frontier tables.
+// The fill's tables in shared memory: band entries and node-table slots of a slice, heap
+// entries, pending incoming columns of a slice.  A slot belongs to a lane, so 32 is the most.
+static constexpr u32 kSmallBand = 32, kSmallHeap = 32, kSmallExtras = 64;
+
+// Capacities of one warp's frontier tables in global memory.
 struct Caps
 {
     u32 band;              // band entries per slice
@@ -96,9 +121,9 @@ struct FillArgs
     u64 arenaBytes;
     unsigned long long* arenaCursor;   // [0] bytes handed out in chunks, [1] bytes the tables took (both start at 0)
     u64 chunkBytes;        // arena bytes a warp takes at once
-    uint8_t* workspace;    // nullptr: the frontier tables live in shared memory
-    u64 workspaceStride;   // bytes of one warp's tables
-    Caps caps;
+    uint8_t* workspace;    // nullptr: the frontier tables live in shared memory (kSmall*), else
+    u64 workspaceStride;   // bytes of one warp's tables there
+    Caps caps;             // and their capacities
     const i32* prevStatus; // when non-null, only extensions whose previous status is GA_CAPACITY run
     ExtState* states;      // [num] where each extension's table is, for the traceback
     // multiseed DP (nullptr otherwise): read i's seeds are [seedOff[i], seedOff[i+1]),
@@ -235,13 +260,13 @@ struct MultiTraceArgs
 
 }
 
-// bytes of one warp's frontier tables for these capacities (the multiseed DP's add each band
+// bytes of one warp's frontier tables in global memory for these capacities (the multiseed DP's add each band
 // node's best X-score)
 uint64_t ga_warp_tables_bytes(const gadev::Caps& caps);
 uint64_t ga_multiseed_tables_bytes(const gadev::Caps& caps);
 // resident blocks of 32 * warpsPerBlock threads per SM of the fill kernel (shared: tables in
 // shared memory) and of the traceback kernel
-int ga_fill_blocks_per_sm(int warpsPerBlock, const gadev::Caps& caps, bool shared);
+int ga_fill_blocks_per_sm(int warpsPerBlock, bool shared);
 int ga_trace_blocks_per_sm(int warpsPerBlock);
 // launches the fill kernel and then the traceback kernel on `stream`, blocks of warpsPerBlock
 // warps, one extension per warp at a time; counters[0] and [1] must be zero
@@ -267,4 +292,6 @@ int ga_launch_multiseed_write(const gadev::MultiTraceArgs& ta, uint32_t* counter
 // exact room: each kept trace's summary into ta.keys
 int ga_launch_multiseed_keys(const gadev::MultiTraceArgs& ta, void* stream);
 int ga_upload_tables();
+// fills rec[0..N) from the graph's arrays
+int ga_build_node_records(const gadev::DevGraph& g, gadev::NodeRec* rec, void* stream);
 void ga_set_last_error(const char* message);

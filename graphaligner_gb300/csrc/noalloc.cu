@@ -45,17 +45,6 @@ void setup_device(int device)
     g_setupError[device] = e;
     if (e == cudaSuccess) g_scratchAddress[device] = p;
 }
-
-// frontier-table capacities: the shared-memory layout of the regular entry point
-Caps small_caps()
-{
-    Caps c;
-    c.band = 32;
-    c.hash = 64;
-    c.heap = 32;
-    c.extras = 64;
-    return c;
-}
 }
 
 extern "C" int ga_extend_batch_noalloc(const ga_graph_desc* device_graph, const ga_extend_params* params,
@@ -120,7 +109,7 @@ extern "C" int ga_extend_batch_noalloc(const ga_graph_desc* device_graph, const 
         return GA_ERR_CUDA;
     }
 
-    DevGraph g;
+    DevGraph g {};
     g.N = gd.num_nodes;
     g.firstAmbiguous = gd.first_ambiguous;
     g.len = gd.node_length;
@@ -152,8 +141,6 @@ extern "C" int ga_extend_batch_noalloc(const ga_graph_desc* device_graph, const 
     fa.arenaCursor = (unsigned long long*)(scratch + 16);
     fa.chunkBytes = 16 * 1024;
     fa.workspace = nullptr;
-    fa.caps = small_caps();
-    fa.workspaceStride = ga_warp_tables_bytes(fa.caps);
     fa.prevStatus = nullptr;
     fa.states = (ExtState*)(scratch + kHeaderBytes);
 

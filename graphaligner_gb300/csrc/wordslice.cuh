@@ -370,7 +370,8 @@ GA_HD int iupac_mask(unsigned char c)
 // libstdc++'s std::priority_queue<..., std::greater<>> (push_heap / pop_heap,
 // bits/stl_heap.h): ties in (component, score) then resolve the same way
 // (ComponentPriorityQueue.h:11-19,153).
-struct HeapItem { u32 component; i32 score; u32 node; };
+// slot: the node's slot in the caller's table, no part of the order.
+struct HeapItem { u32 component; i32 score; u32 node; u32 slot = 0; };
 
 GA_HD bool heap_greater(const HeapItem& a, const HeapItem& b)
 {
@@ -382,9 +383,10 @@ GA_HD void heap_push(HeapItem* h, u32& n, HeapItem v)
     u32 hole = n;
     while (hole > 0)
     {
-        u32 parent = (hole - 1) / 2;
-        if (!heap_greater(h[parent], v)) break;
-        h[hole] = h[parent];
+        const u32 parent = (hole - 1) / 2;
+        const HeapItem up = h[parent];
+        if (!heap_greater(up, v)) break;
+        h[hole] = up;
         hole = parent;
     }
     h[hole] = v;
@@ -393,36 +395,37 @@ GA_HD void heap_push(HeapItem* h, u32& n, HeapItem v)
 
 GA_HD void heap_pop(HeapItem* h, u32& n)
 {
-    if (n > 1)
-    {
-        HeapItem v = h[n - 1];
-        h[n - 1] = h[0];
-        long len = (long)n - 1;
-        long hole = 0;
-        long child = 0;
-        while (child < (len - 1) / 2)
-        {
-            child = 2 * (child + 1);
-            if (heap_greater(h[child], h[child - 1])) child--;
-            h[hole] = h[child];
-            hole = child;
-        }
-        if ((len & 1) == 0 && child == (len - 2) / 2)
-        {
-            child = 2 * (child + 1);
-            h[hole] = h[child - 1];
-            hole = child - 1;
-        }
-        while (hole > 0)
-        {
-            long parent = (hole - 1) / 2;
-            if (!heap_greater(h[parent], v)) break;
-            h[hole] = h[parent];
-            hole = parent;
-        }
-        h[hole] = v;
-    }
     n--;
+    if (n == 0) return;
+    const HeapItem v = h[n];
+    h[n] = h[0];
+    const u32 len = n;
+    u32 hole = 0;
+    u32 child = 0;
+    while (child < (len - 1) / 2)
+    {
+        child = 2 * (child + 1);
+        const HeapItem right = h[child], left = h[child - 1];
+        const bool takeLeft = heap_greater(right, left);
+        if (takeLeft) child--;
+        h[hole] = takeLeft ? left : right;
+        hole = child;
+    }
+    if ((len & 1) == 0 && child == (len - 2) / 2)
+    {
+        child = 2 * (child + 1);
+        h[hole] = h[child - 1];
+        hole = child - 1;
+    }
+    while (hole > 0)
+    {
+        const u32 parent = (hole - 1) / 2;
+        const HeapItem up = h[parent];
+        if (!heap_greater(up, v)) break;
+        h[hole] = up;
+        hole = parent;
+    }
+    h[hole] = v;
 }
 
 }
