@@ -69,22 +69,24 @@ struct NodeVal
     uint16_t tail;
 };
 
-// one recorded column of a node-slice: the fill's epilogue and the traceback read these
-struct __align__(16) Col
-{
-    u64 VP, VN;
-    u64 Mh;             // horizontal -1 deltas of the step (the X-score's candidate mask); in the
-                        // traceback's recomputation the rows with an open diagonal step
-    i32 end;
-    u32 pad;
-};
-
-// A warp's recorded columns and the match mask of each column of its current node, in shared
-// memory in every kernel: dynamic shared memory starts with one of these per warp of the block.
+// A warp's recorded columns of one node-slice, in shared memory in every kernel: dynamic shared
+// memory starts with one of these per warp of the block.
 struct __align__(16) NodeCols
 {
-    Col cols[64];
-    u64 eqcol[64 + 2];  // [64] is read ahead of the last column
+    // what the column loop writes
+    struct __align__(16) V { u64 VP, VN; } v[64];
+    // what is worked out from them across the lanes
+    struct __align__(16) X
+    {
+        u64 rows;       // the fill: horizontal -1 deltas of the step (the X-score's candidate mask);
+                        // the traceback's recomputation: the rows with an open diagonal step
+        i32 end;        // score of the last row
+        u32 pad;
+    } x[64];
+    u64 eqcol[64 + 2];  // match mask of each column with its horizontal -1 input; [64] is read ahead of the last column
+
+    __device__ __forceinline__ WS column(u32 k) const { return ws_make(v[k].VP, v[k].VN, x[k].end); }
+    __device__ __forceinline__ i32 value(u32 k, u32 row) const { return ws_value(column(k), (int)row); }
 };
 extern __shared__ __align__(16) uint8_t dsmem[];
 
@@ -796,7 +798,9 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
 // recurrence, on 32-bit halves: the horizontal -1 input is already in the column's match mask
 // (where it is set the row's bits of VP and VN do not depend on the mask), the +1 input enters
 // through the funnel shift that moves Ph down a row, the next mask is loaded a column ahead, and
-// the bottom-row deltas are read off the recorded scores afterwards.  The reference forces the
+// only VP and VN are recorded: afterwards lanes k and k + 32 run columns k and k + 32's step once
+// more from the columns before them, which gives Ph and Mh, hence the last-row scores, for 64
+// columns in the instructions of two.  The reference forces the
 // first row's delta to -1 where the row above the slice is cheaper than the band above
 // (forceMask); there the input is +1 and the column before it has that delta already, so the
 // recurrence gives it by itself (the first column's merges keep it: the cheaper row above wins
@@ -809,8 +813,8 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     const EqV4& eqv, const PrevInfo& prev, const Extra* pool, uint16_t head, uint16_t nil, const WS* singleIncoming, bool singleInPrevBand,
     i32 seqOffset, WS& endColumn, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
 {
-    Col* const cols = node_cols().cols;
-    u64* const eqcol = node_cols().eqcol;
+    NodeCols& nc = node_cols();
+    u64* const eqcol = nc.eqcol;
     const bool hasExtra = Multi && extra != nullptr;
     bool forceCalculation = false;
     const bool boundOk = seqOffset < kXBoundOffsetLimit;
@@ -941,22 +945,11 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
         const u64 e = mask_at(pos);
         eqcol[pos] = pos == 0 ? e : (e & forceEq) | ((fixedHN >> pos) & 1);
     }
-    if (!Fill)
-    {
-        // the recomputation's column 0, after the merges
-        Col c;
-        c.VP = ws.VP;
-        c.VN = ws.VN;
-        c.Mh = kAllOnes;
-        c.end = ws.end;
-        c.pad = 0;
-        cols[0] = c;
-    }
+    nc.v[0] = { ws.VP, ws.VN };     // column 0 after the merges
     __syncwarp();
     if (!hasExtra)
     {
         u32 vpl = (u32)ws.VP, vph = (u32)(ws.VP >> 32), vnl = (u32)ws.VN, vnh = (u32)(ws.VN >> 32);
-        i32 end = ws.end;
         u32 pos = 1;
         u64 eq = eqcol[1];
         #pragma unroll 1
@@ -980,21 +973,15 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
                 hp <<= 1;
                 hn <<= 1;
                 const u32 xvl = eql | vnl, xvh = eqh | vnh;
-                Col c;
-                c.Mh = Fill ? ((u64)mh << 32) | ml : ((u64)(~(xhh | vnh) | eqh) << 32) | (~(xhl | vnl) | eql);
                 vpl = sml | ~(xvl | spl);
                 vph = smh | ~(xvh | sph);
                 vnl = spl & xvl;
                 vnh = sph & xvh;
-                end = end + (i32)(ph >> 31) - (i32)(mh >> 31);
-                c.VP = ((u64)vph << 32) | vpl;
-                c.VN = ((u64)vnh << 32) | vnl;
-                c.end = end;
-                c.pad = 0;
-                cols[pos] = c;
+                nc.v[pos] = { ((u64)vph << 32) | vpl, ((u64)vnh << 32) | vnl };
             }
         }
-        ws = ws_make(((u64)vph << 32) | vpl, ((u64)vnh << 32) | vnl, end);
+        ws.VP = ((u64)vph << 32) | vpl;
+        ws.VN = ((u64)vnh << 32) | vnl;
     }
     else
     {
@@ -1015,70 +1002,93 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
             hn >>= 1;
             fm >>= 1;
             ws = merge_w(nw, *extra, lane);
-            Col c;
-            c.VP = ws.VP;
-            c.VN = ws.VN;
-            c.Mh = Mh;
-            c.end = ws.end;
-            c.pad = 0;
-            cols[pos] = c;
+            nc.v[pos] = { ws.VP, ws.VN };
+            nc.x[pos] = { Mh, ws.end, 0 };
         }
     }
     __syncwarp();
     steps += columns - 1;
     result.cells = columns;
+    // lane k: columns k and k + 32
+    NodeCols::V col[2];
+    u64 rows[2] = { kAllOnes, kAllOnes };
+    i32 ends[2] = { startEnd, startEnd };
+    u64 outHP, outHN;
+    {
+        bool plus[2] = { false, false }, minus[2] = { false, false };
+#pragma unroll
+        for (u32 h = 0; h < 2; h++)
+        {
+            const u32 pos = lane + 32 * h;
+            col[h] = { 0, 0 };
+            if (pos >= columns) continue;
+            col[h] = nc.v[pos];
+            if (pos == 0) continue;
+            const NodeCols::V before = nc.v[pos - 1];
+            const u64 eq = eqcol[pos];
+            const u64 Xh = (((eq & before.VP) + before.VP) ^ before.VP) | eq;
+            const u64 Ph = before.VN | ~(Xh | before.VP);
+            const u64 Mh = before.VP & Xh;
+            rows[h] = Fill ? Mh : diagonal_rows(eq, Xh, before.VN);
+            plus[h] = (Ph >> 63) != 0;
+            minus[h] = (Mh >> 63) != 0;
+            if (hasExtra)
+            {
+                // the merged columns' deltas are not the step's
+                const NodeCols::X x = nc.x[pos];
+                const i32 last = pos == 1 ? startEnd : nc.x[pos - 1].end;
+                if (Fill) rows[h] = x.rows;
+                ends[h] = x.end;
+                plus[h] = x.end == wadd(last, 1);
+                minus[h] = x.end == wsub(last, 1);
+            }
+        }
+        outHP = (u64)__ballot_sync(kFull, plus[0]) | ((u64)__ballot_sync(kFull, plus[1]) << 32);
+        outHN = (u64)__ballot_sync(kFull, minus[0]) | ((u64)__ballot_sync(kFull, minus[1]) << 32);
+        if (!hasExtra)
+        {
+            const u32 upto = (2u << lane) - 1u;
+            const i32 low = popc32((u32)outHP) - popc32((u32)outHN);
+            ends[0] = startEnd + popc32((u32)outHP & upto) - popc32((u32)outHN & upto);
+            ends[1] = startEnd + low + popc32((u32)(outHP >> 32) & upto) - popc32((u32)(outHN >> 32) & upto);
+            ws.end = startEnd + popc64(outHP) - popc64(outHN);
+        }
+        if (!Fill)
+        {
+#pragma unroll
+            for (u32 h = 0; h < 2; h++)
+                if (lane + 32 * h < columns) nc.x[lane + 32 * h] = { rows[h], ends[h], 0 };
+            __syncwarp();
+        }
+    }
     if (Fill)
     {
-        // Across the lanes (lane k: columns k and k + 32; every lane wrote every column):
-        // the first column of least score, the greatest X-score and the bottom-row deltas.
+        // Across the lanes: the first column of least score and the greatest X-score.
         // A column whose X-score bound is at most the slice's best so far cannot change the
         // slice's choice (it keeps the first node of strictly greatest X-score), so its exact
         // X-score is skipped; every column above that bound is scored exactly.
         u32 loKey = 0xffffffffu, hiKey = 0xffffffffu;
         i32 lmax = kIntMin;
-        i32 loEnd = startEnd, hiEnd = 0;    // the columns' last-row scores (column 0's after the merges)
 #pragma unroll
         for (u32 h = 0; h < 2; h++)
         {
             const u32 pos = lane + 32 * h;
             if (pos < columns)
             {
-                Col c = cols[pos];
-                if (pos == 0)
-                {
-                    // column 0 as it enters the node, every row a candidate
-                    c.VP = ws0.VP;
-                    c.VN = ws0.VN;
-                    c.Mh = kAllOnes;
-                    c.end = ws0.end;
-                }
-                else if (h == 0) loEnd = c.end;
-                else hiEnd = c.end;
-                // column 0's X-score is taken after the seed start's column joins it
-                const WS cw = (Multi && pos == 0) ? wsX : ws_make(c.VP, c.VN, c.end);
-                const u32 key = (u32)c.end ^ 0x80000000u;   // signed order as unsigned
+                // column 0 counts as it enters the node, every row a candidate; its X-score is
+                // taken after the seed start's column joins it
+                const bool first = pos == 0;
+                const u32 key = (u32)(first ? ws0.end : ends[h]) ^ 0x80000000u;   // signed order as unsigned
                 if (h == 0) loKey = key; else hiKey = key;
+                const WS cw = first ? wsX : ws_make(col[h].VP, col[h].VN, ends[h]);
                 if (!boundOk || xscore_bound(cw, seqOffset, cost) > (int64_t)sliceMaxX)
-                    lmax = imax(lmax, ws_max_xscore(cw, seqOffset, cost, 64, c.Mh));
+                    lmax = imax(lmax, ws_max_xscore(cw, seqOffset, cost, 64, rows[h]));
             }
         }
-        // the bottom-row delta of a column is its last-row score less the one before
-        i32 loBefore = __shfl_up_sync(kFull, loEnd, 1);
-        i32 hiBefore = __shfl_up_sync(kFull, hiEnd, 1);
-        const i32 end31 = __shfl_sync(kFull, loEnd, 31);
-        if (lane == 0)
-        {
-            loBefore = loEnd;
-            hiBefore = end31;
-        }
-        const i32 loDelta = lane < columns ? wsub(loEnd, loBefore) : 0;
-        const i32 hiDelta = lane + 32 < columns ? wsub(hiEnd, hiBefore) : 0;
         const u32 gkey = __reduce_min_sync(kFull, loKey < hiKey ? loKey : hiKey);
         const i32 gmax = __reduce_max_sync(kFull, lmax);
         const u32 onLo = __ballot_sync(kFull, loKey == gkey);
         const u32 onHi = __ballot_sync(kFull, hiKey == gkey);
-        const u64 outHP = (u64)__ballot_sync(kFull, loDelta == 1) | ((u64)__ballot_sync(kFull, hiDelta == 1) << 32);
-        const u64 outHN = (u64)__ballot_sync(kFull, loDelta == -1) | ((u64)__ballot_sync(kFull, hiDelta == -1) << 32);
         // column 0 always takes part, so the key is a real score
         result.minScore = (i32)(gkey ^ 0x80000000u);
         result.minScoreOffset = onLo ? (u32)(__ffs((int)onLo) - 1) : (u32)(32 + __ffs((int)onHi) - 1);
@@ -1848,7 +1858,6 @@ template <bool Multi> __device__ __forceinline__ i32 xval(const WS& e, int row) 
 template <bool Multi> __device__ __forceinline__ i32 xbefore(const WS& e) { return Multi ? ws_before(e) : kIntMax; }
 
 
-__device__ __forceinline__ i32 col_value(const Col& c, int row) { return ws_value(ws_make(c.VP, c.VN, c.end), row); }
 
 // pickBacktraceCorner (Common.h:936-1054).  Out of line, like the other crossing rules:
 // the walk inside a node-slice is the hot path.  t is a copy (its record cache is a hint).
@@ -1968,7 +1977,6 @@ template <bool Multi = false>
 __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, u32 node, const EqV4& eqv, u32 lane, u32 lastColumn,
     WS extra = fake_ws())
 {
-    const Col* const cols = node_cols().cols;
     const Item* it = t.template find<Multi>(s, node);
     if (!it) return GA_ASSERT;
     PrevInfo prev;
@@ -1986,9 +1994,9 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
     node_calc<false, Multi>(g, cost, node, L, rec.seq[0], rec.seq[1], copy, it->node, eqv, prev, nullptr, kNil, kNil, &start, false, (i32)j, last,
         steps, err, lane, kIntMin, lastColumn, (Multi && extra.end != kIntMax) ? &extra : nullptr);
     if (err) return err;
-    if (!ws_eq(ws_make(cols[0].VP, cols[0].VN, cols[0].end), start)) return GA_ASSERT;
-    if (lastColumn + 1 >= L && !ws_eq(ws_make(cols[L - 1].VP, cols[L - 1].VN, cols[L - 1].end), ws_make(it->eVP, it->eVN, it->eEnd)))
-        return GA_ASSERT;
+    const NodeCols& nc = node_cols();
+    if (!ws_eq(nc.column(0), start)) return GA_ASSERT;
+    if (lastColumn + 1 >= L && !ws_eq(nc.column(L - 1), ws_make(it->eVP, it->eVN, it->eEnd))) return GA_ASSERT;
     return 0;
 }
 
@@ -1997,7 +2005,7 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
 template <bool Multi>
 __device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* seq, Table t, u32 curSlice, const Item* pself, TPos p, int& err, WS extra)
 {
-    const Col* const cols = node_cols().cols;
+    const NodeCols& nc = node_cols();
     TStep second;
     second.pos = p;
     second.sw = false;
@@ -2006,7 +2014,7 @@ __device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* se
     bool bad = false;
     bool eq = char_match(g, seq[p.seq], p.node, p.off, bad);
     if (bad) { err = GA_ASSERT; return second; }
-    i32 here = col_value(cols[p.off], 0);
+    i32 here = nc.value(p.off, 0);
     // the previous slice's last row at column p.off - 1: its first column plus the deltas of columns 1..p.off-1
     const u64 upto = p.off >= 2 ? ((kAllOnes >> (64 - (p.off - 1))) << 1) : 0;
     i32 diag = pself->sEnd + popc64(pself->HP & upto) - popc64(pself->HN & upto);
@@ -2104,7 +2112,7 @@ struct EndCell
 __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint8_t* arena, Table t, u32 committed, const uint8_t* seq,
     u32 seqLen, u32 lane)
 {
-    const Col* const cols = node_cols().cols;
+    const NodeCols& nc = node_cols();
     EndCell ec;
     ec.err = 0;
     ec.nodeOffset = 0xffffffffu;
@@ -2138,7 +2146,7 @@ __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint
     {
         const u32 i = lane + 32 * h;
         if (i >= L || bad) continue;
-        const WS cw = ws_make(cols[i].VP, cols[i].VN, cols[i].end);
+        const WS cw = nc.column(i);
         i32 mx = ws_max_xscore(cw, (i32)j, cost, cells, kAllOnes);
         if (mx > ec.score) { bad = true; continue; }
         if (mx == ec.score)
@@ -2212,10 +2220,10 @@ __device__ __noinline__ int row_above(const DevGraph& g, Table t, TraceOut& to)
 // The first column of the run of row-0 steps that ends at column off: the least c <= off with
 // score(c') = score(c' - 1) + 1 for every c < c' <= off (pickBacktraceVerticalCrossing's walk
 // along the slice's first row, Common.h:886-900).  Columns 0..off must be in cols.
-__device__ __forceinline__ u32 row0_run_start(const Col* cols, u32 off, u32 lane)
+__device__ __forceinline__ u32 row0_run_start(const NodeCols& nc, u32 off, u32 lane)
 {
-    const i32 v0 = col_value(cols[lane], 0);
-    const i32 v1 = col_value(cols[lane + 32], 0);
+    const i32 v0 = nc.value(lane, 0);
+    const i32 v1 = nc.value(lane + 32, 0);
     i32 p0 = __shfl_up_sync(kFull, v0, 1);
     i32 p1 = __shfl_up_sync(kFull, v1, 1);
     const i32 v31 = __shfl_sync(kFull, v0, 31);
@@ -2234,7 +2242,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     TPos start, i32 startScore, i32& resultScore, u32 lane)
 {
     int err = 0;
-    const Col* const cols = node_cols().cols;
+    const NodeCols& nc = node_cols();
     const u64 guardMax = (u64)((Multi && to.counting) ? (1u << 26) : to.cap) * 4 + 1024;
     resultScore = startScore;
     to.push(start, false);
@@ -2283,8 +2291,8 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
         {
             TStep bt = bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra);
             if (err) break;
-            if (tpos_eq(bt.pos, b) && !bt.sw && col_value(cols[bt.pos.off], (int)mod64(bt.pos.seq)) == xv(mod64(bt.pos.seq))) break;
-            if (Multi && tpos_eq(bt.pos, b) && !bt.sw && col_value(cols[bt.pos.off], (int)mod64(bt.pos.seq)) == ws_before(extra)) break;
+            if (tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == xv(mod64(bt.pos.seq))) break;
+            if (Multi && tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == ws_before(extra)) break;
             to.push(bt.pos, bt.sw);
             if (!to.overflow && trace_circular(to.items, to.ring, to.n, Multi && to.counting)) { err = GA_ASSERT; break; }
             continue;
@@ -2302,10 +2310,10 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             // columns k and k + 32 against their left neighbours, the run ends at the
             // highest failing column at or below b.off (column 0 always ends it)
             TPos p = b;
-            p.off = row0_run_start(cols, b.off, lane);
+            p.off = row0_run_start(nc, b.off, lane);
             TStep second = p.off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : vertical_step<Multi>(g, seq, t, curSlice, pself, p, err, extra);
             if (err) break;
-            if (second.pos.seq == b.seq && col_value(cols[second.pos.off], (int)mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
+            if (second.pos.seq == b.seq && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
             if (p.off != b.off) to.push_run(TPos { p.node, b.off - 1, p.seq }, -1, 0, b.off - p.off);
             if (tpos_eq(second.pos, to.back)) { err = GA_ASSERT; break; }
             to.push(second.pos, second.sw);
@@ -2328,7 +2336,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             const u32 off = mod64(p.seq);
             TStep second = off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : horizontal_step<Multi>(g, seq, t, curSlice, curNode, self, p, off, err, extra);
             if (err) break;
-            if (second.pos.node == b.node && !second.sw && col_value(cols[second.pos.off], (int)mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
+            if (second.pos.node == b.node && !second.sw && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
             if (p.seq != b.seq) to.push_run(TPos { p.node, p.off, b.seq - 1 }, 0, -1, (u32)(b.seq - p.seq));
             if (tpos_eq(second.pos, to.back)) { err = GA_ASSERT; break; }
             to.push(second.pos, second.sw);
@@ -2337,7 +2345,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
         }
         // pickBacktraceInside (Common.h:770-815): up while the column's delta is +1, else
         // diagonally where that step is open, else left.  Inside a node-slice the steps are
-        // bits of the recomputed columns (VP: up, Mh: diagonal; what is neither goes left), so
+        // bits of the recomputed columns (VP: up, rows: diagonal; what is neither goes left), so
         // a run of diagonal steps is found in one ballot, lane k testing the cell k steps down
         // the diagonal, and a run of up steps is a leading-one count.
         // Cell by cell (two scores carried, every lane the same) this walk took 21.9k of the
@@ -2355,9 +2363,8 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 bool diagonal = false;
                 if (lane < most)
                 {
-                    const Col& c = cols[hori - lane];
                     const u64 bit = 1ULL << (vert - lane);
-                    diagonal = (c.Mh & ~c.VP & bit) != 0;
+                    diagonal = (nc.x[hori - lane].rows & ~nc.v[hori - lane].VP & bit) != 0;
                 }
                 const u32 run = (u32)__ffs((int)~__ballot_sync(kFull, diagonal));
                 if (run != 1)
@@ -2369,7 +2376,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                     vert -= count;
                     continue;
                 }
-                const u64 vp = cols[hori].VP;
+                const u64 vp = nc.v[hori].VP;
                 if ((vp >> vert) & 1)
                 {
                     const u32 count = up_run(vp, vert);
@@ -2377,7 +2384,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                     vert -= count;
                     continue;
                 }
-                if (col_value(cols[hori - 1], (int)vert) != col_value(cols[hori], (int)vert) - 1) { err = GA_ASSERT; break; }
+                if (nc.value(hori - 1, vert) != nc.value(hori, vert) - 1) { err = GA_ASSERT; break; }
                 hori--;
                 to.push(TPos { b.node, hori, sj + vert }, false);
             }
@@ -2398,8 +2405,8 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             const u64* eqcol = node_cols().eqcol;
             if (hori > 0 && vert > 0)
             {
-                WS colH = ws_make(cols[hori].VP, cols[hori].VN, cols[hori].end);
-                WS colL = ws_make(cols[hori - 1].VP, cols[hori - 1].VN, cols[hori - 1].end);
+                WS colH = nc.column(hori);
+                WS colL = nc.column(hori - 1);
                 i32 here = ws_value(colH, (int)vert);
                 i32 left = ws_value(colL, (int)vert);
                 u64 eqH = eqcol[hori];
@@ -2425,7 +2432,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                         colH = colL;
                         if (hori > 0)
                         {
-                            colL = ws_make(cols[hori - 1].VP, cols[hori - 1].VN, cols[hori - 1].end);
+                            colL = nc.column(hori - 1);
                             left = ws_value(colL, (int)vert);
                             eqH = eqcol[hori];
                         }
@@ -2438,7 +2445,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                         colH = colL;
                         if (hori > 0)
                         {
-                            colL = ws_make(cols[hori - 1].VP, cols[hori - 1].VN, cols[hori - 1].end);
+                            colL = nc.column(hori - 1);
                             left = ws_value(colL, (int)vert);
                             eqH = eqcol[hori];
                         }
@@ -2452,12 +2459,12 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 }
             }
             if (err || to.overflow) break;
-            if (col_value(cols[to.back.off], (int)mod64(to.back.seq)) == xv(mod64(to.back.seq))) break;
+            if (nc.value(to.back.off, mod64(to.back.seq)) == xv(mod64(to.back.seq))) break;
         }
     }
     if (!err && !to.overflow)
     {
-        const i32 lastScore = lastRow == 0xffffffffu ? kIntMax - 1 : col_value(cols[lastOff], (int)lastRow);
+        const i32 lastScore = lastRow == 0xffffffffu ? kIntMax - 1 : nc.value(lastOff, lastRow);
         if (resultScore < lastScore) err = GA_ASSERT;
         resultScore -= lastScore;
     }
@@ -2489,7 +2496,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
     t.lane = lane;
     t.slots = w.slots;
     t.init();
-    const Col* const cols = node_cols().cols;
+    const NodeCols& nc = node_cols();
     TraceOut to;
     to.items = out;
     to.ring = w.ring;
@@ -2505,7 +2512,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
     {
         // getReverseTraceFromTable (Common.h:571-758)
         TPos start = TPos { ec.node, ec.nodeOffset, ec.j + ec.bvOffset };
-        i32 startScore = col_value(cols[ec.nodeOffset], (int)ec.bvOffset);
+        i32 startScore = nc.value(ec.nodeOffset, ec.bvOffset);
         err = trace_walk<false>(g, a.cost, seq, seqLen, st.committed, t, to, w, start, startScore, resultScore, lane);
         if (!err && !to.overflow) err = row_above(g, t, to);
     }
@@ -2638,7 +2645,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const TraceSpace
     const WS extra = (items[c.index].node & kSeedStart) ? seed_ws(j, seqLen, a.cost) : fake_ws();
     int err = recalc<true>(g, a.cost, t, c.slice, node, eqv, lane, 63, extra);
     if (err) return err;
-    const Col* cols = node_cols().cols;
+    const NodeCols& nc = node_cols();
     const i32 score = c.score;
     const int cells = (int)((int64_t)seqLen - j < 64 ? (int64_t)seqLen - j : 64);
     const u32 L = g.len[node];
@@ -2650,7 +2657,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const TraceSpace
     {
         const u32 i = lane + 32 * h;
         if (i >= L || bad) continue;
-        const WS cw = ws_make(cols[i].VP, cols[i].VN, cols[i].end);
+        const WS cw = nc.column(i);
         const i32 mx = ws_max_xscore(cw, (i32)j, a.cost, cells, kAllOnes);
         if (mx > score) { bad = true; continue; }
         if (mx != score) continue;
@@ -2672,7 +2679,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const TraceSpace
     const u32 gCol = __reduce_min_sync(kFull, candOff == gOff ? candCol : 0xffffffffu);
     if (gOff < 0 || j + gOff >= (int64_t)seqLen) return GA_ASSERT;
     start = TPos { node, gCol, j + gOff };
-    startScore = col_value(cols[gCol], gOff);
+    startScore = nc.value(gCol, gOff);
     return 0;
 }
 
