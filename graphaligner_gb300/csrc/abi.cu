@@ -152,7 +152,9 @@ struct ga_extender
     uint8_t* arena = nullptr;
     uint64_t arenaBytes = 0;
     uint32_t* counters = nullptr;          // [0] work counter, [2] status count; the multiseed DP: work counters [1], [3]-[6], candidate total (u64) [8]-[9]
-    unsigned long long* arenaCursor = nullptr;   // [0] overflow cursor, [1] bytes taken
+    unsigned long long* arenaCursor = nullptr;   // [0] overflow cursor, [1] bytes taken, [2] column store units taken
+    gadev::ColumnUnit* store = nullptr;    // the column store, grown to the largest batch within its bound
+    uint64_t storeUnits = 0;
     float lastFillMs = 0;
     float lastTraceMs = 0;
     float lastH2DMs = 0;                    // host-buffer copies of the last ga_extend_batch
@@ -324,7 +326,7 @@ extern "C" int ga_extender_create(ga_graph_t graph, uint64_t arena_bytes, ga_ext
     e = cudaMalloc((void**)&x->arena, x->arenaBytes);
     if (e != cudaSuccess) { cudaFree(x->workspace); delete x; return cuda_fail(e, "arena"); }
     GA_CUDA(cudaMalloc((void**)&x->counters, 16 * sizeof(uint32_t)));
-    GA_CUDA(cudaMalloc((void**)&x->arenaCursor, 2 * sizeof(unsigned long long)));
+    GA_CUDA(cudaMalloc((void**)&x->arenaCursor, 3 * sizeof(unsigned long long)));
     *out = x;
     return GA_OK;
 }
@@ -346,6 +348,7 @@ extern "C" int ga_extender_free(ga_extender_t x)
     cudaFree(x->arena);
     cudaFree(x->counters);
     cudaFree(x->arenaCursor);
+    cudaFree(x->store);
     x->seq.release(); x->seqOff.release(); x->traceOff.release(); x->traceItems.release(); x->cellSteps.release();
     x->seqLen.release(); x->startNode.release(); x->startOffset.release(); x->traceCap.release(); x->traceLen.release();
     x->order.release(); x->status.release(); x->score.release(); x->prevStatus.release(); x->states.release();
@@ -365,11 +368,37 @@ extern "C" int ga_extender_free(ga_extender_t x)
     return GA_OK;
 }
 
-// Runs one batch whose buffers are all on the device.  order: processing order
+// Room in the column store for a batch of readBp bases: a band of bandwidth 10 computes 2.4
+// columns per base on the variation graphs (5.5 on the tangled ones), 3 and a chunk for every
+// warp are asked for.  The store holds at most four times the arena and half of the memory that
+// is free when it grows; what finds no room in it is recomputed by the traceback.
+static void reserve_store(ga_extender* x, uint64_t readBp, uint64_t warps)
+{
+    const uint64_t unit = sizeof(gadev::ColumnUnit);
+    uint64_t want = readBp * 3 + warps * gadev::kStoreChunk;
+    want = std::min<uint64_t>({want, x->arenaBytes * 4 / unit, (uint64_t)gadev::kNoColumns - 1});
+    if (want <= x->storeUnits) return;
+    size_t freeBytes = 0, totalBytes = 0;
+    if (cudaMemGetInfo(&freeBytes, &totalBytes) != cudaSuccess) return;
+    const uint64_t most = std::min<uint64_t>({(freeBytes / unit + x->storeUnits) / 2, x->arenaBytes * 4 / unit, (uint64_t)gadev::kNoColumns - 1});
+    want = std::min(most, std::max(want, x->storeUnits * 3 / 2));
+    if (want <= x->storeUnits) return;
+    cudaFree(x->store);
+    x->store = nullptr;
+    x->storeUnits = 0;
+    if (cudaMalloc((void**)&x->store, want * unit) == cudaSuccess) x->storeUnits = want;
+    else
+    {
+        x->store = nullptr;
+        cudaGetLastError();
+    }
+}
+
+// Runs one batch whose buffers are all on the device, readBp bases in all.  order: processing order
 // (longest first).  Extensions that outgrow a layout's tables (GA_CAPACITY) run again
 // in the next, larger layout; only those run.
 static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend_batch_desc* b, ga_extend_results* r,
-    const uint32_t* order, int32_t* prevStatus, cudaStream_t stream)
+    const uint32_t* order, int32_t* prevStatus, uint64_t readBp, cudaStream_t stream)
 {
     gadev::FillArgs fa {};
     fa.g = x->graph->d;
@@ -417,6 +446,10 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
     const int wpb = (int)sh.warps_per_block;
     fa.chunkBytes = (uint64_t)sh.chunk_kib << 10;
     uint32_t pending = n;                    // extensions the next round runs
+    reserve_store(x, readBp, std::min<uint64_t>(n, (uint64_t)x->sms * 16));
+    fa.store = x->store;
+    fa.storeUnits = x->storeUnits;
+    ta.store = x->store;
     for (int layout = (int)sh.first_layout; layout < 3; layout++)
     {
         const bool shared = layout == 0;
@@ -445,7 +478,7 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
         fa.prevStatus = layout > (int)sh.first_layout ? prevStatus : nullptr;
         ta.prevStatus = fa.prevStatus;
         GA_CUDA(cudaMemsetAsync(x->counters, 0, 16 * sizeof(uint32_t), stream));
-        GA_CUDA(cudaMemsetAsync(x->arenaCursor, 0, 2 * sizeof(unsigned long long), stream));
+        GA_CUDA(cudaMemsetAsync(x->arenaCursor, 0, 3 * sizeof(unsigned long long), stream));
         GA_CUDA(cudaEventRecord(x->ev[0], stream));
         if (ga_launch_extend(fa, ta, x->counters, (int)fillBlocks, (int)traceBlocks, wpb, stream) != 0)
             return fail(GA_ERR_CUDA, std::string("extension kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
@@ -480,6 +513,8 @@ static int check_lengths(const uint32_t* len, uint32_t n)
             return fail(GA_ERR_ARGUMENT, "extension " + std::to_string(i) + ": sequence longer than GA_MAX_SEQ_LEN (33,554,431 bp)");
     return GA_OK;
 }
+
+static uint64_t sum_lengths(const uint32_t* len, uint32_t n) { return std::accumulate(len, len + n, (uint64_t)0); }
 
 static std::vector<uint32_t> longest_first(const uint32_t* len, uint32_t n)
 {
@@ -560,7 +595,7 @@ extern "C" int ga_extend_batch(ga_extender_t x, const ga_extend_params* p, const
     int rc = stage_host_batch(x, b, &db, &dr, &items);
     if (rc != GA_OK) return rc;
     cudaStream_t s = x->stream;
-    rc = run_device(x, p, &db, &dr, x->order.ptr, x->prevStatus.ptr, s);
+    rc = run_device(x, p, &db, &dr, x->order.ptr, x->prevStatus.ptr, sum_lengths(b->seq_len, n), s);
     if (rc != GA_OK) return rc;
     GA_CUDA(cudaMemcpyAsync(r->status, dr.status, n * 4ULL, cudaMemcpyDeviceToHost, s));
     GA_CUDA(cudaMemcpyAsync(r->score, dr.score, n * 4ULL, cudaMemcpyDeviceToHost, s));
@@ -706,7 +741,11 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
     fa.seedSlice = x->msSeedSlice.ptr;
     fa.seedNode = x->msSeedNode.ptr;
     fa.chunkBytes = (uint64_t)x->shape.chunk_kib << 10;
+    reserve_store(x, 2 * sum_lengths(b->seq_len, n), std::min<uint64_t>(n, (uint64_t)x->sms * 16));
+    fa.store = x->store;
+    fa.storeUnits = x->storeUnits;
     gadev::MultiTraceArgs ta {};
+    ta.store = x->store;
     ta.g = x->graph->d;
     ta.cost = p->xscore_error_cost;
     ta.num = n;
@@ -768,7 +807,7 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
         fa.prevStatus = pass > 0 ? x->prevStatus.ptr : nullptr;
         ta.prevStatus = fa.prevStatus;
         GA_CUDA(cudaMemsetAsync(x->counters, 0, 16 * sizeof(uint32_t), s));
-        GA_CUDA(cudaMemsetAsync(x->arenaCursor, 0, 2 * sizeof(unsigned long long), s));
+        GA_CUDA(cudaMemsetAsync(x->arenaCursor, 0, 3 * sizeof(unsigned long long), s));
         GA_CUDA(cudaEventRecord(x->ev[0], s));
         if (ga_launch_multiseed_fill(fa, ta, x->counters, (int)fillBlocks, (int)readBlocks, wpb, s) != 0)
             return fail(GA_ERR_CUDA, std::string("multiseed kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
@@ -1026,7 +1065,7 @@ extern "C" int ga_extender_autotune(ga_extender_t x, const ga_extend_params* p, 
         std::vector<float> ms;
         for (uint32_t rep = 0; rep < repeats; rep++)
         {
-            rc = run_device(x, p, &db, &dr, x->order.ptr, x->prevStatus.ptr, s);
+            rc = run_device(x, p, &db, &dr, x->order.ptr, x->prevStatus.ptr, sum_lengths(b->seq_len, n), s);
             if (rc != GA_OK) return rc;
             ms.push_back(x->lastFillMs);
         }
@@ -1068,7 +1107,7 @@ extern "C" int ga_extend_batch_device(ga_extender_t x, const ga_extend_params* p
     GA_CUDA(x->order.reserve(n));
     GA_CUDA(x->prevStatus.reserve(n));
     GA_CUDA(cudaMemcpyAsync(x->order.ptr, order.data(), n * 4ULL, cudaMemcpyHostToDevice, s));
-    return run_device(x, p, b, r, x->order.ptr, x->prevStatus.ptr, s);
+    return run_device(x, p, b, r, x->order.ptr, x->prevStatus.ptr, sum_lengths(len.data(), n), s);
 }
 
 extern "C" int ga_extender_last_kernel_ms(ga_extender_t x, float* ms)

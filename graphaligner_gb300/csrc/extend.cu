@@ -163,6 +163,7 @@ struct WSpace
     NodeVal* val[2];
     HeapItem* heap;
     Extra* extras;
+    u32* columns;       // [band] where each band node's columns are in the column store
     i32* nodeMax;       // multiseed DP: [band] each band node's best exact-end-position X-score
 };
 
@@ -170,7 +171,7 @@ __host__ __device__ inline u64 align16(u64 x) { return (x + 15) & ~15ULL; }
 
 __host__ __device__ inline u64 wspace_bytes(const Caps& c, bool multi = false)
 {
-    u64 b = multi ? align16((u64)c.band * 4) : 0;
+    u64 b = (multi ? 2 : 1) * align16((u64)c.band * 4);
     b += 2 * align16((u64)c.band * sizeof(Item));
     b += 2 * align16((u64)c.hash * 8);
     b += 2 * align16((u64)c.hash * sizeof(NodeVal));
@@ -191,6 +192,7 @@ __device__ __forceinline__ WSpace wspace_at(uint8_t* base, const Caps& c)
     w.val[1] = (NodeVal*)(base + off); off += align16((u64)c.hash * sizeof(NodeVal));
     w.heap = (HeapItem*)(base + off); off += align16((u64)c.heap * sizeof(HeapItem));
     w.extras = (Extra*)(base + off); off += align16((u64)c.extras * sizeof(Extra));
+    w.columns = (u32*)(base + off); off += align16((u64)c.band * 4);
     w.nodeMax = (i32*)(base + off);    // inside the stride only when it was sized for the multiseed DP
     return w;
 }
@@ -286,11 +288,12 @@ struct SmallTables
     u32 lane;
     u32 id, val, comp;     // this lane's slot
     u32 bandSlot;          // the slot of band entry `lane`
+    u32 columns;           // where the columns of band entry `lane` are
     u32 prevId, prevComp;  // the previous band's entry `lane`
     bool prevLinear;
     u32 used, heapN, poolN, count, prevCount, side;
 
-    __device__ __forceinline__ SmallTables(const FillArgs&, u64, u32 lane_) : lane(lane_), id(0), val(0), comp(0), bandSlot(0), prevId(0), prevComp(0),
+    __device__ __forceinline__ SmallTables(const FillArgs&, u64, u32 lane_) : lane(lane_), id(0), val(0), comp(0), bandSlot(0), columns(0), prevId(0), prevComp(0),
         prevLinear(false), used(0), heapN(0), poolN(0), count(0), prevCount(0), side(0) {}
     __device__ __forceinline__ Item* band() const { return small_space().band[side]; }
     __device__ __forceinline__ const Item* prev_band() const { return small_space().band[side ^ 1]; }
@@ -380,6 +383,10 @@ struct SmallTables
         if (lane == count) bandSlot = slot;
         return (int)count++;
     }
+    __device__ __forceinline__ u32 columns_of(u32 at) const { return __shfl_sync(kFull, columns, (int)at); }
+    __device__ __forceinline__ void set_columns(u32 at, u32 where) { if (lane == at) columns = where; }
+    // of the band entry this lane commits (entry `lane`, the only one)
+    __device__ __forceinline__ u32 lane_columns(u32) const { return columns; }
     __device__ __forceinline__ int band_of(u32 slot) const
     {
         const u32 b = __shfl_sync(kFull, val, (int)slot) & 0xff;
@@ -494,6 +501,9 @@ struct LargeTables
         w.val[side][slot].band = (int16_t)count;
         return (int)count++;
     }
+    __device__ __forceinline__ u32 columns_of(u32 at) const { return w.columns[at]; }
+    __device__ __forceinline__ void set_columns(u32 at, u32 where) { w.columns[at] = where; }
+    __device__ __forceinline__ u32 lane_columns(u32 at) const { return w.columns[at]; }
     __device__ __forceinline__ int band_of(u32 slot) const { return w.val[side][slot].band; }
     __device__ __forceinline__ NodeRec record(const DevGraph& g, u32, u32 node) { return node_record(g, node); }
     __device__ __forceinline__ u32 prev_component(const DevGraph& g, u32, u32 node) const { return g.comp[node]; }
@@ -784,7 +794,7 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
 // calculateNodeInner (Common.h:1113-1478).  nodeLength, c0, c1: the node's length and 2-bit
 // sequence.  flags: the band entry's, 0 for a node that has none yet.  singleInPrevBand: the
 // node's only in-neighbour is in the previous band.  endColumn: the node's last column in this
-// slice.  Multi = false: the single-seed path, whose extra
+// slice.  kept: the node-slice's units in the column store, or null.  Multi = false: the single-seed path, whose extra
 // slice is always the fake one.  Multi = true: the multiseed DP, where `extra` (non-null for
 // a node that is a seed start in this slice) is merged into every column and an incoming
 // column that starts a seed forces the computation (EdgeWithPriority::forceCalculation).
@@ -811,7 +821,7 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
 template <bool Fill, bool Multi = false>
 __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i, u32 nodeLength, u64 c0, u64 c1, Item& slice, u32 flags,
     const EqV4& eqv, const PrevInfo& prev, const Extra* pool, uint16_t head, uint16_t nil, const WS* singleIncoming, bool singleInPrevBand,
-    i32 seqOffset, WS& endColumn, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
+    i32 seqOffset, WS& endColumn, ColumnUnit* kept, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
 {
     NodeCols& nc = node_cols();
     u64* const eqcol = nc.eqcol;
@@ -1016,6 +1026,7 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     u64 outHP, outHN;
     {
         bool plus[2] = { false, false }, minus[2] = { false, false };
+        bool topPlus[2] = { false, false }, topMinus[2] = { false, false };
 #pragma unroll
         for (u32 h = 0; h < 2; h++)
         {
@@ -1030,6 +1041,12 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
             const u64 Ph = before.VN | ~(Xh | before.VP);
             const u64 Mh = before.VP & Xh;
             rows[h] = Fill ? Mh : diagonal_rows(eq, Xh, before.VN);
+            if (Fill && kept)
+            {
+                kept[pos] = { col[h].VP, diagonal_rows(eq, Xh, before.VN) };
+                topPlus[h] = Ph & 1;
+                topMinus[h] = Mh & 1;
+            }
             plus[h] = (Ph >> 63) != 0;
             minus[h] = (Mh >> 63) != 0;
             if (hasExtra)
@@ -1052,6 +1069,12 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
             ends[0] = startEnd + popc32((u32)outHP & upto) - popc32((u32)outHN & upto);
             ends[1] = startEnd + low + popc32((u32)(outHP >> 32) & upto) - popc32((u32)(outHN >> 32) & upto);
             ws.end = startEnd + popc64(outHP) - popc64(outHN);
+        }
+        if (Fill && kept)
+        {
+            const u64 tp = (u64)__ballot_sync(kFull, topPlus[0]) | ((u64)__ballot_sync(kFull, topPlus[1]) << 32);
+            const u64 tm = (u64)__ballot_sync(kFull, topMinus[0]) | ((u64)__ballot_sync(kFull, topMinus[1]) << 32);
+            if (lane == 0) kept[0] = { tp, tm };
         }
         if (!Fill)
         {
@@ -1110,7 +1133,44 @@ struct ArenaCursor
     u64 pos;
     u64 end;
     u64 used;           // bytes handed out to this warp since the launch began
+    u32 unit;           // this warp's units of the column store
+    u32 unitEnd;
+    bool storeFull;
 };
+
+__device__ __forceinline__ ArenaCursor arena_cursor(const FillArgs& a)
+{
+    ArenaCursor c;
+    c.pos = 0;
+    c.end = 0;
+    c.used = 0;
+    c.unit = 0;
+    c.unitEnd = 0;
+    c.storeFull = a.store == nullptr;
+    return c;
+}
+
+// `columns` units of the column store, or kNoColumns
+__device__ __forceinline__ u32 store_alloc(const FillArgs& a, ArenaCursor& c, u32 columns, u32 lane)
+{
+    if (c.unitEnd - c.unit < columns)
+    {
+        if (c.storeFull) return kNoColumns;
+        unsigned long long p = 0;
+        if (lane == 0) p = atomicAdd(a.arenaCursor + 2, (unsigned long long)kStoreChunk);
+        p = __shfl_sync(kFull, p, 0);
+        if (p + kStoreChunk > a.storeUnits)
+        {
+            c.storeFull = true;
+            return kNoColumns;
+        }
+        c.unit = (u32)p;
+        c.unitEnd = (u32)p + kStoreChunk;
+    }
+    const u32 at = c.unit;
+    c.unit += columns;
+    return at;
+}
 
 // bytes from the warp's current chunk, else a new chunk (one atomic per chunk)
 __device__ __forceinline__ bool arena_alloc(const FillArgs& a, ArenaCursor& c, u64 bytes, u64& out, u32 lane)
@@ -1144,11 +1204,14 @@ __device__ __forceinline__ u32 band_hash_size(u32 count)
     return h;
 }
 
-// write one slice (record, node ids, band in first-pop order and, for the multiseed DP, each
+// write one slice of the tables (record, node ids, band in first-pop order and, for the multiseed DP, each
 // node's best X-score and a large band's index) into the arena, lanes copying
-__device__ bool commit_slice(const FillArgs& a, ArenaCursor& c, u64* dir, u32 index, const Item* band, u32 count,
-    i32 minScore, i32 quit, i32 maxX, u32 maxXNode, bool notValid, u32 lane, const i32* nodeMax = nullptr)
+template <class Tables>
+__device__ __forceinline__ bool commit_slice(const FillArgs& a, ArenaCursor& c, u64* dir, u32 index, const Tables& t, i32 minScore, i32 quit,
+    i32 maxX, u32 maxXNode, bool notValid, u32 lane, const i32* nodeMax = nullptr)
 {
+    const Item* band = t.band();
+    const u32 count = t.count;
     const u64 idBytes = rec_ids_bytes(count);
     u64 off;
     const u64 maxBytes = nodeMax ? rec_ids_bytes(count) : 0;
@@ -1172,11 +1235,19 @@ __device__ bool commit_slice(const FillArgs& a, ArenaCursor& c, u64* dir, u32 in
     }
     u32* ids = (u32*)(base + sizeof(SliceRec));
     #pragma unroll 1
-    for (u32 k = lane; k < count; k += 32) ids[k] = band[k].node & kNodeMask;
-    uint4* dst = (uint4*)(base + sizeof(SliceRec) + idBytes);
-    const uint4* src = (const uint4*)band;
+    for (u32 k = lane; k < count * 4; k += 32)
+    {
+        if ((k & 3) != 3) ((uint4*)(base + sizeof(SliceRec) + idBytes))[k] = ((const uint4*)band)[k];
+    }
     #pragma unroll 1
-    for (u32 k = lane; k < count * 4; k += 32) dst[k] = src[k];
+    for (u32 k = lane; k < count; k += 32)
+    {
+        // the last quarter of an entry, with the place of the node's columns
+        uint4 v = ((const uint4*)(band + k))[3];
+        v.z = t.lane_columns(k);
+        ((uint4*)(base + sizeof(SliceRec) + idBytes))[k * 4 + 3] = v;
+        ids[k] = v.w & kNodeMask;
+    }
     if (nodeMax)
     {
         i32* m = (i32*)(base + sizeof(SliceRec) + idBytes + (u64)count * sizeof(Item));
@@ -1294,8 +1365,8 @@ struct SliceSeeds
 // :228-253) and whose nodes keep their best exact-end-position X-score in the tables' node_max.
 // rows: the slice's read bytes on entry, the next slice's on return (loaded while this one runs).
 template <class Tables, bool Multi = false>
-__device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, const uint8_t* seq, u32 seqLen, RowBytes& rows, int64_t j,
-    i32 prevQuit, i32 prevMin, u64& steps, int& err, u32 lane, const SliceSeeds* seeds = nullptr)
+__device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, ArenaCursor& arena, const uint8_t* seq, u32 seqLen, RowBytes& rows,
+    int64_t j, i32 prevQuit, i32 prevMin, u64& steps, int& err, u32 lane, const SliceSeeds* seeds = nullptr)
 {
     if (Multi)
     {
@@ -1398,6 +1469,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
             ni.node = node | kExists | kSeedStart;
             band[at] = ni;
             nodeMax[at] = 0;
+            t.set_columns((u32)at, kNoColumns);     // a seed start's columns are merged, their steps are not bits
             if (!insert(slot, node, component, ws_value(seeds->ws, 0), seeds->ws, true, true)) { err = GA_CAPACITY; return res; }
         }
     }
@@ -1417,7 +1489,9 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
             at = t.enter(slot);
             if (at < 0) { err = GA_CAPACITY; return res; }
             if (Multi) nodeMax[at] = 0;
+            t.set_columns((u32)at, store_alloc(a, arena, rec_len(rec.meta), lane));
         }
+        const u32 columnsAt = t.columns_of((u32)at);
         Item& thisNode = band[at];
         const u32 flags = fresh ? 0 : thisNode.node & (kExists | kSeedStart);
         WS oldEnd = (flags & kExists) ? ws_make(thisNode.eVP, thisNode.eVN, thisNode.eEnd) : ws_make(0, 0, kIntMax);
@@ -1443,7 +1517,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
         const i32 skipBelow = Multi ? imin(res.maxX, nodeMax[at]) : res.maxX;
         WS newEnd;
         const NodeCalc nc = node_calc<true, Multi>(g, a.cost, i, rec_len(rec.meta), rec.seq[0], rec.seq[1], thisNode, flags, eqv, prev, t.extras(), head,
-            nil, nullptr, singleInPrev, seqOffset, newEnd, steps, err, lane, skipBelow, 63, extra);
+            nil, nullptr, singleInPrev, seqOffset, newEnd, columnsAt == kNoColumns ? nullptr : a.store + columnsAt, steps, err, lane, skipBelow, 63, extra);
         if (err) return res;
         if (Multi) nodeMax[at] = imax(nc.maxX, nodeMax[at]);
         if (nc.minScore > wadd(wadd(seqOffset, bw), 128)) { err = GA_ASSERT; return res; }
@@ -1543,7 +1617,8 @@ __device__ __forceinline__ ExtState fill_extension(const FillArgs& a, Tables& t,
         const int slot = t.add(g, startNode, g.comp[startNode]);
         const int at = t.enter((u32)slot);
         t.band()[at] = it;
-        if (!commit_slice(a, arena, dir, 0, t.band(), 1, 0, 1, 0, startNode, false, lane))
+        t.set_columns((u32)at, kNoColumns);
+        if (!commit_slice(a, arena, dir, 0, t, 0, 1, 0, startNode, false, lane))
         {
             st.status = GA_CAPACITY;
             return st;
@@ -1557,14 +1632,14 @@ __device__ __forceinline__ ExtState fill_extension(const FillArgs& a, Tables& t,
     for (u32 s = 0; s < numSlices; s++)
     {
         const int64_t j = (int64_t)s * 64;
-        SliceResult r = fill_slice(a, t, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane);
+        SliceResult r = fill_slice(a, t, arena, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane);
         if (err) break;
         if (r.maxX > bestX) bestX = r.maxX;
         const bool notValid = r.cells >= a.maxCells;
         if ((int64_t)r.maxX < (int64_t)bestX - (int64_t)a.xdrop) break;
         if (r.minScore < lastMin) { err = GA_ASSERT; break; }
         const i32 quit = wadd(r.minScore, (i32)a.bandwidth);
-        if (!commit_slice(a, arena, dir, committed, t.band(), t.count, r.minScore, quit, r.maxX, r.maxXNode, notValid, lane))
+        if (!commit_slice(a, arena, dir, committed, t, r.minScore, quit, r.maxX, r.maxXNode, notValid, lane))
         {
             err = GA_CAPACITY;
             break;
@@ -1608,7 +1683,7 @@ __device__ ExtState fill_multiseed(const FillArgs& a, LargeTables& t, ArenaCurso
     // getInitialEmptySlice (Common.h:1541-1549): no nodes, minimum 0, bandwidth 1
     t.restart();
     t.next();
-    if (!commit_slice(a, arena, dir, 0, t.band(), 0, 0, 1, kIntMin, 0xffffffffu, false, lane, t.node_max()))
+    if (!commit_slice(a, arena, dir, 0, t, 0, 1, kIntMin, 0xffffffffu, false, lane, t.node_max()))
     {
         st.status = GA_CAPACITY;
         return st;
@@ -1632,7 +1707,7 @@ __device__ ExtState fill_multiseed(const FillArgs& a, LargeTables& t, ArenaCurso
         seeds.count = (u32)(next - k);
         seeds.ws = seed_ws(j, seqLen, a.cost);
         k = next;
-        SliceResult res = fill_slice<LargeTables, true>(a, t, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane, &seeds);
+        SliceResult res = fill_slice<LargeTables, true>(a, t, arena, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane, &seeds);
         if (err) break;
         // fillDPSlice's checks of a slice that started seeds (GraphAlignerBitvectorBanded.h:543-549)
         if (seeds.count > 0)
@@ -1643,7 +1718,7 @@ __device__ ExtState fill_multiseed(const FillArgs& a, LargeTables& t, ArenaCurso
         if (!(res.minScore >= lastMin || res.minScore >= ws_value(seeds.ws, 0) || lastMin == kIntMax - bw - 1)) { err = GA_ASSERT; break; }
         const bool notValid = res.cells >= a.maxCells;
         const i32 quit = wadd(res.minScore, bw);
-        if (!commit_slice(a, arena, dir, committed, t.band(), t.count, res.minScore, quit, res.maxX, res.maxXNode, notValid, lane, t.node_max()))
+        if (!commit_slice(a, arena, dir, committed, t, res.minScore, quit, res.maxX, res.maxXNode, notValid, lane, t.node_max()))
         {
             err = GA_CAPACITY;
             break;
@@ -1702,6 +1777,7 @@ struct TraceSpace
 {
     u64* ring;             // [64] trace items not yet written out
     SliceSlot* slots;      // [2] cached slices (odd and even)
+    ColumnUnit* columns;   // [64] a recomputed node-slice in the column store's form
 };
 
 struct Table
@@ -1992,7 +2068,7 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
     const NodeRec rec = node_record(g, node);
     const u32 L = rec_len(rec.meta);
     node_calc<false, Multi>(g, cost, node, L, rec.seq[0], rec.seq[1], copy, it->node, eqv, prev, nullptr, kNil, kNil, &start, false, (i32)j, last,
-        steps, err, lane, kIntMin, lastColumn, (Multi && extra.end != kIntMax) ? &extra : nullptr);
+        nullptr, steps, err, lane, kIntMin, lastColumn, (Multi && extra.end != kIntMax) ? &extra : nullptr);
     if (err) return err;
     const NodeCols& nc = node_cols();
     if (!ws_eq(nc.column(0), start)) return GA_ASSERT;
@@ -2001,11 +2077,10 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
 }
 
 // pickBacktraceVerticalCrossing (Common.h:886-934), the step out of (p.node, p.off > 0, row 0)
-// into the previous slice; pself is the node's entry there
+// into the previous slice; pself is the node's entry there, here the cell's score
 template <bool Multi>
-__device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* seq, Table t, u32 curSlice, const Item* pself, TPos p, int& err, WS extra)
+__device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* seq, Table t, u32 curSlice, const Item* pself, TPos p, i32 here, int& err, WS extra)
 {
-    const NodeCols& nc = node_cols();
     TStep second;
     second.pos = p;
     second.sw = false;
@@ -2014,7 +2089,6 @@ __device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* se
     bool bad = false;
     bool eq = char_match(g, seq[p.seq], p.node, p.off, bad);
     if (bad) { err = GA_ASSERT; return second; }
-    i32 here = nc.value(p.off, 0);
     // the previous slice's last row at column p.off - 1: its first column plus the deltas of columns 1..p.off-1
     const u64 upto = p.off >= 2 ? ((kAllOnes >> (64 - (p.off - 1))) << 1) : 0;
     i32 diag = pself->sEnd + popc64(pself->HP & upto) - popc64(pself->HN & upto);
@@ -2033,63 +2107,77 @@ __device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* se
     return second;
 }
 
-// pickBacktraceHorizontalCrossing (Common.h:817-884), the step out of (p.node, offset 0,
-// row off > 0) into an in-neighbour; self is the node's entry in the slice
+// pickBacktraceHorizontalCrossing (Common.h:817-884) at a cell whose score the tangle-effort
+// cap left invalid: the least of what the in-neighbours and the cell above offer
 template <bool Multi>
-__device__ __noinline__ TStep horizontal_step(const DevGraph& g, const uint8_t* seq, Table t, u32 curSlice, u32 curNode, const Item* self,
-    TPos p, u32 off, int& err, WS extra)
+__device__ __noinline__ TStep horizontal_step_invalid(const DevGraph& g, Table t, u32 curSlice, u32 curNode, const Item* self, TPos p, u32 off,
+    int& err, WS extra)
+{
+    TStep second;
+    second.pos = p;
+    second.sw = false;
+    WS sws = ws_make(self->sVP, self->sVN, self->sEnd);
+    i32 here = ws_value(sws, (int)off);
+    i32 smallest = ws_value(sws, (int)off - 1);
+    TPos sp = TPos { curNode, 0, p.seq - 1 };
+    bool change = false;
+    #pragma unroll 1
+    for (u32 e = g.inOff[curNode]; e < g.inOff[curNode + 1]; e++)
+    {
+        u32 nb = g.inNb[e];
+        const Item* cn = t.template find<Multi>(curSlice, nb);
+        if (cn)
+        {
+            WS nws = ws_make(cn->eVP, cn->eVN, cn->eEnd);
+            if (ws_value(nws, (int)off - 1) <= smallest)
+            {
+                smallest = ws_value(nws, (int)off - 1);
+                sp = TPos { nb, g.len[nb] - 1, p.seq - 1 };
+                change = true;
+            }
+            if (ws_value(nws, (int)off) < smallest && nb != curNode)
+            {
+                smallest = ws_value(nws, (int)off);
+                sp = TPos { nb, g.len[nb] - 1, p.seq };
+                change = true;
+            }
+        }
+    }
+    if (tpos_eq(sp, p) && here != xval<Multi>(extra, (int)off)) { err = GA_ASSERT; return second; }
+    return TStep { sp, change };
+}
+
+// pickBacktraceHorizontalCrossing (Common.h:817-884), the step out of (p.node, offset 0,
+// row off > 0) into an in-neighbour; self is the node's entry in the slice, the rest of the
+// node's record its in-neighbours
+template <bool Multi>
+__device__ __forceinline__ TStep horizontal_step(const DevGraph& g, const uint8_t* seq, Table& t, u32 curSlice, u32 curNode, const Item* self,
+    TPos p, u32 off, u32 meta, u32 inOff, u32 inNb0, u32 inNb1, int& err, WS extra)
 {
     TStep second;
     second.pos = p;
     second.sw = false;
     const SliceRec* cr = t.rec(curSlice);
     bool bad = false;
-    bool eq = char_match(g, seq[p.seq], p.node, p.off, bad);
+    bool eq = char_match(g, seq[p.seq], p.node, 0, bad);
     if (bad) { err = GA_ASSERT; return second; }
-    WS sws = ws_make(self->sVP, self->sVN, self->sEnd);
-    i32 here = ws_value(sws, (int)off);
-    if (cr->notValid || here > cr->quit)
-    {
-        i32 smallest = ws_value(sws, (int)off - 1);
-        TPos sp = TPos { curNode, 0, p.seq - 1 };
-        bool change = false;
-        #pragma unroll 1
-        for (u32 e = g.inOff[curNode]; e < g.inOff[curNode + 1]; e++)
-        {
-            u32 nb = g.inNb[e];
-            const Item* cn = t.template find<Multi>(curSlice, nb);
-            if (cn)
-            {
-                WS nws = ws_make(cn->eVP, cn->eVN, cn->eEnd);
-                if (ws_value(nws, (int)off - 1) <= smallest)
-                {
-                    smallest = ws_value(nws, (int)off - 1);
-                    sp = TPos { nb, g.len[nb] - 1, p.seq - 1 };
-                    change = true;
-                }
-                if (ws_value(nws, (int)off) < smallest && nb != curNode)
-                {
-                    smallest = ws_value(nws, (int)off);
-                    sp = TPos { nb, g.len[nb] - 1, p.seq };
-                    change = true;
-                }
-            }
-        }
-        if (tpos_eq(sp, p) && here != xval<Multi>(extra, (int)off)) { err = GA_ASSERT; return second; }
-        return TStep { sp, change };
-    }
+    const i32 here = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)off);
+    if (cr->notValid || here > cr->quit) return horizontal_step_invalid<Multi>(g, t, curSlice, curNode, self, p, off, err, extra);
+    u32 degree = rec_in_degree(meta);
+    if (degree >= kRecDegree) degree = g.inOff[curNode + 1] - inOff;
+    const i32 diagonal = here - (eq ? 0 : 1);
     #pragma unroll 1
-    for (u32 e = g.inOff[curNode]; e < g.inOff[curNode + 1]; e++)
+    for (u32 e = 0; e < degree; e++)
     {
-        u32 nb = g.inNb[e];
+        const u32 nb = e == 0 ? inNb0 : e == 1 ? inNb1 : g.inNb[inOff + e];
         const Item* cn = t.template find<Multi>(curSlice, nb);
         if (!cn) continue;
-        WS nws = ws_make(cn->eVP, cn->eVN, cn->eEnd);
-        i32 v0 = ws_value(nws, (int)off);
-        i32 v1 = ws_value(nws, (int)off - 1);
-        if (v0 < here - 1 || v1 < here - (eq ? 0 : 1)) { err = GA_ASSERT; return second; }
+        const u64 vp = cn->eVP, vn = cn->eVN;
+        const i32 v0 = ws_value(ws_make(vp, vn, cn->eEnd), (int)off);
+        const i32 v1 = v0 - (i32)((vp >> off) & 1) + (i32)((vn >> off) & 1);
+        if (v0 < here - 1 || v1 < diagonal) { err = GA_ASSERT; return second; }
         if (v0 == here - 1) return TStep { TPos { nb, g.len[nb] - 1, p.seq }, true };
-        if (v1 == here - (eq ? 0 : 1)) return TStep { TPos { nb, g.len[nb] - 1, p.seq - 1 }, true };
+        if (v1 == diagonal) return TStep { TPos { nb, g.len[nb] - 1, p.seq - 1 }, true };
     }
     if (here != xval<Multi>(extra, (int)off)) { err = GA_ASSERT; return second; }
     return TStep { p, false };
@@ -2217,29 +2305,57 @@ __device__ __noinline__ int row_above(const DevGraph& g, Table t, TraceOut& to)
     return 0;
 }
 
-// The first column of the run of row-0 steps that ends at column off: the least c <= off with
-// score(c') = score(c' - 1) + 1 for every c < c' <= off (pickBacktraceVerticalCrossing's walk
-// along the slice's first row, Common.h:886-900).  Columns 0..off must be in cols.
-__device__ __forceinline__ u32 row0_run_start(const NodeCols& nc, u32 off, u32 lane)
+// Columns 0..off of node-slice (s, node), recomputed into the warp's columns (NodeCols) and, in
+// the column store's form, into `out`.  Returns 0 or the error status.  Out of line: only what
+// found no room in the column store, and the multiseed DP's seed starts, come here.
+template <bool Multi>
+__device__ __noinline__ int recompute(const DevGraph& g, i32 cost, Table t, const uint8_t* seq, u32 seqLen, u32 s, u32 node, u32 off, WS extra,
+    ColumnUnit* out, u32 lane)
 {
-    const i32 v0 = nc.value(lane, 0);
-    const i32 v1 = nc.value(lane + 32, 0);
-    i32 p0 = __shfl_up_sync(kFull, v0, 1);
-    i32 p1 = __shfl_up_sync(kFull, v1, 1);
-    const i32 v31 = __shfl_sync(kFull, v0, 31);
-    if (lane == 0) p1 = v31;
-    // bit c: column c continues the run (column 0 never does)
-    const u64 cont = (u64)(__ballot_sync(kFull, lane > 0 && p0 == v0 - 1)) | ((u64)__ballot_sync(kFull, p1 == v1 - 1) << 32);
-    const u64 stops = ~cont & (off == 63 ? kAllOnes : ((2ULL << off) - 1));
-    return 63 - __clzll((long long)stops);
+    EqV4 eqv;
+    if (!eq_vector(seq, seqLen, ((int64_t)s - 1) * 64, eqv, lane)) return GA_ASSERT;
+    const int err = recalc<Multi>(g, cost, t, s, node, eqv, lane, off, extra);
+    if (err) return err;
+    const NodeCols& nc = node_cols();
+    i32 v[2];
+#pragma unroll
+    for (u32 h = 0; h < 2; h++) v[h] = lane + 32 * h <= off ? nc.value(lane + 32 * h, 0) : 0;
+    i32 p0 = __shfl_up_sync(kFull, v[0], 1);
+    i32 p1 = __shfl_up_sync(kFull, v[1], 1);
+    const i32 v31 = __shfl_sync(kFull, v[0], 31);
+    if (lane == 0)
+    {
+        p0 = v[0];
+        p1 = v31;
+    }
+    const i32 d0 = lane <= off ? wsub(v[0], p0) : 0, d1 = lane + 32 <= off ? wsub(v[1], p1) : 0;
+    const u64 plus = (u64)__ballot_sync(kFull, d0 == 1) | ((u64)__ballot_sync(kFull, d1 == 1) << 32);
+    const u64 minus = (u64)__ballot_sync(kFull, d0 == -1) | ((u64)__ballot_sync(kFull, d1 == -1) << 32);
+    __syncwarp();
+#pragma unroll
+    for (u32 h = 0; h < 2; h++)
+    {
+        const u32 pos = lane + 32 * h;
+        if (pos > 0 && pos <= off) out[pos] = { nc.v[pos].VP, nc.x[pos].rows };
+    }
+    if (lane == 0) out[0] = { plus, minus };
+    __syncwarp();
+    return 0;
 }
+
+// bits 1..off
+__device__ __forceinline__ u64 columns_upto(u32 off) { return (off == 63 ? kAllOnes : (2ULL << off) - 1) & ~1ULL; }
 
 // getReverseTraceFromTable's walk (Common.h:571-720) from `start`, whose score is startScore,
 // up to the row above the read or, in the multiseed DP (Multi), to a seed start.  resultScore:
 // the trace's OnewayTrace::score.  Returns 0 or the error status.
+//
+// The walk is a chain of dependent lookups.  A node-slice's steps come from the column store
+// (recomputed where they are not kept); the crossings whose slices' scores are all valid are
+// done in place, the ones at a tangle's cut-off go through the general rules out of line.
 template <bool Multi>
-__device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uint8_t* seq, u32 seqLen, u32 committed, Table& t, TraceOutT<Multi>& to, const TraceSpace& w,
-    TPos start, i32 startScore, i32& resultScore, u32 lane)
+__device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uint8_t* seq, u32 seqLen, u32 committed, Table& t, TraceOutT<Multi>& to,
+    const TraceSpace& w, const ColumnUnit* store, TPos start, i32 startScore, i32& resultScore, u32 lane)
 {
     int err = 0;
     const NodeCols& nc = node_cols();
@@ -2249,56 +2365,77 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     // the extraSlice of the current node-slice and its score at a row
     WS extra = fake_ws();
     auto xv = [&](u32 row) -> i32 { return Multi ? ws_value(extra, (int)row) : kIntMax; };
-    u32 curSlice = (u32)(start.seq / 64) + 1;
+    u32 curSlice = 0;
     u32 curNode = 0xffffffffu;
-    u32 curLen = 0;
-    u32 colsUpTo = 0;             // columns 0..colsUpTo of (curSlice, curNode) are in cols, their match masks in eqcol
-    EqV4 eqv;
-    if (!eq_vector(seq, seqLen, ((int64_t)curSlice - 1) * 64, eqv, lane)) err = GA_ASSERT;
-    u32 lastOff = 0, lastRow = 0xffffffffu;  // the last cell the walk looked at; its columns stay in cols
+    u32 colsUpTo = 0;             // columns 0..colsUpTo of (curSlice, curNode) are at `columns`
+    const ColumnUnit* columns = nullptr;
+    const Item* self = nullptr;
+    // the node's in-neighbours
+    u32 meta = 0, inOff = 0, inNb0 = 0, inNb1 = 0;
+    i32 lastScore = kIntMax - 1;  // score of the last cell the walk looked at, where it can end
     u64 guard = 0;
     #pragma unroll 1
     while (!err && !to.overflow && to.back.seq != -1)
     {
         if (++guard > guardMax) { err = GA_CAPACITY; break; }
-        TPos b = to.back;
-        u32 newSlice = (u32)(b.seq / 64) + 1;
+        const TPos b = to.back;
+        const u32 newSlice = (u32)(b.seq / 64) + 1;
         if (newSlice >= committed) { err = GA_ASSERT; break; }
         // a self-loop can re-enter the same node-slice further right than it was computed
         if (newSlice != curSlice || b.node != curNode || b.off > colsUpTo)
         {
-            if (newSlice != curSlice && !eq_vector(seq, seqLen, ((int64_t)newSlice - 1) * 64, eqv, lane)) { err = GA_ASSERT; break; }
             curSlice = newSlice;
             curNode = b.node;
-            if (curSlice == 0) { err = GA_ASSERT; break; }
-            if (Multi)
+            self = t.template find<Multi>(curSlice, curNode);
+            if (!self) { err = GA_ASSERT; break; }
+            if (Multi) extra = (self->node & kSeedStart) ? seed_ws(((int64_t)curSlice - 1) * 64, seqLen, cost) : fake_ws();
+            if (g.rec)
             {
-                const Item* here = t.template find<Multi>(curSlice, curNode);
-                if (!here) { err = GA_ASSERT; break; }
-                extra = (here->node & kSeedStart) ? seed_ws(((int64_t)curSlice - 1) * 64, seqLen, cost) : fake_ws();
+                const uint4 q = __ldg((const uint4*)(g.rec + curNode) + 1);
+                const uint2 nb = __ldg((const uint2*)(g.rec + curNode) + 4);
+                meta = q.y; inOff = q.z; inNb0 = nb.x; inNb1 = nb.y;
             }
-            err = recalc<Multi>(g, cost, t, curSlice, curNode, eqv, lane, b.off, extra);
-            if (err) break;
-            colsUpTo = b.off;
-            curLen = g.len[curNode];
+            else
+            {
+                NodeRec x;
+                gather_record(g, curNode, x);
+                meta = x.meta; inOff = x.inOff; inNb0 = x.inNb[0]; inNb1 = x.inNb[1];
+            }
+            const u32 at = (u32)self->minScore;
+            if (at != kNoColumns)
+            {
+                columns = store + at;
+                colsUpTo = 63;
+            }
+            else
+            {
+                err = recompute<Multi>(g, cost, t, seq, seqLen, curSlice, curNode, b.off, extra, w.columns, lane);
+                if (err) break;
+                columns = w.columns;
+                colsUpTo = b.off;
+            }
         }
+        const bool seeded = Multi && extra.end != kIntMax;
         const int64_t sj = ((int64_t)curSlice - 1) * 64;
-        if (b.off >= curLen) { err = GA_ASSERT; break; }
+        if (b.off >= rec_len(meta)) { err = GA_ASSERT; break; }
         const u32 row = mod64(b.seq);
-        lastOff = b.off;
-        lastRow = row;
-        if (row == 0 && b.off == 0)
-        {
-            TStep bt = bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra);
-            if (err) break;
-            if (tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == xv(mod64(bt.pos.seq))) break;
-            if (Multi && tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == ws_before(extra)) break;
-            to.push(bt.pos, bt.sw);
-            if (!to.overflow && trace_circular(to.items, to.ring, to.n, Multi && to.counting)) { err = GA_ASSERT; break; }
-            continue;
-        }
+        // the walk ends above the read, so from row 0 or up column 0 to it, or at a seed start
+        if (seeded) lastScore = nc.value(b.off, row);
         if (row == 0)
         {
+            const i32 first = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), 0);
+            const ColumnUnit top = columns[0];
+            if (!seeded) lastScore = first + popc64(top.x & columns_upto(b.off)) - popc64(top.y & columns_upto(b.off));
+            if (b.off == 0)
+            {
+                TStep bt = bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra);
+                if (err) break;
+                if (seeded && tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == xv(mod64(bt.pos.seq))) break;
+                if (seeded && tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == ws_before(extra)) break;
+                to.push(bt.pos, bt.sw);
+                if (!to.overflow && trace_circular(to.items, to.ring, to.n, Multi && to.counting)) { err = GA_ASSERT; break; }
+                continue;
+            }
             const Item* pself = t.template find<Multi>(curSlice - 1, curNode);
             if (!pself)
             {
@@ -2306,14 +2443,19 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 continue;
             }
             // pickBacktraceVerticalCrossing (Common.h:886-934)
-            // step left along row 0 while the score falls by one per column: lane k tests
-            // columns k and k + 32 against their left neighbours, the run ends at the
-            // highest failing column at or below b.off (column 0 always ends it)
+            // step left along row 0 while the score falls by one per column: the run ends at the
+            // highest column at or below b.off without a +1 delta (column 0 has none)
             TPos p = b;
-            p.off = row0_run_start(nc, b.off, lane);
-            TStep second = p.off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : vertical_step<Multi>(g, seq, t, curSlice, pself, p, err, extra);
+            p.off = 63 - (u32)__clzll((long long)(~top.x & (columns_upto(b.off) | 1)));
+            TStep second;
+            if (p.off == 0) second = bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra);
+            else
+            {
+                const i32 here = seeded ? nc.value(p.off, 0) : first + popc64(top.x & columns_upto(p.off)) - popc64(top.y & columns_upto(p.off));
+                second = vertical_step<Multi>(g, seq, t, curSlice, pself, p, here, err, extra);
+            }
             if (err) break;
-            if (second.pos.seq == b.seq && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
+            if (seeded && second.pos.seq == b.seq && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
             if (p.off != b.off) to.push_run(TPos { p.node, b.off - 1, p.seq }, -1, 0, b.off - p.off);
             if (tpos_eq(second.pos, to.back)) { err = GA_ASSERT; break; }
             to.push(second.pos, second.sw);
@@ -2322,21 +2464,18 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
         if (b.off == 0)
         {
             // pickBacktraceHorizontalCrossing (Common.h:817-884)
-            const Item* self = t.template find<Multi>(curSlice, curNode);
-            if (!self) { err = GA_ASSERT; break; }
             // step up column 0 while its score falls by one per row (the start column's VP
             // bits): the run ends at the highest row at or below this one whose bit is clear
             // (row 0 always ends it)
             TPos p = b;
-            {
-                const u32 r = mod64(b.seq);
-                const u64 stops = (~self->sVP | 1ULL) & (r == 63 ? kAllOnes : ((2ULL << r) - 1));
-                p.seq -= (int64_t)(r - (63 - __clzll((long long)stops)));
-            }
-            const u32 off = mod64(p.seq);
-            TStep second = off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : horizontal_step<Multi>(g, seq, t, curSlice, curNode, self, p, off, err, extra);
+            const u64 stops = (~self->sVP | 1ULL) & (row == 63 ? kAllOnes : ((2ULL << row) - 1));
+            const u32 off = 63 - (u32)__clzll((long long)stops);
+            p.seq -= (int64_t)(row - off);
+            if (!seeded && off == 0) lastScore = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)row);
+            TStep second = off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra)
+                : horizontal_step<Multi>(g, seq, t, curSlice, curNode, self, p, off, meta, inOff, inNb0, inNb1, err, extra);
             if (err) break;
-            if (second.pos.node == b.node && !second.sw && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
+            if (seeded && second.pos.node == b.node && !second.sw && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
             if (p.seq != b.seq) to.push_run(TPos { p.node, p.off, b.seq - 1 }, 0, -1, (u32)(b.seq - p.seq));
             if (tpos_eq(second.pos, to.back)) { err = GA_ASSERT; break; }
             to.push(second.pos, second.sw);
@@ -2345,14 +2484,11 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
         }
         // pickBacktraceInside (Common.h:770-815): up while the column's delta is +1, else
         // diagonally where that step is open, else left.  Inside a node-slice the steps are
-        // bits of the recomputed columns (VP: up, rows: diagonal; what is neither goes left), so
-        // a run of diagonal steps is found in one ballot, lane k testing the cell k steps down
-        // the diagonal, and a run of up steps is a leading-one count.
+        // bits of its columns, so a run of diagonal steps is found in one ballot, lane k testing
+        // the cell k steps down the diagonal, and a run of up steps is a leading-one count.
         // Cell by cell (two scores carried, every lane the same) this walk took 21.9k of the
-        // traceback's 58.8k cycles per 64-row slice of an extension alone; by runs, one seed of a
-        // 10 kbp read takes 4.72 ms instead of 5.60 and 50,000 extensions (250 Mbp) 115.6 ms
-        // instead of 128.2.
-        if (!Multi || extra.end == kIntMax)
+        // traceback's 58.8k cycles per 64-row slice of an extension alone.
+        if (!seeded)
         {
             u32 hori = b.off;
             u32 vert = row;
@@ -2360,13 +2496,10 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             while (hori > 0 && vert > 0 && !to.overflow)
             {
                 const u32 most = hori < vert ? hori : vert;
-                bool diagonal = false;
-                if (lane < most)
-                {
-                    const u64 bit = 1ULL << (vert - lane);
-                    diagonal = (nc.x[hori - lane].rows & ~nc.v[hori - lane].VP & bit) != 0;
-                }
-                const u32 run = (u32)__ffs((int)~__ballot_sync(kFull, diagonal));
+                ColumnUnit c { 0, 0 };
+                if (lane < most) c = columns[hori - lane];
+                const u64 bit = 1ULL << ((vert - lane) & 63);
+                const u32 run = (u32)__ffs((int)~__ballot_sync(kFull, (c.y & ~c.x & bit) != 0));
                 if (run != 1)
                 {
                     // __ffs(0) = 0: all 32 lanes' steps are diagonal
@@ -2376,7 +2509,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                     vert -= count;
                     continue;
                 }
-                const u64 vp = nc.v[hori].VP;
+                const u64 vp = __shfl_sync(kFull, c.x, 0);
                 if ((vp >> vert) & 1)
                 {
                     const u32 count = up_run(vp, vert);
@@ -2384,11 +2517,9 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                     vert -= count;
                     continue;
                 }
-                if (nc.value(hori - 1, vert) != nc.value(hori, vert) - 1) { err = GA_ASSERT; break; }
                 hori--;
                 to.push(TPos { b.node, hori, sj + vert }, false);
             }
-            if (err || to.overflow) break;
             continue;
         }
         // A seed start's columns are merged with its seed column, so their steps are not the
@@ -2464,7 +2595,6 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     }
     if (!err && !to.overflow)
     {
-        const i32 lastScore = lastRow == 0xffffffffu ? kIntMax - 1 : nc.value(lastOff, lastRow);
         if (resultScore < lastScore) err = GA_ASSERT;
         resultScore -= lastScore;
     }
@@ -2513,7 +2643,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
         // getReverseTraceFromTable (Common.h:571-758)
         TPos start = TPos { ec.node, ec.nodeOffset, ec.j + ec.bvOffset };
         i32 startScore = nc.value(ec.nodeOffset, ec.bvOffset);
-        err = trace_walk<false>(g, a.cost, seq, seqLen, st.committed, t, to, w, start, startScore, resultScore, lane);
+        err = trace_walk<false>(g, a.cost, seq, seqLen, st.committed, t, to, w, a.store, start, startScore, resultScore, lane);
         if (!err && !to.overflow) err = row_above(g, t, to);
     }
     to.finish();
@@ -2739,7 +2869,7 @@ __device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const TraceSp
     i32 traceScore = 0;
     if (!err)
     {
-        err = trace_walk<true>(a.g, a.cost, seq, seqLen, st.committed, t, to, w, start, startScore, traceScore, lane);
+        err = trace_walk<true>(a.g, a.cost, seq, seqLen, st.committed, t, to, w, a.store, start, startScore, traceScore, lane);
         to.finish();
         // a walk past its step guard or its counted length is broken, not short of room
         if (err == GA_CAPACITY || (!err && to.overflow)) err = GA_ASSERT;
@@ -2909,10 +3039,7 @@ __device__ __forceinline__ void fill_extensions(const FillArgs& fa, u32* counter
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
     Tables t(fa, (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane);
-    ArenaCursor arena;
-    arena.pos = 0;
-    arena.end = 0;
-    arena.used = 0;
+    ArenaCursor arena = arena_cursor(fa);
     u32 ext;
 #pragma unroll 1
     while (next_extension(counter, fa.num, fa.order, fa.prevStatus, lane, ext))
@@ -2924,15 +3051,15 @@ __device__ __forceinline__ void fill_extensions(const FillArgs& fa, u32* counter
     if (lane == 0 && arena.used) atomicAdd(fa.arenaCursor + 1, (unsigned long long)arena.used);
 }
 
-__global__ void __launch_bounds__(128, 4) fill_kernel(FillArgs fa, u32* counter) { fill_extensions<SmallTables>(fa, counter); }
-__global__ void __launch_bounds__(128, 4) fill_large_kernel(FillArgs fa, u32* counter) { fill_extensions<LargeTables>(fa, counter); }
+__global__ void __launch_bounds__(128, 4) fill_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<SmallTables>(fa, counter); }
+__global__ void __launch_bounds__(128, 4) fill_large_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<LargeTables>(fa, counter); }
 
 // the traceback's shared memory of one warp behind the block's NodeCols
-static constexpr u32 kTraceSpaceBytes = 64 * 8 + 2 * sizeof(SliceSlot);
+static constexpr u32 kTraceSpaceBytes = 64 * 8 + 2 * sizeof(SliceSlot) + 64 * sizeof(ColumnUnit);
 
 // The traceback: a warp takes the next filled extension and walks its table back.  Its
 // shared memory holds the recomputed columns, the match masks and the trace staging.
-__global__ void __launch_bounds__(128, 6) trace_kernel(TraceArgs ta, u32* counter)
+__global__ void __launch_bounds__(128, 6) trace_kernel(const __grid_constant__ TraceArgs ta, u32* counter)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
@@ -2940,6 +3067,7 @@ __global__ void __launch_bounds__(128, 6) trace_kernel(TraceArgs ta, u32* counte
     TraceSpace w;
     w.ring = (u64*)base;
     w.slots = (SliceSlot*)(base + 64 * 8);
+    w.columns = (ColumnUnit*)(base + 64 * 8 + 2 * sizeof(SliceSlot));
     u32 ext;
 #pragma unroll 1
     while (next_extension(counter, ta.num, ta.order, ta.prevStatus, lane, ext))
@@ -2952,15 +3080,12 @@ __global__ void __launch_bounds__(128, 6) trace_kernel(TraceArgs ta, u32* counte
 
 // The multiseed DP's fill: a warp takes the next read and fills its whole DP table; its
 // frontier tables and per-node X-scores live in the global workspace.
-__global__ void __launch_bounds__(128, 4) fill_multiseed_kernel(FillArgs fa, u32* counter)
+__global__ void __launch_bounds__(128, 4) fill_multiseed_kernel(const __grid_constant__ FillArgs fa, u32* counter)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
     LargeTables t(fa, (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane);
-    ArenaCursor arena;
-    arena.pos = 0;
-    arena.end = 0;
-    arena.used = 0;
+    ArenaCursor arena = arena_cursor(fa);
     u32 r;
 #pragma unroll 1
     while (next_extension(counter, fa.num, fa.order, fa.prevStatus, lane, r))
@@ -2974,7 +3099,7 @@ __global__ void __launch_bounds__(128, 4) fill_multiseed_kernel(FillArgs fa, u32
 
 // The per-read passes of the multiseed traceback (write = false: count the candidates and
 // reserve their run; write = true: list them), a warp per read.
-__global__ void __launch_bounds__(128, 6) ms_candidates_kernel(MultiTraceArgs ta, u32* counter, int write)
+__global__ void __launch_bounds__(128, 6) ms_candidates_kernel(const __grid_constant__ MultiTraceArgs ta, u32* counter, int write)
 {
     const u32 lane = threadIdx.x & 31;
     u32 r;
@@ -3006,7 +3131,7 @@ __global__ void ms_keys_kernel(MultiTraceArgs ta)
     }
 }
 
-__global__ void __launch_bounds__(128, 6) ms_resolve_kernel(MultiTraceArgs ta, u32* counter)
+__global__ void __launch_bounds__(128, 6) ms_resolve_kernel(const __grid_constant__ MultiTraceArgs ta, u32* counter)
 {
     const u32 lane = threadIdx.x & 31;
     u32 r;
@@ -3021,7 +3146,7 @@ __global__ void __launch_bounds__(128, 6) ms_resolve_kernel(MultiTraceArgs ta, u
 // The candidates' traces, a warp per candidate (write = false: the round's queued walks,
 // counted; write = true: the kept ones written).  A read's traces spread over as many warps
 // as it has walks in the round.
-__global__ void __launch_bounds__(128, 6) ms_trace_kernel(MultiTraceArgs ta, u32* counter, int write)
+__global__ void __launch_bounds__(128, 6) ms_trace_kernel(const __grid_constant__ MultiTraceArgs ta, u32* counter, int write)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
@@ -3029,6 +3154,7 @@ __global__ void __launch_bounds__(128, 6) ms_trace_kernel(MultiTraceArgs ta, u32
     TraceSpace w;
     w.ring = (u64*)base;
     w.slots = (SliceSlot*)(base + 64 * 8);
+    w.columns = (ColumnUnit*)(base + 64 * 8 + 2 * sizeof(SliceSlot));
     const u64 total = write ? (*ta.candTotal < ta.candCap ? *ta.candTotal : ta.candCap) : *ta.workCount;
 #pragma unroll 1
     while (true)

@@ -51,13 +51,27 @@ struct __align__(16) Item
     u64 eVP, eVN;          // last column
     u64 HP, HN;            // horizontal deltas along the slice's last row
     i32 sEnd, eEnd;
-    i32 minScore;
+    i32 minScore;          // in a committed slice: where the node's columns are (u32, kNoColumns: not kept)
     u32 node;              // bit 31: the node has been computed ("exists"); bit 30: it is a
                            // seed start in this slice (multiseed DP, DPSlice::seedstartNodes)
 };
 static constexpr u32 kExists = 0x80000000u;
 static constexpr u32 kSeedStart = 0x40000000u;
 static constexpr u32 kNodeMask = 0x3fffffffu;
+
+// The column store: what the traceback needs of a node-slice's columns, kept by the fill in
+// 16-byte units while there is room.  Unit 0 holds the +1 and -1 deltas along the slice's first
+// row (bit c: column c against column c - 1), unit c > 0 column c's VP and its rows with an open
+// diagonal step.  About 37 bytes per read base at bandwidth 10, written once and about half of it
+// read, where memory bandwidth is otherwise idle (below 1 % of the copy peak).  Recomputing the
+// columns, with the lookups, loads and masks that takes, was half of the traceback: 50,000
+// extensions (250 Mbp) 89.5 -> 61.5 ms, one seed of a 10 kbp read 3.95 -> 3.15 ms.
+struct __align__(16) ColumnUnit
+{
+    u64 x, y;
+};
+static constexpr u32 kNoColumns = 0xffffffffu;
+static constexpr u32 kStoreChunk = 2048;   // units a warp takes at once
 
 // A committed DP slice in the arena: this 32-byte record, then the band's node ids
 // (count u32, padded to 16 bytes), then count Items, all in first-pop order (the multiseed
@@ -119,7 +133,10 @@ struct FillArgs
     const u32* startOffset;
     uint8_t* arena;        // DP tables of the batch, handed out in chunks
     u64 arenaBytes;
-    unsigned long long* arenaCursor;   // [0] bytes handed out in chunks, [1] bytes the tables took (both start at 0)
+    unsigned long long* arenaCursor;   // [0] bytes handed out in chunks, [1] bytes the tables took, [2] units of the column store
+                                       // handed out (all start at 0)
+    ColumnUnit* store;     // the column store, or null
+    u64 storeUnits;        // below kNoColumns
     u64 chunkBytes;        // arena bytes a warp takes at once
     uint8_t* workspace;    // nullptr: the frontier tables live in shared memory (kSmall*), else
     u64 workspaceStride;   // bytes of one warp's tables there
@@ -145,6 +162,7 @@ struct TraceArgs
     const u64* seqOff;
     const u32* seqLen;
     const uint8_t* arena;
+    const ColumnUnit* store;
     const u64* traceOffset;
     const u32* traceCap;
     i32* status;
@@ -224,6 +242,7 @@ struct MultiTraceArgs
     const u64* seqOff;
     const u32* seqLen;
     const uint8_t* arena;
+    const ColumnUnit* store;
     const u64* traceOffset;
     const u64* traceCap;
     u32 maxTraces;

@@ -140,6 +140,7 @@ extern "C" int ga_extend_batch_noalloc(const ga_graph_desc* device_graph, const 
     fa.arenaBytes = arenaBytes;
     fa.arenaCursor = (unsigned long long*)(scratch + 16);
     fa.chunkBytes = 16 * 1024;
+    fa.store = nullptr;        // no column store: the traceback recomputes
     fa.workspace = nullptr;
     fa.prevStatus = nullptr;
     fa.states = (ExtState*)(scratch + kHeaderBytes);
