@@ -323,7 +323,7 @@ extern "C" int ga_extender_create(ga_graph_t graph, uint64_t arena_bytes, ga_ext
     if (e != cudaSuccess) { delete x; return cuda_fail(e, "workspace"); }
     if (arena_bytes == 0) arena_bytes = 4ULL << 30;
     x->arenaBytes = arena_bytes;
-    e = cudaMalloc((void**)&x->arena, x->arenaBytes);
+    e = cudaMalloc((void**)&x->arena, x->arenaBytes + gadev::kArenaPad);
     if (e != cudaSuccess) { cudaFree(x->workspace); delete x; return cuda_fail(e, "arena"); }
     GA_CUDA(cudaMalloc((void**)&x->counters, 16 * sizeof(uint32_t)));
     GA_CUDA(cudaMalloc((void**)&x->arenaCursor, 3 * sizeof(unsigned long long)));
@@ -386,7 +386,7 @@ static void reserve_store(ga_extender* x, uint64_t readBp, uint64_t warps)
     cudaFree(x->store);
     x->store = nullptr;
     x->storeUnits = 0;
-    if (cudaMalloc((void**)&x->store, want * unit) == cudaSuccess) x->storeUnits = want;
+    if (cudaMalloc((void**)&x->store, (want + gadev::kStorePad) * unit) == cudaSuccess) x->storeUnits = want;
     else
     {
         x->store = nullptr;

@@ -69,8 +69,8 @@ struct NodeVal
     uint16_t tail;
 };
 
-// A warp's recorded columns of one node-slice, in shared memory in every kernel: dynamic shared
-// memory starts with one of these per warp of the block.
+// A warp's recorded columns of one node-slice, in shared memory in every kernel: the fills' dynamic
+// shared memory starts with one of these per warp of the block.
 struct __align__(16) NodeCols
 {
     // what the column loop writes
@@ -90,7 +90,7 @@ struct __align__(16) NodeCols
 };
 extern __shared__ __align__(16) uint8_t dsmem[];
 
-__device__ __forceinline__ NodeCols& node_cols() { return ((NodeCols*)dsmem)[threadIdx.x >> 5]; }
+__device__ __forceinline__ NodeCols& fill_cols() { return ((NodeCols*)dsmem)[threadIdx.x >> 5]; }
 
 __device__ __forceinline__ u32 hash_node(u32 node)
 {
@@ -510,6 +510,50 @@ struct LargeTables
     __device__ __forceinline__ bool prev_linear(const DevGraph& g, u32, u32 node) const { return g.lin[node] != 0; }
 };
 
+// ---- the traceback's shared memory ----
+
+// A copy of one committed slice whose band has at most kCachedBand nodes
+static constexpr u32 kCachedBand = 12;
+
+struct __align__(16) SliceSlot
+{
+    SliceRec rec;
+    Item items[kCachedBand];
+    u32 slice;             // the slice, 0xffffffff = none
+    u32 pad[3];
+};
+
+// One warp's.  The walk works on one slice and the one before it while the next one is on its
+// way, so three slots (by the slice's number) hold them; the columns of a slice's whole band are
+// copied from the column store while the walk is in the slice after it.
+static constexpr u32 kKeptUnits = 128;
+
+struct __align__(16) TraceWarp
+{
+    union
+    {
+        NodeCols cols;                         // a node-slice recomputed
+        ColumnUnit kept[2][kKeptUnits];        // or the columns of two slices (odd and even)
+    };
+    ColumnUnit columns[64];                    // the recomputed node-slice in the column store's form
+    u64 ring[64];                              // trace items not yet written out
+    SliceSlot slots[3];
+};
+
+__device__ __forceinline__ TraceWarp& trace_warp() { return ((TraceWarp*)dsmem)[threadIdx.x >> 5]; }
+__device__ __forceinline__ NodeCols& trace_cols() { return trace_warp().cols; }
+
+// 16 bytes from global to shared memory, not waited for
+__device__ __forceinline__ void copy_ahead(void* to, const void* from)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"((u32)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void copies_done()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+}
+
 // IUPAC membership of every byte value (bit0 A, bit1 C, bit2 G, bit3 T; 0 = '-',
 // -1 = not a sequence character), filled from iupac_mask on the host at load time and
 // copied into shared memory by every block (lanes index it by data: the constant
@@ -823,7 +867,7 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     const EqV4& eqv, const PrevInfo& prev, const Extra* pool, uint16_t head, uint16_t nil, const WS* singleIncoming, bool singleInPrevBand,
     i32 seqOffset, WS& endColumn, ColumnUnit* kept, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
 {
-    NodeCols& nc = node_cols();
+    NodeCols& nc = Fill ? fill_cols() : trace_cols();
     u64* const eqcol = nc.eqcol;
     const bool hasExtra = Multi && extra != nullptr;
     bool forceCalculation = false;
@@ -1204,7 +1248,7 @@ __device__ __forceinline__ u32 band_hash_size(u32 count)
     return h;
 }
 
-// write one slice of the tables (record, node ids, band in first-pop order and, for the multiseed DP, each
+// write one slice of the tables (record, band in first-pop order, node ids and, for the multiseed DP, each
 // node's best X-score and a large band's index) into the arena, lanes copying
 template <class Tables>
 __device__ __forceinline__ bool commit_slice(const FillArgs& a, ArenaCursor& c, u64* dir, u32 index, const Tables& t, i32 minScore, i32 quit,
@@ -1233,11 +1277,12 @@ __device__ __forceinline__ bool commit_slice(const FillArgs& a, ArenaCursor& c, 
         *(SliceRec*)base = r;
         dir[index] = off;
     }
-    u32* ids = (u32*)(base + sizeof(SliceRec));
+    uint4* const items = (uint4*)(base + sizeof(SliceRec));
+    u32* const ids = (u32*)(items + count * 4);
     #pragma unroll 1
     for (u32 k = lane; k < count * 4; k += 32)
     {
-        if ((k & 3) != 3) ((uint4*)(base + sizeof(SliceRec) + idBytes))[k] = ((const uint4*)band)[k];
+        if ((k & 3) != 3) items[k] = ((const uint4*)band)[k];
     }
     #pragma unroll 1
     for (u32 k = lane; k < count; k += 32)
@@ -1245,7 +1290,7 @@ __device__ __forceinline__ bool commit_slice(const FillArgs& a, ArenaCursor& c, 
         // the last quarter of an entry, with the place of the node's columns
         uint4 v = ((const uint4*)(band + k))[3];
         v.z = t.lane_columns(k);
-        ((uint4*)(base + sizeof(SliceRec) + idBytes))[k * 4 + 3] = v;
+        items[k * 4 + 3] = v;
         ids[k] = v.w & kNodeMask;
     }
     if (nodeMax)
@@ -1272,6 +1317,10 @@ __device__ __forceinline__ bool commit_slice(const FillArgs& a, ArenaCursor& c, 
     }
     return true;
 }
+
+// the band entries of committed slice r, and their node ids
+__device__ __forceinline__ const Item* rec_items(const SliceRec* r) { return (const Item*)((const uint8_t*)r + sizeof(SliceRec)); }
+__device__ __forceinline__ const u32* rec_ids(const SliceRec* r) { return (const u32*)(rec_items(r) + r->count); }
 
 // position of node's entry in committed slice r (whose node ids are `ids`) through its band
 // index: 32 slots per probe step, the first slot in probe order that is empty or the node's
@@ -1737,82 +1786,53 @@ __device__ ExtState fill_multiseed(const FillArgs& a, LargeTables& t, ArenaCurso
 
 // ---------------------------------------------------------------- traceback
 
-// A copy in shared memory of one committed slice whose band has at most kCachedBand nodes:
-// the traceback works on one slice and the one before it, so two slots (by the slice's
-// parity) hold both, and their band lookups are ballots over shared memory.
-static constexpr u32 kCachedBand = 16;
-
-struct __align__(16) SliceSlot
-{
-    SliceRec rec;
-    u32 slice;             // the cached slice, 0xffffffff = none
-    u32 pad[3];
-    u32 ids[kCachedBand];
-    Item items[kCachedBand];
-};
-
-// The record of slice s; a band of at most kCachedBand nodes is first copied into the
-// slot of the slice's parity (lanes copy 16 bytes each)
-__device__ __noinline__ const SliceRec* load_slice(const uint8_t* arena, const u64* dir, SliceSlot* slots, u32 s, u32 lane)
+// The record of slice s; a slice of at most kCachedBand nodes is first copied into its slot
+// (lanes copy 16 bytes each)
+__device__ __noinline__ const SliceRec* load_slice(const uint8_t* arena, const u64* dir, u32 s, u32 lane)
 {
     const SliceRec* r = (const SliceRec*)(arena + dir[s]);
     const u32 n = r->count;
     if (n > kCachedBand) return r;
-    SliceSlot& sl = slots[s & 1];
+    SliceSlot& sl = trace_warp().slots[s % 3];
     __syncwarp();
-    const uint4* src = (const uint4*)r;
-    const u32* ids = (const u32*)((const uint8_t*)r + sizeof(SliceRec));
-    const uint4* items = (const uint4*)((const uint8_t*)ids + rec_ids_bytes(n));
-    if (lane < 2) ((uint4*)&sl.rec)[lane] = src[lane];
-    if (lane < n) sl.ids[lane] = ids[lane];
 #pragma unroll 1
-    for (u32 k = lane; k < n * 4; k += 32) ((uint4*)sl.items)[k] = items[k];
+    for (u32 k = lane; k < 2 + n * 4; k += 32) ((uint4*)&sl)[k] = ((const uint4*)r)[k];
     sl.slice = s;
     __syncwarp();
     return &sl.rec;
 }
 
-// One warp's shared memory of the traceback, besides its columns
-struct TraceSpace
-{
-    u64* ring;             // [64] trace items not yet written out
-    SliceSlot* slots;      // [2] cached slices (odd and even)
-    ColumnUnit* columns;   // [64] a recomputed node-slice in the column store's form
-};
-
 struct Table
 {
     const uint8_t* arena;
     const u64* dir;
-    u32 count;
     u32 lane;
-    SliceSlot* slots;
     __device__ __forceinline__ void init()
     {
-        slots[0].slice = 0xffffffffu;
-        slots[1].slice = 0xffffffffu;
+        for (u32 k = 0; k < 3; k++) trace_warp().slots[k].slice = 0xffffffffu;
         __syncwarp();
     }
     // the slice's record: its shared copy (made on first use when the band is small), else
     // the arena's
     __device__ __forceinline__ const SliceRec* rec(u32 s)
     {
-        SliceSlot& sl = slots[s & 1];
+        SliceSlot& sl = trace_warp().slots[s % 3];
         if (sl.slice == s) return &sl.rec;
-        return load_slice(arena, dir, slots, s, lane);
+        return load_slice(arena, dir, s, lane);
     }
     // the band entry of node in slice s, or nullptr (Hashed: the multiseed DP's tables)
     template <bool Hashed = false>
     __device__ __forceinline__ const Item* find(u32 s, u32 node)
     {
         const SliceRec* r = rec(s);
-        const u32 n = r->count;
-        const SliceSlot& sl = slots[s & 1];
-        const bool cached = sl.slice == s;
-        const u32* ids = cached ? sl.ids : (const u32*)((const uint8_t*)r + sizeof(SliceRec));
-        const Item* items = cached ? sl.items : (const Item*)((const uint8_t*)ids + rec_ids_bytes(n));
-        const int k = rec_index<Hashed>(r, ids, node, lane);
-        return k < 0 ? nullptr : &items[k];
+        const SliceSlot& sl = trace_warp().slots[s % 3];
+        if (sl.slice == s)
+        {
+            const u32 hit = __ballot_sync(kFull, lane < r->count && (sl.items[lane < kCachedBand ? lane : 0].node & kNodeMask) == node);
+            return hit ? &sl.items[__ffs((int)hit) - 1] : nullptr;
+        }
+        const int k = rec_index<Hashed>(r, rec_ids(r), node, lane);
+        return k < 0 ? nullptr : rec_items(r) + k;
     }
 };
 
@@ -2070,25 +2090,21 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
     node_calc<false, Multi>(g, cost, node, L, rec.seq[0], rec.seq[1], copy, it->node, eqv, prev, nullptr, kNil, kNil, &start, false, (i32)j, last,
         nullptr, steps, err, lane, kIntMin, lastColumn, (Multi && extra.end != kIntMax) ? &extra : nullptr);
     if (err) return err;
-    const NodeCols& nc = node_cols();
+    const NodeCols& nc = trace_cols();
     if (!ws_eq(nc.column(0), start)) return GA_ASSERT;
     if (lastColumn + 1 >= L && !ws_eq(nc.column(L - 1), ws_make(it->eVP, it->eVN, it->eEnd))) return GA_ASSERT;
     return 0;
 }
 
 // pickBacktraceVerticalCrossing (Common.h:886-934), the step out of (p.node, p.off > 0, row 0)
-// into the previous slice; pself is the node's entry there, here the cell's score
+// into the previous slice; pself is the node's entry there, here the cell's score, eq whether its
+// characters match
 template <bool Multi>
-__device__ __noinline__ TStep vertical_step(const DevGraph& g, const uint8_t* seq, Table t, u32 curSlice, const Item* pself, TPos p, i32 here, int& err, WS extra)
+__device__ __forceinline__ TStep vertical_step(const SliceRec* cr, const SliceRec* pr, const Item* pself, TPos p, i32 here, bool eq, int& err, const WS& extra)
 {
     TStep second;
     second.pos = p;
     second.sw = false;
-    const SliceRec* cr = t.rec(curSlice);
-    const SliceRec* pr = t.rec(curSlice - 1);
-    bool bad = false;
-    bool eq = char_match(g, seq[p.seq], p.node, p.off, bad);
-    if (bad) { err = GA_ASSERT; return second; }
     // the previous slice's last row at column p.off - 1: its first column plus the deltas of columns 1..p.off-1
     const u64 upto = p.off >= 2 ? ((kAllOnes >> (64 - (p.off - 1))) << 1) : 0;
     i32 diag = pself->sEnd + popc64(pself->HP & upto) - popc64(pself->HN & upto);
@@ -2147,42 +2163,6 @@ __device__ __noinline__ TStep horizontal_step_invalid(const DevGraph& g, Table t
     return TStep { sp, change };
 }
 
-// pickBacktraceHorizontalCrossing (Common.h:817-884), the step out of (p.node, offset 0,
-// row off > 0) into an in-neighbour; self is the node's entry in the slice, the rest of the
-// node's record its in-neighbours
-template <bool Multi>
-__device__ __forceinline__ TStep horizontal_step(const DevGraph& g, const uint8_t* seq, Table& t, u32 curSlice, u32 curNode, const Item* self,
-    TPos p, u32 off, u32 meta, u32 inOff, u32 inNb0, u32 inNb1, int& err, WS extra)
-{
-    TStep second;
-    second.pos = p;
-    second.sw = false;
-    const SliceRec* cr = t.rec(curSlice);
-    bool bad = false;
-    bool eq = char_match(g, seq[p.seq], p.node, 0, bad);
-    if (bad) { err = GA_ASSERT; return second; }
-    const i32 here = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)off);
-    if (cr->notValid || here > cr->quit) return horizontal_step_invalid<Multi>(g, t, curSlice, curNode, self, p, off, err, extra);
-    u32 degree = rec_in_degree(meta);
-    if (degree >= kRecDegree) degree = g.inOff[curNode + 1] - inOff;
-    const i32 diagonal = here - (eq ? 0 : 1);
-    #pragma unroll 1
-    for (u32 e = 0; e < degree; e++)
-    {
-        const u32 nb = e == 0 ? inNb0 : e == 1 ? inNb1 : g.inNb[inOff + e];
-        const Item* cn = t.template find<Multi>(curSlice, nb);
-        if (!cn) continue;
-        const u64 vp = cn->eVP, vn = cn->eVN;
-        const i32 v0 = ws_value(ws_make(vp, vn, cn->eEnd), (int)off);
-        const i32 v1 = v0 - (i32)((vp >> off) & 1) + (i32)((vn >> off) & 1);
-        if (v0 < here - 1 || v1 < diagonal) { err = GA_ASSERT; return second; }
-        if (v0 == here - 1) return TStep { TPos { nb, g.len[nb] - 1, p.seq }, true };
-        if (v1 == diagonal) return TStep { TPos { nb, g.len[nb] - 1, p.seq - 1 }, true };
-    }
-    if (here != xval<Multi>(extra, (int)off)) { err = GA_ASSERT; return second; }
-    return TStep { p, false };
-}
-
 struct EndCell
 {
     u32 node;
@@ -2200,7 +2180,7 @@ struct EndCell
 __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint8_t* arena, Table t, u32 committed, const uint8_t* seq,
     u32 seqLen, u32 lane)
 {
-    const NodeCols& nc = node_cols();
+    const NodeCols& nc = trace_cols();
     EndCell ec;
     ec.err = 0;
     ec.nodeOffset = 0xffffffffu;
@@ -2309,14 +2289,14 @@ __device__ __noinline__ int row_above(const DevGraph& g, Table t, TraceOut& to)
 // the column store's form, into `out`.  Returns 0 or the error status.  Out of line: only what
 // found no room in the column store, and the multiseed DP's seed starts, come here.
 template <bool Multi>
-__device__ __noinline__ int recompute(const DevGraph& g, i32 cost, Table t, const uint8_t* seq, u32 seqLen, u32 s, u32 node, u32 off, WS extra,
-    ColumnUnit* out, u32 lane)
+__device__ __noinline__ int recompute(const DevGraph& g, i32 cost, Table t, const uint8_t* seq, u32 seqLen, u32 s, u32 node, u32 off, WS extra, u32 lane)
 {
+    ColumnUnit* const out = trace_warp().columns;
     EqV4 eqv;
     if (!eq_vector(seq, seqLen, ((int64_t)s - 1) * 64, eqv, lane)) return GA_ASSERT;
     const int err = recalc<Multi>(g, cost, t, s, node, eqv, lane, off, extra);
     if (err) return err;
-    const NodeCols& nc = node_cols();
+    const NodeCols& nc = trace_cols();
     i32 v[2];
 #pragma unroll
     for (u32 h = 0; h < 2; h++) v[h] = lane + 32 * h <= off ? nc.value(lane + 32 * h, 0) : 0;
@@ -2350,15 +2330,23 @@ __device__ __forceinline__ u64 columns_upto(u32 off) { return (off == 63 ? kAllO
 // up to the row above the read or, in the multiseed DP (Multi), to a seed start.  resultScore:
 // the trace's OnewayTrace::score.  Returns 0 or the error status.
 //
-// The walk is a chain of dependent lookups.  A node-slice's steps come from the column store
-// (recomputed where they are not kept); the crossings whose slices' scores are all valid are
-// done in place, the ones at a tangle's cut-off go through the general rules out of line.
+// The walk is a chain of dependent lookups, so it is bound by how long each takes: with a
+// slice's record, entries and columns, the node's record, its neighbours' lengths and the read's
+// bytes each loaded where they were needed, a warp waited six cycles for every instruction.  They
+// are all on their way beforehand: when the walk enters slice s, the band's columns in s - 1 and
+// the record and entries of s - 2 are copied to shared memory (in pieces of fixed sizes, larger
+// bands are read in place), the read's rows of s - 1 loaded; when it enters a node, lanes 0-15 and
+// 16-31 load the records of its first two in-neighbours, a word each.  Columns that are not kept
+// are recomputed; the crossings whose slices' scores are all valid are done in place, the ones at
+// a tangle's cut-off go through the general rules out of line.
+// Ahead of time against on demand: one seed of a 10 kbp read 3.12 -> 2.80 ms, 50,000 extensions
+// (250 Mbp) 61.5 -> 58.5 ms, the multiseed DP of 40 tangled reads 107 -> 92 ms.
 template <bool Multi>
 __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uint8_t* seq, u32 seqLen, u32 committed, Table& t, TraceOutT<Multi>& to,
-    const TraceSpace& w, const ColumnUnit* store, TPos start, i32 startScore, i32& resultScore, u32 lane)
+    const ColumnUnit* store, TPos start, i32 startScore, i32& resultScore, u32 lane)
 {
     int err = 0;
-    const NodeCols& nc = node_cols();
+    const NodeCols& nc = trace_cols();
     const u64 guardMax = (u64)((Multi && to.counting) ? (1u << 26) : to.cap) * 4 + 1024;
     resultScore = startScore;
     to.push(start, false);
@@ -2370,10 +2358,78 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     u32 colsUpTo = 0;             // columns 0..colsUpTo of (curSlice, curNode) are at `columns`
     const ColumnUnit* columns = nullptr;
     const Item* self = nullptr;
-    // the node's in-neighbours
-    u32 meta = 0, inOff = 0, inNb0 = 0, inNb1 = 0;
     i32 lastScore = kIntMax - 1;  // score of the last cell the walk looked at, where it can end
     u64 guard = 0;
+    // the current slice and the one before it
+    const SliceRec* recCur = nullptr;
+    const SliceRec* recPrev = nullptr;
+    u32 idCur = 0xffffffffu, idPrev = 0xffffffffu;     // their bands' node ids where they have a slot (lane k: entry k)
+    bool slotCur = false, slotPrev = false;
+    RowBytes rows { -1, -1 }, rowsNext { -1, -1 };
+    u32 rowsSlice = 0, ahead = 0xffffffffu;            // the slice of rowsNext, the slice on its way to a slot
+    u64 dirNext = 0;                                   // where slice dirSlice lies
+    u32 dirSlice = 0xffffffffu;
+    u32 keptCur = kNoColumns, keptNext = kNoColumns, keptSlice = 0;    // first unit of the copied columns of the current slice and of keptSlice
+    // the current node's record (lane k: word k & 15) and its first two in-neighbours'
+    u32 word = 0, nbWord = 0;
+    u32 meta = 0, inOff = 0, inNb0 = 0xffffffffu, inNb1 = 0xffffffffu;
+
+    auto find_cur = [&](u32 node) -> const Item*
+    {
+        if (!slotCur) return t.template find<Multi>(curSlice, node);
+        const u32 hit = __ballot_sync(kFull, idCur == node);
+        return hit ? &trace_warp().slots[curSlice % 3].items[__ffs((int)hit) - 1] : nullptr;
+    };
+    auto find_prev = [&](u32 node) -> const Item*
+    {
+        if (!slotPrev) return t.template find<Multi>(curSlice - 1, node);
+        const u32 hit = __ballot_sync(kFull, idPrev == node);
+        return hit ? &trace_warp().slots[(curSlice - 1) % 3].items[__ffs((int)hit) - 1] : nullptr;
+    };
+    // a slice's band in the lanes; false when it has no slot
+    auto band_ids = [&](u32 s, const SliceRec* r, u32& id) -> bool
+    {
+        const SliceSlot& sl = trace_warp().slots[s % 3];
+        id = 0xffffffffu;
+        if (sl.slice != s) return false;
+        if (lane < r->count) id = sl.items[lane].node & kNodeMask;
+        return true;
+    };
+    // whether the read's character at `row` of the current slice matches column `off` of the node
+    auto matches = [&](u32 off, u32 row) -> bool
+    {
+        const u32 byte = row < 32 ? (u32)__shfl_sync(kFull, rows.lo, (int)row) : (u32)__shfl_sync(kFull, rows.hi, (int)row - 32);
+        const u32 base = (__shfl_sync(kFull, word, (int)(off >> 4)) >> ((off & 15) * 2)) & 3;
+        const u32 mask = curNode < g.firstAmbiguous ? 1u << base : (u32)node_char_mask(g, curNode, off);
+        return ((u32)s_iupac[byte & 0xff] & mask) != 0;
+    };
+    // pickBacktraceHorizontalCrossing (Common.h:817-884), the step out of (p.node, offset 0,
+    // row off > 0) into an in-neighbour
+    auto horizontal = [&](const TPos& p, u32 off) -> TStep
+    {
+        const i32 here = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)off);
+        if (recCur->notValid || here > recCur->quit) return horizontal_step_invalid<Multi>(g, t, curSlice, curNode, self, p, off, err, extra);
+        const i32 diagonal = here - (matches(0, off) ? 0 : 1);
+        u32 degree = rec_in_degree(meta);
+        if (degree >= kRecDegree) degree = g.inOff[curNode + 1] - inOff;
+        #pragma unroll 1
+        for (u32 e = 0; e < degree; e++)
+        {
+            const u32 nb = e == 0 ? inNb0 : e == 1 ? inNb1 : g.inNb[inOff + e];
+            const Item* cn = find_cur(nb);
+            if (!cn) continue;
+            const u64 vp = cn->eVP, vn = cn->eVN;
+            const i32 v0 = ws_value(ws_make(vp, vn, cn->eEnd), (int)off);
+            const i32 v1 = v0 - (i32)((vp >> off) & 1) + (i32)((vn >> off) & 1);
+            if (v0 < here - 1 || v1 < diagonal) { err = GA_ASSERT; return TStep { p, false }; }
+            if (v0 != here - 1 && v1 != diagonal) continue;
+            const u32 last = (e < 2 && g.rec ? rec_len(__shfl_sync(kFull, nbWord, (int)(16 * e + 5))) : g.len[nb]) - 1;
+            return TStep { TPos { nb, last, v0 == here - 1 ? p.seq : p.seq - 1 }, true };
+        }
+        if (here != xval<Multi>(extra, (int)off)) err = GA_ASSERT;
+        return TStep { p, false };
+    };
+
     #pragma unroll 1
     while (!err && !to.overflow && to.back.seq != -1)
     {
@@ -2384,34 +2440,88 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
         // a self-loop can re-enter the same node-slice further right than it was computed
         if (newSlice != curSlice || b.node != curNode || b.off > colsUpTo)
         {
-            curSlice = newSlice;
-            curNode = b.node;
-            self = t.template find<Multi>(curSlice, curNode);
+            if (newSlice != curSlice)
+            {
+                TraceWarp& tw = trace_warp();
+                copies_done();
+                if (ahead != 0xffffffffu)
+                {
+                    SliceSlot& sl = tw.slots[ahead % 3];
+                    sl.slice = sl.rec.count <= kCachedBand ? ahead : 0xffffffffu;
+                    ahead = 0xffffffffu;
+                    __syncwarp();
+                }
+                curSlice = newSlice;
+                keptCur = keptSlice == curSlice ? keptNext : kNoColumns;
+                keptNext = kNoColumns;
+                recCur = t.rec(curSlice);
+                recPrev = t.rec(curSlice - 1);
+                slotCur = band_ids(curSlice, recCur, idCur);
+                slotPrev = band_ids(curSlice - 1, recPrev, idPrev);
+                rows = rowsSlice == curSlice ? rowsNext : row_bytes(seq, seqLen, ((int64_t)curSlice - 1) * 64, lane);
+                if (curSlice >= 2)
+                {
+                    rowsNext = row_bytes(seq, seqLen, ((int64_t)curSlice - 2) * 64, lane);
+                    rowsSlice = curSlice - 1;
+                    const u32 first = slotPrev && recPrev->count ? (u32)tw.slots[(curSlice - 1) % 3].items[0].minScore : kNoColumns;
+                    if (first != kNoColumns)
+                    {
+                        keptNext = first;
+                        keptSlice = curSlice - 1;
+                        ColumnUnit* to16 = tw.kept[keptSlice & 1];
+#pragma unroll
+                        for (u32 k = 0; k < kKeptUnits; k += 32) copy_ahead(to16 + k + lane, store + first + k + lane);
+                    }
+                    ahead = curSlice - 2;
+                    SliceSlot& sl = tw.slots[ahead % 3];
+                    sl.slice = 0xffffffffu;
+                    const uint4* from = (const uint4*)(t.arena + (dirSlice == ahead ? dirNext : t.dir[ahead]));
+                    if (ahead > 0)
+                    {
+                        dirSlice = ahead - 1;
+                        dirNext = t.dir[dirSlice];
+                    }
+                    #pragma unroll 1
+                    for (u32 k = lane; k < 2 + 4 * kCachedBand; k += 32) copy_ahead((uint4*)&sl + k, from + k);
+                }
+            }
+            if (b.node != curNode)
+            {
+                curNode = b.node;
+                if (g.rec && curNode == inNb0) word = __shfl_sync(kFull, nbWord, (int)(lane & 15));
+                else if (g.rec && curNode == inNb1) word = __shfl_sync(kFull, nbWord, (int)(16 + (lane & 15)));
+                else if (g.rec) word = __ldg((const u32*)(g.rec + curNode) + (lane & 15));
+                else
+                {
+                    NodeRec x;
+                    gather_record(g, curNode, x);
+                    word = ((const u32*)&x)[lane & 15];
+                }
+                meta = __shfl_sync(kFull, word, 5);
+                inOff = __shfl_sync(kFull, word, 6);
+                inNb0 = __shfl_sync(kFull, word, 8);
+                inNb1 = __shfl_sync(kFull, word, 9);
+                const u32 nb = lane < 16 ? inNb0 : inNb1;
+                if (g.rec && nb != 0xffffffffu) nbWord = __ldg((const u32*)(g.rec + nb) + (lane & 15));
+            }
+            self = find_cur(curNode);
             if (!self) { err = GA_ASSERT; break; }
             if (Multi) extra = (self->node & kSeedStart) ? seed_ws(((int64_t)curSlice - 1) * 64, seqLen, cost) : fake_ws();
-            if (g.rec)
-            {
-                const uint4 q = __ldg((const uint4*)(g.rec + curNode) + 1);
-                const uint2 nb = __ldg((const uint2*)(g.rec + curNode) + 4);
-                meta = q.y; inOff = q.z; inNb0 = nb.x; inNb1 = nb.y;
-            }
-            else
-            {
-                NodeRec x;
-                gather_record(g, curNode, x);
-                meta = x.meta; inOff = x.inOff; inNb0 = x.inNb[0]; inNb1 = x.inNb[1];
-            }
             const u32 at = (u32)self->minScore;
             if (at != kNoColumns)
             {
-                columns = store + at;
+                columns = keptCur != kNoColumns && at - keptCur <= kKeptUnits - rec_len(meta) ? trace_warp().kept[curSlice & 1] + (at - keptCur)
+                    : store + at;
                 colsUpTo = 63;
             }
             else
             {
-                err = recompute<Multi>(g, cost, t, seq, seqLen, curSlice, curNode, b.off, extra, w.columns, lane);
+                // the recomputed columns lie where the kept ones are copied to
+                copies_done();
+                keptCur = keptNext = kNoColumns;
+                err = recompute<Multi>(g, cost, t, seq, seqLen, curSlice, curNode, b.off, extra, lane);
                 if (err) break;
-                columns = w.columns;
+                columns = trace_warp().columns;
                 colsUpTo = b.off;
             }
         }
@@ -2436,7 +2546,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 if (!to.overflow && trace_circular(to.items, to.ring, to.n, Multi && to.counting)) { err = GA_ASSERT; break; }
                 continue;
             }
-            const Item* pself = t.template find<Multi>(curSlice - 1, curNode);
+            const Item* pself = find_prev(curNode);
             if (!pself)
             {
                 to.push_run(TPos { curNode, b.off - 1, b.seq }, -1, 0, b.off);
@@ -2452,7 +2562,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             else
             {
                 const i32 here = seeded ? nc.value(p.off, 0) : first + popc64(top.x & columns_upto(p.off)) - popc64(top.y & columns_upto(p.off));
-                second = vertical_step<Multi>(g, seq, t, curSlice, pself, p, here, err, extra);
+                second = vertical_step<Multi>(recCur, recPrev, pself, p, here, matches(p.off, 0), err, extra);
             }
             if (err) break;
             if (seeded && second.pos.seq == b.seq && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
@@ -2472,8 +2582,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             const u32 off = 63 - (u32)__clzll((long long)stops);
             p.seq -= (int64_t)(row - off);
             if (!seeded && off == 0) lastScore = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)row);
-            TStep second = off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra)
-                : horizontal_step<Multi>(g, seq, t, curSlice, curNode, self, p, off, meta, inOff, inNb0, inNb1, err, extra);
+            TStep second = off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : horizontal(p, off);
             if (err) break;
             if (seeded && second.pos.node == b.node && !second.sw && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
             if (p.seq != b.seq) to.push_run(TPos { p.node, p.off, b.seq - 1 }, 0, -1, (u32)(b.seq - p.seq));
@@ -2533,7 +2642,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             u32 hori = b.off;
             u32 vert = row;
             // the recomputation left each column's match mask (the fill's Eq) in eqcol
-            const u64* eqcol = node_cols().eqcol;
+            const u64* eqcol = nc.eqcol;
             if (hori > 0 && vert > 0)
             {
                 WS colH = nc.column(hori);
@@ -2593,6 +2702,8 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             if (nc.value(to.back.off, mod64(to.back.seq)) == xv(mod64(to.back.seq))) break;
         }
     }
+    // the next trace writes where copies may still be on their way
+    copies_done();
     if (!err && !to.overflow)
     {
         if (resultScore < lastScore) err = GA_ASSERT;
@@ -2601,7 +2712,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     return err;
 }
 
-__device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st, const TraceSpace& w, u32 lane)
+__device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st, u32 lane)
 {
     const DevGraph& g = a.g;
     u64* out = a.traceItems + a.traceOffset[ext];
@@ -2622,14 +2733,12 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
     Table t;
     t.arena = a.arena;
     t.dir = (const u64*)(a.arena + st.dir);
-    t.count = st.committed;
     t.lane = lane;
-    t.slots = w.slots;
     t.init();
-    const NodeCols& nc = node_cols();
+    const NodeCols& nc = trace_cols();
     TraceOut to;
     to.items = out;
-    to.ring = w.ring;
+    to.ring = trace_warp().ring;
     to.cap = cap;
     to.n = 0;
     to.lane = lane;
@@ -2643,7 +2752,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
         // getReverseTraceFromTable (Common.h:571-758)
         TPos start = TPos { ec.node, ec.nodeOffset, ec.j + ec.bvOffset };
         i32 startScore = nc.value(ec.nodeOffset, ec.bvOffset);
-        err = trace_walk<false>(g, a.cost, seq, seqLen, st.committed, t, to, w, a.store, start, startScore, resultScore, lane);
+        err = trace_walk<false>(g, a.cost, seq, seqLen, st.committed, t, to, a.store, start, startScore, resultScore, lane);
         if (!err && !to.overflow) err = row_above(g, t, to);
     }
     to.finish();
@@ -2661,7 +2770,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
 __device__ __forceinline__ bool slice_node_max(const uint8_t* arena, const u64* dir, u32 s, u32 node, u32 lane, i32& out)
 {
     const SliceRec* r = (const SliceRec*)(arena + dir[s]);
-    const int k = rec_index<true>(r, (const u32*)((const uint8_t*)r + sizeof(SliceRec)), node, lane);
+    const int k = rec_index<true>(r, rec_ids(r), node, lane);
     if (k < 0) return false;
     out = rec_node_max(r)[k];
     return true;
@@ -2713,8 +2822,8 @@ __device__ void ms_candidates(const MultiTraceArgs& a, u32 r, const ExtState& st
             const SliceRec* cr = (const SliceRec*)(a.arena + dir[cs]);
             if (cr->maxX <= 0) continue;
             const u32 n = cr->count;
-            const u32* ids = (const u32*)((const uint8_t*)cr + sizeof(SliceRec));
-            const Item* items = (const Item*)((const uint8_t*)ids + rec_ids_bytes(n));
+            const u32* ids = rec_ids(cr);
+            const Item* items = rec_items(cr);
             const i32* nodeMax = rec_node_max(cr);
             const double threshold = (double)sliceMax[cs] * a.multimapScoreFraction;
 #pragma unroll 1
@@ -2762,12 +2871,12 @@ __device__ void ms_candidates(const MultiTraceArgs& a, u32 r, const ExtState& st
 // The first cell of a candidate's trace (getLocalMaximaTracesFromTable): among the node's
 // columns, recomputed with its seed start, the cell of greatest row that scores the node's
 // best X-score (the first column on ties); a cell above it is GA_ASSERT.
-__device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const TraceSpace& w, const uint8_t* seq, u32 seqLen, const MsCand& c,
+__device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const uint8_t* seq, u32 seqLen, const MsCand& c,
     TPos& start, i32& startScore, u32 lane)
 {
     const DevGraph& g = a.g;
     const SliceRec* cr = (const SliceRec*)(a.arena + t.dir[c.slice]);
-    const Item* items = (const Item*)((const uint8_t*)cr + sizeof(SliceRec) + rec_ids_bytes(cr->count));
+    const Item* items = rec_items(cr);
     const u32 node = items[c.index].node & kNodeMask;
     const int64_t j = ((int64_t)c.slice - 1) * 64;
     EqV4 eqv;
@@ -2775,7 +2884,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const TraceSpace
     const WS extra = (items[c.index].node & kSeedStart) ? seed_ws(j, seqLen, a.cost) : fake_ws();
     int err = recalc<true>(g, a.cost, t, c.slice, node, eqv, lane, 63, extra);
     if (err) return err;
-    const NodeCols& nc = node_cols();
+    const NodeCols& nc = trace_cols();
     const i32 score = c.score;
     const int cells = (int)((int64_t)seqLen - j < 64 ? (int64_t)seqLen - j : 64);
     const u32 L = g.len[node];
@@ -2818,7 +2927,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const TraceSpace
 // span and last cell.  write = true (a kept trace of a read whose traces all fit and, with
 // exact room, that removeDuplicateTraces kept): walks it again into the read's output at
 // the place the read's selection (or the host, with exact room) gave it.
-__device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const TraceSpace& w, bool write, u32 lane)
+__device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, bool write, u32 lane)
 {
     const MsCand c = *cp;
     const u32 r = c.read;
@@ -2836,9 +2945,7 @@ __device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const TraceSp
     Table t;
     t.arena = a.arena;
     t.dir = (const u64*)(a.arena + st.dir);
-    t.count = st.committed;
     t.lane = lane;
-    t.slots = w.slots;
     t.init();
     TPos start;
     i32 startScore = 0;
@@ -2850,7 +2957,7 @@ __device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const TraceSp
     }
     else
     {
-        err = ms_start_cell(a, t, w, seq, seqLen, c, start, startScore, lane);
+        err = ms_start_cell(a, t, seq, seqLen, c, start, startScore, lane);
     }
     const bool exact = a.traceBase != nullptr;
     // exact room: the kept trace's place after the duplicates went, or none
@@ -2859,7 +2966,7 @@ __device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const TraceSp
     if (exact && write && outSlot == kNoSlot) return;
     TraceOutT<true> to;
     to.items = write ? a.traceItems + (exact ? a.keptItem[kept] : a.traceOffset[r] + c.outOff) : nullptr;
-    to.ring = w.ring;
+    to.ring = trace_warp().ring;
     to.lane = lane;
     to.counting = !write;
     to.cap = write ? c.len : 0xffffffffu;
@@ -2869,7 +2976,7 @@ __device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, const TraceSp
     i32 traceScore = 0;
     if (!err)
     {
-        err = trace_walk<true>(a.g, a.cost, seq, seqLen, st.committed, t, to, w, a.store, start, startScore, traceScore, lane);
+        err = trace_walk<true>(a.g, a.cost, seq, seqLen, st.committed, t, to, a.store, start, startScore, traceScore, lane);
         to.finish();
         // a walk past its step guard or its counted length is broken, not short of room
         if (err == GA_CAPACITY || (!err && to.overflow)) err = GA_ASSERT;
@@ -3054,26 +3161,20 @@ __device__ __forceinline__ void fill_extensions(const FillArgs& fa, u32* counter
 __global__ void __launch_bounds__(128, 4) fill_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<SmallTables>(fa, counter); }
 __global__ void __launch_bounds__(128, 4) fill_large_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<LargeTables>(fa, counter); }
 
-// the traceback's shared memory of one warp behind the block's NodeCols
-static constexpr u32 kTraceSpaceBytes = 64 * 8 + 2 * sizeof(SliceSlot) + 64 * sizeof(ColumnUnit);
-
-// The traceback: a warp takes the next filled extension and walks its table back.  Its
+// The traceback: a warp takes the next filled extension and walks its table back.  Four blocks of
+// 128 registers a thread on an SM: with six of 80 the walk's state spills, and the batch above
+// takes 67.5 ms instead of 58.5 (five of 96: 62.8).  Its
 // shared memory holds the recomputed columns, the match masks and the trace staging.
-__global__ void __launch_bounds__(128, 6) trace_kernel(const __grid_constant__ TraceArgs ta, u32* counter)
+__global__ void __launch_bounds__(128, 4) trace_kernel(const __grid_constant__ TraceArgs ta, u32* counter)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
-    uint8_t* base = dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (threadIdx.x >> 5) * kTraceSpaceBytes;
-    TraceSpace w;
-    w.ring = (u64*)base;
-    w.slots = (SliceSlot*)(base + 64 * 8);
-    w.columns = (ColumnUnit*)(base + 64 * 8 + 2 * sizeof(SliceSlot));
     u32 ext;
 #pragma unroll 1
     while (next_extension(counter, ta.num, ta.order, ta.prevStatus, lane, ext))
     {
         __syncwarp();
-        trace_extension(ta, ext, ta.states[ext], w, lane);
+        trace_extension(ta, ext, ta.states[ext], lane);
     }
 }
 
@@ -3146,15 +3247,10 @@ __global__ void __launch_bounds__(128, 6) ms_resolve_kernel(const __grid_constan
 // The candidates' traces, a warp per candidate (write = false: the round's queued walks,
 // counted; write = true: the kept ones written).  A read's traces spread over as many warps
 // as it has walks in the round.
-__global__ void __launch_bounds__(128, 6) ms_trace_kernel(const __grid_constant__ MultiTraceArgs ta, u32* counter, int write)
+__global__ void __launch_bounds__(128, 4) ms_trace_kernel(const __grid_constant__ MultiTraceArgs ta, u32* counter, int write)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
-    uint8_t* base = dsmem + (blockDim.x >> 5) * sizeof(NodeCols) + (threadIdx.x >> 5) * kTraceSpaceBytes;
-    TraceSpace w;
-    w.ring = (u64*)base;
-    w.slots = (SliceSlot*)(base + 64 * 8);
-    w.columns = (ColumnUnit*)(base + 64 * 8 + 2 * sizeof(SliceSlot));
     const u64 total = write ? (*ta.candTotal < ta.candCap ? *ta.candTotal : ta.candCap) : *ta.workCount;
 #pragma unroll 1
     while (true)
@@ -3164,7 +3260,7 @@ __global__ void __launch_bounds__(128, 6) ms_trace_kernel(const __grid_constant_
         i = __shfl_sync(kFull, i, 0);
         if (i >= total) break;
         __syncwarp();
-        ms_trace_cand(ta, ta.cands + (write ? i : ta.work[i]), w, write != 0, lane);
+        ms_trace_cand(ta, ta.cands + (write ? i : ta.work[i]), write != 0, lane);
     }
 }
 }
@@ -3172,7 +3268,7 @@ __global__ void __launch_bounds__(128, 6) ms_trace_kernel(const __grid_constant_
 // dynamic shared memory of a block of the fill kernels (shared: with its frontier tables) and of
 // the traceback kernels
 static size_t fill_smem(int warpsPerBlock, bool shared) { return (sizeof(gadev::NodeCols) + (shared ? sizeof(gadev::SmallSpace) : 0)) * warpsPerBlock; }
-static size_t trace_smem(int warpsPerBlock) { return (sizeof(gadev::NodeCols) + gadev::kTraceSpaceBytes) * warpsPerBlock; }
+static size_t trace_smem(int warpsPerBlock) { return sizeof(gadev::TraceWarp) * warpsPerBlock; }
 
 uint64_t ga_warp_tables_bytes(const gadev::Caps& c) { return gadev::wspace_bytes(c); }
 uint64_t ga_multiseed_tables_bytes(const gadev::Caps& c) { return gadev::wspace_bytes(c, true); }

@@ -73,9 +73,14 @@ struct __align__(16) ColumnUnit
 static constexpr u32 kNoColumns = 0xffffffffu;
 static constexpr u32 kStoreChunk = 2048;   // units a warp takes at once
 
-// A committed DP slice in the arena: this 32-byte record, then the band's node ids
-// (count u32, padded to 16 bytes), then count Items, all in first-pop order (the multiseed
-// DP's seed starts first), then for the multiseed DP each node's best exact-end-position
+// The traceback copies slices and their columns ahead in pieces of fixed sizes, which may reach
+// past the last one: so much is readable behind the arena (bytes) and the store (units).
+static constexpr u32 kArenaPad = 1024;
+static constexpr u32 kStorePad = 128;
+
+// A committed DP slice in the arena: this 32-byte record, then count Items in first-pop order
+// (the multiseed DP's seed starts first), then their node ids (u32, padded to 16 bytes), then
+// for the multiseed DP each node's best exact-end-position
 // X-score (count i32, DPSlice::nodeMaxExactEndposScore) and, for a band of more than
 // kHashedBand nodes, an open-addressing index of the band (hashSize u32 slots, each an
 // entry's position or kEmptySlot, linear probing from the node's hash).  The traceback finds
@@ -132,7 +137,7 @@ struct FillArgs
     const u32* startNode;
     const u32* startOffset;
     uint8_t* arena;        // DP tables of the batch, handed out in chunks
-    u64 arenaBytes;
+    u64 arenaBytes;        // kArenaPad more are readable behind them
     unsigned long long* arenaCursor;   // [0] bytes handed out in chunks, [1] bytes the tables took, [2] units of the column store
                                        // handed out (all start at 0)
     ColumnUnit* store;     // the column store, or null

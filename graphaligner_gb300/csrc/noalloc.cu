@@ -29,7 +29,7 @@ constexpr u32 kMaxExtensions = 4096;              // per call
 constexpr u64 kMaxReadBp = 8000000;               // per call, summed over the batch
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) uint8_t g_scratch[kScratchBytes];
+static __device__ __align__(256) uint8_t g_scratch[kScratchBytes + kArenaPad];
 
 // the scratch array's device address, per device, looked up once with that device current
 void* g_scratchAddress[kMaxDevices] = {};
