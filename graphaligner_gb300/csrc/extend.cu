@@ -142,17 +142,14 @@ __device__ __forceinline__ NodeRec node_record(const DevGraph& g, u32 node)
     return r;
 }
 
-// in- and out-degree (beyond what the record's field holds: from the arrays)
-__device__ __forceinline__ u32 in_degree(const DevGraph& g, u32 node, const NodeRec& r)
+// What a node's computation needs of its record; the out-neighbours are asked for afterwards,
+// so that they do not take registers meanwhile
+struct NodeHead
 {
-    const u32 n = rec_in_degree(r.meta);
-    return n < kRecDegree ? n : g.inOff[node + 1] - r.inOff;
-}
-__device__ __forceinline__ u32 out_degree(const DevGraph& g, u32 node, const NodeRec& r)
-{
-    const u32 n = rec_out_degree(r.meta);
-    return n < kRecDegree ? n : g.outOff[node + 1] - r.outOff;
-}
+    u64 seq[2];
+    u32 meta;
+    u32 inNb;              // the first in-neighbour
+};
 
 // One warp's tables in global memory.  A node-table key is (generation << 32) | node; a slot whose
 // generation is not the slice's is empty, so tables are never cleared between slices.
@@ -392,14 +389,17 @@ struct SmallTables
         const u32 b = __shfl_sync(kFull, val, (int)slot) & 0xff;
         return b == 0xff ? -1 : (int)b;
     }
-    __device__ __forceinline__ NodeRec record(const DevGraph&, u32 slot, u32)
+    __device__ __forceinline__ NodeHead head(const DevGraph&, u32 slot, u32)
     {
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncwarp();
-        const NodeRec r = small_space().rec[slot];
-        if ((r.meta & kRecLinearizable) && lane == slot) val |= kLinear;
-        return r;
+        const NodeRec& r = small_space().rec[slot];
+        const NodeHead h { { r.seq[0], r.seq[1] }, r.meta, r.inNb[0] };
+        if ((h.meta & kRecLinearizable) && lane == slot) val |= kLinear;
+        return h;
     }
+    // the record, for its out-neighbours
+    __device__ __forceinline__ const NodeRec* record(const DevGraph&, u32 slot, u32, NodeRec&) const { return &small_space().rec[slot]; }
     __device__ __forceinline__ u32 prev_component(const DevGraph&, u32 k, u32) const { return __shfl_sync(kFull, prevComp, (int)k); }
     __device__ __forceinline__ bool prev_linear(const DevGraph&, u32 k, u32) const { return __shfl_sync(kFull, (int)prevLinear, (int)k) != 0; }
 };
@@ -505,7 +505,17 @@ struct LargeTables
     __device__ __forceinline__ void set_columns(u32 at, u32 where) { w.columns[at] = where; }
     __device__ __forceinline__ u32 lane_columns(u32 at) const { return w.columns[at]; }
     __device__ __forceinline__ int band_of(u32 slot) const { return w.val[side][slot].band; }
-    __device__ __forceinline__ NodeRec record(const DevGraph& g, u32, u32 node) { return node_record(g, node); }
+    __device__ __forceinline__ NodeHead head(const DevGraph& g, u32, u32 node)
+    {
+        const NodeRec r = node_record(g, node);
+        return NodeHead { { r.seq[0], r.seq[1] }, r.meta, r.inNb[0] };
+    }
+    __device__ __forceinline__ const NodeRec* record(const DevGraph& g, u32, u32 node, NodeRec& room) const
+    {
+        if (g.rec) return g.rec + node;
+        gather_record(g, node, room);
+        return &room;
+    }
     __device__ __forceinline__ u32 prev_component(const DevGraph& g, u32, u32 node) const { return g.comp[node]; }
     __device__ __forceinline__ bool prev_linear(const DevGraph& g, u32, u32 node) const { return g.lin[node] != 0; }
 };
@@ -739,50 +749,60 @@ __device__ __forceinline__ int64_t xscore_bound(const WS& w, i32 seqOffset, i32 
 static constexpr i32 kXBoundOffsetLimit = 10000000;
 
 // The part of calculateNodeInner (Common.h:1209-1300) that runs when the node already
-// has a column in this slice: merge the new first column into it.  Returns true when the
-// reference leaves the node early (nothing changed).  Out of line: a node is computed
-// again within a slice only inside cyclic components.
-__device__ __noinline__ bool merge_existing(WS& ws, const Item& slice, bool hasSkipless, bool singleInEdge, u32 lane)
+// has a column in this slice: merge the new first column into it.  leave: the reference leaves
+// the node early (nothing changed).  Out of line: a node is computed again within a slice only
+// inside cyclic components.  (Out of line functions take and return values: a variable handed
+// over by reference stays in local memory wherever it is used, and the walk's and the fill's own
+// variables are read all the time.)
+struct Merged
+{
+    WS ws;
+    bool leave;
+};
+
+__device__ __noinline__ Merged merge_existing(WS ws, const Item& slice, bool hasSkipless, bool singleInEdge, u32 lane)
 {
     WS s = ws_make(slice.sVP, slice.sVN, slice.sEnd);
     if (hasSkipless && singleInEdge)
     {
-        if (ws.end > s.end) return true;
-        if (ws.end < s.end) return false;
+        if (ws.end > s.end) return Merged { ws, true };
+        if (ws.end < s.end) return Merged { ws, false };
         u64 newBigger = (ws.VP & ~s.VP) | (s.VN & ~ws.VN);
         u64 oldBigger = (s.VP & ~ws.VP) | (ws.VN & ~s.VN);
-        if (newBigger > oldBigger) return false;
-        if (oldBigger > newBigger) return true;
-        if (newBigger == 0 && oldBigger == 0) return true;
+        if (newBigger > oldBigger) return Merged { ws, false };
+        if (oldBigger > newBigger) return Merged { ws, true };
+        if (newBigger == 0 && oldBigger == 0) return Merged { ws, true };
         WS t = merge_w(ws, s, lane);
-        if (ws_eq(t, s)) return true;
-        ws = t;
-        return false;
+        return Merged { ws_eq(t, s) ? ws : t, ws_eq(t, s) };
     }
     WS t = merge_w(ws, s, lane);
     // the reference compares test.VP against the stored VN here (Common.h:1282)
-    if (t.end == s.end && t.VP == s.VP && t.VP == s.VN) return true;
-    ws = t;
-    return false;
+    if (t.end == s.end && t.VP == s.VP && t.VP == s.VN) return Merged { ws, true };
+    return Merged { t, false };
 }
 
 // The horizontal input along the slice's first row when the column enters below the
-// previous slice's last row (Common.h:1310-1343): fixedHP/HN and the rows whose first
-// cell is forced.  False where the reference asserts.  Out of line: rarely taken.
-__device__ __noinline__ bool fix_horizontal(i32 scoreBefore, i32 scoreComparison, u64& fixedHP, u64& fixedHN, u64& forceMask)
+// previous slice's last row (Common.h:1310-1343): fixedHP/HN and, for a seed start, the
+// columns whose first row is forced.  ok = false where the reference asserts.  Out of line:
+// rarely taken.
+struct FixedRow
 {
-    forceMask |= 1;
+    u64 HP, HN, force;
+    bool ok;
+};
+
+__device__ __noinline__ FixedRow fix_horizontal(i32 scoreBefore, i32 scoreComparison, u64 fixedHP, u64 fixedHN)
+{
     #pragma unroll 1
     for (int off = 1; off < 64; off++)
     {
         i32 next = scoreComparison + (i32)((fixedHP >> off) & 1) - (i32)((fixedHN >> off) & 1);
         u64 mask = 1ULL << off;
-        if (scoreBefore > next) return false;
+        if (scoreBefore > next) return FixedRow { fixedHP, fixedHN, 0, false };
         if (scoreBefore < next)
         {
             fixedHP |= mask;
             fixedHN &= ~mask;
-            forceMask |= mask;
         }
         else
         {
@@ -793,15 +813,15 @@ __device__ __noinline__ bool fix_horizontal(i32 scoreBefore, i32 scoreComparison
         scoreComparison = next;
         if (scoreBefore >= scoreComparison) break;
     }
-    return true;
+    return FixedRow { fixedHP, fixedHN, 0, true };
 }
 
 // The same when the node is a seed start of the multiseed DP (Common.h:1314-1362): the row
 // above follows the lower of the previous slice's last row and the seed start's score
 // before the slice, and every column of the first row takes its delta from that.
-__device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComparison, i32 extraBefore, u32 nodeLength, u64& fixedHP,
-    u64& fixedHN, u64& forceMask)
+__device__ __noinline__ FixedRow fix_horizontal_extra(i32 scoreBefore, i32 scoreComparison, i32 extraBefore, u32 nodeLength, u64 fixedHP, u64 fixedHN)
 {
+    u64 forceMask = 0;
     scoreBefore = imin(scoreBefore, extraBefore);
     if (scoreBefore < scoreComparison) forceMask |= 1;
     i32 adjust = imin(scoreBefore, scoreComparison);
@@ -813,7 +833,7 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
         const u64 mask = 1ULL << off;
         if (scoreBefore < next) forceMask |= mask;
         const i32 na = imin(next, scoreBefore);
-        if (na < adjust - 1 || na > adjust + 1) return false;
+        if (na < adjust - 1 || na > adjust + 1) return FixedRow { fixedHP, fixedHN, forceMask, false };
         if (na == adjust - 1)
         {
             fixedHN |= mask;
@@ -832,7 +852,7 @@ __device__ __noinline__ bool fix_horizontal_extra(i32 scoreBefore, i32 scoreComp
         adjust = na;
         scoreComparison = next;
     }
-    return true;
+    return FixedRow { fixedHP, fixedHN, forceMask, true };
 }
 
 // calculateNodeInner (Common.h:1113-1478).  nodeLength, c0, c1: the node's length and 2-bit
@@ -949,7 +969,14 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     if (hasExtra) ws = merge_w(ws, *extra, lane);
     const WS wsX = ws;
     // (the recomputation starts from the stored first column, whose merge with itself changes nothing)
-    if (Fill && !forceCalculation && (flags & kExists) != 0 && merge_existing(ws, slice, hasSkipless, singleInPrevBand, lane))
+    bool leave = false;
+    if (Fill && !forceCalculation && (flags & kExists) != 0)
+    {
+        const Merged m = merge_existing(ws, slice, hasSkipless, singleInPrevBand, lane);
+        ws = m.ws;
+        leave = m.leave;
+    }
+    if (leave)
     {
         endColumn = ws_make(slice.eVP, slice.eVN, slice.eEnd);
         if (!boundOk || xscore_bound(wsX, seqOffset, cost) > (int64_t)sliceMaxX)
@@ -965,18 +992,14 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
         i32 scoreBefore = ws_before(ws);
         i32 scoreComparison = prev.sEnd;
         if (scoreBefore > scoreComparison) { err = GA_ASSERT; return result; }
-        if (hasExtra)
+        if (hasExtra || scoreBefore < scoreComparison)
         {
-            if (!fix_horizontal_extra(scoreBefore, scoreComparison, ws_before(*extra), nodeLength, fixedHP, fixedHN, forceMask))
-            {
-                err = GA_ASSERT;
-                return result;
-            }
-        }
-        else if (scoreBefore < scoreComparison && !fix_horizontal(scoreBefore, scoreComparison, fixedHP, fixedHN, forceMask))
-        {
-            err = GA_ASSERT;
-            return result;
+            const FixedRow r = hasExtra ? fix_horizontal_extra(scoreBefore, scoreComparison, ws_before(*extra), nodeLength, fixedHP, fixedHN)
+                : fix_horizontal(scoreBefore, scoreComparison, fixedHP, fixedHN);
+            if (!r.ok) { err = GA_ASSERT; return result; }
+            fixedHP = r.HP;
+            fixedHN = r.HN;
+            forceMask = r.force;
         }
     }
     else
@@ -1529,7 +1552,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
     {
         const u32 i = t.heap()[0].node;
         const u32 slot = t.heap()[0].slot;
-        const NodeRec rec = t.record(g, slot, i);
+        const NodeHead rec = t.head(g, slot, i);
         int at;
         const uint16_t head = t.take(slot, at);
         const bool fresh = at < 0;
@@ -1560,7 +1583,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
             prev.HN = pi.HN;
         }
         // asked for only when a node is computed again
-        const bool singleInPrev = (flags & kExists) && rec_in_degree(rec.meta) == 1 && t.prev_of(rec.inNb[0]) >= 0;
+        const bool singleInPrev = (flags & kExists) && rec_in_degree(rec.meta) == 1 && t.prev_of(rec.inNb) >= 0;
         // a column whose X-score bound is at most both the slice's and the node's best so far
         // changes neither, so the node computation may skip its exact X-score
         const i32 skipBelow = Multi ? imin(res.maxX, nodeMax[at]) : res.maxX;
@@ -1578,19 +1601,22 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
             if (newEndMin == kIntMax) { err = GA_ASSERT; return res; }
             if (newEndMin <= wadd(curMin, bw))
             {
-                const u32 degree = out_degree(g, i, rec);
+                NodeRec room;
+                const NodeRec* r = t.record(g, slot, i, room);
+                u32 degree = rec_out_degree(rec.meta);
+                if (degree >= kRecDegree) degree = g.outOff[i + 1] - r->outOff;
                 #pragma unroll 1
                 for (u32 e = 0; e < degree; e++)
                 {
                     u32 target, component;
                     if (e < kRecOut)
                     {
-                        target = e == 0 ? rec.outNb[0] : e == 1 ? rec.outNb[1] : rec.outNb[2];
-                        component = e == 0 ? rec.outComp[0] : e == 1 ? rec.outComp[1] : rec.outComp[2];
+                        target = r->outNb[e];
+                        component = r->outComp[e];
                     }
                     else
                     {
-                        target = g.outNb[rec.outOff + e];
+                        target = g.outNb[r->outOff + e];
                         component = g.comp[target];
                     }
                     if (!insert(t.slot_of(g, target, component), target, component, newEndMin, newEnd, false, false))
@@ -2374,6 +2400,13 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     u32 word = 0, nbWord = 0;
     u32 meta = 0, inOff = 0, inNb0 = 0xffffffffu, inNb1 = 0xffffffffu;
 
+    auto corner = [&]() -> TStep
+    {
+        int e = 0;
+        const TStep step = bt_corner<Multi>(g, seq, t, curSlice, curNode, ((int64_t)curSlice - 1) * 64, e, extra);
+        if (e) err = e;
+        return step;
+    };
     auto find_cur = [&](u32 node) -> const Item*
     {
         if (!slotCur) return t.template find<Multi>(curSlice, node);
@@ -2408,7 +2441,13 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     auto horizontal = [&](const TPos& p, u32 off) -> TStep
     {
         const i32 here = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)off);
-        if (recCur->notValid || here > recCur->quit) return horizontal_step_invalid<Multi>(g, t, curSlice, curNode, self, p, off, err, extra);
+        if (recCur->notValid || here > recCur->quit)
+        {
+            int x = 0;
+            const TStep step = horizontal_step_invalid<Multi>(g, t, curSlice, curNode, self, p, off, x, extra);
+            if (x) err = x;
+            return step;
+        }
         const i32 diagonal = here - (matches(0, off) ? 0 : 1);
         u32 degree = rec_in_degree(meta);
         if (degree >= kRecDegree) degree = g.inOff[curNode + 1] - inOff;
@@ -2538,7 +2577,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             if (!seeded) lastScore = first + popc64(top.x & columns_upto(b.off)) - popc64(top.y & columns_upto(b.off));
             if (b.off == 0)
             {
-                TStep bt = bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra);
+                TStep bt = corner();
                 if (err) break;
                 if (seeded && tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == xv(mod64(bt.pos.seq))) break;
                 if (seeded && tpos_eq(bt.pos, b) && !bt.sw && nc.value(bt.pos.off, mod64(bt.pos.seq)) == ws_before(extra)) break;
@@ -2558,7 +2597,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             TPos p = b;
             p.off = 63 - (u32)__clzll((long long)(~top.x & (columns_upto(b.off) | 1)));
             TStep second;
-            if (p.off == 0) second = bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra);
+            if (p.off == 0) second = corner();
             else
             {
                 const i32 here = seeded ? nc.value(p.off, 0) : first + popc64(top.x & columns_upto(p.off)) - popc64(top.y & columns_upto(p.off));
@@ -2582,7 +2621,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             const u32 off = 63 - (u32)__clzll((long long)stops);
             p.seq -= (int64_t)(row - off);
             if (!seeded && off == 0) lastScore = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)row);
-            TStep second = off == 0 ? bt_corner<Multi>(g, seq, t, curSlice, curNode, sj, err, extra) : horizontal(p, off);
+            TStep second = off == 0 ? corner() : horizontal(p, off);
             if (err) break;
             if (seeded && second.pos.node == b.node && !second.sw && nc.value(second.pos.off, mod64(second.pos.seq)) == xv(mod64(second.pos.seq))) break;
             if (p.seq != b.seq) to.push_run(TPos { p.node, p.off, b.seq - 1 }, 0, -1, (u32)(b.seq - p.seq));
@@ -2753,7 +2792,12 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
         TPos start = TPos { ec.node, ec.nodeOffset, ec.j + ec.bvOffset };
         i32 startScore = nc.value(ec.nodeOffset, ec.bvOffset);
         err = trace_walk<false>(g, a.cost, seq, seqLen, st.committed, t, to, a.store, start, startScore, resultScore, lane);
-        if (!err && !to.overflow) err = row_above(g, t, to);
+        if (!err && !to.overflow)
+        {
+            TraceOut end = to;
+            err = row_above(g, t, end);
+            to = end;
+        }
     }
     to.finish();
     int status = err ? err : (to.overflow ? GA_CAPACITY : GA_OK);
