@@ -69,8 +69,20 @@ struct NodeVal
     uint16_t tail;
 };
 
+// A fill warp's place in the arena and in the column store, in shared memory: it is asked for
+// once a slice and once a node, and its registers are missed in between
+struct ArenaCursor
+{
+    u64 pos;
+    u64 end;
+    u64 used;           // bytes handed out to this warp since the launch began
+    u32 unit;           // this warp's units of the column store
+    u32 unitEnd;
+    u32 storeFull;
+};
+
 // A warp's recorded columns of one node-slice, in shared memory in every kernel: the fills' dynamic
-// shared memory starts with one of these per warp of the block.
+// shared memory starts with a FillWarp per warp of the block.
 struct __align__(16) NodeCols
 {
     // what the column loop writes
@@ -83,14 +95,21 @@ struct __align__(16) NodeCols
         i32 end;        // score of the last row
         u32 pad;
     } x[64];
+    u64 base[4];        // the slice's match masks, one per base
     u64 eqcol[64 + 2];  // match mask of each column with its horizontal -1 input; [64] is read ahead of the last column
 
     __device__ __forceinline__ WS column(u32 k) const { return ws_make(v[k].VP, v[k].VN, x[k].end); }
     __device__ __forceinline__ i32 value(u32 k, u32 row) const { return ws_value(column(k), (int)row); }
 };
+struct __align__(16) FillWarp
+{
+    NodeCols cols;
+    ArenaCursor arena;
+};
 extern __shared__ __align__(16) uint8_t dsmem[];
 
-__device__ __forceinline__ NodeCols& fill_cols() { return ((NodeCols*)dsmem)[threadIdx.x >> 5]; }
+__device__ __forceinline__ FillWarp& fill_warp() { return ((FillWarp*)dsmem)[threadIdx.x >> 5]; }
+__device__ __forceinline__ NodeCols& fill_cols() { return fill_warp().cols; }
 
 __device__ __forceinline__ u32 hash_node(u32 node)
 {
@@ -267,7 +286,7 @@ struct SmallSpace
 
 __device__ __forceinline__ SmallSpace& small_space()
 {
-    return ((SmallSpace*)(dsmem + (blockDim.x >> 5) * sizeof(NodeCols)))[threadIdx.x >> 5];
+    return ((SmallSpace*)(dsmem + (blockDim.x >> 5) * sizeof(FillWarp)))[threadIdx.x >> 5];
 }
 
 // The tables of a warp whose bands hold at most 32 nodes: slot k of the node table is lane k's
@@ -594,8 +613,8 @@ __device__ __forceinline__ RowBytes row_bytes(const uint8_t* seq, u32 len, int64
 
 // Match masks of 64 rows (getEqVector, Common.h:279-318): the masks come from ballots.  False
 // when a row holds a non-sequence byte, or a gap inside a full 64-row window (the reference
-// asserts).
-__device__ __forceinline__ bool eq_of_rows(const RowBytes& r, EqV4& eq)
+// asserts).  eq: NodeCols::base.
+__device__ __forceinline__ bool eq_of_rows(const RowBytes& r, u64* eq)
 {
     const bool full = __ballot_sync(kFull, r.hi < 0) == 0;
     int m0 = 0, m1 = 0;
@@ -610,16 +629,18 @@ __device__ __forceinline__ bool eq_of_rows(const RowBytes& r, EqV4& eq)
         m1 = s_iupac[r.hi];
         bad |= m1 < 0 || (m1 == 0 && full);
     }
-    eq.a = (u64)__ballot_sync(kFull, m0 & 1) | ((u64)__ballot_sync(kFull, m1 & 1) << 32);
-    eq.c = (u64)__ballot_sync(kFull, m0 & 2) | ((u64)__ballot_sync(kFull, m1 & 2) << 32);
-    eq.g = (u64)__ballot_sync(kFull, m0 & 4) | ((u64)__ballot_sync(kFull, m1 & 4) << 32);
-    eq.t = (u64)__ballot_sync(kFull, m0 & 8) | ((u64)__ballot_sync(kFull, m1 & 8) << 32);
-    return __ballot_sync(kFull, bad) == 0;
-}
-
-__device__ __noinline__ bool eq_vector(const uint8_t* seq, u32 len, int64_t j, EqV4& eq, u32 lane)
-{
-    return eq_of_rows(row_bytes(seq, len, j, lane), eq);
+    const u64 e0 = (u64)__ballot_sync(kFull, m0 & 1) | ((u64)__ballot_sync(kFull, m1 & 1) << 32);
+    const u64 e1 = (u64)__ballot_sync(kFull, m0 & 2) | ((u64)__ballot_sync(kFull, m1 & 2) << 32);
+    const u64 e2 = (u64)__ballot_sync(kFull, m0 & 4) | ((u64)__ballot_sync(kFull, m1 & 4) << 32);
+    const u64 e3 = (u64)__ballot_sync(kFull, m0 & 8) | ((u64)__ballot_sync(kFull, m1 & 8) << 32);
+    __syncwarp();
+    eq[0] = e0;
+    eq[1] = e1;
+    eq[2] = e2;
+    eq[3] = e3;
+    const bool ok = __ballot_sync(kFull, bad) == 0;
+    __syncwarp();
+    return ok;
 }
 
 // graph character of node n at pos (AlignmentGraph::NodeSequences) as an IUPAC mask
@@ -884,7 +905,7 @@ __device__ __noinline__ FixedRow fix_horizontal_extra(i32 scoreBefore, i32 score
 // 10 kbp read 13 % less.
 template <bool Fill, bool Multi = false>
 __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i, u32 nodeLength, u64 c0, u64 c1, Item& slice, u32 flags,
-    const EqV4& eqv, const PrevInfo& prev, const Extra* pool, uint16_t head, uint16_t nil, const WS* singleIncoming, bool singleInPrevBand,
+    const PrevInfo& prev, const Extra* pool, uint16_t head, uint16_t nil, const WS* singleIncoming, bool singleInPrevBand,
     i32 seqOffset, WS& endColumn, ColumnUnit* kept, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
 {
     NodeCols& nc = Fill ? fill_cols() : trace_cols();
@@ -908,8 +929,8 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     }
     auto mask_at = [&](u32 pos) -> u64
     {
-        if (!amb) return eq_pick(eqv, (u32)(((pos < 32 ? c0 : c1) >> ((pos & 31) * 2)) & 3));
-        return eq_amb(eqv, (u32)(((a0 >> pos) & 1) | (((a1 >> pos) & 1) << 1) | (((a2 >> pos) & 1) << 2) | (((a3 >> pos) & 1) << 3)));
+        if (!amb) return nc.base[((pos < 32 ? c0 : c1) >> ((pos & 31) * 2)) & 3];
+        return eq_amb(EqV4 { nc.base[0], nc.base[1], nc.base[2], nc.base[3] }, (u32)(((a0 >> pos) & 1) | (((a1 >> pos) & 1) << 1) | (((a2 >> pos) & 1) << 2) | (((a3 >> pos) & 1) << 3)));
     };
     const u64 eq0 = mask_at(0);
 
@@ -1195,32 +1216,13 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
 
 // ---------------------------------------------------------------- arena
 
-struct ArenaCursor
-{
-    u64 pos;
-    u64 end;
-    u64 used;           // bytes handed out to this warp since the launch began
-    u32 unit;           // this warp's units of the column store
-    u32 unitEnd;
-    bool storeFull;
-};
-
-__device__ __forceinline__ ArenaCursor arena_cursor(const FillArgs& a)
-{
-    ArenaCursor c;
-    c.pos = 0;
-    c.end = 0;
-    c.used = 0;
-    c.unit = 0;
-    c.unitEnd = 0;
-    c.storeFull = a.store == nullptr;
-    return c;
-}
-
+// (the cursor is every lane's: each one has read it before any of them moves it)
 // `columns` units of the column store, or kNoColumns
 __device__ __forceinline__ u32 store_alloc(const FillArgs& a, ArenaCursor& c, u32 columns, u32 lane)
 {
-    if (c.unitEnd - c.unit < columns)
+    u32 at = c.unit;
+    const u32 end = c.unitEnd;
+    if (end - at < columns)
     {
         if (c.storeFull) return kNoColumns;
         unsigned long long p = 0;
@@ -1228,14 +1230,16 @@ __device__ __forceinline__ u32 store_alloc(const FillArgs& a, ArenaCursor& c, u3
         p = __shfl_sync(kFull, p, 0);
         if (p + kStoreChunk > a.storeUnits)
         {
-            c.storeFull = true;
+            c.storeFull = 1;
+            __syncwarp();
             return kNoColumns;
         }
-        c.unit = (u32)p;
+        at = (u32)p;
         c.unitEnd = (u32)p + kStoreChunk;
     }
-    const u32 at = c.unit;
-    c.unit += columns;
+    __syncwarp();
+    c.unit = at + columns;
+    __syncwarp();
     return at;
 }
 
@@ -1243,19 +1247,23 @@ __device__ __forceinline__ u32 store_alloc(const FillArgs& a, ArenaCursor& c, u3
 __device__ __forceinline__ bool arena_alloc(const FillArgs& a, ArenaCursor& c, u64 bytes, u64& out, u32 lane)
 {
     bytes = align16(bytes);
-    if (c.pos + bytes > c.end)
+    u64 at = c.pos;
+    const u64 end = c.end, used = c.used;
+    if (at + bytes > end)
     {
         const u64 grab = bytes > a.chunkBytes ? bytes : a.chunkBytes;
         unsigned long long p = 0;
         if (lane == 0) p = atomicAdd(a.arenaCursor, (unsigned long long)grab);
         p = __shfl_sync(kFull, p, 0);
         if (p + grab > a.arenaBytes) return false;
-        c.pos = p;
+        at = p;
         c.end = p + grab;
     }
-    out = c.pos;
-    c.pos += bytes;
-    c.used += bytes;
+    __syncwarp();
+    out = at;
+    c.pos = at + bytes;
+    c.used = used + bytes;
+    __syncwarp();
     return true;
 }
 
@@ -1466,8 +1474,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
     res.maxX = kIntMin;
     res.maxXNode = 0;
     res.cells = 0;
-    EqV4 eqv;
-    if (!eq_of_rows(rows, eqv)) { err = GA_ASSERT; return res; }
+    if (!eq_of_rows(rows, fill_cols().base)) { err = GA_ASSERT; return res; }
     rows = row_bytes(seq, seqLen, j + 64, lane);
 
     auto insert = [&](int slot, u32 node, u32 component, i32 score, const WS& c, bool skip, bool force) -> bool
@@ -1588,7 +1595,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
         // changes neither, so the node computation may skip its exact X-score
         const i32 skipBelow = Multi ? imin(res.maxX, nodeMax[at]) : res.maxX;
         WS newEnd;
-        const NodeCalc nc = node_calc<true, Multi>(g, a.cost, i, rec_len(rec.meta), rec.seq[0], rec.seq[1], thisNode, flags, eqv, prev, t.extras(), head,
+        const NodeCalc nc = node_calc<true, Multi>(g, a.cost, i, rec_len(rec.meta), rec.seq[0], rec.seq[1], thisNode, flags, prev, t.extras(), head,
             nil, nullptr, singleInPrev, seqOffset, newEnd, columnsAt == kNoColumns ? nullptr : a.store + columnsAt, steps, err, lane, skipBelow, 63, extra);
         if (err) return res;
         if (Multi) nodeMax[at] = imax(nc.maxX, nodeMax[at]);
@@ -2091,12 +2098,18 @@ __device__ __noinline__ TStep bt_corner(const DevGraph& g, const uint8_t* seq, T
     return out;
 }
 
-// recalcNodeWordslice (Common.h:1078-1102): the columns 0..lastColumn of one node-slice
+// The match masks of slice s into the warp's columns
+__device__ __forceinline__ bool slice_masks(const uint8_t* seq, u32 seqLen, u32 s, u32 lane)
+{
+    return eq_of_rows(row_bytes(seq, seqLen, ((int64_t)s - 1) * 64, lane), trace_cols().base);
+}
+
+// recalcNodeWordslice (Common.h:1078-1102), after slice_masks: the columns 0..lastColumn of one node-slice
 // into cols (the traceback only moves left inside a node, so it never needs the columns
 // after the one it enters at).  When every column is recomputed the last one must equal
 // the stored end column, as the reference asserts.  Returns 0 or the error status.
 template <bool Multi = false>
-__device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, u32 node, const EqV4& eqv, u32 lane, u32 lastColumn,
+__device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, u32 node, u32 lane, u32 lastColumn,
     WS extra = fake_ws())
 {
     const Item* it = t.template find<Multi>(s, node);
@@ -2113,7 +2126,7 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
     int64_t j = ((int64_t)s - 1) * 64;
     const NodeRec rec = node_record(g, node);
     const u32 L = rec_len(rec.meta);
-    node_calc<false, Multi>(g, cost, node, L, rec.seq[0], rec.seq[1], copy, it->node, eqv, prev, nullptr, kNil, kNil, &start, false, (i32)j, last,
+    node_calc<false, Multi>(g, cost, node, L, rec.seq[0], rec.seq[1], copy, it->node, prev, nullptr, kNil, kNil, &start, false, (i32)j, last,
         nullptr, steps, err, lane, kIntMin, lastColumn, (Multi && extra.end != kIntMax) ? &extra : nullptr);
     if (err) return err;
     const NodeCols& nc = trace_cols();
@@ -2226,9 +2239,8 @@ __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint
     ec.score = br->maxX;
     ec.j = ((int64_t)best - 1) * 64;
     const int64_t j = ec.j;
-    EqV4 eqv;
-    if (!eq_vector(seq, seqLen, j, eqv, lane)) { ec.err = GA_ASSERT; return ec; }
-    ec.err = recalc(g, cost, t, best, ec.node, eqv, lane, 63);
+    if (!slice_masks(seq, seqLen, best, lane)) { ec.err = GA_ASSERT; return ec; }
+    ec.err = recalc(g, cost, t, best, ec.node, lane, 63);
     if (ec.err) return ec;
     const int cells = (int)((int64_t)seqLen - j < 64 ? (int64_t)seqLen - j : 64);
     const u32 L = g.len[ec.node];
@@ -2318,9 +2330,8 @@ template <bool Multi>
 __device__ __noinline__ int recompute(const DevGraph& g, i32 cost, Table t, const uint8_t* seq, u32 seqLen, u32 s, u32 node, u32 off, WS extra, u32 lane)
 {
     ColumnUnit* const out = trace_warp().columns;
-    EqV4 eqv;
-    if (!eq_vector(seq, seqLen, ((int64_t)s - 1) * 64, eqv, lane)) return GA_ASSERT;
-    const int err = recalc<Multi>(g, cost, t, s, node, eqv, lane, off, extra);
+    if (!slice_masks(seq, seqLen, s, lane)) return GA_ASSERT;
+    const int err = recalc<Multi>(g, cost, t, s, node, lane, off, extra);
     if (err) return err;
     const NodeCols& nc = trace_cols();
     i32 v[2];
@@ -2923,10 +2934,9 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const uint8_t* s
     const Item* items = rec_items(cr);
     const u32 node = items[c.index].node & kNodeMask;
     const int64_t j = ((int64_t)c.slice - 1) * 64;
-    EqV4 eqv;
-    if (!eq_vector(seq, seqLen, j, eqv, lane)) return GA_ASSERT;
+    if (!slice_masks(seq, seqLen, c.slice, lane)) return GA_ASSERT;
     const WS extra = (items[c.index].node & kSeedStart) ? seed_ws(j, seqLen, a.cost) : fake_ws();
-    int err = recalc<true>(g, a.cost, t, c.slice, node, eqv, lane, 63, extra);
+    int err = recalc<true>(g, a.cost, t, c.slice, node, lane, 63, extra);
     if (err) return err;
     const NodeCols& nc = trace_cols();
     const i32 score = c.score;
@@ -3190,7 +3200,9 @@ __device__ __forceinline__ void fill_extensions(const FillArgs& fa, u32* counter
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
     Tables t(fa, (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane);
-    ArenaCursor arena = arena_cursor(fa);
+    ArenaCursor& arena = fill_warp().arena;
+    arena = { 0, 0, 0, 0, 0, fa.store == nullptr ? 1u : 0u };
+    __syncwarp();
     u32 ext;
 #pragma unroll 1
     while (next_extension(counter, fa.num, fa.order, fa.prevStatus, lane, ext))
@@ -3230,7 +3242,9 @@ __global__ void __launch_bounds__(128, 4) fill_multiseed_kernel(const __grid_con
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
     LargeTables t(fa, (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane);
-    ArenaCursor arena = arena_cursor(fa);
+    ArenaCursor& arena = fill_warp().arena;
+    arena = { 0, 0, 0, 0, 0, fa.store == nullptr ? 1u : 0u };
+    __syncwarp();
     u32 r;
 #pragma unroll 1
     while (next_extension(counter, fa.num, fa.order, fa.prevStatus, lane, r))
@@ -3311,7 +3325,7 @@ __global__ void __launch_bounds__(128, 4) ms_trace_kernel(const __grid_constant_
 
 // dynamic shared memory of a block of the fill kernels (shared: with its frontier tables) and of
 // the traceback kernels
-static size_t fill_smem(int warpsPerBlock, bool shared) { return (sizeof(gadev::NodeCols) + (shared ? sizeof(gadev::SmallSpace) : 0)) * warpsPerBlock; }
+static size_t fill_smem(int warpsPerBlock, bool shared) { return (sizeof(gadev::FillWarp) + (shared ? sizeof(gadev::SmallSpace) : 0)) * warpsPerBlock; }
 static size_t trace_smem(int warpsPerBlock) { return sizeof(gadev::TraceWarp) * warpsPerBlock; }
 
 uint64_t ga_warp_tables_bytes(const gadev::Caps& c) { return gadev::wspace_bytes(c); }
