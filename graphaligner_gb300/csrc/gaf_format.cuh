@@ -1,6 +1,7 @@
 // GAF line formatting (GraphAlignerGAFAlignment::traceToAlignment, GraphAlignerGAFAlignment.h:37-200),
-// host- and device-callable: the device formats every selected alignment of a batch, one thread
-// per line, and the host tests check the number formatting against std::ostream.
+// host- and device-callable: the device formats every selected alignment of a batch (a warp per
+// line with these numbers, gaf_device.cu; write_line is the same line by one thread, for the host),
+// and the host tests check the number formatting against std::ostream.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -464,7 +465,7 @@ GAF_HD inline bool classify_line(GetItem item, uint32_t count, uint32_t readLen,
 
 // Writes one classified GAF line (no newline) to out, or only measures it when out is null;
 // returns its length.
-GAF_HD inline int64_t write_line(const Names& nm, const LineMeta& m, const uint8_t* ops, const int32_t* entries, char* out)
+inline int64_t write_line(const Names& nm, const LineMeta& m, const uint8_t* ops, const int32_t* entries, char* out)
 {
     const char codes[5] = { '=', 'X', 'M', 'I', 'D' };
     int64_t n = 0;
