@@ -169,6 +169,7 @@ struct ga_extender
     DevBuf<uint32_t> seqLen, startNode, startOffset, traceCap, traceLen, order;
     DevBuf<int32_t> status, score, prevStatus;
     DevBuf<gadev::ExtState> states;        // where the fill left each extension's table
+    DevBuf<gadev::ResumeRec> resume;       // extensions handed on from the small tables to the medium ones
     // multiseed DP staging
     DevBuf<uint64_t> msSeedOff, msTraceCap, msTraceStart, msItemsNeeded;
     DevBuf<uint32_t> msSeedSlice, msSeedNode, msNumTraces, msTraceLen, msTracesNeeded;
@@ -298,6 +299,10 @@ static gadev::Caps layout_caps(int layout)
     return c;
 }
 
+// Extensions that one call hands on from the small tables to the medium ones (2 KB each); more
+// start again in the next layout
+static constexpr uint32_t kResumeCap = 8192;
+
 static const char* kShapeError = "launch shape: warps_per_block within 1..4, first_layout within 0..2, chunk_kib within 1..2^20";
 
 extern "C" int ga_extender_create(ga_graph_t graph, uint64_t arena_bytes, ga_extender_t* out)
@@ -351,7 +356,7 @@ extern "C" int ga_extender_free(ga_extender_t x)
     cudaFree(x->store);
     x->seq.release(); x->seqOff.release(); x->traceOff.release(); x->traceItems.release(); x->cellSteps.release();
     x->seqLen.release(); x->startNode.release(); x->startOffset.release(); x->traceCap.release(); x->traceLen.release();
-    x->order.release(); x->status.release(); x->score.release(); x->prevStatus.release(); x->states.release();
+    x->order.release(); x->status.release(); x->score.release(); x->prevStatus.release(); x->states.release(); x->resume.release();
     x->msSeedOff.release(); x->msTraceCap.release(); x->msTraceStart.release(); x->msItemsNeeded.release();
     x->msSeedSlice.release(); x->msSeedNode.release(); x->msNumTraces.release(); x->msTraceLen.release(); x->msTracesNeeded.release();
     x->msTraceScore.release(); x->msCandBegin.release(); x->msCandCount.release(); x->msCands.release();
@@ -435,6 +440,8 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
     const uint32_t n = b->num;
     GA_CUDA(x->states.reserve(n));
     fa.states = x->states.ptr;
+    const uint32_t resumeCap = std::min<uint32_t>(n, kResumeCap);
+    GA_CUDA(x->resume.reserve(resumeCap));
     ta.num = n;
     ta.order = order;
     ta.states = x->states.ptr;
@@ -455,7 +462,9 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
         const bool shared = layout == 0;
         const gadev::Caps caps = layout_caps(layout);
         const uint64_t stride = ga_warp_tables_bytes(caps);
-        int fillPerSm = ga_fill_blocks_per_sm(wpb, shared);
+        const gadev::FillTables tables = shared ? gadev::FillTables::Small : gadev::FillTables::Global;
+        int fillPerSm = ga_fill_blocks_per_sm(wpb, tables);
+        const int mediumPerSm = shared ? ga_fill_blocks_per_sm(1, gadev::FillTables::Medium) : 0;
         int tracePerSm = ga_trace_blocks_per_sm(wpb);
         if (fillPerSm <= 0 || tracePerSm <= 0) return fail(GA_ERR_CUDA, "the extension kernels do not fit an SM with this launch shape");
         if (sh.blocks_per_sm > 0)
@@ -473,26 +482,33 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
             GA_CUDA(cudaMemcpyAsync(prevStatus, r->status, (size_t)n * 4, cudaMemcpyDeviceToDevice, stream));
         }
         fa.caps = caps;
+        fa.tables = tables;
         fa.workspace = shared ? nullptr : x->workspace;
         fa.workspaceStride = stride;
+        fa.resume = mediumPerSm > 0 ? x->resume.ptr : nullptr;
+        fa.resumeCap = resumeCap;
+        fa.resumeCount = x->counters + 4;
         fa.prevStatus = layout > (int)sh.first_layout ? prevStatus : nullptr;
         ta.prevStatus = fa.prevStatus;
         GA_CUDA(cudaMemsetAsync(x->counters, 0, 16 * sizeof(uint32_t), stream));
         GA_CUDA(cudaMemsetAsync(x->arenaCursor, 0, 3 * sizeof(unsigned long long), stream));
         GA_CUDA(cudaEventRecord(x->ev[0], stream));
-        if (ga_launch_extend(fa, ta, x->counters, (int)fillBlocks, (int)traceBlocks, wpb, stream) != 0)
+        if (ga_launch_extend(fa, ta, x->counters, (int)fillBlocks, (int)std::min<uint64_t>((uint64_t)x->sms * mediumPerSm, resumeCap),
+                (int)traceBlocks, wpb, stream) != 0)
             return fail(GA_ERR_CUDA, std::string("extension kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
-        x->lastLaunches += 2;
-        x->lastRounds[layout] = pending;
+        x->lastLaunches += fa.resume ? 3 : 2;
+        x->lastRounds[layout] += pending;
         GA_CUDA(cudaEventRecord(x->ev[1], stream));
         count_status_kernel<<<64, 256, 0, stream>>>(r->status, n, GA_CAPACITY, x->counters + 2);
         GA_CUDA(cudaGetLastError());
         x->lastLaunches += 1;
-        uint32_t capFails = 0;
+        uint32_t counts[3] = {0, 0, 0};          // capacity failures, -, extensions handed on
         unsigned long long used[2] = {0, 0};
-        GA_CUDA(cudaMemcpyAsync(&capFails, x->counters + 2, 4, cudaMemcpyDeviceToHost, stream));
+        GA_CUDA(cudaMemcpyAsync(counts, x->counters + 2, 12, cudaMemcpyDeviceToHost, stream));
         GA_CUDA(cudaMemcpyAsync(used, x->arenaCursor, 16, cudaMemcpyDeviceToHost, stream));
         GA_CUDA(cudaStreamSynchronize(stream));
+        const uint32_t capFails = counts[0];
+        if (layout == 0) x->lastRounds[1] += std::min(counts[2], resumeCap);
         if (layout == (int)sh.first_layout) x->lastArenaBytes = used[1];
         float ms = 0;
         GA_CUDA(cudaEventElapsedTime(&ms, x->ev[0], x->ev[1]));

@@ -297,6 +297,7 @@ __device__ __forceinline__ SmallSpace& small_space()
 // read 8 % less, 1,000 tangled extensions of 20 kbp reads 14 % less.
 struct SmallTables
 {
+    static constexpr bool kSmall = true;
     static constexpr uint16_t kNoExtra = 0xff;
     static constexpr u32 kFresh = 0x00ffffffu;     // bits 0-7 band, 8-15 first and 16-23 last pending column (0xff: none), 24 queued
     static constexpr u32 kQueued = 1u << 24;
@@ -423,9 +424,12 @@ struct SmallTables
     __device__ __forceinline__ bool prev_linear(const DevGraph&, u32 k, u32) const { return __shfl_sync(kFull, (int)prevLinear, (int)k) != 0; }
 };
 
-// The tables in global memory: a hash table with generation stamps.
-struct LargeTables
+// Larger tables, a hash table with generation stamps: in global memory, or (Shared) in the block's
+// shared memory for the extensions that outgrow the tables above.
+template <bool Shared>
+struct HashTables
 {
+    static constexpr bool kSmall = false;
     static constexpr uint16_t kNoExtra = kNil;
     WSpace w;
     Caps caps;
@@ -433,7 +437,12 @@ struct LargeTables
     u32 gen, prevGen;
     u32 used, heapN, poolN, count, prevCount, side;
 
-    __device__ __forceinline__ LargeTables(const FillArgs& a, u64 gwarp, u32 lane_) : w(wspace_at(a.workspace + gwarp * a.workspaceStride, a.caps)),
+    __device__ __forceinline__ static uint8_t* place(const FillArgs& a, u64 gwarp)
+    {
+        if (Shared) return dsmem + (blockDim.x >> 5) * sizeof(FillWarp) + (u64)(threadIdx.x >> 5) * a.workspaceStride;
+        return a.workspace + gwarp * a.workspaceStride;
+    }
+    __device__ __forceinline__ HashTables(const FillArgs& a, u64 gwarp, u32 lane_) : w(wspace_at(place(a, gwarp), a.caps)),
         caps(a.caps), lane(lane_), gen(0), prevGen(0), used(0), heapN(0), poolN(0), count(0), prevCount(0), side(0)
     {
         clear();
@@ -538,6 +547,9 @@ struct LargeTables
     __device__ __forceinline__ u32 prev_component(const DevGraph& g, u32, u32 node) const { return g.comp[node]; }
     __device__ __forceinline__ bool prev_linear(const DevGraph& g, u32, u32 node) const { return g.lin[node] != 0; }
 };
+
+using LargeTables = HashTables<false>;
+using MediumTables = HashTables<true>;
 
 // ---- the traceback's shared memory ----
 
@@ -956,7 +968,7 @@ __device__ __noinline__ FixedRow fix_horizontal_extra(i32 scoreBefore, i32 score
 template <bool Fill, bool Multi = false>
 __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i, u32 nodeLength, u64 c0, u64 c1, Item& slice, u32 flags,
     const PrevInfo& prev, const Extra* pool, uint16_t head, uint16_t nil, const WS* singleIncoming, bool singleInPrevBand,
-    i32 seqOffset, WS& endColumn, ColumnUnit* kept, u64& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
+    i32 seqOffset, WS& endColumn, ColumnUnit* kept, u32& steps, int& err, u32 lane, i32 sliceMaxX = kIntMin, u32 lastColumn = 63, const WS* extra = nullptr)
 {
     NodeCols& nc = Fill ? fill_cols() : trace_cols();
     u64* const eqcol = nc.eqcol;
@@ -1502,7 +1514,7 @@ struct SliceSeeds
 // rows: the slice's read bytes on entry, the next slice's on return (loaded while this one runs).
 template <class Tables, bool Multi = false>
 __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, ArenaCursor& arena, const uint8_t* seq, u32 seqLen, RowBytes& rows,
-    int64_t j, i32 prevQuit, i32 prevMin, u64& steps, int& err, u32 lane, const SliceSeeds* seeds = nullptr)
+    int64_t j, i32 prevQuit, i32 prevMin, u32& steps, int& err, u32 lane, const SliceSeeds* seeds = nullptr)
 {
     if (Multi)
     {
@@ -1708,6 +1720,71 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
     return res;
 }
 
+// Writes down an extension for the medium tables, if there is room.  Out of line: rare, and the
+// fill's registers are full.
+__device__ __noinline__ void hand_on(ResumeRec* resume, u32 cap, u32* count, const Item* prevBand, u32 prevCount, FillState f, u32 ext, u32 lane)
+{
+    u32 k = 0;
+    if (lane == 0) k = atomicAdd(count, 1u);
+    k = __shfl_sync(kFull, k, 0);
+    if (k >= cap) return;
+    ResumeRec& rec = resume[k];
+    #pragma unroll 1
+    for (u32 q = lane; q < prevCount * 4; q += 32) ((uint4*)rec.band)[q] = ((const uint4*)prevBand)[q];
+    if (lane == 0)
+    {
+        rec.state = f;
+        rec.ext = ext;
+        rec.count = prevCount;
+    }
+}
+
+// The slices of an extension from f.slice on.  With the small tables, an extension that outgrows
+// them at a slice is handed on to the medium ones while there is room for it.
+template <class Tables>
+__device__ __forceinline__ ExtState fill_slices(const FillArgs& a, Tables& t, ArenaCursor& arena, u32 ext, FillState& f, u32 lane)
+{
+    const uint8_t* seq = a.seq + a.seqOff[ext];
+    const u32 seqLen = a.seqLen[ext];
+    const u32 numSlices = (seqLen + 63) / 64;
+    u64* dir = (u64*)(a.arena + f.dir);
+    int err = 0;
+    RowBytes rows = row_bytes(seq, seqLen, (int64_t)f.slice * 64, lane);
+    #pragma unroll 1
+    for (; f.slice < numSlices; f.slice++)
+    {
+        const int64_t j = (int64_t)f.slice * 64;
+        u32 steps = 0;
+        SliceResult r = fill_slice(a, t, arena, seq, seqLen, rows, j, f.lastQuit, f.lastMin, steps, err, lane);
+        if (Tables::kSmall && err == GA_CAPACITY && a.resume)
+        {
+            hand_on(a.resume, a.resumeCap, a.resumeCount, t.prev_band(), t.prevCount, f, ext, lane);
+        }
+        f.steps += steps;
+        if (err) break;
+        if (r.maxX > f.bestX) f.bestX = r.maxX;
+        const bool notValid = r.cells >= a.maxCells;
+        if ((int64_t)r.maxX < (int64_t)f.bestX - (int64_t)a.xdrop) break;
+        if (r.minScore < f.lastMin) { err = GA_ASSERT; break; }
+        const i32 quit = wadd(r.minScore, (i32)a.bandwidth);
+        if (!commit_slice(a, arena, dir, f.committed, t, r.minScore, quit, r.maxX, r.maxXNode, notValid, lane))
+        {
+            err = GA_CAPACITY;
+            break;
+        }
+        f.committed++;
+        f.lastMin = r.minScore;
+        f.lastQuit = quit;
+    }
+    ExtState st;
+    st.dir = f.dir;
+    st.committed = f.committed;
+    st.status = err ? err : f.committed <= 1 ? GA_TRACE_FAILED : GA_OK;
+    st.steps = f.steps;
+    st.aux = 0;
+    return st;
+}
+
 template <class Tables>
 __device__ __forceinline__ ExtState fill_extension(const FillArgs& a, Tables& t, ArenaCursor& arena, u32 ext, u32 lane)
 {
@@ -1718,12 +1795,10 @@ __device__ __forceinline__ ExtState fill_extension(const FillArgs& a, Tables& t,
     st.status = GA_OK;
     st.steps = 0;
     st.aux = 0;
-    const uint8_t* seq = a.seq + a.seqOff[ext];
     const u32 seqLen = a.seqLen[ext];
     const u32 startNode = a.startNode[ext];
     const u32 startOff = a.startOffset[ext];
     const u32 numSlices = (seqLen + 63) / 64;
-    int err = 0;
     if (startNode >= g.N || startOff >= g.len[startNode])
     {
         st.status = GA_BAD_REQUEST;
@@ -1737,7 +1812,6 @@ __device__ __forceinline__ ExtState fill_extension(const FillArgs& a, Tables& t,
     }
     u64* dir = (u64*)(a.arena + dirOff);
     st.dir = dirOff;
-    RowBytes rows = row_bytes(seq, seqLen, 0, lane);
     // start slice (getInitialSliceExactPosition, Common.h:1551-1587): one node, scores = distance from the offset
     t.restart();
     t.next();
@@ -1762,34 +1836,15 @@ __device__ __forceinline__ ExtState fill_extension(const FillArgs& a, Tables& t,
             return st;
         }
     }
-    u32 committed = 1;
-    i32 bestX = 0;
-    i32 lastMin = 0;
-    i32 lastQuit = 1;
-    #pragma unroll 1
-    for (u32 s = 0; s < numSlices; s++)
-    {
-        const int64_t j = (int64_t)s * 64;
-        SliceResult r = fill_slice(a, t, arena, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane);
-        if (err) break;
-        if (r.maxX > bestX) bestX = r.maxX;
-        const bool notValid = r.cells >= a.maxCells;
-        if ((int64_t)r.maxX < (int64_t)bestX - (int64_t)a.xdrop) break;
-        if (r.minScore < lastMin) { err = GA_ASSERT; break; }
-        const i32 quit = wadd(r.minScore, (i32)a.bandwidth);
-        if (!commit_slice(a, arena, dir, committed, t, r.minScore, quit, r.maxX, r.maxXNode, notValid, lane))
-        {
-            err = GA_CAPACITY;
-            break;
-        }
-        committed++;
-        lastMin = r.minScore;
-        lastQuit = quit;
-    }
-    st.committed = committed;
-    if (err) st.status = err;
-    else if (committed <= 1) st.status = GA_TRACE_FAILED;
-    return st;
+    FillState f;
+    f.dir = dirOff;
+    f.steps = 0;
+    f.slice = 0;
+    f.committed = 1;
+    f.bestX = 0;
+    f.lastMin = 0;
+    f.lastQuit = 1;
+    return fill_slices(a, t, arena, ext, f, lane);
 }
 
 // GraphAlignerBitvectorBanded::getMultiseedSlices (GraphAlignerBitvectorBanded.h:727-822): every
@@ -1845,7 +1900,9 @@ __device__ ExtState fill_multiseed(const FillArgs& a, LargeTables& t, ArenaCurso
         seeds.count = (u32)(next - k);
         seeds.ws = seed_ws(j, seqLen, a.cost);
         k = next;
-        SliceResult res = fill_slice<LargeTables, true>(a, t, arena, seq, seqLen, rows, j, lastQuit, lastMin, st.steps, err, lane, &seeds);
+        u32 steps = 0;
+        SliceResult res = fill_slice<LargeTables, true>(a, t, arena, seq, seqLen, rows, j, lastQuit, lastMin, steps, err, lane, &seeds);
+        st.steps += steps;
         if (err) break;
         // fillDPSlice's checks of a slice that started seeds (GraphAlignerBitvectorBanded.h:543-549)
         if (seeds.count > 0)
@@ -2177,7 +2234,7 @@ __device__ __noinline__ int recalc(const DevGraph& g, i32 cost, Table t, u32 s, 
     Item copy;
     WS start = ws_make(it->sVP, it->sVN, it->sEnd);
     WS last;
-    u64 steps = 0;
+    u32 steps = 0;
     int err = 0;
     int64_t j = ((int64_t)s - 1) * 64;
     const NodeRec rec = node_record(g, node);
@@ -3271,6 +3328,40 @@ __device__ __forceinline__ void fill_extensions(const FillArgs& fa, u32* counter
 }
 
 __global__ void __launch_bounds__(128, 4) fill_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<SmallTables>(fa, counter); }
+
+// The extensions that the fill above handed on, each from the slice it stopped at.
+__global__ void __launch_bounds__(128, 1) fill_medium_kernel(const __grid_constant__ FillArgs fa, u32* counter)
+{
+    load_iupac_table();
+    const u32 lane = threadIdx.x & 31;
+    const u32 handed = fa.resumeCount[0] < fa.resumeCap ? fa.resumeCount[0] : fa.resumeCap;
+    if (handed == 0) return;
+    MediumTables t(fa, 0, lane);
+    ArenaCursor& arena = fill_warp().arena;
+    arena = { 0, 0, 0, 0, 0, fa.store == nullptr ? 1u : 0u };
+    __syncwarp();
+    u32 k;
+#pragma unroll 1
+    while (next_extension(counter, handed, nullptr, nullptr, lane, k))
+    {
+        __syncwarp();
+        const ResumeRec& r = fa.resume[k];
+        t.restart();
+        t.next();
+        #pragma unroll 1
+        for (u32 e = 0; e < r.count; e++)
+        {
+            const u32 node = r.band[e].node & kNodeMask;
+            const int at = t.enter((u32)t.slot_of(fa.g, node, 0));
+            t.band()[at] = r.band[e];
+        }
+        __syncwarp();
+        FillState f = r.state;
+        const ExtState st = fill_slices(fa, t, arena, r.ext, f, lane);
+        if (lane == 0) fa.states[r.ext] = st;
+    }
+    if (lane == 0 && arena.used) atomicAdd(fa.arenaCursor + 1, (unsigned long long)arena.used);
+}
 __global__ void __launch_bounds__(128, 4) fill_large_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<LargeTables>(fa, counter); }
 
 // The traceback: a warp takes the next filled extension and walks its table back.  Four blocks of
@@ -3379,9 +3470,18 @@ __global__ void __launch_bounds__(128, 4) ms_trace_kernel(const __grid_constant_
 }
 }
 
-// dynamic shared memory of a block of the fill kernels (shared: with its frontier tables) and of
-// the traceback kernels
-static size_t fill_smem(int warpsPerBlock, bool shared) { return (sizeof(gadev::FillWarp) + (shared ? sizeof(gadev::SmallSpace) : 0)) * warpsPerBlock; }
+// dynamic shared memory of a block of the fill kernels and of the traceback kernels
+static size_t fill_smem(int warpsPerBlock, gadev::FillTables tables)
+{
+    const size_t own = tables == gadev::FillTables::Small ? sizeof(gadev::SmallSpace)
+        : tables == gadev::FillTables::Medium ? (size_t)gadev::wspace_bytes(gadev::medium_caps()) : 0;
+    return (sizeof(gadev::FillWarp) + own) * warpsPerBlock;
+}
+static auto fill_function(gadev::FillTables tables)
+{
+    return tables == gadev::FillTables::Small ? gadev::fill_kernel : tables == gadev::FillTables::Medium ? gadev::fill_medium_kernel
+        : gadev::fill_large_kernel;
+}
 static size_t trace_smem(int warpsPerBlock) { return sizeof(gadev::TraceWarp) * warpsPerBlock; }
 
 uint64_t ga_warp_tables_bytes(const gadev::Caps& c) { return gadev::wspace_bytes(c); }
@@ -3392,10 +3492,10 @@ static bool set_smem(const void* kernel, size_t smem)
     return smem <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
 }
 
-int ga_fill_blocks_per_sm(int warpsPerBlock, bool shared)
+int ga_fill_blocks_per_sm(int warpsPerBlock, gadev::FillTables tables)
 {
-    const size_t smem = fill_smem(warpsPerBlock, shared);
-    const auto kernel = shared ? gadev::fill_kernel : gadev::fill_large_kernel;
+    const size_t smem = fill_smem(warpsPerBlock, tables);
+    const auto kernel = fill_function(tables);
     if (!set_smem((const void*)kernel, smem)) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, warpsPerBlock * 32, smem) != cudaSuccess) return 0;
@@ -3411,15 +3511,26 @@ int ga_trace_blocks_per_sm(int warpsPerBlock)
     return n;
 }
 
-int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int traceBlocks,
-    int warpsPerBlock, void* stream)
+int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int mediumBlocks,
+    int traceBlocks, int warpsPerBlock, void* stream)
 {
-    const size_t fillSmem = fill_smem(warpsPerBlock, fa.workspace == nullptr);
-    const auto fill = fa.workspace ? gadev::fill_large_kernel : gadev::fill_kernel;
+    const size_t fillSmem = fill_smem(warpsPerBlock, fa.tables);
+    const auto fill = fill_function(fa.tables);
     const size_t traceSmem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)fill, fillSmem) || !set_smem((const void*)gadev::trace_kernel, traceSmem)) return -1;
     fill<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;
+    if (fa.resume)
+    {
+        gadev::FillArgs fm = fa;
+        fm.tables = gadev::FillTables::Medium;
+        fm.caps = gadev::medium_caps();
+        fm.workspaceStride = gadev::wspace_bytes(fm.caps);
+        const size_t smem = fill_smem(1, gadev::FillTables::Medium);
+        if (!set_smem((const void*)gadev::fill_medium_kernel, smem)) return -1;
+        gadev::fill_medium_kernel<<<mediumBlocks, 32, smem, (cudaStream_t)stream>>>(fm, counters + 3);
+        if (cudaGetLastError() != cudaSuccess) return -1;
+    }
     gadev::trace_kernel<<<traceBlocks, warpsPerBlock * 32, traceSmem, (cudaStream_t)stream>>>(ta, counters + 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -3428,7 +3539,7 @@ int ga_launch_multiseed_fill(const gadev::FillArgs& fa, const gadev::MultiTraceA
     int warpsPerBlock, void* stream)
 {
     if (!fa.workspace) return -1;
-    const size_t fillSmem = fill_smem(warpsPerBlock, false);
+    const size_t fillSmem = fill_smem(warpsPerBlock, gadev::FillTables::Global);
     if (!set_smem((const void*)gadev::fill_multiseed_kernel, fillSmem)) return -1;
     gadev::fill_multiseed_kernel<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;

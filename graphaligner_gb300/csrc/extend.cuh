@@ -122,6 +122,42 @@ struct Caps
     u32 extras;            // pending incoming columns per slice
 };
 
+// How far an extension's fill has come: its next slice and what the slices before it left.
+struct FillState
+{
+    u64 dir;               // as in ExtState
+    u64 steps;
+    u32 slice;
+    u32 committed;
+    i32 bestX;
+    i32 lastMin;
+    i32 lastQuit;
+};
+
+// An extension that outgrew the small tables at a slice, with the band of the slice before it: the
+// medium tables go on from there.  Started again with the tables in global memory, after a pass of
+// their own, the 233 of 1,000 tangled extensions that this happens to took the call from 39.0 ms to
+// 45.8; started again with the medium ones 41.7.
+struct __align__(16) ResumeRec
+{
+    Item band[kSmallBand];
+    FillState state;
+    u32 ext;
+    u32 count;             // band entries
+};
+
+// Where a warp's frontier tables are: in lane registers and shared memory (kSmall*), in shared
+// memory with medium_caps(), or in global memory with FillArgs::caps.
+enum class FillTables { Small, Medium, Global };
+
+// 35 KB a warp: four to five warps on an SM, for the few extensions that outgrow the small tables
+inline Caps medium_caps()
+{
+    Caps c;
+    c.band = 128; c.hash = 256; c.heap = 128; c.extras = 256;
+    return c;
+}
+
 struct FillArgs
 {
     DevGraph g;
@@ -143,8 +179,12 @@ struct FillArgs
     ColumnUnit* store;     // the column store, or null
     u64 storeUnits;        // below kNoColumns
     u64 chunkBytes;        // arena bytes a warp takes at once
-    uint8_t* workspace;    // nullptr: the frontier tables live in shared memory (kSmall*), else
-    u64 workspaceStride;   // bytes of one warp's tables there
+    FillTables tables;
+    ResumeRec* resume;     // small tables: [resumeCap] the extensions handed on to the medium tables, or null
+    u32 resumeCap;
+    u32* resumeCount;      // starts at 0
+    uint8_t* workspace;    // global tables: where they are
+    u64 workspaceStride;   // medium and global tables: bytes of one warp's
     Caps caps;             // and their capacities
     const i32* prevStatus; // when non-null, only extensions whose previous status is GA_CAPACITY run
     ExtState* states;      // [num] where each extension's table is, for the traceback
@@ -290,12 +330,13 @@ uint64_t ga_warp_tables_bytes(const gadev::Caps& caps);
 uint64_t ga_multiseed_tables_bytes(const gadev::Caps& caps);
 // resident blocks of 32 * warpsPerBlock threads per SM of the fill kernel (shared: tables in
 // shared memory) and of the traceback kernel
-int ga_fill_blocks_per_sm(int warpsPerBlock, bool shared);
+int ga_fill_blocks_per_sm(int warpsPerBlock, gadev::FillTables tables);
 int ga_trace_blocks_per_sm(int warpsPerBlock);
-// launches the fill kernel and then the traceback kernel on `stream`, blocks of warpsPerBlock
-// warps, one extension per warp at a time; counters[0] and [1] must be zero
-int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int traceBlocks,
-    int warpsPerBlock, void* stream);
+// launches the fill kernel, with fa.resume the medium tables' (mediumBlocks blocks of one warp),
+// and then the traceback kernel on `stream`, blocks of warpsPerBlock warps, one extension per warp
+// at a time; counters[0], [1] and [3] must be zero
+int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int mediumBlocks,
+    int traceBlocks, int warpsPerBlock, void* stream);
 // the multiseed DP's fill and traceback kernels (the frontier tables always in the global workspace)
 // the multiseed DP in steps, blocks of warpsPerBlock warps, each on `stream`:
 // - fill: the fill and the count of each read's trace candidates (counters[0], [1] and

@@ -141,6 +141,8 @@ extern "C" int ga_extend_batch_noalloc(const ga_graph_desc* device_graph, const 
     fa.arenaCursor = (unsigned long long*)(scratch + 16);
     fa.chunkBytes = 16 * 1024;
     fa.store = nullptr;        // no column store: the traceback recomputes
+    fa.tables = FillTables::Small;
+    fa.resume = nullptr;       // what outgrows the tables reports GA_CAPACITY
     fa.workspace = nullptr;
     fa.prevStatus = nullptr;
     fa.states = (ExtState*)(scratch + kHeaderBytes);
@@ -164,7 +166,7 @@ extern "C" int ga_extend_batch_noalloc(const ga_graph_desc* device_graph, const 
     ta.prevStatus = nullptr;
     ta.states = fa.states;
 
-    if (ga_launch_extend(fa, ta, (u32*)scratch, (int)kBlocks, (int)kBlocks, (int)kWarpsPerBlock, s) != 0)
+    if (ga_launch_extend(fa, ta, (u32*)scratch, (int)kBlocks, 0, (int)kBlocks, (int)kWarpsPerBlock, s) != 0)
     {
         ga_set_last_error("ga_extend_batch_noalloc: kernel launch failed");
         return GA_ERR_CUDA;
