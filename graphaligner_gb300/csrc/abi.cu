@@ -175,7 +175,7 @@ struct ga_extender
     DevBuf<uint32_t> msSeedSlice, msSeedNode, msNumTraces, msTraceLen, msTracesNeeded;
     DevBuf<int32_t> msTraceScore;
     DevBuf<uint64_t> msCandBegin, msTraceBase, msKeptItem;
-    DevBuf<uint32_t> msCandCount, msWork, msKeptSlot;
+    DevBuf<uint32_t> msCandCount, msCandPart, msWork, msKeptSlot;
     DevBuf<gadev::MsKey> msKeys;
     DevBuf<gadev::MsCand> msCands;
     DevBuf<gadev::MsSel> msSel;
@@ -359,7 +359,7 @@ extern "C" int ga_extender_free(ga_extender_t x)
     x->order.release(); x->status.release(); x->score.release(); x->prevStatus.release(); x->states.release(); x->resume.release();
     x->msSeedOff.release(); x->msTraceCap.release(); x->msTraceStart.release(); x->msItemsNeeded.release();
     x->msSeedSlice.release(); x->msSeedNode.release(); x->msNumTraces.release(); x->msTraceLen.release(); x->msTracesNeeded.release();
-    x->msTraceScore.release(); x->msCandBegin.release(); x->msCandCount.release(); x->msCands.release();
+    x->msTraceScore.release(); x->msCandBegin.release(); x->msCandCount.release(); x->msCandPart.release(); x->msCands.release();
     x->msTraceBase.release(); x->msKeptItem.release(); x->msWork.release(); x->msSel.release();
     x->msKeptSlot.release(); x->msKeys.release();
     for (auto& e : x->ev) cudaEventDestroy(e);
@@ -718,6 +718,7 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
     GA_CUDA(x->states.reserve(n));
     GA_CUDA(x->msCandBegin.reserve(n));
     GA_CUDA(x->msCandCount.reserve(n));
+    GA_CUDA(x->msCandPart.reserve((size_t)n * gadev::kCandParts));
     GA_CUDA(x->msSel.reserve(n));
     cudaStream_t s = x->stream;
     GA_CUDA(cudaMemcpyAsync(x->seq.ptr, b->seq, seqBytes, cudaMemcpyHostToDevice, s));
@@ -788,6 +789,7 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
     ta.tracesNeeded = x->msTracesNeeded.ptr;
     ta.candBegin = x->msCandBegin.ptr;
     ta.candCount = x->msCandCount.ptr;
+    ta.candPart = x->msCandPart.ptr;
     ta.candTotal = (unsigned long long*)(x->counters + 8);
 
     x->lastFillMs = 0;
@@ -816,6 +818,7 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
         uint64_t fillBlocks = std::min<uint64_t>((uint64_t)x->sms * 4, pendingBlocks);
         fillBlocks = std::max<uint64_t>(1, std::min<uint64_t>(fillBlocks, x->workspaceBytes / stride / wpb));
         const uint64_t readBlocks = std::min<uint64_t>((uint64_t)x->sms * 6, pendingBlocks);
+        const uint64_t partBlocks = std::min<uint64_t>((uint64_t)x->sms * 6, ((uint64_t)pending * gadev::kCandParts + wpb - 1) / wpb);
         if (pass > 0) GA_CUDA(cudaMemcpyAsync(x->prevStatus.ptr, x->status.ptr, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
         fa.caps = caps;
         fa.workspace = x->workspace;
@@ -825,7 +828,7 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
         GA_CUDA(cudaMemsetAsync(x->counters, 0, 16 * sizeof(uint32_t), s));
         GA_CUDA(cudaMemsetAsync(x->arenaCursor, 0, 3 * sizeof(unsigned long long), s));
         GA_CUDA(cudaEventRecord(x->ev[0], s));
-        if (ga_launch_multiseed_fill(fa, ta, x->counters, (int)fillBlocks, (int)readBlocks, wpb, s) != 0)
+        if (ga_launch_multiseed_fill(fa, ta, x->counters, (int)fillBlocks, (int)partBlocks, wpb, s) != 0)
             return fail(GA_ERR_CUDA, std::string("multiseed kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
         unsigned long long candTotal = 0;
         GA_CUDA(cudaMemcpyAsync(&candTotal, ta.candTotal, 8, cudaMemcpyDeviceToHost, s));
@@ -841,9 +844,9 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
         ta.sel = x->msSel.ptr;
         const uint64_t candBlocks = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)x->sms * 6, (candTotal + wpb - 1) / wpb));
         GA_CUDA(cudaMemsetAsync(x->msSel.ptr, 0, n * sizeof(gadev::MsSel), s));
-        if (ga_launch_multiseed_list(ta, x->counters, (int)readBlocks, wpb, s) != 0)
+        if (ga_launch_multiseed_list(ta, x->counters, (int)partBlocks, wpb, s) != 0)
             return fail(GA_ERR_CUDA, std::string("multiseed kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
-        x->lastLaunches += 3;
+        x->lastLaunches += 4;
         // rounds: each read decides its candidates as far as their walks are known and queues
         // the next walks, twice as many each round, up to 1024
         for (uint32_t round = 0;; round++)

@@ -274,6 +274,8 @@ struct MsSel
 // the room it needs; the batch does not run it again as it does a read whose tables ran out)
 static constexpr i32 kMsRoom = 100;
 
+static constexpr u32 kCandParts = 32;
+
 // The multiseed DP's traceback outputs (ga_multiseed_results).
 struct MultiTraceArgs
 {
@@ -319,6 +321,7 @@ struct MultiTraceArgs
     u64 candCap;
     u64* candBegin;        // [num] read i's candidates are [candBegin[i], candBegin[i] + candCount[i])
     u32* candCount;
+    u32* candPart;         // [num][kCandParts] candidates of each part of a read's slices, then where they start in its run
     unsigned long long* candTotal;   // candidates of the batch
 };
 
@@ -348,9 +351,9 @@ int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint
 //   and *ta.workCount zero) and walk (the queued candidates' traces counted; counters[5] zero);
 // - write: the kept traces written (counters[6] zero).
 // counters[2] is left to the caller.
-int ga_launch_multiseed_fill(const gadev::FillArgs& fa, const gadev::MultiTraceArgs& ta, uint32_t* counters, int fillBlocks, int readBlocks,
+int ga_launch_multiseed_fill(const gadev::FillArgs& fa, const gadev::MultiTraceArgs& ta, uint32_t* counters, int fillBlocks, int partBlocks,
     int warpsPerBlock, void* stream);
-int ga_launch_multiseed_list(const gadev::MultiTraceArgs& ta, uint32_t* counters, int readBlocks, int warpsPerBlock, void* stream);
+int ga_launch_multiseed_list(const gadev::MultiTraceArgs& ta, uint32_t* counters, int partBlocks, int warpsPerBlock, void* stream);
 int ga_launch_multiseed_resolve(const gadev::MultiTraceArgs& ta, uint32_t* counters, int readBlocks, int warpsPerBlock, void* stream);
 int ga_launch_multiseed_walk(const gadev::MultiTraceArgs& ta, uint32_t* counters, int candBlocks, int warpsPerBlock, void* stream);
 int ga_launch_multiseed_write(const gadev::MultiTraceArgs& ta, uint32_t* counters, int candBlocks, int warpsPerBlock, void* stream);
