@@ -848,11 +848,14 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
             return fail(GA_ERR_CUDA, std::string("multiseed kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
         x->lastLaunches += 4;
         // rounds: each read decides its candidates as far as their walks are known and queues
-        // the next walks, twice as many each round, up to 1024
+        // the next walks, twice as many each round, up to 1024, and at least as many as there are
+        // warps for: a round takes as long as its longest walk, so walks that may turn out not to be
+        // needed cost nothing on warps that would be idle (40 reads: 7 rounds of 5 ms without)
+        const uint32_t idle = std::min<uint32_t>(1024, std::max<uint32_t>(1, (uint32_t)x->sms * 16 / pending));
         for (uint32_t round = 0;; round++)
         {
             GA_CUDA(cudaMemsetAsync(x->counters + 4, 0, 4 * sizeof(uint32_t), s));
-            ta.window = round < 10 ? 1u << round : 1024u;
+            ta.window = std::max(idle, round < 10 ? 1u << round : 1024u);
             if (ga_launch_multiseed_resolve(ta, x->counters, (int)readBlocks, wpb, s) != 0)
                 return fail(GA_ERR_CUDA, std::string("multiseed kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
             uint32_t walks = 0;
