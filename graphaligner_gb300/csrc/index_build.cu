@@ -2,7 +2,8 @@
 // initMaxCount with one bucket, MinimizerSeeder.cpp:104-189, 299-491, 557-575).
 //
 // It produces the arrays of the host build in seeding.cpp, element for element:
-//   1. one thread per bigraph node (AlignmentGraph::nodeLookup order) walks the node's
+//   1. one thread per bigraph node (AlignmentGraph::nodeLookup order), or for a node of kLongNode
+//      bases and more one thread per base, walks the node's
 //      sequence over its pieces and reports its window minimizers (iterateMinimizersReal,
 //      ties in hash reported together, restarts after non-ACGT characters) from the end
 //      of the last piece entered from another bigraph node on (MinimizerSeeder.cpp:323-340),
@@ -28,10 +29,19 @@
 namespace gadev
 {
 
+// Nodes of at least this many bases are not walked by one thread but by a thread per base
+// (minimizers_at), in chunks of kChunk bases a block.  A thread's walk takes 1.4 us a base (its
+// window lies in local memory), so the unitigs of a de Bruijn graph, up to 100 kbp long, set the
+// time of the whole build: 143 ms on the graph of a 1 Mbp genome, 2.0 ms by bases.  The nodes of
+// a variation graph are shorter and many, where a block for each would be mostly idle.
+static constexpr uint32_t kLongNode = 256;
+static constexpr uint32_t kChunk = 256;
+static constexpr uint32_t kHalo = 128;      // bases before a chunk that its windows reach: w + 3 <= 31 + 63 + 3
+
 __global__ void count_minimizers_kernel(IndexGraph g, uint32_t k, uint32_t w, uint32_t* counts, uint32_t* error)
 {
     const uint32_t li = blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= g.numLookup) return;
+    if (li >= g.numLookup || g.originalSize[li] >= kLongNode) return;
     bool bad = false;
     counts[li] = node_minimizers(g, li, k, w, nullptr, nullptr, bad);
     if (bad) atomicOr(error, 1u);
@@ -41,12 +51,149 @@ __global__ void write_minimizers_kernel(IndexGraph g, uint32_t k, uint32_t w, co
     uint32_t* order, uint32_t* error)
 {
     const uint32_t li = blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= g.numLookup) return;
+    if (li >= g.numLookup || g.originalSize[li] >= kLongNode) return;
     const uint32_t from = first[li];
     bool bad = false;
     const uint32_t n = node_minimizers(g, li, k, w, kmers + from, positions + from, bad);
     if (bad) atomicOr(error, 1u);
     for (uint32_t i = 0; i < n; i++) order[from + i] = from + i;
+}
+
+// chunks[li] = the chunks of node li if it is long, else 0
+__global__ void count_chunks_kernel(IndexGraph g, uint32_t* chunks)
+{
+    const uint32_t li = blockIdx.x * blockDim.x + threadIdx.x;
+    if (li < g.numLookup) chunks[li] = g.originalSize[li] >= kLongNode ? (g.originalSize[li] + kChunk - 1) / kChunk : 0;
+}
+
+// the node of each chunk
+__global__ void chunk_nodes_kernel(IndexGraph g, const uint32_t* firstChunk, uint32_t* chunkNode)
+{
+    const uint32_t li = blockIdx.x * blockDim.x + threadIdx.x;
+    if (li >= g.numLookup) return;
+    for (uint32_t c = firstChunk[li]; c < firstChunk[li + 1]; c++) chunkNode[c] = li;
+}
+
+// A block per chunk: its share of the node's pieces checked (they tile the node in order) and of
+// the search for the last piece entered from another bigraph node (minStart, zeroed before).
+__global__ void long_nodes_kernel(IndexGraph g, const uint32_t* firstChunk, const uint32_t* chunkNode, uint32_t* minStart, uint32_t* error)
+{
+    const uint32_t li = chunkNode[blockIdx.x];
+    const uint32_t part = blockIdx.x - firstChunk[li], parts = firstChunk[li + 1] - firstChunk[li];
+    const uint32_t from = g.lookupOff[li], to = g.lookupOff[li + 1];
+    bool bad = from == to;
+    uint32_t start = 0;
+    for (uint32_t e = from + part * blockDim.x + threadIdx.x; e < to; e += parts * blockDim.x)
+    {
+        const uint32_t piece = g.lookupNodes[e];
+        if (piece >= g.N)
+        {
+            bad = true;
+            continue;
+        }
+        const uint32_t end = g.nodeOffset[piece] + g.len[piece];
+        const uint32_t next = e + 1 < to ? g.lookupNodes[e + 1] : 0;
+        if (e + 1 < to ? (next >= g.N || g.nodeOffset[next] != end) : end != g.originalSize[li]) bad = true;
+        if (e == from && g.nodeOffset[piece] != 0) bad = true;
+        for (uint32_t p = g.inOff[piece]; p < g.inOff[piece + 1]; p++)
+            if (g.nodeIds[g.inNb[p]] != g.nodeIds[piece] && g.nodeOffset[piece] > start) start = g.nodeOffset[piece];
+    }
+    if (bad) atomicOr(error, 1u);
+    if (start) atomicMax(&minStart[li], start);
+}
+
+// The minimizers of one chunk of a long node, a thread per base: counted (kmers == nullptr), or
+// written behind the chunks before it.  The bases of the chunk and of the windows that reach into
+// it are laid out in shared memory first, then the k-mers' hashes.
+__global__ void __launch_bounds__(kChunk) long_minimizers_kernel(IndexGraph g, uint32_t k, uint32_t w, const uint32_t* firstChunk, const uint32_t* chunkNode,
+    const uint32_t* minStart, const uint32_t* error, uint32_t* chunkCount, uint32_t* nodeCount, const uint32_t* first, uint64_t* kmers, uint64_t* positions,
+    uint32_t* order)
+{
+    constexpr uint32_t kBases = kChunk + kHalo;
+    __shared__ int8_t code[kBases];
+    __shared__ uint32_t pieceOf[kBases];
+    __shared__ uint64_t kmerAt[kBases], hashOf[kBases];
+    __shared__ uint32_t warpSum[kChunk / 32];
+    if (*error) return;                 // pieces that do not tile their node
+    const uint32_t li = chunkNode[blockIdx.x];
+    const uint32_t size = g.originalSize[li];
+    const uint32_t chunkStart = (blockIdx.x - firstChunk[li]) * kChunk;
+    const uint32_t base = chunkStart > kHalo ? chunkStart - kHalo : 0;     // node offset of the first base laid out
+    const uint32_t end = chunkStart + kChunk < size ? chunkStart + kChunk : size;
+    // the last piece that starts at or before `base`
+    uint32_t lo = g.lookupOff[li], hi = g.lookupOff[li + 1];
+    while (hi - lo > 1)
+    {
+        const uint32_t mid = (lo + hi) / 2;
+        if (g.nodeOffset[g.lookupNodes[mid]] <= base) lo = mid;
+        else hi = mid;
+    }
+    for (uint32_t e = lo + threadIdx.x; e < g.lookupOff[li + 1]; e += kChunk)
+    {
+        const uint32_t piece = g.lookupNodes[e];
+        const uint32_t at = g.nodeOffset[piece];
+        if (at >= end) break;
+        const uint32_t stop = at + g.len[piece] < end ? at + g.len[piece] : end;
+        for (uint32_t p = at < base ? base : at; p < stop; p++)
+        {
+            code[p - base] = (int8_t)piece_code(g, piece, p - at);
+            pieceOf[p - base] = piece;
+        }
+    }
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < end - base; q += kChunk)
+    {
+        uint64_t kmer = 0;
+        for (uint32_t i = q + 1 < k ? 0 : q + 1 - k; i <= q; i++) kmer = (kmer << 2) | (uint64_t)(code[i] & 3);
+        kmerAt[q] = kmer;
+        hashOf[q] = kmer_hash(kmer);
+    }
+    __syncthreads();
+    const uint32_t P = chunkStart + threadIdx.x;
+    uint32_t run = 0;
+    if (P < end)
+        while (run < w + 3 && run <= P - base && code[P - base - run] >= 0) run++;
+    const uint32_t from = minStart[li];
+    auto hashAt = [&](uint32_t p) { return hashOf[p - base]; };
+    uint32_t n = 0;
+    minimizers_at(P, run, k, w, hashAt, [&](uint32_t p) { if (p >= from) n++; });
+    // this thread's place among the chunk's minimizers
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = n;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1)
+    {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += up;
+    }
+    if (lane == 31) warpSum[warp] = incl;
+    __syncthreads();
+    uint32_t before = incl - n, all = 0;
+    for (uint32_t q = 0; q < kChunk / 32; q++)
+    {
+        if (q < warp) before += warpSum[q];
+        all += warpSum[q];
+    }
+    if (!kmers)
+    {
+        if (threadIdx.x == 0)
+        {
+            chunkCount[blockIdx.x] = all;
+            if (all) atomicAdd(&nodeCount[li], all);
+        }
+        return;
+    }
+    // chunkCount is scanned by now
+    uint32_t to = first[li] + chunkCount[blockIdx.x] - chunkCount[firstChunk[li]] + before;
+    minimizers_at(P, run, k, w, hashAt, [&](uint32_t p)
+    {
+        if (p < from) return;
+        const uint32_t piece = pieceOf[p - base];
+        kmers[to] = kmerAt[p - base];
+        positions[to] = ((uint64_t)piece << 6) + (p - g.nodeOffset[piece]);
+        order[to] = to;
+        to++;
+    });
 }
 
 // ---------------------------------------------------------------- exclusive scan (u32)
@@ -325,8 +472,33 @@ int ga_build_index_gpu(const gahost::HostGraph& hg, size_t k, size_t w, double k
     keep.push_back(errorFlag);
     IDX_CUDA(cudaMemsetAsync(errorFlag, 0, 4, s), "flag");
     IDX_CUDA(cudaMemsetAsync(first + numLookup, 0, 4, s), "counts");
-    if (numLookup) count_minimizers_kernel<<<(numLookup + 127) / 128, 128, 0, s>>>(g, (uint32_t)k, (uint32_t)w, first, errorFlag);
+    // the long nodes' chunks
+    uint32_t *firstChunk, *minStart, *chunkNode = nullptr, *chunkCount = nullptr;
+    IDX_CUDA(cudaMallocAsync((void**)&firstChunk, ((size_t)numLookup + 1) * 4, s), "chunks"); keep.push_back(firstChunk);
+    IDX_CUDA(cudaMallocAsync((void**)&minStart, std::max<size_t>(numLookup, 1) * 4, s), "chunks"); keep.push_back(minStart);
+    IDX_CUDA(cudaMemsetAsync(firstChunk + numLookup, 0, 4, s), "chunks");
+    IDX_CUDA(cudaMemsetAsync(first, 0, (size_t)numLookup * 4, s), "counts");
+    IDX_CUDA(cudaMemsetAsync(minStart, 0, (size_t)numLookup * 4, s), "chunks");
+    const uint32_t nodeBlocks = (numLookup + 127) / 128;
+    if (numLookup) count_chunks_kernel<<<nodeBlocks, 128, 0, s>>>(g, firstChunk);
+    IDX_CUDA(cudaGetLastError(), "chunks");
+    IDX_CUDA(exclusive_scan(firstChunk, numLookup + 1, s, scanScratch), "chunk scan");
+    uint32_t chunks = 0;
+    IDX_CUDA(cudaMemcpyAsync(&chunks, firstChunk + numLookup, 4, cudaMemcpyDeviceToHost, s), "chunks");
+    if (numLookup) count_minimizers_kernel<<<nodeBlocks, 128, 0, s>>>(g, (uint32_t)k, (uint32_t)w, first, errorFlag);
     IDX_CUDA(cudaGetLastError(), "minimizer count");
+    IDX_CUDA(cudaStreamSynchronize(s), "chunks");
+    if (chunks)
+    {
+        IDX_CUDA(cudaMallocAsync((void**)&chunkNode, (size_t)chunks * 4, s), "chunks"); keep.push_back(chunkNode);
+        IDX_CUDA(cudaMallocAsync((void**)&chunkCount, (size_t)chunks * 4, s), "chunks"); keep.push_back(chunkCount);
+        chunk_nodes_kernel<<<nodeBlocks, 128, 0, s>>>(g, firstChunk, chunkNode);
+        long_nodes_kernel<<<chunks, 128, 0, s>>>(g, firstChunk, chunkNode, minStart, errorFlag);
+        long_minimizers_kernel<<<chunks, kChunk, 0, s>>>(g, (uint32_t)k, (uint32_t)w, firstChunk, chunkNode, minStart, errorFlag, chunkCount, first, nullptr,
+            nullptr, nullptr, nullptr);
+        IDX_CUDA(cudaGetLastError(), "minimizer count");
+        IDX_CUDA(exclusive_scan(chunkCount, chunks, s, scanScratch), "chunk scan");
+    }
     // counts in [0, numLookup), 0 at numLookup: the exclusive scan leaves the total there
     IDX_CUDA(exclusive_scan(first, numLookup + 1, s, scanScratch), "scan");
     uint32_t total = 0, bad = 0;
@@ -344,6 +516,9 @@ int ga_build_index_gpu(const gahost::HostGraph& hg, size_t k, size_t w, double k
     IDX_CUDA(cudaMallocAsync((void**)&order, cells * 4, s), "occurrences"); keep.push_back(order);
     IDX_CUDA(cudaMallocAsync((void**)&order2, cells * 4, s), "occurrences"); keep.push_back(order2);
     if (numLookup) write_minimizers_kernel<<<(numLookup + 127) / 128, 128, 0, s>>>(g, (uint32_t)k, (uint32_t)w, first, kmers, positions, order, errorFlag);
+    if (chunks)
+        long_minimizers_kernel<<<chunks, kChunk, 0, s>>>(g, (uint32_t)k, (uint32_t)w, firstChunk, chunkNode, minStart, errorFlag, chunkCount, nullptr, first,
+            kmers, positions, order);
     IDX_CUDA(cudaGetLastError(), "minimizer write");
 
     // 2. stable LSD radix sort of (k-mer, occurrence) by the k-mer's 2k bits

@@ -249,4 +249,56 @@ GA_HOST_DEVICE inline uint32_t node_minimizers(const IndexGraph& g, uint32_t li,
     }
 }
 
+// The walk above without its state: what it reports when it has read the base at P, from the
+// hashes of the k-mers that end at P and before it.
+//
+// run: how many A, C, G and T in a row end at P, counted up to w + 3.  The walk reports nothing
+// before w + 1 of them; there its first window, the w - k + 2 k-mers so far, reports every k-mer of
+// least hash.  From then on the window is the last w - k + 1 k-mers.  Where its least hash is the
+// one of the window before, only the k-mer at P is reported, if it has it.  Where it is not, the
+// k-mer at P is reported if it has it, after the last of the others that have it: as a front runs
+// out of the window the walk drops the ones before that (MinimizerSeeder.cpp:160-168).
+// hashAt(p): the hash of the k-mer ending at p.  at(p): called for each reported position, in order.
+template <typename HashAt, typename Report>
+GA_HOST_DEVICE inline void minimizers_at(uint32_t P, uint32_t run, uint32_t k, uint32_t w, HashAt hashAt, Report report)
+{
+    if (run < w + 1) return;
+    const uint32_t realWindow = w - k + 1;
+    const uint64_t own = hashAt(P);
+    if (run == w + 1)
+    {
+        uint64_t least = own;
+        for (uint32_t p = P - realWindow; p < P; p++)
+        {
+            const uint64_t h = hashAt(p);
+            if (h < least) least = h;
+        }
+        for (uint32_t p = P - realWindow; p <= P; p++)
+            if (hashAt(p) == least) report(p);
+        return;
+    }
+    uint64_t others = ~0ULL;
+    uint32_t lastOther = P;
+    for (uint32_t p = P - realWindow + 1; p < P; p++)
+    {
+        const uint64_t h = hashAt(p);
+        if (lastOther == P || h <= others)
+        {
+            others = h;
+            lastOther = p;
+        }
+    }
+    const bool some = lastOther != P;
+    const uint64_t now = some && others < own ? others : own;
+    uint64_t before = hashAt(P - realWindow);
+    if (some && others < before) before = others;
+    if (run == w + 2)
+    {
+        const uint64_t h = hashAt(P - realWindow - 1);
+        if (h < before) before = h;
+    }
+    if (now != before && some && others == now) report(lastOther);
+    if (own == now) report(P);
+}
+
 }
