@@ -1986,7 +1986,7 @@ struct TPos
 {
     u32 node;
     u32 off;
-    int64_t seq;      // -1 = the row above the read
+    i32 seq;          // below GA_MAX_SEQ_LEN; -1 = the row above the read
 };
 
 __device__ __forceinline__ bool tpos_eq(const TPos& a, const TPos& b) { return a.node == b.node && a.off == b.off && a.seq == b.seq; }
@@ -1997,29 +1997,12 @@ struct TStep
     bool sw;
 };
 
-// Stages `count` (<= 32) trace items, item i = first + i * step, behind the n already there, as
-// far as they fit cap; a filled group of 32 goes out, one item per lane.  Returns the new n.
-// Out of line: the walk emits from many places, and its code has to stay in the instruction cache.
-__device__ __noinline__ u32 emit_run(u64* items, u64* ring, u32 n, u32 cap, u64 first, u64 step, u32 count, u32 lane)
-{
-    if (count > cap - n) count = cap - n;
-    if (lane < count) ring[(n + lane) & 63] = first + lane * step;
-    __syncwarp();
-    const u32 to = n + count;
-    if (items && ((n ^ to) & ~31u))
-    {
-        const u32 k = (n & ~31u) + lane;
-        items[k] = ring[k & 63];
-        __syncwarp();
-    }
-    return to;
-}
+// What a step takes off an item's upper word: a column (bits 32-37) or a row (bits 39-63).  Runs
+// of steps of one kind lie inside one node, so the lower word, the node, stays.
+static constexpr u32 kColumnStep = 1u, kRowStep = 1u << 7;
 
-static constexpr u64 kStepLeft = ~(1ULL << 32) + 1;                 // one column left
-static constexpr u64 kStepUp = ~(1ULL << 39) + 1;                   // one row up
-
-// Trace items go to a 64-entry ring in shared memory and out to the caller's buffer 32 at a
-// time, one item per lane.  A run of steps inside one node goes in at once.
+// Trace items go out one per lane, a run of steps of one kind at once, and into a 64-entry ring in
+// shared memory that the circularity check reads.
 // counting (MayCount only, the multiseed traceback): nothing goes out, the items are only
 // counted.
 template <bool MayCount>
@@ -2033,15 +2016,31 @@ struct TraceOutT
     TPos back;
     bool overflow;
     bool counting = false;
-    __device__ __forceinline__ static u64 pack(const TPos& p, bool sw)
+    // `count` (1..64) items, each `step` less in the upper word than the one before
+    __device__ __forceinline__ void emit(u32 node, u32 upper, u32 step, u32 count)
     {
-        const u64 sp1 = p.seq < 0 ? 0 : (u64)p.seq + 1;
-        return (u64)p.node | ((u64)(p.off & 63) << 32) | ((u64)(sw ? 1 : 0) << 38) | (sp1 << 39);
+#pragma unroll 1
+        for (u32 from = 0; from < count; from += 32)
+        {
+            const u32 k = from + lane;
+            if (k < count)
+            {
+                const u64 x = ((u64)(upper - k * step) << 32) | node;
+                ring[(n + k) & 63] = x;
+                if (!(MayCount && counting)) items[n + k] = x;
+            }
+        }
+        n += count;
+        __syncwarp();
+    }
+    __device__ __forceinline__ static u32 upper_word(const TPos& p, bool sw)
+    {
+        return (p.off & 63) | (sw ? 1u << 6 : 0) | ((u32)(p.seq + 1) << 7);
     }
     __device__ __forceinline__ void push(const TPos& p, bool sw)
     {
         if (n >= cap) { overflow = true; return; }
-        n = emit_run((MayCount && counting) ? nullptr : items, ring, n, cap, pack(p, sw), 0, 1, lane);
+        emit(p.node, upper_word(p, sw), 0, 1);
         back = p;
     }
     // `count` (1..64) steps of the same kind from `p`, which is the first item; every item stays
@@ -2049,28 +2048,16 @@ struct TraceOutT
     __device__ __forceinline__ void push_run(TPos p, int dOff, int dSeq, u32 count)
     {
         if (count > cap - n) { overflow = true; count = cap - n; }
-        const u64 step = (dOff ? kStepLeft : 0) + (dSeq ? kStepUp : 0);
-        const u64 first = pack(p, false);
-        u64* out = (MayCount && counting) ? nullptr : items;
-        n = emit_run(out, ring, n, cap, first, step, count < 32 ? count : 32, lane);
-        if (count > 32) n = emit_run(out, ring, n, cap, first + 32 * step, step, count - 32, lane);
         if (count == 0) return;
+        emit(p.node, upper_word(p, false), (dOff ? kColumnStep : 0) + (dSeq ? kRowStep : 0), count);
         p.off += (u32)(dOff * (int)(count - 1));
-        p.seq += dSeq * (int64_t)(count - 1);
+        p.seq += dSeq * (int)(count - 1);
         back = p;
-    }
-    // writes the items of the last, partial group of 32
-    __device__ __forceinline__ void finish()
-    {
-        if (MayCount && counting) return;
-        const u32 k = (n & ~31u) + lane;
-        if (k < n) items[k] = ring[k & 63];
-        __syncwarp();
     }
 };
 using TraceOut = TraceOutT<false>;
 
-__device__ __forceinline__ u32 mod64(int64_t seq) { return (u32)((u64)seq & 63); }
+__device__ __forceinline__ u32 mod64(i32 seq) { return (u32)seq & 63; }
 
 // checkBacktraceCircularity (Common.h:760-768): the newest item must not repeat an
 // earlier item of the same read position.  Items still in the ring are read there, older
@@ -2104,7 +2091,7 @@ template <bool Multi> __device__ __forceinline__ i32 xbefore(const WS& e) { retu
 // pickBacktraceCorner (Common.h:936-1054).  Out of line, like the other crossing rules:
 // the walk inside a node-slice is the hot path.  t is a copy (its record cache is a hint).
 template <bool Multi>
-__device__ __noinline__ TStep bt_corner(const DevGraph& g, const uint8_t* seq, Table t, u32 cs, u32 node, int64_t j, int& err, WS extra)
+__device__ __noinline__ TStep bt_corner(const DevGraph& g, const uint8_t* seq, Table t, u32 cs, u32 node, i32 j, int& err, WS extra)
 {
     const SliceRec* cr = t.rec(cs);
     const SliceRec* pr = t.rec(cs - 1);
@@ -2321,7 +2308,7 @@ struct EndCell
     u32 nodeOffset;
     u32 bvOffset;
     i32 score;
-    int64_t j;
+    i32 j;
     int err;
 };
 
@@ -2350,12 +2337,12 @@ __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint
     const SliceRec* br = t.rec(best);
     ec.node = br->maxXNode;
     ec.score = br->maxX;
-    ec.j = ((int64_t)best - 1) * 64;
-    const int64_t j = ec.j;
+    ec.j = ((i32)best - 1) * 64;
+    const i32 j = ec.j;
     if (!slice_masks(seq, seqLen, best, lane)) { ec.err = GA_ASSERT; return ec; }
     ec.err = recalc(g, cost, t, best, ec.node, lane, 63);
     if (ec.err) return ec;
-    const int cells = (int)((int64_t)seqLen - j < 64 ? (int64_t)seqLen - j : 64);
+    const int cells = (i32)seqLen - j < 64 ? (i32)seqLen - j : 64;
     const u32 L = g.len[ec.node];
     bool bad = false;
     int candOff = -1;
@@ -2373,7 +2360,7 @@ __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint
             #pragma unroll 1
             for (int off = 63; off >= 0; off--)
             {
-                if (j + off >= (int64_t)seqLen) continue;
+                if (j + off >= (i32)seqLen) continue;
                 i32 here = ws_xscore(cw, (i32)j, off, cost);
                 if (here > ec.score) { bad = true; break; }
                 if (here == ec.score && off > candOff)
@@ -2387,7 +2374,7 @@ __device__ __noinline__ EndCell end_cell(const DevGraph& g, i32 cost, const uint
     if (__ballot_sync(kFull, bad)) { ec.err = GA_ASSERT; return ec; }
     const int gOff = __reduce_max_sync(kFull, candOff);
     const u32 gCol = __reduce_min_sync(kFull, candOff == gOff ? candCol : 0xffffffffu);
-    if (gOff < 0 || j + gOff >= (int64_t)seqLen) { ec.err = GA_ASSERT; return ec; }
+    if (gOff < 0 || j + gOff >= (i32)seqLen) { ec.err = GA_ASSERT; return ec; }
     ec.nodeOffset = gCol;
     ec.bvOffset = (u32)gOff;
     return ec;
@@ -2497,7 +2484,9 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
 {
     int err = 0;
     const NodeCols& nc = trace_cols();
-    const u64 guardMax = (u64)((Multi && to.counting) ? (1u << 26) : to.cap) * 4 + 1024;
+    // steps a walk may take (a trace that needs 2^32 has no room anywhere)
+    const u32 guardCap = (Multi && to.counting) ? 1u << 26 : to.cap;
+    const u32 guardMax = guardCap < (1u << 29) ? guardCap * 4 + 1024 : 0xffffffffu;
     resultScore = startScore;
     to.push(start, false);
     // the extraSlice of the current node-slice and its score at a row
@@ -2509,7 +2498,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     const ColumnUnit* columns = nullptr;
     const Item* self = nullptr;
     i32 lastScore = kIntMax - 1;  // score of the last cell the walk looked at, where it can end
-    u64 guard = 0;
+    u32 guard = 0;
     // the current slice and the one before it
     const SliceRec* recCur = nullptr;
     const SliceRec* recPrev = nullptr;
@@ -2527,7 +2516,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     auto corner = [&]() -> TStep
     {
         int e = 0;
-        const TStep step = bt_corner<Multi>(g, seq, t, curSlice, curNode, ((int64_t)curSlice - 1) * 64, e, extra);
+        const TStep step = bt_corner<Multi>(g, seq, t, curSlice, curNode, ((i32)curSlice - 1) * 64, e, extra);
         if (e) err = e;
         return step;
     };
@@ -2598,7 +2587,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
     {
         if (++guard > guardMax) { err = GA_CAPACITY; break; }
         const TPos b = to.back;
-        const u32 newSlice = (u32)(b.seq / 64) + 1;
+        const u32 newSlice = ((u32)b.seq >> 6) + 1;
         if (newSlice >= committed) { err = GA_ASSERT; break; }
         // a self-loop can re-enter the same node-slice further right than it was computed
         if (newSlice != curSlice || b.node != curNode || b.off > colsUpTo)
@@ -2689,7 +2678,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             }
         }
         const bool seeded = Multi && extra.end != kIntMax;
-        const int64_t sj = ((int64_t)curSlice - 1) * 64;
+        const i32 sj = ((i32)curSlice - 1) * 64;
         if (b.off >= rec_len(meta)) { err = GA_ASSERT; break; }
         const u32 row = mod64(b.seq);
         // the walk ends above the read, so from row 0 or up column 0 to it, or at a seed start
@@ -2743,7 +2732,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             TPos p = b;
             const u64 stops = (~self->sVP | 1ULL) & (row == 63 ? kAllOnes : ((2ULL << row) - 1));
             const u32 off = 63 - (u32)__clzll((long long)stops);
-            p.seq -= (int64_t)(row - off);
+            p.seq -= (i32)(row - off);
             if (!seeded && off == 0) lastScore = ws_value(ws_make(self->sVP, self->sVN, self->sEnd), (int)row);
             TStep second = off == 0 ? corner() : horizontal(p, off);
             if (err) break;
@@ -2776,7 +2765,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 {
                     // __ffs(0) = 0: all 32 lanes' steps are diagonal
                     const u32 count = run ? run - 1 : 32;
-                    to.push_run(TPos { b.node, hori - 1, sj + vert - 1 }, -1, -1, count);
+                    to.push_run(TPos { b.node, hori - 1, sj + (i32)vert - 1 }, -1, -1, count);
                     hori -= count;
                     vert -= count;
                     continue;
@@ -2785,12 +2774,12 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 if ((vp >> vert) & 1)
                 {
                     const u32 count = up_run(vp, vert);
-                    to.push_run(TPos { b.node, hori, sj + vert - 1 }, 0, -1, count);
+                    to.push_run(TPos { b.node, hori, sj + (i32)vert - 1 }, 0, -1, count);
                     vert -= count;
                     continue;
                 }
                 hori--;
-                to.push(TPos { b.node, hori, sj + vert }, false);
+                to.push(TPos { b.node, hori, sj + (i32)vert }, false);
             }
             continue;
         }
@@ -2822,7 +2811,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                     if (vs == here - 1)
                     {
                         vert--;
-                        to.push(TPos { b.node, hori, sj + vert }, false);
+                        to.push(TPos { b.node, hori, sj + (i32)vert }, false);
                         here = vs;
                         left = ds;
                     }
@@ -2830,7 +2819,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                     {
                         hori--;
                         vert--;
-                        to.push(TPos { b.node, hori, sj + vert }, false);
+                        to.push(TPos { b.node, hori, sj + (i32)vert }, false);
                         here = ds;
                         colH = colL;
                         if (hori > 0)
@@ -2843,7 +2832,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                     else if (left == here - 1)
                     {
                         hori--;
-                        to.push(TPos { b.node, hori, sj + vert }, false);
+                        to.push(TPos { b.node, hori, sj + (i32)vert }, false);
                         here = left;
                         colH = colL;
                         if (hori > 0)
@@ -2913,7 +2902,7 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
     if (!err)
     {
         // getReverseTraceFromTable (Common.h:571-758)
-        TPos start = TPos { ec.node, ec.nodeOffset, ec.j + ec.bvOffset };
+        TPos start = TPos { ec.node, ec.nodeOffset, ec.j + (i32)ec.bvOffset };
         i32 startScore = nc.value(ec.nodeOffset, ec.bvOffset);
         err = trace_walk<false>(g, a.cost, seq, seqLen, st.committed, t, to, a.store, start, startScore, resultScore, lane);
         if (!err && !to.overflow)
@@ -2923,7 +2912,6 @@ __device__ void trace_extension(const TraceArgs& a, u32 ext, const ExtState& st,
             to = end;
         }
     }
-    to.finish();
     int status = err ? err : (to.overflow ? GA_CAPACITY : GA_OK);
     if (lane == 0)
     {
@@ -3046,14 +3034,14 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const uint8_t* s
     const SliceRec* cr = (const SliceRec*)(a.arena + t.dir[c.slice]);
     const Item* items = rec_items(cr);
     const u32 node = items[c.index].node & kNodeMask;
-    const int64_t j = ((int64_t)c.slice - 1) * 64;
+    const i32 j = ((i32)c.slice - 1) * 64;
     if (!slice_masks(seq, seqLen, c.slice, lane)) return GA_ASSERT;
     const WS extra = (items[c.index].node & kSeedStart) ? seed_ws(j, seqLen, a.cost) : fake_ws();
     int err = recalc<true>(g, a.cost, t, c.slice, node, lane, 63, extra);
     if (err) return err;
     const NodeCols& nc = trace_cols();
     const i32 score = c.score;
-    const int cells = (int)((int64_t)seqLen - j < 64 ? (int64_t)seqLen - j : 64);
+    const int cells = (i32)seqLen - j < 64 ? (i32)seqLen - j : 64;
     const u32 L = g.len[node];
     bool bad = false;
     int candOff = -1;
@@ -3070,7 +3058,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const uint8_t* s
 #pragma unroll 1
         for (int off = 63; off >= 0; off--)
         {
-            if (j + off >= (int64_t)seqLen) continue;
+            if (j + off >= (i32)seqLen) continue;
             const i32 here = ws_xscore(cw, (i32)j, off, a.cost);
             if (here > score) { bad = true; break; }
             if (here == score && off > candOff)
@@ -3083,7 +3071,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const uint8_t* s
     if (__ballot_sync(kFull, bad)) return GA_ASSERT;
     const int gOff = __reduce_max_sync(kFull, candOff);
     const u32 gCol = __reduce_min_sync(kFull, candOff == gOff ? candCol : 0xffffffffu);
-    if (gOff < 0 || j + gOff >= (int64_t)seqLen) return GA_ASSERT;
+    if (gOff < 0 || j + gOff >= (i32)seqLen) return GA_ASSERT;
     start = TPos { node, gCol, j + gOff };
     startScore = nc.value(gCol, gOff);
     return 0;
@@ -3119,7 +3107,7 @@ __device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, bool write, u
     int err = 0;
     if (write)
     {
-        start = TPos { c.startNode, c.startOff, c.startSeq };
+        start = TPos { c.startNode, c.startOff, (i32)c.startSeq };
         startScore = c.startScore;
     }
     else
@@ -3144,8 +3132,7 @@ __device__ void ms_trace_cand(const MultiTraceArgs& a, MsCand* cp, bool write, u
     if (!err)
     {
         err = trace_walk<true>(a.g, a.cost, seq, seqLen, st.committed, t, to, a.store, start, startScore, traceScore, lane);
-        to.finish();
-        // a walk past its step guard or its counted length is broken, not short of room
+            // a walk past its step guard or its counted length is broken, not short of room
         if (err == GA_CAPACITY || (!err && to.overflow)) err = GA_ASSERT;
         if (!err && (to.back.seq < 0 || start.seq < to.back.seq)) err = GA_ASSERT;
     }
