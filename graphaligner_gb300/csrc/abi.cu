@@ -189,6 +189,23 @@ extern "C" const char* ga_last_error(void) { return g_lastError.c_str(); }
 void ga_set_last_error(const char* message) { g_lastError = message; }
 extern "C" const char* ga_version(void) { return "graphaligner_gb300 0.1 (sm_103a)"; }
 
+// whether no two of the n component numbers are the same (0 also where they are spread too widely to tell cheaply)
+static uint32_t unique_components(const uint32_t* component, uint32_t n)
+{
+    uint32_t most = 0;
+    for (uint32_t i = 0; i < n; i++) most = std::max(most, component[i]);
+    if (most >= 16ull * n + 1024 || most == 0xffffffffu) return 0;
+    std::vector<uint64_t> seen((size_t)most / 64 + 1, 0);
+    for (uint32_t i = 0; i < n; i++)
+    {
+        uint64_t& word = seen[component[i] / 64];
+        const uint64_t bit = 1ull << (component[i] % 64);
+        if (word & bit) return 0;
+        word |= bit;
+    }
+    return 1;
+}
+
 extern "C" int ga_graph_upload(const ga_graph_desc* desc, int device, ga_graph_t* out)
 {
     if (!desc || !out) return fail(GA_ERR_ARGUMENT, "null argument");
@@ -232,6 +249,7 @@ extern "C" int ga_graph_upload(const ga_graph_desc* desc, int device, ga_graph_t
         return cuda_fail(e, "graph upload");
     }
     g->d.N = N;
+    g->d.uniqueComponents = unique_components(desc->component, N);
     g->d.firstAmbiguous = desc->first_ambiguous;
     g->d.len = (const uint32_t*)len;
     g->d.seq2 = (const uint64_t*)seq2;
@@ -463,8 +481,8 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
         const gadev::Caps caps = layout_caps(layout);
         const uint64_t stride = ga_warp_tables_bytes(caps);
         const gadev::FillTables tables = shared ? gadev::FillTables::Small : gadev::FillTables::Global;
-        int fillPerSm = ga_fill_blocks_per_sm(wpb, tables);
-        const int mediumPerSm = shared ? ga_fill_blocks_per_sm(1, gadev::FillTables::Medium) : 0;
+        int fillPerSm = ga_fill_blocks_per_sm(wpb, tables, x->graph->d.uniqueComponents != 0);
+        const int mediumPerSm = shared ? ga_fill_blocks_per_sm(1, gadev::FillTables::Medium, false) : 0;
         int tracePerSm = ga_trace_blocks_per_sm(wpb);
         if (fillPerSm <= 0 || tracePerSm <= 0) return fail(GA_ERR_CUDA, "the extension kernels do not fit an SM with this launch shape");
         if (sh.blocks_per_sm > 0)

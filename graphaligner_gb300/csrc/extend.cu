@@ -54,6 +54,7 @@ struct Extra
 {
     u64 VP, VN;
     i32 end;
+    i32 before;         // the score above the column's first row
     uint16_t next;
     uint16_t skip;      // bit 0 EdgeWithPriority::skipFirst, bit 1 ::forceCalculation
 };
@@ -293,8 +294,14 @@ __device__ __forceinline__ SmallSpace& small_space()
 // registers, a lookup one ballot, and the nodes' records are copied into shared memory while
 // they wait in the queue.  With a hash table and the records' fields read from global memory
 // the pops and inserts took 17k of the fill's 45k cycles per slice of an extension alone.
+//
+// Unique: no two nodes of the graph share a component number, as in a variation graph.  The
+// component queue then has one order whatever its heap looks like, the component numbers', so the
+// queued slots are not in a heap at all and the next one is found by a minimum over the lanes.
+// (Where numbers are shared, equal scores come off in the order the heap's layout gives.)
 // This form against that: 50,000 extensions (250 Mbp) 102.9 -> 92.7 ms, one seed of a 10 kbp
 // read 8 % less, 1,000 tangled extensions of 20 kbp reads 14 % less.
+template <bool Unique>
 struct SmallTables
 {
     static constexpr bool kSmall = true;
@@ -368,9 +375,13 @@ struct SmallTables
         if (!(v & kQueued))
         {
             if (heapN >= kSmallHeap) return false;
-            HeapItem h;
-            h.component = component; h.score = score; h.node = node; h.slot = (u32)slot;
-            heap_push(heap(), heapN, h);
+            if (Unique) heapN++;
+            else
+            {
+                HeapItem h;
+                h.component = component; h.score = score; h.node = node; h.slot = (u32)slot;
+                heap_push(heap(), heapN, h);
+            }
             v = (v & (kLinear | 0xffu)) | 0xffff00u | kQueued;
         }
         if (poolN >= kSmallExtras) return false;
@@ -383,10 +394,24 @@ struct SmallTables
         if (lane == (u32)slot) val = v;
         return true;
     }
+    // the queue's first node, and its slot
+    __device__ __forceinline__ u32 top(u32& slot) const
+    {
+        if (!Unique)
+        {
+            slot = heap()[0].slot;
+            return heap()[0].node;
+        }
+        const u32 key = lane < used && (val & kQueued) ? comp : 0xffffffffu;
+        const u32 least = __reduce_min_sync(kFull, key);
+        slot = (u32)__ffs((int)__ballot_sync(kFull, key == least && lane < used && (val & kQueued))) - 1;
+        return __shfl_sync(kFull, id, (int)slot);
+    }
     // takes the node off the queue; its first pending column
     __device__ __forceinline__ uint16_t take(u32 slot, int& bandIndex)
     {
-        heap_pop(heap(), heapN);
+        if (Unique) heapN--;
+        else heap_pop(heap(), heapN);
         const u32 v = __shfl_sync(kFull, val, (int)slot);
         if (lane == slot) val = (v & (kLinear | 0xffu)) | 0xffff00u;
         bandIndex = (v & 0xff) == 0xff ? -1 : (int)(v & 0xff);
@@ -511,6 +536,11 @@ struct HashTables
         else w.extras[s.tail].next = e;
         s.tail = e;
         return true;
+    }
+    __device__ __forceinline__ u32 top(u32& slot) const
+    {
+        slot = w.heap[0].slot;
+        return w.heap[0].node;
     }
     __device__ __forceinline__ uint16_t take(u32 slot, int& bandIndex)
     {
@@ -724,22 +754,22 @@ __device__ __forceinline__ WS ws_from_rows(i32 before, i32 m0, i32 m1, u32 lane)
 __device__ __noinline__ WS merge_seq(WS a, WS b) { return ws_merge(a, b); }
 __device__ __noinline__ i32 changed_min_seq(WS w, WS old) { return ws_changed_min(w, old); }
 
-// mergeTwoSlices (WordSlice.h:502-541) across the lanes
-__device__ __forceinline__ WS merge_w(const WS& a, const WS& b, u32 lane)
+// mergeTwoSlices (WordSlice.h:502-541) across the lanes; ba and bb: ws_before of a and b
+__device__ __forceinline__ WS merge_w(const WS& a, i32 ba, const WS& b, i32 bb, u32 lane)
 {
-    const i32 ba = ws_before(a), bb = ws_before(b);
     if (!(score_ok(ba) && score_ok(bb) && score_ok(a.end) && score_ok(b.end))) return merge_seq(a, b);
     i32 a0, a1, b0, b1;
     ws_rows(a, ba, lane, a0, a1);
     ws_rows(b, bb, lane, b0, b1);
     return ws_from_rows(imin(ba, bb), imin(a0, b0), imin(a1, b1), lane);
 }
+__device__ __forceinline__ WS merge_w(const WS& a, const WS& b, u32 lane) { return merge_w(a, ws_before(a), b, ws_before(b), lane); }
 
 // changedMinScoreLocalMinima (WordSlice.h:438-472) across the lanes; old may be the
-// never-computed column (0, 0, INT32_MAX), whose every score is INT32_MAX
-__device__ __forceinline__ i32 changed_min_w(const WS& w, const WS& old, u32 lane)
+// never-computed column (0, 0, INT32_MAX), whose every score is INT32_MAX.  bw: ws_before(w)
+__device__ __forceinline__ i32 changed_min_w(const WS& w, i32 bw, const WS& old, u32 lane)
 {
-    const i32 bw = ws_before(w), bo = ws_before(old);
+    const i32 bo = ws_before(old);
     const bool oldUnset = old.VP == 0 && old.VN == 0 && old.end == kIntMax;
     if (!(score_ok(bw) && score_ok(w.end) && (oldUnset || (score_ok(bo) && score_ok(old.end))))) return changed_min_seq(w, old);
     i32 w0, w1, o0, o1;
@@ -997,12 +1027,14 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     const u64 eq0 = mask_at(0);
 
     WS ws = ws_make(0, 0, 0);
+    i32 wsBefore = 0;           // ws_before(ws), carried along: a column's popcounts are a dozen instructions
     bool hasWs = false;
     bool hasSkipless = false;
     if (singleIncoming)
     {
         result.cells = 1;
         ws = *singleIncoming;
+        wsBefore = ws_before(ws);
         hasWs = true;
     }
     else
@@ -1017,26 +1049,31 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
             if (Multi && (inc.skip & 2)) forceCalculation = true;
             if (inc.skip & 1)
             {
-                ws = hasWs ? merge_w(ws, incWs, lane) : incWs;
+                ws = hasWs ? merge_w(ws, wsBefore, incWs, inc.before, lane) : incWs;
+                wsBefore = hasWs ? imin(wsBefore, inc.before) : inc.before;
                 hasWs = true;
                 continue;
             }
             hasSkipless = true;
             i32 compareHin = prev.exists ? prev.sEnd : kIntMax;
             if (hasExtra) compareHin = imin(compareHin, ws_before(*extra));
-            i32 incBefore = ws_before(incWs);
+            const i32 incBefore = inc.before;
             u64 hinP = 0, hinN = 0;
             if (compareHin < incBefore) hinN = 1;
             else if (compareHin > incBefore) hinP = 1;
             u64 Ph, Mh;
             WS nw = myers_step(eq0, incWs, hinP, hinN, Ph, Mh);
             steps++;
-            if (!prev.exists || ws_before(nw) < prev.sEnd)
+            // (as popcounts give it, the forced first row included)
+            i32 nwBefore = incBefore + (i32)hinP - (i32)hinN;
+            if (!prev.exists || nwBefore < prev.sEnd)
             {
+                nwBefore += 1 - (i32)(nw.VN & 1) + (i32)(nw.VP & 1);
                 nw.VP &= kAllOnes ^ 1;
                 nw.VN |= 1;
             }
-            ws = hasWs ? merge_w(ws, nw, lane) : nw;
+            ws = hasWs ? merge_w(ws, wsBefore, nw, nwBefore, lane) : nw;
+            wsBefore = hasWs ? imin(wsBefore, nwBefore) : nwBefore;
             hasWs = true;
         }
     }
@@ -1049,7 +1086,11 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     result.minScoreOffset = 0;
     result.maxXNode = i;
     // the seed start's column joins after the first minimum and before the first X-score
-    if (hasExtra) ws = merge_w(ws, *extra, lane);
+    if (hasExtra)
+    {
+        ws = merge_w(ws, *extra, lane);
+        wsBefore = ws_before(ws);
+    }
     const WS wsX = ws;
     // (the recomputation starts from the stored first column, whose merge with itself changes nothing)
     bool leave = false;
@@ -1057,6 +1098,7 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     {
         const Merged m = merge_existing(ws, slice, hasSkipless, singleInPrevBand, lane);
         ws = m.ws;
+        wsBefore = ws_before(ws);
         leave = m.leave;
     }
     if (leave)
@@ -1066,13 +1108,17 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
             result.maxX = ws_max_xscore(wsX, seqOffset, cost, 64, kAllOnes);
         return result;
     }
-    if (prev.exists && ws_before(ws) > prev.sEnd) ws = merge_w(ws, ws_source(prev.sEnd), lane);
+    if (prev.exists && wsBefore > prev.sEnd)
+    {
+        ws = merge_w(ws, wsBefore, ws_source(prev.sEnd), prev.sEnd, lane);
+        wsBefore = prev.sEnd;
+    }
     u64 forceMask = 0;
     u64 fixedHP = prev.HP;
     u64 fixedHN = prev.HN;
     if (prev.exists)
     {
-        i32 scoreBefore = ws_before(ws);
+        i32 scoreBefore = wsBefore;
         i32 scoreComparison = prev.sEnd;
         if (scoreBefore > scoreComparison) { err = GA_ASSERT; return result; }
         if (hasExtra || scoreBefore < scoreComparison)
@@ -1545,11 +1591,11 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
     if (!eq_of_rows(rows, fill_cols().base)) { err = GA_ASSERT; return res; }
     rows = row_bytes(seq, seqLen, j + 64, lane);
 
-    auto insert = [&](int slot, u32 node, u32 component, i32 score, const WS& c, bool skip, bool force) -> bool
+    auto insert = [&](int slot, u32 node, u32 component, i32 score, const WS& c, i32 before, bool skip, bool force) -> bool
     {
         if (slot < 0) return false;
         Extra x;
-        x.VP = c.VP; x.VN = c.VN; x.end = c.end; x.next = nil; x.skip = (skip ? 1 : 0) | (force ? 2 : 0);
+        x.VP = c.VP; x.VN = c.VN; x.end = c.end; x.before = before; x.next = nil; x.skip = (skip ? 1 : 0) | (force ? 2 : 0);
         return t.queue(slot, node, component, score, x);
     };
 
@@ -1585,9 +1631,9 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
                 }
             }
             const u32 component = t.prev_component(g, from + k, node);
-            const WS src = ws_source(__shfl_sync(kFull, sEnd, (int)k));
+            const i32 above = __shfl_sync(kFull, sEnd, (int)k);
             // the band's nodes are distinct and the table is still empty of them
-            if (!insert(t.add(g, node, component), node, component, __shfl_sync(kFull, minScore, (int)k), src, true, false))
+            if (!insert(t.add(g, node, component), node, component, __shfl_sync(kFull, minScore, (int)k), ws_source(above), above, true, false))
             {
                 err = GA_CAPACITY;
                 return res;
@@ -1617,7 +1663,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
             band[at] = ni;
             nodeMax[at] = 0;
             t.set_columns((u32)at, kNoColumns);     // a seed start's columns are merged, their steps are not bits
-            if (!insert(slot, node, component, ws_value(seeds->ws, 0), seeds->ws, true, true)) { err = GA_CAPACITY; return res; }
+            if (!insert(slot, node, component, ws_value(seeds->ws, 0), seeds->ws, ws_before(seeds->ws), true, true)) { err = GA_CAPACITY; return res; }
         }
     }
     i32 curMin = res.minScore;
@@ -1625,8 +1671,8 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
     #pragma unroll 1
     while (t.heapN > 0)
     {
-        const u32 i = t.heap()[0].node;
-        const u32 slot = t.heap()[0].slot;
+        u32 slot;
+        const u32 i = t.top(slot);
         const NodeHead rec = t.head(g, slot, i);
         int at;
         const uint16_t head = t.take(slot, at);
@@ -1672,7 +1718,8 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
         if (fresh || nc.minScore < thisNode.minScore) thisNode.minScore = nc.minScore;
         if (!ws_eq(newEnd, oldEnd))
         {
-            const i32 newEndMin = changed_min_w(newEnd, oldEnd, lane);
+            const i32 newEndBefore = ws_before(newEnd);
+            const i32 newEndMin = changed_min_w(newEnd, newEndBefore, oldEnd, lane);
             if (newEndMin == kIntMax) { err = GA_ASSERT; return res; }
             if (newEndMin <= wadd(curMin, bw))
             {
@@ -1694,7 +1741,7 @@ __device__ __forceinline__ SliceResult fill_slice(const FillArgs& a, Tables& t, 
                         target = g.outNb[r->outOff + e];
                         component = g.comp[target];
                     }
-                    if (!insert(t.slot_of(g, target, component), target, component, newEndMin, newEnd, false, false))
+                    if (!insert(t.slot_of(g, target, component), target, component, newEndMin, newEnd, newEndBefore, false, false))
                     {
                         err = GA_CAPACITY;
                         return res;
@@ -3314,7 +3361,9 @@ __device__ __forceinline__ void fill_extensions(const FillArgs& fa, u32* counter
     if (lane == 0 && arena.used) atomicAdd(fa.arenaCursor + 1, (unsigned long long)arena.used);
 }
 
-__global__ void __launch_bounds__(128, 4) fill_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<SmallTables>(fa, counter); }
+__global__ void __launch_bounds__(128, 4) fill_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<SmallTables<true>>(fa, counter); }
+// the same for graphs that share component numbers
+__global__ void __launch_bounds__(128, 4) fill_shared_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<SmallTables<false>>(fa, counter); }
 
 // The extensions that the fill above handed on, each from the slice it stopped at.
 __global__ void __launch_bounds__(128, 1) fill_medium_kernel(const __grid_constant__ FillArgs fa, u32* counter)
@@ -3494,9 +3543,9 @@ static size_t fill_smem(int warpsPerBlock, gadev::FillTables tables)
         : tables == gadev::FillTables::Medium ? (size_t)gadev::wspace_bytes(gadev::medium_caps()) : 0;
     return (sizeof(gadev::FillWarp) + own) * warpsPerBlock;
 }
-static auto fill_function(gadev::FillTables tables)
+static auto fill_function(gadev::FillTables tables, bool unique)
 {
-    return tables == gadev::FillTables::Small ? gadev::fill_kernel : tables == gadev::FillTables::Medium ? gadev::fill_medium_kernel
+    return tables == gadev::FillTables::Small ? (unique ? gadev::fill_kernel : gadev::fill_shared_kernel) : tables == gadev::FillTables::Medium ? gadev::fill_medium_kernel
         : gadev::fill_large_kernel;
 }
 static size_t trace_smem(int warpsPerBlock) { return sizeof(gadev::TraceWarp) * warpsPerBlock; }
@@ -3509,10 +3558,10 @@ static bool set_smem(const void* kernel, size_t smem)
     return smem <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
 }
 
-int ga_fill_blocks_per_sm(int warpsPerBlock, gadev::FillTables tables)
+int ga_fill_blocks_per_sm(int warpsPerBlock, gadev::FillTables tables, bool unique)
 {
     const size_t smem = fill_smem(warpsPerBlock, tables);
-    const auto kernel = fill_function(tables);
+    const auto kernel = fill_function(tables, unique);
     if (!set_smem((const void*)kernel, smem)) return 0;
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, warpsPerBlock * 32, smem) != cudaSuccess) return 0;
@@ -3532,7 +3581,7 @@ int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint
     int traceBlocks, int warpsPerBlock, void* stream)
 {
     const size_t fillSmem = fill_smem(warpsPerBlock, fa.tables);
-    const auto fill = fill_function(fa.tables);
+    const auto fill = fill_function(fa.tables, fa.g.uniqueComponents != 0);
     const size_t traceSmem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)fill, fillSmem) || !set_smem((const void*)gadev::trace_kernel, traceSmem)) return -1;
     fill<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);

@@ -30,6 +30,7 @@ GA_HD u32 rec_out_degree(u32 meta) { return meta >> 20; }
 struct DevGraph
 {
     const NodeRec* rec;    // [N], or null: the records are put together from the arrays as they are needed
+    u32 uniqueComponents;  // no two nodes share a component number (0: they may)
     u32 N;
     u32 firstAmbiguous;
     const u32* len;
@@ -333,7 +334,7 @@ uint64_t ga_warp_tables_bytes(const gadev::Caps& caps);
 uint64_t ga_multiseed_tables_bytes(const gadev::Caps& caps);
 // resident blocks of 32 * warpsPerBlock threads per SM of the fill kernel (shared: tables in
 // shared memory) and of the traceback kernel
-int ga_fill_blocks_per_sm(int warpsPerBlock, gadev::FillTables tables);
+int ga_fill_blocks_per_sm(int warpsPerBlock, gadev::FillTables tables, bool unique);
 int ga_trace_blocks_per_sm(int warpsPerBlock);
 // launches the fill kernel, with fa.resume the medium tables' (mediumBlocks blocks of one warp),
 // and then the traceback kernel on `stream`, blocks of warpsPerBlock warps, one extension per warp
