@@ -100,7 +100,6 @@ struct GafDevice
     DevGrow<uint64_t> nodeNameOff;
     DevGrow<uint32_t> originalSize, idVal;
     DevGrow<int32_t> idKey;
-    uint64_t idCap = 0;
     gaf::NamesHost host;                  // the same tables on the host (node sizes for the classification)
     // one chunk of lines
     Pinned<uint8_t> hOps, hNames;

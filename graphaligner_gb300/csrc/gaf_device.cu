@@ -220,9 +220,7 @@ gaf::Names device_names(const GafDevice& d)
     nm.nodeNames = d.nodeNames.p;
     nm.nodeNameOff = d.nodeNameOff.p;
     nm.originalSize = d.originalSize.p;
-    nm.idKey = d.idKey.p;
-    nm.idVal = d.idVal.p;
-    nm.idCap = d.idCap;
+    nm.ids = gaf::IdView { d.host.ids.key.empty() ? nullptr : d.idKey.p, d.idVal.p, d.host.ids.val.size(), d.host.ids.base };
     return nm;
 }
 
@@ -347,9 +345,8 @@ int ga_gaf_device_init(GafDevice& d, const gahost::HostGraph& g)
     gaf::build_names(g.lookupIds, g.names, g.originalSize, d.host);
     cudaStream_t s = d.stream;
     if (!upload(d.nodeNames, d.host.nodeNames, s) || !upload(d.nodeNameOff, d.host.nodeNameOff, s) || !upload(d.originalSize, d.host.originalSize, s)
-        || !upload(d.idKey, d.host.idKey, s) || !upload(d.idVal, d.host.idVal, s) || cudaStreamSynchronize(s) != cudaSuccess)
+        || !upload(d.idKey, d.host.ids.key, s) || !upload(d.idVal, d.host.ids.val, s) || cudaStreamSynchronize(s) != cudaSuccess)
         return GA_ERR_CUDA;
-    d.idCap = d.host.idCap;
     return GA_OK;
 }
 
@@ -419,14 +416,8 @@ extern "C" int ga_aligner_format_gaf(ga_aligner_t a, uint32_t num_lines, const g
     const gaf::NamesHost& nh = d.host;
     auto sizeOf = [&nh](int32_t bignode) -> uint64_t
     {
-        uint64_t h = gaf::id_hash(bignode) & (nh.idCap - 1);
-        for (uint64_t k = 0; k < nh.idCap; k++)
-        {
-            if (nh.idKey[h] == bignode) return nh.originalSize[nh.idVal[h]];
-            if (nh.idKey[h] == INT32_MIN) return 0;
-            h = (h + 1) & (nh.idCap - 1);
-        }
-        return 0;
+        const uint32_t i = nh.ids.find(bignode);
+        return i == gaf::kNoId ? 0 : nh.originalSize[i];
     };
     std::vector<gahost::ClassifiedLines> cls(num_lines);
     std::vector<std::string> names(num_lines);

@@ -131,24 +131,24 @@ HostGraph::HostGraph(const ga_host_graph_desc& d) :
     for (size_t i = 0; i < d.num_lookup; i++)
     {
         if (d.names && d.names[i]) names[i] = d.names[i];
-        lookupIndex[lookupIds[i]] = i;
     }
+    lookupIndex.build(lookupIds);
     bpSize = 0;
     for (uint32_t i = 0; i < N; i++) bpSize += len[i];
     // each split node's bigraph node size, so reversing a trace item needs no hash lookup
     bigSize.resize(N);
     for (uint32_t i = 0; i < N; i++)
     {
-        auto f = lookupIndex.find(nodeIds[i]);
-        bigSize[i] = f == lookupIndex.end() ? 0 : originalSize[f->second];
+        const uint32_t f = lookupIndex.find(nodeIds[i]);
+        bigSize[i] = f == gaf::kNoId ? 0 : originalSize[f];
     }
 }
 
 size_t HostGraph::lookup(int bignode) const
 {
-    auto f = lookupIndex.find(bignode);
-    GAH_ASSERT(f != lookupIndex.end());
-    return f->second;
+    const uint32_t f = lookupIndex.find(bignode);
+    GAH_ASSERT(f != gaf::kNoId);
+    return f;
 }
 
 char HostGraph::charAt(size_t node, size_t pos) const
@@ -889,8 +889,8 @@ static void formatFinished(const HostGraph& g, const ReadAlignParams& p, const s
     }
     auto sizeOf = [&g](int32_t bignode) -> uint64_t
     {
-        auto f = g.lookupIndex.find(bignode);
-        return f == g.lookupIndex.end() ? 0 : g.originalSize[f->second];
+        const uint32_t f = g.lookupIndex.find(bignode);
+        return f == gaf::kNoId ? 0 : g.originalSize[f];
     };
     parallelFor(n, [&](size_t i)
     {

@@ -26,7 +26,7 @@ struct HostGraph
     std::vector<int32_t> lookupIds;
     std::vector<uint32_t> originalSize, lookupOff, lookupNodes;
     std::vector<std::string> names;
-    std::unordered_map<int, size_t> lookupIndex;
+    gaf::IdTable lookupIndex;           // bigraph node id -> index in the lookup arrays
     std::vector<uint32_t> bigSize;      // per split node: originalSize of its bigraph node
     size_t bpSize;
     size_t lookup(int bignode) const;
