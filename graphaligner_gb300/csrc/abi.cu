@@ -132,6 +132,7 @@ struct ga_graph
     int device = 0;
     uint32_t N = 0;
     gadev::DevGraph d {};
+    bool tangled = false;     // at least half of the nodes share their component number
     std::vector<void*> allocations;
 };
 
@@ -189,21 +190,27 @@ extern "C" const char* ga_last_error(void) { return g_lastError.c_str(); }
 void ga_set_last_error(const char* message) { g_lastError = message; }
 extern "C" const char* ga_version(void) { return "graphaligner_gb300 0.1 (sm_103a)"; }
 
-// whether no two of the n component numbers are the same (0 also where they are spread too widely to tell cheaply)
-static uint32_t unique_components(const uint32_t* component, uint32_t n)
+// How many of the n nodes share their component number with another, or n + 1 where the numbers are
+// spread too widely to tell cheaply
+static uint64_t shared_components(const uint32_t* component, uint32_t n)
 {
     uint32_t most = 0;
     for (uint32_t i = 0; i < n; i++) most = std::max(most, component[i]);
-    if (most >= 16ull * n + 1024 || most == 0xffffffffu) return 0;
-    std::vector<uint64_t> seen((size_t)most / 64 + 1, 0);
+    if (most >= 16ull * n + 1024 || most == 0xffffffffu) return (uint64_t)n + 1;
+    std::vector<uint64_t> seen((size_t)most / 64 + 1, 0), again(seen.size(), 0);
+    bool any = false;
     for (uint32_t i = 0; i < n; i++)
     {
         uint64_t& word = seen[component[i] / 64];
         const uint64_t bit = 1ull << (component[i] % 64);
-        if (word & bit) return 0;
+        again[component[i] / 64] |= word & bit;
+        any |= (word & bit) != 0;
         word |= bit;
     }
-    return 1;
+    uint64_t shared = 0;
+    if (any)
+        for (uint32_t i = 0; i < n; i++) shared += (again[component[i] / 64] >> (component[i] % 64)) & 1;
+    return shared;
 }
 
 extern "C" int ga_graph_upload(const ga_graph_desc* desc, int device, ga_graph_t* out)
@@ -249,7 +256,9 @@ extern "C" int ga_graph_upload(const ga_graph_desc* desc, int device, ga_graph_t
         return cuda_fail(e, "graph upload");
     }
     g->d.N = N;
-    g->d.uniqueComponents = unique_components(desc->component, N);
+    const uint64_t shared = shared_components(desc->component, N);
+    g->d.uniqueComponents = shared == 0;
+    g->tangled = shared <= N && 2 * shared >= N;
     g->d.firstAmbiguous = desc->first_ambiguous;
     g->d.len = (const uint32_t*)len;
     g->d.seq2 = (const uint64_t*)seq2;
@@ -478,20 +487,23 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
     for (int layout = (int)sh.first_layout; layout < 3; layout++)
     {
         const bool shared = layout == 0;
-        const gadev::Caps caps = layout_caps(layout);
-        const uint64_t stride = ga_warp_tables_bytes(caps);
-        const gadev::FillTables tables = shared ? gadev::FillTables::Small : gadev::FillTables::Global;
-        int fillPerSm = ga_fill_blocks_per_sm(wpb, tables, x->graph->d.uniqueComponents != 0);
         const int mediumPerSm = shared ? ga_fill_blocks_per_sm(1, gadev::FillTables::Medium, false) : 0;
+        // (the line is explained at medium_caps)
+        const bool medium = x->graph->tangled && mediumPerSm > 0 && pending <= (uint64_t)gadev::kMediumWaves * x->sms * mediumPerSm;
+        const gadev::FillTables tables = medium ? gadev::FillTables::Medium : shared ? gadev::FillTables::Small : gadev::FillTables::Global;
+        const int fillWarps = medium ? 1 : wpb;
+        const gadev::Caps caps = medium ? gadev::medium_caps() : layout_caps(layout);
+        const uint64_t stride = ga_warp_tables_bytes(caps);
+        int fillPerSm = ga_fill_blocks_per_sm(fillWarps, tables, x->graph->d.uniqueComponents != 0);
         int tracePerSm = ga_trace_blocks_per_sm(wpb);
         if (fillPerSm <= 0 || tracePerSm <= 0) return fail(GA_ERR_CUDA, "the extension kernels do not fit an SM with this launch shape");
         if (sh.blocks_per_sm > 0)
         {
-            fillPerSm = std::min<int>(fillPerSm, (int)sh.blocks_per_sm);
+            fillPerSm = (int)std::min<uint64_t>(fillPerSm, (uint64_t)sh.blocks_per_sm * wpb / fillWarps);
             tracePerSm = std::min<int>(tracePerSm, (int)sh.blocks_per_sm);
         }
         const uint64_t pendingBlocks = std::max<uint64_t>(1, ((uint64_t)pending + wpb - 1) / wpb);
-        uint64_t fillBlocks = std::min<uint64_t>((uint64_t)x->sms * fillPerSm, pendingBlocks);
+        uint64_t fillBlocks = std::min<uint64_t>((uint64_t)x->sms * fillPerSm, std::max<uint64_t>(1, ((uint64_t)pending + fillWarps - 1) / fillWarps));
         if (!shared) fillBlocks = std::max<uint64_t>(1, std::min<uint64_t>(fillBlocks, x->workspaceBytes / stride / wpb));
         const uint64_t traceBlocks = std::min<uint64_t>((uint64_t)x->sms * tracePerSm, pendingBlocks);
         if (layout > (int)sh.first_layout)
@@ -503,7 +515,7 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
         fa.tables = tables;
         fa.workspace = shared ? nullptr : x->workspace;
         fa.workspaceStride = stride;
-        fa.resume = mediumPerSm > 0 ? x->resume.ptr : nullptr;
+        fa.resume = mediumPerSm > 0 && !medium ? x->resume.ptr : nullptr;
         fa.resumeCap = resumeCap;
         fa.resumeCount = x->counters + 4;
         fa.prevStatus = layout > (int)sh.first_layout ? prevStatus : nullptr;

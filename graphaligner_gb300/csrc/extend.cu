@@ -3398,6 +3398,8 @@ __global__ void __launch_bounds__(128, 1) fill_medium_kernel(const __grid_consta
     }
     if (lane == 0 && arena.used) atomicAdd(fa.arenaCursor + 1, (unsigned long long)arena.used);
 }
+// the extensions of a graph that is mostly cycles, with the medium tables from the start
+__global__ void __launch_bounds__(32, 6) fill_tangled_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<MediumTables>(fa, counter); }
 __global__ void __launch_bounds__(128, 4) fill_large_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<LargeTables>(fa, counter); }
 
 // The traceback: a warp takes the next filled extension and walks its table back.  Four blocks of
@@ -3545,7 +3547,7 @@ static size_t fill_smem(int warpsPerBlock, gadev::FillTables tables)
 }
 static auto fill_function(gadev::FillTables tables, bool unique)
 {
-    return tables == gadev::FillTables::Small ? (unique ? gadev::fill_kernel : gadev::fill_shared_kernel) : tables == gadev::FillTables::Medium ? gadev::fill_medium_kernel
+    return tables == gadev::FillTables::Small ? (unique ? gadev::fill_kernel : gadev::fill_shared_kernel) : tables == gadev::FillTables::Medium ? gadev::fill_tangled_kernel
         : gadev::fill_large_kernel;
 }
 static size_t trace_smem(int warpsPerBlock) { return sizeof(gadev::TraceWarp) * warpsPerBlock; }
@@ -3580,11 +3582,12 @@ int ga_trace_blocks_per_sm(int warpsPerBlock)
 int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int mediumBlocks,
     int traceBlocks, int warpsPerBlock, void* stream)
 {
-    const size_t fillSmem = fill_smem(warpsPerBlock, fa.tables);
+    const int fillWarps = fa.tables == gadev::FillTables::Medium ? 1 : warpsPerBlock;
+    const size_t fillSmem = fill_smem(fillWarps, fa.tables);
     const auto fill = fill_function(fa.tables, fa.g.uniqueComponents != 0);
     const size_t traceSmem = trace_smem(warpsPerBlock);
     if (!set_smem((const void*)fill, fillSmem) || !set_smem((const void*)gadev::trace_kernel, traceSmem)) return -1;
-    fill<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
+    fill<<<fillBlocks, fillWarps * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;
     if (fa.resume)
     {

@@ -151,7 +151,19 @@ struct __align__(16) ResumeRec
 // memory with medium_caps(), or in global memory with FillArgs::caps.
 enum class FillTables { Small, Medium, Global };
 
-// 35 KB a warp: four to five warps on an SM, for the few extensions that outgrow the small tables
+// 35 KB a warp, six warps on an SM: for the few extensions that outgrow the small tables, and from
+// the start for graphs that are mostly cycles (ga_graph::tangled).  There one extension in four to
+// twenty outgrows the small tables, and those, which go on only when all others have ended, are
+// what the call waits for: the 1,000 extensions of 500 tangled reads of 20 kbp take 28.7 ms instead
+// of 38.1, 1,000 of accurate 1 kbp reads 2.7 instead of 4.5, those of 16 such reads 2.1 instead of
+// 2.6.  With 64 band entries, eleven warps on an SM and the rest handed on: 30.2 ms.
+//
+// The small tables let sixteen warps on an SM, and their nodes cost a tenth less.  So all other
+// graphs keep them (a variation graph's reads would take 1.08 times as long), and batches of more
+// than kMediumWaves times the warps that fit the GPU at once (152 SMs: 3,648 extensions): 4,000
+// extensions take 34.5 against 42.9 ms with tangles, 4,800 take 37.5 against 45.4, but 6.7 against
+// 4.6 where a graph has none; 10,000 take 67 against 62.
+static constexpr u32 kMediumWaves = 4;
 inline Caps medium_caps()
 {
     Caps c;
