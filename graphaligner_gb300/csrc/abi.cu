@@ -845,8 +845,8 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
         const gadev::Caps caps = layout_caps(layout);
         const uint64_t stride = ga_multiseed_tables_bytes(caps);
         const uint64_t pendingBlocks = std::max<uint64_t>(1, ((uint64_t)pending + wpb - 1) / wpb);
-        uint64_t fillBlocks = std::min<uint64_t>((uint64_t)x->sms * 4, pendingBlocks);
-        fillBlocks = std::max<uint64_t>(1, std::min<uint64_t>(fillBlocks, x->workspaceBytes / stride / wpb));
+        uint64_t fillBlocks = std::min<uint64_t>((uint64_t)x->sms * 16, std::max<uint64_t>(1, pending));
+        fillBlocks = std::max<uint64_t>(1, std::min<uint64_t>(fillBlocks, x->workspaceBytes / stride));
         const uint64_t readBlocks = std::min<uint64_t>((uint64_t)x->sms * 6, pendingBlocks);
         const uint64_t partBlocks = std::min<uint64_t>((uint64_t)x->sms * 6, ((uint64_t)pending * gadev::kCandParts + wpb - 1) / wpb);
         if (pass > 0) GA_CUDA(cudaMemcpyAsync(x->prevStatus.ptr, x->status.ptr, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));

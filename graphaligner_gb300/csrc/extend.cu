@@ -968,6 +968,33 @@ __device__ __noinline__ FixedRow fix_horizontal_extra(i32 scoreBefore, i32 score
     return FixedRow { fixedHP, fixedHN, forceMask, true };
 }
 
+// The columns 1.. of a seed start of the multiseed DP: its column `extra` joins every column.  hp, hn and
+// fm: the horizontal inputs and the forced columns, bit 0: column 1.  Out of line: 1 node in 300 is one,
+// and inside node_calc this loop made the other columns' 83 cycles a column instead of 36.
+template <bool Fill>
+__device__ __noinline__ WS seeded_columns(WS ws, WS extra, u64 hp, u64 hn, u64 fm, u32 columns, u32 lane)
+{
+    NodeCols& nc = Fill ? fill_cols() : trace_cols();
+    #pragma unroll 1
+    for (u32 pos = 1; pos < columns; pos++)
+    {
+        u64 Ph, Mh;
+        WS nw = myers_step(nc.eqcol[pos], ws, hp & 1, hn & 1, Ph, Mh);
+        if (fm & 1)
+        {
+            nw.VP &= kAllOnes ^ 1;
+            nw.VN |= 1;
+        }
+        hp >>= 1;
+        hn >>= 1;
+        fm >>= 1;
+        ws = merge_w(nw, extra, lane);
+        nc.v[pos] = { ws.VP, ws.VN };
+        nc.x[pos] = { Mh, ws.end, 0 };
+    }
+    return ws;
+}
+
 // calculateNodeInner (Common.h:1113-1478).  nodeLength, c0, c1: the node's length and 2-bit
 // sequence.  flags: the band entry's, 0 for a node that has none yet.  singleInPrevBand: the
 // node's only in-neighbour is in the previous band.  endColumn: the node's last column in this
@@ -1191,26 +1218,7 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
     }
     else
     {
-        // a seed start of the multiseed DP: its column joins every column
-        u64 hp = fixedHP >> 1, hn = fixedHN >> 1, fm = forceMask >> 1;   // bit 0: column 1
-        #pragma unroll 1
-        for (u32 pos = 1; pos < columns; pos++)
-        {
-            const u64 eq = eqcol[pos];
-            u64 Ph, Mh;
-            WS nw = myers_step(eq, ws, hp & 1, hn & 1, Ph, Mh);
-            if (fm & 1)
-            {
-                nw.VP &= kAllOnes ^ 1;
-                nw.VN |= 1;
-            }
-            hp >>= 1;
-            hn >>= 1;
-            fm >>= 1;
-            ws = merge_w(nw, *extra, lane);
-            nc.v[pos] = { ws.VP, ws.VN };
-            nc.x[pos] = { Mh, ws.end, 0 };
-        }
+        ws = seeded_columns<Fill>(ws, *extra, fixedHP >> 1, fixedHN >> 1, forceMask >> 1, columns, lane);
     }
     __syncwarp();
     steps += columns - 1;
@@ -1525,25 +1533,21 @@ struct SliceResult
 
 // getSeedSlice (Common.h:320-353): the column of starting an alignment at each row of the slice
 // at j, each row scored as the X-score's error cost of the read before it (rows past the read's
-// end one more each)
-__device__ __noinline__ WS seed_ws(int64_t j, u32 seqLen, i32 cost)
+// end one more each).  A row's score needs a 64-bit division, so lane k takes rows k and k + 32: row
+// by row in every lane it was 19k of the multiseed fill's 123k cycles per slice.
+__device__ __noinline__ WS seed_ws(int64_t j, u32 seqLen, i32 cost, u32 lane)
 {
-    u64 vp = 0;
-    i32 old = j > 0 ? (i32)((j * 100 + cost / 2) / cost) : 0;
-    #pragma unroll 1
-    for (u32 off = 0; off < 64; off++)
-    {
-        if (j + off >= (int64_t)seqLen)
-        {
-            vp |= 1ULL << off;
-            old += 1;
-            continue;
-        }
-        const i32 score = (i32)(((j + off + 1) * 100 + cost / 2) / cost);
-        if (score == old + 1) vp |= 1ULL << off;
-        old = score;
-    }
-    return ws_make(vp & ~1ULL, 1, old);
+    auto score = [&](u32 before) { return (i32)(((j + before) * 100 + cost / 2) / cost); };
+    const u32 inRead = j + 64 <= (int64_t)seqLen ? 64 : (u32)((int64_t)seqLen - j);     // a slice has one row at least
+    const i32 lo = score(lane + 1), hi = score(lane + 33);
+    const i32 start = j > 0 ? score(0) : 0;
+    const i32 upLo = __shfl_up_sync(kFull, lo, 1), upHi = __shfl_up_sync(kFull, hi, 1), mid = __shfl_sync(kFull, lo, 31);
+    const i32 beforeLo = lane == 0 ? start : upLo, beforeHi = lane == 0 ? mid : upHi;
+    const u32 bitsLo = __ballot_sync(kFull, lane >= inRead || lo == wadd(beforeLo, 1));
+    const u32 bitsHi = __ballot_sync(kFull, lane + 32 >= inRead || hi == wadd(beforeHi, 1));
+    const u32 last = inRead - 1;
+    const i32 endLo = __shfl_sync(kFull, lo, (int)(last & 31)), endHi = __shfl_sync(kFull, hi, (int)(last & 31));
+    return ws_make((((u64)bitsHi << 32) | bitsLo) & ~1ULL, 1, wadd(last < 32 ? endLo : endHi, (i32)(64 - inRead)));
 }
 
 // The seeds the multiseed DP starts in one slice, with the slice's seed-start column.
@@ -1945,7 +1949,7 @@ __device__ ExtState fill_multiseed(const FillArgs& a, LargeTables& t, ArenaCurso
         SliceSeeds seeds;
         seeds.nodes = a.seedNode + k;
         seeds.count = (u32)(next - k);
-        seeds.ws = seed_ws(j, seqLen, a.cost);
+        seeds.ws = seed_ws(j, seqLen, a.cost, lane);
         k = next;
         u32 steps = 0;
         SliceResult res = fill_slice<LargeTables, true>(a, t, arena, seq, seqLen, rows, j, lastQuit, lastMin, steps, err, lane, &seeds);
@@ -2705,7 +2709,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
             }
             self = find_cur(curNode);
             if (!self) { err = GA_ASSERT; break; }
-            if (Multi) extra = (self->node & kSeedStart) ? seed_ws(((int64_t)curSlice - 1) * 64, seqLen, cost) : fake_ws();
+            if (Multi) extra = (self->node & kSeedStart) ? seed_ws(((int64_t)curSlice - 1) * 64, seqLen, cost, lane) : fake_ws();
             const u32 at = (u32)self->minScore;
             if (at != kNoColumns)
             {
@@ -3083,7 +3087,7 @@ __device__ int ms_start_cell(const MultiTraceArgs& a, Table& t, const uint8_t* s
     const u32 node = items[c.index].node & kNodeMask;
     const i32 j = ((i32)c.slice - 1) * 64;
     if (!slice_masks(seq, seqLen, c.slice, lane)) return GA_ASSERT;
-    const WS extra = (items[c.index].node & kSeedStart) ? seed_ws(j, seqLen, a.cost) : fake_ws();
+    const WS extra = (items[c.index].node & kSeedStart) ? seed_ws(j, seqLen, a.cost, lane) : fake_ws();
     int err = recalc<true>(g, a.cost, t, c.slice, node, lane, 63, extra);
     if (err) return err;
     const NodeCols& nc = trace_cols();
@@ -3421,8 +3425,11 @@ __global__ void __launch_bounds__(128, 4) trace_kernel(const __grid_constant__ T
 
 
 // The multiseed DP's fill: a warp takes the next read and fills its whole DP table; its
-// frontier tables and per-node X-scores live in the global workspace.
-__global__ void __launch_bounds__(128, 4) fill_multiseed_kernel(const __grid_constant__ FillArgs fa, u32* counter)
+// frontier tables and per-node X-scores live in the global workspace.  A batch has few reads and waits
+// for its longest one's chain, so a block is one warp, with all the registers it can use: 40 tangled reads
+// of 20 kbp 57.8 -> 53.7 ms with the two functions taken out of line (seed_ws, seeded_columns), 20.5 -> 17.3
+// on a variation graph; 1,000 reads take as long as with four blocks of four warps on an SM.
+__global__ void __launch_bounds__(32, 8) fill_multiseed_kernel(const __grid_constant__ FillArgs fa, u32* counter)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
@@ -3608,9 +3615,9 @@ int ga_launch_multiseed_fill(const gadev::FillArgs& fa, const gadev::MultiTraceA
     int warpsPerBlock, void* stream)
 {
     if (!fa.workspace) return -1;
-    const size_t fillSmem = fill_smem(warpsPerBlock, gadev::FillTables::Global);
+    const size_t fillSmem = fill_smem(1, gadev::FillTables::Global);
     if (!set_smem((const void*)gadev::fill_multiseed_kernel, fillSmem)) return -1;
-    gadev::fill_multiseed_kernel<<<fillBlocks, warpsPerBlock * 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
+    gadev::fill_multiseed_kernel<<<fillBlocks, 32, fillSmem, (cudaStream_t)stream>>>(fa, counters);
     if (cudaGetLastError() != cudaSuccess) return -1;
     gadev::ms_candidates_kernel<<<partBlocks, warpsPerBlock * 32, 0, (cudaStream_t)stream>>>(ta, counters + 1, 0);
     if (cudaGetLastError() != cudaSuccess) return -1;
