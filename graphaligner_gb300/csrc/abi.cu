@@ -1,9 +1,8 @@
 // C ABI of the GB300 seed-extension path (declared in include/graphaligner_gb300.h).
 //
 // Handles own their device memory.  ga_extend_batch copies a host batch in,
-// runs the fill and traceback kernels (with an on-GPU retry at larger
-// per-thread capacities for the few extensions whose band, frontier or trace
-// outgrew the first pass), and copies the results out.  No CPU fallback exists:
+// runs the fill and traceback kernels (and again with larger frontier tables for
+// the few extensions that outgrew the first pass's), and copies the results out.  No CPU fallback exists:
 // every extension is computed by the kernels or reported with its status.
 #include <cuda_runtime.h>
 #include <algorithm>

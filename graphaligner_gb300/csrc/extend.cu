@@ -1,10 +1,12 @@
 // Batched seed extension on GB300: one warp per extension.
 //
-// Two persistent kernels run back to back.  In the fill kernel a warp owns one
+// Persistent kernels run back to back.  In the fill kernel a warp owns one
 // extension at a time and runs the banded Myers DP over the graph with the
 // component-ordered frontier and X-drop, writing each committed slice into the
-// batch's DP-table arena; the traceback kernel then gives each warp one filled
-// extension to walk back.  The DP of one extension is a sequential chain: each
+// batch's DP-table arena and, while there is room, each column into the column
+// store; a second fill goes on with the extensions that outgrew the first one's
+// tables; the traceback kernel then gives each warp one filled extension to walk
+// back.  The DP of one extension is a sequential chain: each
 // 64-row slice depends on the whole band of the previous one, and inside a slice
 // nodes are computed one at a time in frontier order, the admission test using the
 // running minimum.  So a warp runs that control flow warp-uniformly (every lane
@@ -12,22 +14,25 @@
 // work that is parallel inside it:
 //   - the match masks of a slice (lane k reads rows k and k + 32; ballots),
 //   - the match mask of every column of a node, before its column loop,
-//   - per node: the X-score of every column (lane k scores columns k and k + 32),
-//     the minimum and its first column (reduce + ballot) and the bottom-row
-//     horizontal deltas (ballots), so the column loop itself only runs the
-//     Myers recurrence,
+//   - per node: the horizontal deltas of every column, its X-score (lane k:
+//     columns k and k + 32), the minimum and its first column (reduce + ballot) and
+//     the bottom-row deltas (ballots), so the column loop itself only runs the
+//     Myers recurrence on VP and VN,
 //   - cellwise merges of columns and the changed-minimum test (row scores by
 //     popcount, then a shuffle, ballots and a reduction),
-//   - node-table lookups: 32 probes of the open-addressing table per step (ballot),
+//   - the small tables' node table, a slot per lane (ballots); the larger tables'
+//     lookups, 32 probes of the open-addressing table per step,
 //   - committing a slice to the DP table (coalesced copies),
-//   - the traceback's end-cell choice (slices and columns across lanes) and its
-//     band lookups (ballot over the slice's node ids),
-//   - trace output, staged in shared memory and written 32 items at a time.
-// The fill's frontier tables (two bands, two node tables, the heap, the pending
-// incoming columns) and a node's recorded columns live in shared memory; an
-// extension that outgrows them is re-run with larger tables in global memory.
+//   - the traceback's end-cell choice (slices and columns across lanes), its band
+//     lookups (ballot over the slice's node ids), and its walk inside a node and
+//     slice: whole runs of one direction at a time, found in the columns' bits.
+// The fill's frontier tables come in three sizes (see FillTables): the small ones
+// in lane registers and shared memory, the medium ones in shared memory, the large
+// ones in global memory.  A node's recorded columns are in shared memory always.
 // Fill and traceback are separate kernels so that the warps of an SM share one
-// phase's code: fused, the two phases' code did not fit the instruction caches.
+// phase's code.  With the traceback run by the fill's warps right after it, 50,000
+// extensions (250 Mbp) took 95 ms instead of 51: the two phases' code does not fit
+// the instruction caches.
 // Cold paths (crossing rules, end-cell choice, sequential fallbacks) are out of line.
 //
 // Warps take extensions from a device counter over a longest-first order.

@@ -247,10 +247,11 @@ int ga_extender_last_launches(ga_extender_t ext, uint32_t* launches);
  * each warp taking the next of the batch's longest-first order.  warps_per_block
  * (1..4) warps share a block; blocks_per_sm caps the resident blocks per SM (0 = as
  * many as registers and shared memory allow).  first_layout picks the fill's frontier
- * tables in the first pass: 0 = small tables in shared memory (variation graphs),
- * 1 = medium tables in global memory, 2 = large tables in global memory (tangled de
- * Bruijn graphs); extensions that outgrow them (GA_CAPACITY) run again with the next
- * layout.  chunk_kib (1..2^20): the arena bytes a warp takes at once for the DP
+ * tables in the first pass: 0 = tables in shared memory (band 32, and where an extension
+ * outgrows that a second fill goes on with band 128; band 128 at once, in blocks of one
+ * warp, for batches of moderate size on graphs that are mostly cycles), 1 = tables in
+ * global memory (band 512), 2 = large ones in global memory; extensions that outgrow
+ * them (GA_CAPACITY) run again with the next layout.  chunk_kib (1..2^20): the arena bytes a warp takes at once for the DP
  * tables of the extensions it fills. */
 typedef struct ga_launch_shape {
     uint32_t warps_per_block;
@@ -272,7 +273,8 @@ int ga_extender_autotune(ga_extender_t ext, const ga_extend_params* params,
                          uint32_t count, uint32_t repeats, float* ms_out);
 /* DP-table bytes the first pass of the last call wrote to the arena. */
 int ga_extender_last_arena_bytes(ga_extender_t ext, uint64_t* bytes);
-/* Extensions run with each table layout (0, 1, 2) by the last call (0 = layout not run). */
+/* Extensions run with each table layout (0, 1, 2) by the last call (0 = layout not run).  Layout 1's
+ * include those that layout 0's second fill went on with. */
 int ga_extender_last_layout_counts(ga_extender_t ext, uint32_t counts[3]);
 /* The last multiseed call's local-maximum candidates, the walks that counted their traces
  * (candidates the traces kept before them ruled out are not walked), the traces it kept and
