@@ -3531,9 +3531,8 @@ __global__ void __launch_bounds__(128, 6) ms_resolve_kernel(const __grid_constan
 
 // The candidates' traces, a warp per candidate (write = false: the round's queued walks,
 // counted; write = true: the kept ones written).  A read's traces spread over as many warps
-// as it has walks in the round.  A round waits for its longest walk, so the state of a walk stays in
-// registers (at four blocks on an SM 222 bytes a thread did not): 200 reads 86.9 -> 85.0 ms.
-__global__ void __launch_bounds__(128, 2) ms_trace_kernel(const __grid_constant__ MultiTraceArgs ta, u32* counter, int write)
+// as it has walks in the round.
+__global__ void __launch_bounds__(128, 4) ms_trace_kernel(const __grid_constant__ MultiTraceArgs ta, u32* counter, int write)
 {
     load_iupac_table();
     const u32 lane = threadIdx.x & 31;
