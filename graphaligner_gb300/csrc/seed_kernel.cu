@@ -64,23 +64,27 @@ __device__ __forceinline__ bool probe(const SeedTable& t, uint64_t kmer, uint32_
 // included, 0.46 -> 0.11 ms; of 200 reads 1.06 -> 0.40 ms; of 100 reads of 20 kbp 1.26 -> 0.42 ms).
 constexpr int kSteps = 4, kWarps = 8;
 
-// The last position before `at` that was looked up, when the k-mer ending at `at` repeats the one
-// before it: a run of one base that began at some b, so that its first k-mer was looked up, then
-// every realWindow-th (and every one below realWindow).
-__device__ __noinline__ int64_t lookup_before(const uint8_t* s, int64_t at, int64_t k, int64_t realWindow, uint32_t lane)
+// Where the run of base code c that ends before `at` began.  It is looked for back to `round`, the start of
+// the segments that are walked together (32 divides at - round); a run that is older than that began
+// at `carried`, which the round before left.  So a read takes time linear in its length: with every
+// segment of a homopolymer walking back to its beginning, the lookups of a run of 131 kbp took 32 ms
+// and twice the length four times as long; now 2.1 ms, and 16 ms for 1 Mbp.
+__device__ __noinline__ int64_t run_start(const uint8_t* s, int64_t at, int c, int64_t round, int64_t carried, uint32_t lane)
 {
-    const int c = base_code(s[at]);
-    int64_t first = 0;
-    for (int64_t end = at; end > 0; end -= 32)
+#pragma unroll 1
+    for (int64_t end = at; end > round; end -= 32)
     {
-        const int64_t p = end - 1 - lane;
-        const uint32_t other = __ballot_sync(kAllLanes, p < 0 || base_code(s[p]) != c);
-        if (other)
-        {
-            first = end - (__ffs((int)other) - 1);
-            break;
-        }
+        const uint32_t other = __ballot_sync(kAllLanes, base_code(s[end - 1 - lane]) != c);
+        if (other) return end - (__ffs((int)other) - 1);
     }
+    return round > 0 && base_code(s[round - 1]) == c ? carried : round;
+}
+
+// The last position before `at` that was looked up, when the k-mer ending at `at` repeats the one
+// before it: a run of one base that began at `first`, so that its first k-mer was looked up, then
+// every realWindow-th (and every one below realWindow).
+__device__ __forceinline__ int64_t lookup_before(int64_t at, int64_t first, int64_t k, int64_t realWindow)
+{
     int64_t last = first + k - 1;
     if (last < realWindow - 1) last = at - 1 < realWindow - 1 ? at - 1 : realWindow - 1;
     return last + (at - 1 - last) / realWindow * realWindow;
@@ -90,6 +94,7 @@ __global__ void __launch_bounds__(32 * kWarps) seed_lookup_kernel(SeedTable t, u
     const uint8_t* seq, const uint64_t* seqOff, const uint32_t* seqLen, const uint64_t* outOff, SeedMatch* out, uint32_t* outCount)
 {
     __shared__ uint32_t found[2][kWarps];
+    __shared__ int64_t runBefore[2];        // where the run of one base that ends before the round began
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t r = blockIdx.x;
     const uint8_t* s = seq + seqOff[r];
@@ -166,7 +171,8 @@ __global__ void __launch_bounds__(32 * kWarps) seed_lookup_kernel(SeedTable t, u
                 {
                     // positions in order: a repeat is looked up when the last lookup lies w-k+1 back
                     // (or the position is below w-k+1)
-                    if (q == 0 && (repeats & 1) && from > 0) lastPos = lookup_before(s, from, k, realWindow, lane);
+                    if (q == 0 && (repeats & 1) && from > 0)
+                        lastPos = lookup_before(from, run_start(s, from, __shfl_sync(kAllLanes, c, 0), round, round ? runBefore[turn] : 0, lane), k, realWindow);
                     look = 0;
                     const uint32_t validMask = __ballot_sync(kAllLanes, valid);
 #pragma unroll 1
@@ -216,6 +222,12 @@ __global__ void __launch_bounds__(32 * kWarps) seed_lookup_kernel(SeedTable t, u
                 hits[q] = __ballot_sync(kAllLanes, hit[q] && slot[q].count < t.maxCount);
                 own += __popc(hits[q]);
             }
+        }
+        const int64_t next = round + 32 * kSteps * kWarps;
+        if (warp == kWarps - 1 && next < len)
+        {
+            const int64_t began = run_start(s, next, base_code(s[next - 1]), round, round ? runBefore[turn] : 0, lane);
+            if (lane == 0) runBefore[turn ^ 1] = began;
         }
         // the segments' matches one behind the other (two rows: a warp may be a round ahead)
         if (lane == 0) found[turn][warp] = own;
