@@ -37,25 +37,6 @@ __device__ __forceinline__ int base_code(uint8_t c)
     return -1;
 }
 
-__device__ __forceinline__ bool probe(const SeedTable& t, uint64_t kmer, uint32_t& start, uint32_t& count)
-{
-    uint64_t h = seed_slot_hash(kmer) & (t.capacity - 1);
-#pragma unroll 1
-    for (uint64_t n = 0; n < t.capacity; n++)
-    {
-        const SeedSlot s = t.slots[h];
-        if (s.key == kEmptyKmer) return false;
-        if (s.key == kmer)
-        {
-            start = s.start;
-            count = s.count;
-            return true;
-        }
-        h = (h + 1) & (t.capacity - 1);
-    }
-    return false;
-}
-
 // A block per read, kWarps segments of 32 kSteps positions at a time.  A warp knows what it needs of
 // the positions before its segment from the 32 bases there (and, inside a homopolymer longer than a
 // k-mer, from where that began); the segments' matches are placed by a sum over the warps.  The
