@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 #include "extend.cuh"
+#include "launch_grid.h"
 #include "trace_dedupe.h"
 #include "../../include/graphaligner_gb300.h"
 
@@ -493,18 +494,11 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
         const int fillWarps = medium ? 1 : wpb;
         const gadev::Caps caps = medium ? gadev::medium_caps() : layout_caps(layout);
         const uint64_t stride = ga_warp_tables_bytes(caps);
-        int fillPerSm = ga_fill_blocks_per_sm(fillWarps, tables, x->graph->d.uniqueComponents != 0);
-        int tracePerSm = ga_trace_blocks_per_sm(wpb);
+        const int fillPerSm = ga_fill_blocks_per_sm(fillWarps, tables, x->graph->d.uniqueComponents != 0);
+        const int tracePerSm = ga_trace_blocks_per_sm(wpb);
         if (fillPerSm <= 0 || tracePerSm <= 0) return fail(GA_ERR_CUDA, "the extension kernels do not fit an SM with this launch shape");
-        if (sh.blocks_per_sm > 0)
-        {
-            fillPerSm = (int)std::min<uint64_t>(fillPerSm, (uint64_t)sh.blocks_per_sm * wpb / fillWarps);
-            tracePerSm = std::min<int>(tracePerSm, (int)sh.blocks_per_sm);
-        }
-        const uint64_t pendingBlocks = std::max<uint64_t>(1, ((uint64_t)pending + wpb - 1) / wpb);
-        uint64_t fillBlocks = std::min<uint64_t>((uint64_t)x->sms * fillPerSm, std::max<uint64_t>(1, ((uint64_t)pending + fillWarps - 1) / fillWarps));
-        if (!shared) fillBlocks = std::max<uint64_t>(1, std::min<uint64_t>(fillBlocks, x->workspaceBytes / stride / wpb));
-        const uint64_t traceBlocks = std::min<uint64_t>((uint64_t)x->sms * tracePerSm, pendingBlocks);
+        gadev::LaunchGrid grid = gadev::launch_grid(sh, x->sms, fillPerSm, fillWarps, mediumPerSm, tracePerSm, pending, resumeCap);
+        if (!shared) grid.fill = std::max<uint64_t>(1, std::min<uint64_t>(grid.fill, x->workspaceBytes / stride / wpb));
         if (layout > (int)sh.first_layout)
         {
             // only extensions that ran out of a capacity in the previous round run again
@@ -522,8 +516,7 @@ static int run_device(ga_extender* x, const ga_extend_params* p, const ga_extend
         GA_CUDA(cudaMemsetAsync(x->counters, 0, 16 * sizeof(uint32_t), stream));
         GA_CUDA(cudaMemsetAsync(x->arenaCursor, 0, 3 * sizeof(unsigned long long), stream));
         GA_CUDA(cudaEventRecord(x->ev[0], stream));
-        if (ga_launch_extend(fa, ta, x->counters, (int)fillBlocks, (int)std::min<uint64_t>((uint64_t)x->sms * mediumPerSm, resumeCap),
-                (int)traceBlocks, wpb, stream) != 0)
+        if (ga_launch_extend(fa, ta, x->counters, (int)grid.fill, (int)grid.medium, (int)grid.trace, wpb, stream) != 0)
             return fail(GA_ERR_CUDA, std::string("extension kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
         x->lastLaunches += fa.resume ? 3 : 2;
         x->lastRounds[layout] += pending;
