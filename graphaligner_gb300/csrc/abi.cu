@@ -19,6 +19,7 @@
 namespace
 {
 thread_local std::string g_lastError;
+thread_local cudaError_t g_lastCuda = cudaSuccess;     // of the last call that GA_CUDA refused
 
 int fail(int code, const std::string& msg)
 {
@@ -28,6 +29,7 @@ int fail(int code, const std::string& msg)
 
 int cuda_fail(cudaError_t e, const char* what)
 {
+    g_lastCuda = e;
     return fail(GA_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -156,6 +158,7 @@ struct ga_extender
     unsigned long long* arenaCursor = nullptr;   // [0] overflow cursor, [1] bytes taken, [2] column store units taken
     gadev::ColumnUnit* store = nullptr;    // the column store, grown to the largest batch within its bound
     uint64_t storeUnits = 0;
+    bool storeWithheld = false;            // this call goes without a column store
     float lastFillMs = 0;
     float lastTraceMs = 0;
     float lastH2DMs = 0;                    // host-buffer copies of the last ga_extend_batch
@@ -400,12 +403,42 @@ extern "C" int ga_extender_free(ga_extender_t x)
     return GA_OK;
 }
 
+static void release_store(ga_extender* x)
+{
+    cudaFree(x->store);
+    x->store = nullptr;
+    x->storeUnits = 0;
+}
+
+bool ga_extender_give_back_store(ga_extender_t x)
+{
+    if (!x || !x->store) return false;
+    cudaGetLastError();
+    release_store(x);
+    return true;
+}
+
+// Runs a call that may find no memory for its buffers while the column store, which only saves
+// time, holds some: the store is then given back and the call made again without one.
+template <class Call>
+static int with_store_given_back(ga_extender* x, Call call)
+{
+    g_lastCuda = cudaSuccess;
+    int rc = call();
+    if (rc != GA_ERR_CUDA || g_lastCuda != cudaErrorMemoryAllocation || !ga_extender_give_back_store(x)) return rc;
+    x->storeWithheld = true;
+    rc = call();
+    x->storeWithheld = false;
+    return rc;
+}
+
 // Room in the column store for a batch of readBp bases: a band of bandwidth 10 computes 2.4
 // columns per base on the variation graphs (5.5 on the tangled ones), 3 and a chunk for every
 // warp are asked for.  The store holds at most four times the arena and half of the memory that
 // is free when it grows; what finds no room in it is recomputed by the traceback.
 static void reserve_store(ga_extender* x, uint64_t readBp, uint64_t warps)
 {
+    if (x->storeWithheld) return;
     const uint64_t unit = sizeof(gadev::ColumnUnit);
     uint64_t want = readBp * 3 + warps * gadev::kStoreChunk;
     want = std::min<uint64_t>({want, x->arenaBytes * 4 / unit, (uint64_t)gadev::kNoColumns - 1});
@@ -415,9 +448,7 @@ static void reserve_store(ga_extender* x, uint64_t readBp, uint64_t warps)
     const uint64_t most = std::min<uint64_t>({(freeBytes / unit + x->storeUnits) / 2, x->arenaBytes * 4 / unit, (uint64_t)gadev::kNoColumns - 1});
     want = std::min(most, std::max(want, x->storeUnits * 3 / 2));
     if (want <= x->storeUnits) return;
-    cudaFree(x->store);
-    x->store = nullptr;
-    x->storeUnits = 0;
+    release_store(x);
     if (cudaMalloc((void**)&x->store, (want + gadev::kStorePad) * unit) == cudaSuccess) x->storeUnits = want;
     else
     {
@@ -620,9 +651,8 @@ static int stage_host_batch(ga_extender* x, const ga_extend_batch_desc* b, ga_ex
     return GA_OK;
 }
 
-extern "C" int ga_extend_batch(ga_extender_t x, const ga_extend_params* p, const ga_extend_batch_desc* b, ga_extend_results* r)
+static int extend_host_batch(ga_extender* x, const ga_extend_params* p, const ga_extend_batch_desc* b, ga_extend_results* r)
 {
-    if (!x || !p || !b || !r) return fail(GA_ERR_ARGUMENT, "null argument");
     GA_CUDA(cudaSetDevice(x->graph->device));
     x->lastH2DMs = x->lastD2HMs = 0;
     const uint32_t n = b->num;
@@ -656,6 +686,12 @@ extern "C" int ga_extend_batch(ga_extender_t x, const ga_extend_params* p, const
     GA_CUDA(cudaEventElapsedTime(&x->lastH2DMs, x->ev[3], x->ev[4]));
     GA_CUDA(cudaEventElapsedTime(&x->lastD2HMs, x->ev[2], x->ev[5]));
     return GA_OK;
+}
+
+extern "C" int ga_extend_batch(ga_extender_t x, const ga_extend_params* p, const ga_extend_batch_desc* b, ga_extend_results* r)
+{
+    if (!x || !p || !b || !r) return fail(GA_ERR_ARGUMENT, "null argument");
+    return with_store_given_back(x, [&] { return extend_host_batch(x, p, b, r); });
 }
 
 // ---- multiseed DP ----
@@ -1072,23 +1108,19 @@ static int multiseed_run(ga_extender_t x, const ga_extend_params* p, const ga_mu
 
 extern "C" int ga_multiseed_batch(ga_extender_t x, const ga_extend_params* p, const ga_multiseed_batch_desc* b, ga_multiseed_results* r)
 {
-    if (!r) return fail(GA_ERR_ARGUMENT, "null argument");
-    return multiseed_run(x, p, b, r, nullptr);
+    if (!x || !r) return fail(GA_ERR_ARGUMENT, "null argument");
+    return with_store_given_back(x, [&] { return multiseed_run(x, p, b, r, nullptr); });
 }
 
 extern "C" int ga_multiseed_batch_exact(ga_extender_t x, const ga_extend_params* p, const ga_multiseed_batch_desc* b, ga_multiseed_output* out)
 {
-    if (!out) return fail(GA_ERR_ARGUMENT, "null argument");
-    return multiseed_run(x, p, b, nullptr, out);
+    if (!x || !out) return fail(GA_ERR_ARGUMENT, "null argument");
+    return with_store_given_back(x, [&] { return multiseed_run(x, p, b, nullptr, out); });
 }
 
-extern "C" int ga_extender_autotune(ga_extender_t x, const ga_extend_params* p, const ga_extend_batch_desc* b,
-    const ga_launch_shape* shapes, uint32_t count, uint32_t repeats, float* ms_out)
+static int autotune(ga_extender* x, const ga_extend_params* p, const ga_extend_batch_desc* b, const ga_launch_shape* shapes, uint32_t count,
+    uint32_t repeats, float* ms_out)
 {
-    if (!x || !p || !b || !shapes) return fail(GA_ERR_ARGUMENT, "null argument");
-    if (count == 0) return fail(GA_ERR_ARGUMENT, "no launch shapes");
-    for (uint32_t i = 0; i < count; i++)
-        if (!shape_ok(shapes[i])) return fail(GA_ERR_ARGUMENT, kShapeError);
     GA_CUDA(cudaSetDevice(x->graph->device));
     x->lastH2DMs = x->lastD2HMs = 0;
     const uint32_t n = b->num;
@@ -1132,10 +1164,18 @@ extern "C" int ga_extender_autotune(ga_extender_t x, const ga_extend_params* p, 
     return GA_OK;
 }
 
-extern "C" int ga_extend_batch_device(ga_extender_t x, const ga_extend_params* p, const ga_extend_batch_desc* b,
-    ga_extend_results* r, void* stream)
+extern "C" int ga_extender_autotune(ga_extender_t x, const ga_extend_params* p, const ga_extend_batch_desc* b,
+    const ga_launch_shape* shapes, uint32_t count, uint32_t repeats, float* ms_out)
 {
-    if (!x || !p || !b || !r) return fail(GA_ERR_ARGUMENT, "null argument");
+    if (!x || !p || !b || !shapes) return fail(GA_ERR_ARGUMENT, "null argument");
+    if (count == 0) return fail(GA_ERR_ARGUMENT, "no launch shapes");
+    for (uint32_t i = 0; i < count; i++)
+        if (!shape_ok(shapes[i])) return fail(GA_ERR_ARGUMENT, kShapeError);
+    return with_store_given_back(x, [&] { return autotune(x, p, b, shapes, count, repeats, ms_out); });
+}
+
+static int extend_device_batch(ga_extender* x, const ga_extend_params* p, const ga_extend_batch_desc* b, ga_extend_results* r, void* stream)
+{
     GA_CUDA(cudaSetDevice(x->graph->device));
     x->lastH2DMs = x->lastD2HMs = 0;
     const uint32_t n = b->num;
@@ -1152,6 +1192,13 @@ extern "C" int ga_extend_batch_device(ga_extender_t x, const ga_extend_params* p
     GA_CUDA(x->prevStatus.reserve(n));
     GA_CUDA(cudaMemcpyAsync(x->order.ptr, order.data(), n * 4ULL, cudaMemcpyHostToDevice, s));
     return run_device(x, p, b, r, x->order.ptr, x->prevStatus.ptr, sum_lengths(len.data(), n), s);
+}
+
+extern "C" int ga_extend_batch_device(ga_extender_t x, const ga_extend_params* p, const ga_extend_batch_desc* b,
+    ga_extend_results* r, void* stream)
+{
+    if (!x || !p || !b || !r) return fail(GA_ERR_ARGUMENT, "null argument");
+    return with_store_given_back(x, [&] { return extend_device_batch(x, p, b, r, stream); });
 }
 
 extern "C" int ga_extender_last_kernel_ms(ga_extender_t x, float* ms)

@@ -226,6 +226,18 @@ int ga_aligner_seed(ga_aligner* a, uint32_t n, const char* const* names, const u
     return GA_OK;
 }
 
+// The same between the aligner's extensions: where the device has no memory for the buffers, once more
+// without the lanes' column stores.
+static int seed_idle(ga_aligner* a, uint32_t n, const char* const* names, const uint8_t* seq, const uint64_t* seqOffset, const uint32_t* seqLen,
+    std::vector<gahost::ReadInput>& reads)
+{
+    int rc = ga_aligner_seed(a, n, names, seq, seqOffset, seqLen, reads);
+    if (rc != GA_ERR_CUDA) return rc;
+    bool given = false;
+    for (auto& l : a->lanes) given |= ga_extender_give_back_store(l.ext);
+    return given ? ga_aligner_seed(a, n, names, seq, seqOffset, seqLen, reads) : rc;
+}
+
 extern "C" int ga_aligner_create(ga_extender_t ext, const ga_host_graph_desc* graph, const ga_align_params* params, ga_aligner_t* out)
 {
     if (!ext || !graph || !params || !out) return GA_ERR_ARGUMENT;
@@ -325,7 +337,7 @@ extern "C" int ga_align_reads(ga_aligner_t a, uint32_t n, const char* const* nam
     // ---- k-mer lookups on the GPU, seed selection on the host ----
     auto ts = std::chrono::steady_clock::now();
     std::vector<gahost::ReadInput> reads;
-    int rc = ga_aligner_seed(a, n, names, seq, seqOffset, seqLen, reads);
+    int rc = seed_idle(a, n, names, seq, seqOffset, seqLen, reads);
     if (rc != GA_OK) return rc;
     for (const auto& r : reads) if (!r.seeds.empty()) a->stats.reads_with_seeds++;
     a->stats.seed_ms = ms_since(ts);
@@ -407,7 +419,7 @@ extern "C" int ga_aligner_get_seeds(ga_aligner_t a, uint32_t n, const uint8_t* s
     cudaSetDevice(a->device);
     std::vector<const char*> names(n, nullptr);
     std::vector<gahost::ReadInput> reads;
-    int rc = ga_aligner_seed(a, n, names.data(), seq, seqOffset, seqLen, reads);
+    int rc = seed_idle(a, n, names.data(), seq, seqOffset, seqLen, reads);
     if (rc != GA_OK) return rc;
     a->seedOffsets.assign(n + 1, 0);
     for (uint32_t i = 0; i < n; i++) a->seedOffsets[i + 1] = a->seedOffsets[i] + reads[i].seeds.size();

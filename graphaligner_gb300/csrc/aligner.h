@@ -184,6 +184,9 @@ struct ga_aligner
 int ga_aligner_seed(ga_aligner* a, uint32_t n, const char* const* names, const uint8_t* seq, const uint64_t* seqOffset,
     const uint32_t* seqLen, std::vector<gahost::ReadInput>& reads);
 
+// Gives back the column store of an extender none of whose calls is running (abi.cu); false if it has none
+bool ga_extender_give_back_store(ga_extender_t x);
+
 // gahost::ExtendFn over ga_extend_batch (ctx = ExtendLane*)
 void ga_aligner_extend(void* ctx, const std::vector<gahost::ExtensionRequest>& rq, std::vector<gahost::ExtensionResult>& rs);
 
