@@ -447,7 +447,9 @@ static void reserve_store(ga_extender* x, uint64_t readBp, uint64_t warps)
     if (cudaMemGetInfo(&freeBytes, &totalBytes) != cudaSuccess) return;
     const uint64_t most = std::min<uint64_t>({(freeBytes / unit + x->storeUnits) / 2, x->arenaBytes * 4 / unit, (uint64_t)gadev::kNoColumns - 1});
     want = std::min(most, std::max(want, x->storeUnits * 3 / 2));
-    if (want <= x->storeUnits) return;
+    // where free memory is the bound it moves with every other allocation of the process: a store that
+    // would gain less than a quarter stays as it is (growing it frees it first, which waits for the device)
+    if (want <= x->storeUnits || (want == most && want < x->storeUnits + x->storeUnits / 4)) return;
     release_store(x);
     if (cudaMalloc((void**)&x->store, (want + gadev::kStorePad) * unit) == cudaSuccess) x->storeUnits = want;
     else

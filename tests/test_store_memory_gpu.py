@@ -134,3 +134,28 @@ def test_seeding(cuda_lib, other):
     assert list(got[:3]) == list(want) and not any(len(x) for x in got[3:])
     a.close()
     ext.close()
+
+
+def test_bounded_store_stays(cuda_lib, other):
+    """Where free memory bounds the store, a little more of it does not make the store move."""
+    g, one = golden_case("vg50k")
+    params = ExtendParams(bandwidth=10)
+    dgraph = DeviceGraph(g)
+    load_kernels(dgraph, params, one)
+    ext = Extender(dgraph, arena_bytes=ARENA)
+    batch = filling_batch(g)[1]
+    spare = OtherUser()
+    other.leave(STORE + batch.total_items * 8 + 32 * MB)
+    spare.leave(free_bytes() - 32 * MB)
+    before = free_bytes()
+    ext.run(params, batch)
+    held = before - free_bytes()
+    assert held > batch.total_items * 8 + 64 * MB        # a store, and not the whole one
+    assert held < batch.total_items * 8 + STORE
+    left = free_bytes()
+    spare.close()
+    freed = free_bytes() - left
+    assert freed >= 32 * MB
+    ext.run(params, batch)
+    assert free_bytes() == left + freed
+    ext.close()
