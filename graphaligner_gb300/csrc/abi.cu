@@ -30,6 +30,7 @@ int fail(int code, const std::string& msg)
 int cuda_fail(cudaError_t e, const char* what)
 {
     g_lastCuda = e;
+    cudaGetLastError();      // reported here: the next launch's check must not find it again
     return fail(GA_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -71,7 +72,11 @@ struct HostPinned
         if (n <= count) return true;
         const size_t grow = std::max(n, count * 3 / 2);
         T* q = nullptr;
-        if (cudaHostAlloc((void**)&q, grow * sizeof(T), cudaHostAllocDefault) != cudaSuccess) return false;
+        if (cudaHostAlloc((void**)&q, grow * sizeof(T), cudaHostAllocDefault) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return false;
+        }
         if (keep) memcpy(q, ptr, keep * sizeof(T));
         if (ptr) cudaFreeHost(ptr);
         ptr = q;
@@ -413,7 +418,6 @@ static void release_store(ga_extender* x)
 bool ga_extender_give_back_store(ga_extender_t x)
 {
     if (!x || !x->store) return false;
-    cudaGetLastError();
     release_store(x);
     return true;
 }

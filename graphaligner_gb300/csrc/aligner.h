@@ -20,7 +20,11 @@ struct Pinned
         if (n <= cap) return true;
         size_t want = std::max(n, cap + cap / 2);
         void* q = nullptr;
-        if (cudaHostAlloc(&q, want * sizeof(T), cudaHostAllocDefault) != cudaSuccess) return false;
+        if (cudaHostAlloc(&q, want * sizeof(T), cudaHostAllocDefault) != cudaSuccess)
+        {
+            cudaGetLastError();      // reported by the result: the next launch's check must not find it again
+            return false;
+        }
         if (p) cudaFreeHost(p);
         p = (T*)q;
         cap = want;
@@ -43,7 +47,11 @@ struct DevGrow
         if (n <= cap) return true;
         size_t want = std::max(n, cap + cap / 2);
         void* q = nullptr;
-        if (cudaMalloc(&q, want * sizeof(T)) != cudaSuccess) return false;
+        if (cudaMalloc(&q, want * sizeof(T)) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return false;
+        }
         if (p) cudaFree(p);
         p = (T*)q;
         cap = want;

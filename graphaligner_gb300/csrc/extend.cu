@@ -3666,6 +3666,7 @@ int ga_launch_multiseed_write(const gadev::MultiTraceArgs& ta, uint32_t* counter
 
 int ga_build_node_records(const gadev::DevGraph& g, gadev::NodeRec* rec, void* stream)
 {
+    cudaGetLastError();      // an upload fails by its own errors only, not by one that the process has left
     gadev::node_records_kernel<<<(g.N + 255) / 256, 256, 0, (cudaStream_t)stream>>>(g, rec);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -454,6 +454,7 @@ int ga_build_index_gpu(const gahost::HostGraph& hg, size_t k, size_t w, double k
     {
         error = std::string("index build: ") + what + (e != cudaSuccess ? std::string(": ") + cudaGetErrorString(e) : std::string());
         release();
+        cudaGetLastError();      // reported here: the next launch's check must not find it again
         return e != cudaSuccess ? -2 : -1;
     };
 #define IDX_CUDA(call, what) do { cudaError_t _e = (call); if (_e != cudaSuccess) return fail(what, _e); } while (0)
