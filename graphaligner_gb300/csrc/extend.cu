@@ -128,6 +128,9 @@ __device__ __noinline__ void gather_record(const DevGraph& g, u32 node, NodeRec&
 {
     const u32 in = g.inOff[node], inN = g.inOff[node + 1] - in;
     const u32 out = g.outOff[node], outN = g.outOff[node + 1] - out;
+    // a record is made of every node, whether an extension comes near it or not: what an inconsistent
+    // graph's arrays say about a node is not followed outside them
+    const u32 inEnd = g.inOff[g.N], outEnd = g.outOff[g.N];
     r.seq[0] = node < g.firstAmbiguous ? g.seq2[(u64)node * 2] : 0;
     r.seq[1] = node < g.firstAmbiguous ? g.seq2[(u64)node * 2 + 1] : 0;
     r.comp = g.comp[node];
@@ -135,11 +138,11 @@ __device__ __noinline__ void gather_record(const DevGraph& g, u32 node, NodeRec&
         | ((outN < kRecDegree ? outN : kRecDegree) << 20);
     r.inOff = in;
     r.outOff = out;
-    for (u32 k = 0; k < kRecIn; k++) r.inNb[k] = k < inN ? g.inNb[in + k] : 0xffffffffu;
+    for (u32 k = 0; k < kRecIn; k++) r.inNb[k] = k < inN && in < inEnd && k < inEnd - in ? g.inNb[in + k] : 0xffffffffu;
     for (u32 k = 0; k < kRecOut; k++)
     {
-        r.outNb[k] = k < outN ? g.outNb[out + k] : 0xffffffffu;
-        r.outComp[k] = k < outN ? g.comp[r.outNb[k]] : 0;
+        r.outNb[k] = k < outN && out < outEnd && k < outEnd - out ? g.outNb[out + k] : 0xffffffffu;
+        r.outComp[k] = r.outNb[k] < g.N ? g.comp[r.outNb[k]] : 0;
     }
 }
 
@@ -2710,7 +2713,7 @@ __device__ __forceinline__ int trace_walk(const DevGraph& g, i32 cost, const uin
                 inNb0 = __shfl_sync(kFull, word, 8);
                 inNb1 = __shfl_sync(kFull, word, 9);
                 const u32 nb = lane < 16 ? inNb0 : inNb1;
-                if (g.rec && nb != 0xffffffffu) nbWord = __ldg((const u32*)(g.rec + nb) + (lane & 15));
+                if (g.rec && nb < g.N) nbWord = __ldg((const u32*)(g.rec + nb) + (lane & 15));
             }
             self = find_cur(curNode);
             if (!self) { err = GA_ASSERT; break; }
