@@ -163,6 +163,7 @@ struct ga_extender
     unsigned long long* arenaCursor = nullptr;   // [0] overflow cursor, [1] bytes taken, [2] column store units taken
     gadev::ColumnUnit* store = nullptr;    // the column store, grown to the largest batch within its bound
     uint64_t storeUnits = 0;
+    uint64_t storeLimit = 0;               // the store's bound in bytes
     bool storeWithheld = false;            // this call goes without a column store
     float lastFillMs = 0;
     float lastTraceMs = 0;
@@ -363,6 +364,7 @@ extern "C" int ga_extender_create(ga_graph_t graph, uint64_t arena_bytes, ga_ext
     if (e != cudaSuccess) { delete x; return cuda_fail(e, "workspace"); }
     if (arena_bytes == 0) arena_bytes = 4ULL << 30;
     x->arenaBytes = arena_bytes;
+    x->storeLimit = arena_bytes * 4;
     e = cudaMalloc((void**)&x->arena, x->arenaBytes + gadev::kArenaPad);
     if (e != cudaSuccess) { cudaFree(x->workspace); delete x; return cuda_fail(e, "arena"); }
     GA_CUDA(cudaMalloc((void**)&x->counters, 16 * sizeof(uint32_t)));
@@ -375,8 +377,10 @@ extern "C" int ga_extender_create_like(ga_extender_t x, ga_extender_t* out)
 {
     if (!x || !out) return fail(GA_ERR_ARGUMENT, "null argument");
     int rc = ga_extender_create(x->graph, x->arenaBytes, out);
-    if (rc == GA_OK) (*out)->shape = x->shape;
-    return rc;
+    if (rc != GA_OK) return rc;
+    (*out)->shape = x->shape;
+    (*out)->storeLimit = x->storeLimit;
+    return GA_OK;
 }
 
 extern "C" int ga_extender_free(ga_extender_t x)
@@ -438,18 +442,22 @@ static int with_store_given_back(ga_extender* x, Call call)
 
 // Room in the column store for a batch of readBp bases: a band of bandwidth 10 computes 2.4
 // columns per base on the variation graphs (5.5 on the tangled ones), 3 and a chunk for every
-// warp are asked for.  The store holds at most four times the arena and half of the memory that
-// is free when it grows; what finds no room in it is recomputed by the traceback.
+// warp are asked for.  The store holds at most its limit (four times the arena unless the caller
+// sets another) and half of the memory that is free when it grows; what finds no room in it is
+// recomputed by the traceback.
 static void reserve_store(ga_extender* x, uint64_t readBp, uint64_t warps)
 {
     if (x->storeWithheld) return;
     const uint64_t unit = sizeof(gadev::ColumnUnit);
     uint64_t want = readBp * 3 + warps * gadev::kStoreChunk;
-    want = std::min<uint64_t>({want, x->arenaBytes * 4 / unit, (uint64_t)gadev::kNoColumns - 1});
+    // (what is allocated ends kStorePad units behind the store)
+    const uint64_t limit = x->storeLimit / unit;
+    const uint64_t bound = std::min<uint64_t>(limit - std::min<uint64_t>(limit, gadev::kStorePad), (uint64_t)gadev::kNoColumns - 1);
+    want = std::min(want, bound);
     if (want <= x->storeUnits) return;
     size_t freeBytes = 0, totalBytes = 0;
     if (cudaMemGetInfo(&freeBytes, &totalBytes) != cudaSuccess) return;
-    const uint64_t most = std::min<uint64_t>({(freeBytes / unit + x->storeUnits) / 2, x->arenaBytes * 4 / unit, (uint64_t)gadev::kNoColumns - 1});
+    const uint64_t most = std::min<uint64_t>((freeBytes / unit + x->storeUnits) / 2, bound);
     want = std::min(most, std::max(want, x->storeUnits * 3 / 2));
     // where free memory is the bound it moves with every other allocation of the process: a store that
     // would gain less than a quarter stays as it is (growing it frees it first, which waits for the device)
@@ -1242,6 +1250,15 @@ extern "C" int ga_extender_set_launch_shape(ga_extender_t x, const ga_launch_sha
     if (!x || !shape) return fail(GA_ERR_ARGUMENT, "null argument");
     if (!shape_ok(*shape)) return fail(GA_ERR_ARGUMENT, kShapeError);
     x->shape = *shape;
+    return GA_OK;
+}
+
+extern "C" int ga_extender_set_store_limit(ga_extender_t x, uint64_t max_bytes)
+{
+    if (!x) return fail(GA_ERR_ARGUMENT, "null argument");
+    GA_CUDA(cudaSetDevice(x->graph->device));
+    x->storeLimit = max_bytes;
+    if (x->store && (x->storeUnits + gadev::kStorePad) * sizeof(gadev::ColumnUnit) > max_bytes) release_store(x);
     return GA_OK;
 }
 

@@ -360,6 +360,10 @@ class Extender:
         sh = LaunchShape(warps_per_block, blocks_per_sm, first_layout, chunk_kib)
         check(lib().ga_extender_set_launch_shape(self.handle, ctypes.byref(sh)))
 
+    def set_store_limit(self, max_bytes: int):
+        """Bounds the device memory of the extender's column store (0: none)."""
+        check(lib().ga_extender_set_store_limit(self.handle, ctypes.c_uint64(max_bytes)))
+
     def autotune(self, params: ExtendParams, batch: PackedBatch, candidates=None, sample_every: int = 4, repeats: int = 2) -> dict:
         """Times each launch shape on an evenly spaced sample of the batch (device time of the
         kernels, ``ga_extender_autotune``) and keeps the fastest.  The sample stays on the

@@ -111,7 +111,8 @@ typedef struct ga_extend_results {
 typedef struct ga_graph* ga_graph_t;
 /* Replaces the AlignmentGraph the DP reads (src/AlignmentGraph.h:121-139), as
  * AlignmentGraph::Finalize leaves it (src/AlignmentGraph.cpp:252-296): copied to
- * `device` once, read-only afterwards, shared by every extender made on it. */
+ * `device` once, with a record of 64 bytes a node beside the arrays where there is room,
+ * read-only afterwards, shared by every extender made on it. */
 int ga_graph_upload(const ga_graph_desc* desc, int device, ga_graph_t* out);
 int ga_graph_free(ga_graph_t graph);
 
@@ -119,12 +120,22 @@ int ga_graph_free(ga_graph_t graph);
 typedef struct ga_extender* ga_extender_t;
 /* The device side of the per-thread AlignerGraphsizedState
  * (src/GraphAlignerCommon.h:52-81), for a whole batch: per-warp frontier tables and
- * the DP-table arena.  arena_bytes: device bytes for per-extension DP tables; 0 = 4 GiB. */
+ * the DP-table arena.  arena_bytes: device bytes for per-extension DP tables; 0 = 4 GiB.
+ * Beside the arena an extender holds 256 MiB of frontier tables, its batches' staging
+ * (grown to the largest batch) and the column store: the DP's columns, kept for the
+ * traceback in 48 bytes a read base (the multiseed calls: 96), at most four times the arena and half of the device
+ * memory that is free when the store grows.  It is kept until the extender is freed or a
+ * call finds no memory for its staging.  ga_extender_set_store_limit bounds it. */
 int ga_extender_create(ga_graph_t graph, uint64_t arena_bytes, ga_extender_t* out);
 /* A second extender on the same device graph with the same arena size and launch shape
  * (no reference counterpart): two extenders let two batches run while the host works. */
 int ga_extender_create_like(ga_extender_t ext, ga_extender_t* out);
 int ga_extender_free(ga_extender_t ext);
+/* Bounds the extender's column store (no reference counterpart: it never changes a result):
+ * at most max_bytes, 0 = none; a larger one is freed at once.  Columns that find no room
+ * in the store are computed again by the traceback, which takes longer.  Not while a call
+ * of the extender runs; ga_extender_create_like passes the bound on. */
+int ga_extender_set_store_limit(ga_extender_t ext, uint64_t max_bytes);
 /* A batch of GraphAlignerBitvectorBanded::getReverseTraceFromSeed calls
  * (src/GraphAlignerBitvectorBanded.h:59-76).  Host buffers in, host buffers out:
  * copies, launches and waits.  Status GA_TRACE_FAILED is OnewayTrace::TraceFailed(),

@@ -159,3 +159,36 @@ def test_bounded_store_stays(cuda_lib, other):
     ext.run(params, batch)
     assert free_bytes() == left + freed
     ext.close()
+
+
+@pytest.mark.parametrize("limit", [0, 1, 4096 * 16, 40 * MB])
+def test_store_limit(cuda_lib, limit):
+    """A store of at most the caller's bound, from the start or once it is larger, and the same results."""
+    g, one = golden_case("vg50k")
+    expected = load_digests("vg50k", 10)
+    params = ExtendParams(bandwidth=10)
+    dgraph = DeviceGraph(g)
+    load_kernels(dgraph, params, one)
+    slack = 4 * MB               # allocations are whole pages, and the store ends some units early
+
+    def grown_by(ext, calls):
+        before = free_bytes()
+        for _ in range(calls):
+            assert not compare(ext.run(params, one), expected)
+        return before - free_bytes()
+    ext = Extender(dgraph, arena_bytes=ARENA)
+    ext.set_store_limit(0)
+    staging = grown_by(ext, 1)
+    ext.close()
+    ext = Extender(dgraph, arena_bytes=ARENA)
+    ext.set_store_limit(limit)
+    assert abs(grown_by(ext, 2) - staging - limit) <= slack
+    ext.close()
+    ext = Extender(dgraph, arena_bytes=ARENA)
+    full = grown_by(ext, 1) - staging
+    assert full > 40 * MB + slack
+    before = free_bytes()
+    ext.set_store_limit(limit)
+    assert abs(free_bytes() - before - full) <= slack
+    assert abs(grown_by(ext, 2) - limit) <= slack
+    ext.close()
