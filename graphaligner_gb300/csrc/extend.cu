@@ -33,6 +33,11 @@
 // phase's code.  With the traceback run by the fill's warps right after it, 50,000
 // extensions (250 Mbp) took 95 ms instead of 51: the two phases' code does not fit
 // the instruction caches.
+//
+// Times below that go from one figure to another are of the change that made the form, with the
+// code around it as it was then.  As it stands, that batch takes 48.0 ms in these kernels
+// (fill and traceback), one seed of a 10 kbp read 2.67 ms, 1,000 tangled extensions of 20 kbp
+// reads 28.2 ms.
 // Cold paths (crossing rules, end-cell choice, sequential fallbacks) are out of line.
 //
 // Warps take extensions from a device counter over a longest-first order.
@@ -307,8 +312,9 @@ __device__ __forceinline__ SmallSpace& small_space()
 // component queue then has one order whatever its heap looks like, the component numbers', so the
 // queued slots are not in a heap at all and the next one is found by a minimum over the lanes.
 // (Where numbers are shared, equal scores come off in the order the heap's layout gives.)
-// This form against that: 50,000 extensions (250 Mbp) 102.9 -> 92.7 ms, one seed of a 10 kbp
-// read 8 % less, 1,000 tangled extensions of 20 kbp reads 14 % less.
+// With the heap instead, 50,000 extensions (250 Mbp) take 48.9 ms instead of 48.0, one seed of a
+// 10 kbp read 2.72 instead of 2.67.  The lane tables and records against a hash table and the
+// graph's arrays: 102.9 -> 92.7 ms, one seed 8 % less, 1,000 tangled extensions 14 % less.
 template <bool Unique>
 struct SmallTables
 {
@@ -3415,8 +3421,8 @@ __global__ void __launch_bounds__(32, 6) fill_tangled_kernel(const __grid_consta
 __global__ void __launch_bounds__(128, 4) fill_large_kernel(const __grid_constant__ FillArgs fa, u32* counter) { fill_extensions<LargeTables>(fa, counter); }
 
 // The traceback: a warp takes the next filled extension and walks its table back.  Four blocks of
-// 128 registers a thread on an SM: with six of 80 the walk's state spills, and the batch above
-// takes 67.5 ms instead of 58.5 (five of 96: 62.8).  Its
+// 128 registers a thread on an SM: with six of 80 the walk's state spills, and 50,000 extensions
+// (250 Mbp) take 52.9 ms instead of 48.0, with five of 96 49.5.  Its
 // shared memory holds the recomputed columns, the match masks and the trace staging.
 __global__ void __launch_bounds__(128, 4) trace_kernel(const __grid_constant__ TraceArgs ta, u32* counter)
 {

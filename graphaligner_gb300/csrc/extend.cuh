@@ -64,9 +64,10 @@ static constexpr u32 kNodeMask = 0x3fffffffu;
 // 16-byte units while there is room.  Unit 0 holds the +1 and -1 deltas along the slice's first
 // row (bit c: column c against column c - 1), unit c > 0 column c's VP and its rows with an open
 // diagonal step.  About 37 bytes per read base at bandwidth 10, written once and about half of it
-// read, where memory bandwidth is otherwise idle (below 1 % of the copy peak).  Recomputing the
-// columns, with the lookups, loads and masks that takes, was half of the traceback: 50,000
-// extensions (250 Mbp) 89.5 -> 61.5 ms, one seed of a 10 kbp read 3.95 -> 3.15 ms.
+// read, where memory bandwidth is otherwise idle (below 1 % of the copy peak).  Without the store
+// the traceback recomputes the columns, with the lookups, loads and masks that takes: 50,000
+// extensions (250 Mbp) take 74.3 ms instead of 48.0, one seed of a 10 kbp read 3.59 instead of
+// 2.67, 1,000 tangled extensions 29.1 instead of 28.2.
 struct __align__(16) ColumnUnit
 {
     u64 x, y;
@@ -151,18 +152,24 @@ struct __align__(16) ResumeRec
 // memory with medium_caps(), or in global memory with FillArgs::caps.
 enum class FillTables { Small, Medium, Global };
 
-// 35 KB a warp, six warps on an SM: for the few extensions that outgrow the small tables, and from
-// the start for graphs that are mostly cycles (ga_graph::tangled).  There one extension in four to
-// twenty outgrows the small tables, and those, which go on only when all others have ended, are
-// what the call waits for: the 1,000 extensions of 500 tangled reads of 20 kbp take 28.7 ms instead
-// of 38.1, 1,000 of accurate 1 kbp reads 2.7 instead of 4.5, those of 16 such reads 2.1 instead of
-// 2.6.  With 64 band entries, eleven warps on an SM and the rest handed on: 30.2 ms.
+// 35 KB a warp, 38 with its recorded columns, five warps on an SM: for the few extensions that
+// outgrow the small tables, and from the start for graphs that are mostly cycles
+// (ga_graph::tangled).  There one extension in four to twenty outgrows the small tables, and those,
+// which go on only when all others have ended, are what the call waits for.  With 64 band entries,
+// ten warps on an SM and the rest handed on, 1,000 extensions of tangled 20 kbp reads took 30.2 ms
+// instead of 28.7.
 //
-// The small tables let sixteen warps on an SM, and their nodes cost a tenth less.  So all other
-// graphs keep them (a variation graph's reads would take 1.08 times as long), and batches of more
-// than kMediumWaves times the warps that fit the GPU at once (152 SMs: 3,648 extensions): 4,000
-// extensions take 34.5 against 42.9 ms with tangles, 4,800 take 37.5 against 45.4, but 6.7 against
-// 4.6 where a graph has none; 10,000 take 67 against 62.
+// The small tables let sixteen warps on an SM, and their nodes cost a tenth less, so all other graphs
+// keep them.  The line for the graphs that are mostly cycles is kMediumWaves times the warps that are
+// on the GPU at once (152 SMs: 3,040 extensions), a bound of what is lost where a graph's numbers
+// are shared but its reads meet no tangles, at the price of the tangled batches between it and
+// the crossing.  Milliseconds with the medium tables / with the small ones:
+//   extensions                                1,000       3,000       4,800      10,000
+//   tangled graph, 20 kbp reads at 12 %   28.5/36.1   31.1/43.2   36.4/41.4   66.2/61.8
+//   tangled graph, accurate 1 kbp reads     3.0/4.5     3.7/5.9     3.4/5.4     4.3/6.5
+//   variation graph with its numbers
+//     shared in pairs, 10 kbp at 10 %       4.1/3.5     7.3/5.1    10.7/5.9   22.1/11.0
+//   the same, accurate 1 kbp reads         0.52/0.49   0.92/0.72   1.38/0.92   2.75/1.66
 static constexpr u32 kMediumWaves = 4;
 inline Caps medium_caps()
 {
@@ -353,8 +360,8 @@ int ga_trace_blocks_per_sm(int warpsPerBlock);
 // at a time; counters[0], [1] and [3] must be zero
 int ga_launch_extend(const gadev::FillArgs& fa, const gadev::TraceArgs& ta, uint32_t* counters, int fillBlocks, int mediumBlocks,
     int traceBlocks, int warpsPerBlock, void* stream);
-// the multiseed DP's fill and traceback kernels (the frontier tables always in the global workspace)
-// the multiseed DP in steps, blocks of warpsPerBlock warps, each on `stream`:
+// the multiseed DP in steps, each on `stream`, its frontier tables always in the global workspace; blocks
+// of warpsPerBlock warps but for the fill, whose fillBlocks are of one:
 // - fill: the fill and the count of each read's trace candidates (counters[0], [1] and
 //   ta.candTotal zero);
 // - list: once ta.cands has room for *ta.candTotal, the candidates listed (counters[3] zero,

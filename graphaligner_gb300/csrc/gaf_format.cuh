@@ -1,7 +1,8 @@
 // GAF line formatting (GraphAlignerGAFAlignment::traceToAlignment, GraphAlignerGAFAlignment.h:37-200),
 // host- and device-callable: the device formats every selected alignment of a batch (a warp per
-// line with these numbers, gaf_device.cu; write_line is the same line by one thread, for the host),
-// and the host tests check the number formatting against std::ostream.
+// line with these numbers, warp_line in gaf_device.cu; write_line is the same line by one thread, which
+// only the host tests' harness calls), and the host tests check the number formatting against
+// std::ostream.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -483,7 +484,8 @@ GAF_HD inline bool classify_line(GetItem item, uint32_t count, uint32_t readLen,
 }
 
 // Writes one classified GAF line (no newline) to out, or only measures it when out is null;
-// returns its length.
+// returns its length.  The form the host tests write their lines with: what the library writes is
+// warp_line's, whose lines are compared with the reference's on the GPU.
 inline int64_t write_line(const Names& nm, const LineMeta& m, const uint8_t* ops, const int32_t* entries, char* out)
 {
     const char codes[5] = { '=', 'X', 'M', 'I', 'D' };

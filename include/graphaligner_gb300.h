@@ -65,7 +65,9 @@ typedef struct ga_extend_params {
     uint32_t bandwidth;               /* alignmentBandwidth */
     int32_t  xdrop;                   /* Xdropcutoff */
     uint64_t max_cells_per_slice;     /* maxCellsPerSlice (tangle effort); UINT64_MAX = unlimited */
-    int32_t  xscore_error_cost;       /* XscoreErrorCost = int(100*(c/(1-c)+1)) */
+    int32_t  xscore_error_cost;       /* XscoreErrorCost = int(100*(c/(1-c)+1)), at least 100.  Below that the
+                                         multiseed calls do not report every read in which the
+                                         reference asserts (a seed column's rows may rise by two) */
 } ga_extend_params;
 
 /* A batch of extensions.  Extension i aligns seq[seq_offset[i] .. +seq_len[i]) starting
