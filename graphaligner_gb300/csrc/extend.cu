@@ -837,6 +837,7 @@ __device__ __forceinline__ int64_t xscore_bound(const WS& w, i32 seqOffset, i32 
 // X-scores were 17 % of the fill (50,000 extensions 56.4 -> 55.2 ms, 1,000 tangled ones 45.6 ->
 // 42.7 ms).
 static constexpr i32 kCostLimit = 1 << 16;
+static constexpr int64_t kOriginLimit = -(1LL << 30);     // with the greatest terms (4,160 kCostLimit) still within 32 bits
 __device__ __forceinline__ bool near(i32 a, i32 b) { return (u32)a - (u32)b + 4096u <= 8192u; }
 
 __device__ __forceinline__ i32 column_xscore(const WS& w, i32 ref, i32 cost, u64 rows, i32 beat)
@@ -1311,8 +1312,11 @@ __device__ __forceinline__ NodeCalc node_calc(const DevGraph& g, i32 cost, u32 i
         u32 loKey = 0xffffffffu, hiKey = 0xffffffffu;
         i32 lmax = kIntMin;
         // scores and X-scores are counted from the node's first column
-        const bool small = boundOk && cost >= 0 && cost < kCostLimit && score_ok(startEnd) && near(ws0.end, startEnd) && near(wsX.end, startEnd);
         const int64_t origin = (int64_t)seqOffset * 100 - (int64_t)cost * startEnd;
+        // (far below zero a column's X-score leaves the 32 bits: each column is then bounded in 64 bits before
+        // it is scored, and one that is out of their range does not come back as a great one)
+        const bool small = boundOk && cost >= 0 && cost < kCostLimit && score_ok(startEnd) && near(ws0.end, startEnd) && near(wsX.end, startEnd)
+            && origin > kOriginLimit;
         const int64_t toBeat = (int64_t)sliceMaxX - origin;
         const i32 beat = toBeat < -kWarpScoreLimit ? -kWarpScoreLimit : toBeat > kWarpScoreLimit ? kWarpScoreLimit : (i32)toBeat;
 #pragma unroll
